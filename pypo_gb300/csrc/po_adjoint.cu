@@ -26,9 +26,9 @@
 //                 dL/d delta_s = n_s . sum_t Re[-t j k G (conj(gS_J).J' + conj(gS_M).M')] r.
 // The illumination mask is piecewise constant: its derivative is dropped.
 //
-// This file holds the formulas in generic form, the cotangent mapping, the
-// plain FP64 adjoint kernels (the comparison path) and the epilogues. The
-// mixed-precision kernels, pair-packed, are in po_adjoint_pk.cu.
+// This file holds the formulas, the cotangent mapping and the epilogues. The
+// mixed-precision kernels, pair-packed, are in po_adjoint_pk.cu, the plain
+// FP64 ones in po_fp64.cu.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <cstdint>
@@ -37,207 +37,6 @@
 #include "po_kernels.cuh"
 
 namespace po {
-
-template <typename F>
-struct cx {
-    F r, i;
-};
-
-template <typename F>
-__device__ __forceinline__ cx<F> cmul(cx<F> a, cx<F> b)
-{
-    return {a.r * b.r - a.i * b.i, a.r * b.i + a.i * b.r};
-}
-template <typename F>
-__device__ __forceinline__ cx<F> cadd(cx<F> a, cx<F> b)
-{
-    return {a.r + b.r, a.i + b.i};
-}
-template <typename F>
-__device__ __forceinline__ cx<F> csub(cx<F> a, cx<F> b)
-{
-    return {a.r - b.r, a.i - b.i};
-}
-template <typename F>
-__device__ __forceinline__ cx<F> cconj(cx<F> a)
-{
-    return {a.r, -a.i};
-}
-// complex 3-vector . real 3-vector
-template <typename F>
-__device__ __forceinline__ cx<F> cdot_r(const cx<F> *v, F x, F y, F z)
-{
-    return {v[0].r * x + v[1].r * y + v[2].r * z, v[0].i * x + v[1].i * y + v[2].i * z};
-}
-// complex 3-vector . complex 3-vector (bilinear, no conjugation)
-template <typename F>
-__device__ __forceinline__ cx<F> cdot_c(const cx<F> *a, const cx<F> *b)
-{
-    return cadd(cadd(cmul(a[0], b[0]), cmul(a[1], b[1])), cmul(a[2], b[2]));
-}
-// complex 3-vector x real 3-vector
-template <typename F>
-__device__ __forceinline__ void ccross_r(const cx<F> *v, F x, F y, F z, cx<F> *o)
-{
-    o[0] = {v[1].r * z - v[2].r * y, v[1].i * z - v[2].i * y};
-    o[1] = {v[2].r * x - v[0].r * z, v[2].i * x - v[0].i * z};
-    o[2] = {v[0].r * y - v[1].r * x, v[0].i * y - v[1].i * x};
-}
-
-// Forward coefficients (and radial derivatives) of one lit pair, in the
-// units of d (mm for the FP64 kernels): rinv = 1/R,
-// u = 1/(kR) given, G = (gc, gs) = e^{t j k R} (zero when not lit).
-template <typename F, int T>
-struct Coef {
-    cx<F> c1, c2, c3, d1, d2, d3;
-};
-
-template <typename F, int T, bool WANT_C1, bool WANT_D>
-__device__ __forceinline__ Coef<F, T> coefficients(F rinv, F u, F gc, F gs)
-{
-    Coef<F, T> k;
-    const cx<F> G = {gc, gs};
-    const F u2 = u * u, u3 = u2 * u;
-    const F tf = (F)T;
-    const cx<F> s1 = {tf * u2, u3 - u};
-    const cx<F> c1 = cmul(G, s1);
-    if (WANT_C1) k.c1 = c1;
-    const F rinv2 = rinv * rinv;
-    // c2' = (-3 c1 - 2 j u G) / R^2
-    k.c2 = {(-(F)3 * c1.r + (F)2 * u * gs) * rinv2, (-(F)3 * c1.i - (F)2 * u * gc) * rinv2};
-    k.c3 = cmul(G, cx<F>{-u2 * rinv, tf * u * rinv});
-    if (WANT_D) {
-        const F rinv3 = rinv2 * rinv;
-        k.d1 = cmul(G, cx<F>{tf * ((F)1 - (F)3 * u2) * rinv2, ((F)2 * u - (F)3 * u3) * rinv2});
-        k.d2 = cmul(G, cx<F>{-tf * ((F)1 - (F)15 * u2) * rinv2 * rinv2, (-(F)6 * u + (F)15 * u3) * rinv2 * rinv2});
-        k.d3 = cmul(G, cx<F>{-((F)1 - (F)3 * u2) * rinv3, -(F)3 * tf * u * rinv3});
-    }
-    return k;
-}
-
-// Per-thread constants of one source (its folded currents and normal).
-template <typename F>
-struct SrcConst {
-    cx<F> J[3], M[3];
-    F n[3];
-    cx<F> Jn, Mn;        // J.n, M.n
-    cx<F> Jxn[3], Mxn[3];
-};
-
-template <typename F, bool HAS_M>
-__device__ __forceinline__ void src_const_finish(SrcConst<F> &s)
-{
-    s.Jn = cdot_r(s.J, s.n[0], s.n[1], s.n[2]);
-    ccross_r(s.J, s.n[0], s.n[1], s.n[2], s.Jxn);
-    if (HAS_M) {
-        s.Mn = cdot_r(s.M, s.n[0], s.n[1], s.n[2]);
-        ccross_r(s.M, s.n[0], s.n[1], s.n[2], s.Mxn);
-    }
-}
-
-// Near-field source-side pair: adjoint currents (acc[0..11]) and the source
-// displacement term n_s . grad_d phi (acc[12]).
-template <typename F, int T, bool HAS_M, bool WANT_D>
-__device__ __forceinline__ void nf_adj_src_algebra(F *acc, F dx, F dy, F dz, F rinv, F u, F gc, F gs, F ndn,
-                                                   const cx<F> *gE, const cx<F> *gH, const SrcConst<F> &sc)
-{
-    const Coef<F, T> k = coefficients<F, T, true, WANT_D>(rinv, u, gc, gs);
-    const cx<F> c1c = cconj(k.c1), c2c = cconj(k.c2), c3c = cconj(k.c3);
-    const cx<F> ged = cdot_r(gE, dx, dy, dz), ghd = cdot_r(gH, dx, dy, dz);
-    const cx<F> P = cmul(c2c, ged), Q = cmul(c2c, ghd);
-    cx<F> ghxd[3], gexd[3];
-    ccross_r(gH, dx, dy, dz, ghxd);
-    ccross_r(gE, dx, dy, dz, gexd);
-    const F dv[3] = {dx, dy, dz};
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        const cx<F> jb = cadd(cadd(cmul(c1c, gE[c]), cx<F>{P.r * dv[c], P.i * dv[c]}), cmul(c3c, ghxd[c]));
-        const cx<F> mb = csub(cadd(cmul(c1c, gH[c]), cx<F>{Q.r * dv[c], Q.i * dv[c]}), cmul(c3c, gexd[c]));
-        acc[c] += jb.r;
-        acc[3 + c] += jb.i;
-        acc[6 + c] += mb.r;
-        acc[9 + c] += mb.i;
-    }
-    if (WANT_D) {
-        // a = conj(gE), b = conj(gH)
-        cx<F> a[3], b[3];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            a[c] = cconj(gE[c]);
-            b[c] = cconj(gH[c]);
-        }
-        const cx<F> ad = cconj(ged), bd = cconj(ghd);
-        const cx<F> Jd = cdot_r(sc.J, dx, dy, dz);
-        cx<F> alpha = cdot_c(a, sc.J);
-        cx<F> beta = cmul(Jd, ad);
-        cx<F> Jxd[3];
-        ccross_r(sc.J, dx, dy, dz, Jxd);
-        cx<F> Wd = {-cdot_c(b, Jxd).r, -cdot_c(b, Jxd).i};
-        cx<F> Wn = {-cdot_c(b, sc.Jxn).r, -cdot_c(b, sc.Jxn).i};
-        const cx<F> an = cdot_r(a, sc.n[0], sc.n[1], sc.n[2]);
-        cx<F> gbn = cadd(cmul(ad, sc.Jn), cmul(Jd, an));
-        if (HAS_M) {
-            const cx<F> Md = cdot_r(sc.M, dx, dy, dz);
-            alpha = cadd(alpha, cdot_c(b, sc.M));
-            beta = cadd(beta, cmul(Md, bd));
-            cx<F> Mxd[3];
-            ccross_r(sc.M, dx, dy, dz, Mxd);
-            Wd = cadd(Wd, cdot_c(a, Mxd));
-            Wn = cadd(Wn, cdot_c(a, sc.Mxn));
-            const cx<F> bn = cdot_r(b, sc.n[0], sc.n[1], sc.n[2]);
-            gbn = cadd(gbn, cadd(cmul(bd, sc.Mn), cmul(Md, bn)));
-        }
-        const cx<F> sig = cadd(cadd(cmul(k.d1, alpha), cmul(k.d2, beta)), cmul(k.d3, Wd));
-        acc[12] += sig.r * ndn + cmul(k.c2, gbn).r + cmul(k.c3, Wn).r;
-    }
-}
-
-// Near-field target-side pair: n_t . grad_d phi for one source (J, M, d).
-template <typename F, int T, bool HAS_M>
-__device__ __forceinline__ F nf_adj_tgt_algebra(F dx, F dy, F dz, F rinv, F u, F gc, F gs, F ndn,
-                                                const cx<F> *a, const cx<F> *b, const cx<F> *nxa,
-                                                const cx<F> *nxb, cx<F> an, cx<F> bn, const F *n,
-                                                const cx<F> *J, const cx<F> *M)
-{
-    const Coef<F, T> k = coefficients<F, T, false, true>(rinv, u, gc, gs);
-    const cx<F> Jd = cdot_r(J, dx, dy, dz);
-    const cx<F> ad = cdot_r(a, dx, dy, dz);
-    cx<F> alpha = cdot_c(a, J);
-    cx<F> beta = cmul(Jd, ad);
-    // W.d = M.(d x a) - J.(d x b);  W.n = M.(n x a) - J.(n x b)
-    cx<F> dxb[3];
-    {
-        cx<F> t3[3];
-        ccross_r(b, dx, dy, dz, t3);   // b x d = -(d x b)
-        dxb[0] = {-t3[0].r, -t3[0].i};
-        dxb[1] = {-t3[1].r, -t3[1].i};
-        dxb[2] = {-t3[2].r, -t3[2].i};
-    }
-    cx<F> Wd = {-cdot_c(J, dxb).r, -cdot_c(J, dxb).i};
-    cx<F> Wn = {-cdot_c(J, nxb).r, -cdot_c(J, nxb).i};
-    const cx<F> Jn = cdot_r(J, n[0], n[1], n[2]);
-    cx<F> gbn = cadd(cmul(ad, Jn), cmul(Jd, an));
-    if (HAS_M) {
-        const cx<F> Md = cdot_r(M, dx, dy, dz);
-        const cx<F> bd = cdot_r(b, dx, dy, dz);
-        alpha = cadd(alpha, cdot_c(b, M));
-        beta = cadd(beta, cmul(Md, bd));
-        cx<F> dxa[3];
-        {
-            cx<F> t3[3];
-            ccross_r(a, dx, dy, dz, t3);
-            dxa[0] = {-t3[0].r, -t3[0].i};
-            dxa[1] = {-t3[1].r, -t3[1].i};
-            dxa[2] = {-t3[2].r, -t3[2].i};
-        }
-        Wd = cadd(Wd, cdot_c(M, dxa));
-        Wn = cadd(Wn, cdot_c(M, nxa));
-        const cx<F> Mn = cdot_r(M, n[0], n[1], n[2]);
-        gbn = cadd(gbn, cadd(cmul(bd, Mn), cmul(Md, bn)));
-    }
-    const cx<F> sig = cadd(cadd(cmul(k.d1, alpha), cmul(k.d2, beta)), cmul(k.d3, Wd));
-    return sig.r * ndn + cmul(k.c2, gbn).r + cmul(k.c3, Wn).r;
-}
 
 // ------------------------------------------------------- cotangent mapping
 
@@ -326,233 +125,6 @@ __global__ void po_adj_ehp_cot_kernel(long nt, const double *__restrict__ cot, c
     }
 }
 
-// ------------------------------------------------------------- FP64 kernels
-
-// One (source, target) pair of the plain FP64 source-side adjoint, added into
-// acc (kAccAdj): sp the source position (mm), sc its constants, r the target
-// as the kernel stages it (point or direction, then the 12 cotangent rows
-// gE re xyz, gE im, gH re, gH im). Unlit pairs add nothing.
-template <int KIND, int T>
-__device__ __forceinline__ void adj_src_pair_fp64(const double *sp, const SrcConst<double> &sc, const double *r,
-                                                  double k, double *acc)
-{
-    const cx<double> gE[3] = {{r[3], r[6]}, {r[4], r[7]}, {r[5], r[8]}};
-    const cx<double> gH[3] = {{r[9], r[12]}, {r[10], r[13]}, {r[11], r[14]}};
-    if (KIND == kKindScalar) {
-        // c = e^{-t j k R} / R; Sbar' += conj(c) g; n . grad_d phi = Re[conj(g) S' dc/dR] (n.d) / R
-        const double dx = r[0] - sp[0], dy = r[1] - sp[1], dz = r[2] - sp[2];
-        const double R = sqrt(dx * dx + dy * dy + dz * dz), rinv = 1.0 / R;
-        double sn, cs;
-        sincos(k * R, &sn, &cs);
-        const cx<double> c = {cs * rinv, -T * sn * rinv};
-        const cx<double> g = gE[0];
-        const cx<double> sb = cmul(cconj(c), g);
-        acc[0] += sb.r;
-        acc[3] += sb.i;
-        const cx<double> y = cmul(cmul(cconj(g), sc.J[0]), c);
-        const double dphi = -y.r * rinv + T * k * y.i;
-        acc[12] += dphi * rinv * (sc.n[0] * dx + sc.n[1] * dy + sc.n[2] * dz);
-    } else if (KIND == kKindNF) {
-        const double dx = r[0] - sp[0], dy = r[1] - sp[1], dz = r[2] - sp[2];
-        const double R = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
-                                              __dmul_rn(dz, dz)));
-        const double rinv = __ddiv_rn(1.0, R);
-        if (lit_fp64(sc.n, dx, dy, dz, rinv) == false) return;
-        const double ndd = sc.n[0] * dx + sc.n[1] * dy + sc.n[2] * dz;
-        double sn, cs;
-        sincos(k * R, &sn, &cs);
-        nf_adj_src_algebra<double, T, true, true>(acc, dx, dy, dz, rinv, rinv / k, cs, T * sn, ndd, gE, gH,
-                                                  sc);
-    } else {
-        const double ndr = sc.n[0] * r[0] + sc.n[1] * r[1] + sc.n[2] * r[2];
-        if (__dadd_rn(__dadd_rn(__dmul_rn(sc.n[0], r[0]), __dmul_rn(sc.n[1], r[1])),
-                      __dmul_rn(sc.n[2], r[2])) < 0.0)
-            return;
-        double sn, cs;
-        sincos(k * (sp[0] * r[0] + sp[1] * r[1] + sp[2] * r[2]), &sn, &cs);
-        const cx<double> G = {cs, -T * sn};
-        const cx<double> Gc = cconj(G);
-        for (int c = 0; c < 3; ++c) {
-            const cx<double> jb = cmul(Gc, gE[c]), mb = cmul(Gc, gH[c]);
-            acc[c] += jb.r;
-            acc[3 + c] += jb.i;
-            acc[6 + c] += mb.r;
-            acc[9 + c] += mb.i;
-        }
-        cx<double> gEc[3] = {cconj(gE[0]), cconj(gE[1]), cconj(gE[2])};
-        cx<double> gHc[3] = {cconj(gH[0]), cconj(gH[1]), cconj(gH[2])};
-        const cx<double> Z = cmul(G, cadd(cdot_c(gEc, sc.J), cdot_c(gHc, sc.M)));
-        acc[12] += T * k * Z.i * ndr;
-    }
-}
-
-// Plain FP64 source-side adjoint: thread = source, loop over every target.
-template <int KIND, int T>
-__global__ void __launch_bounds__(kThreadsD)
-po_adj_src_fp64_kernel(const double *__restrict__ srcd, long ns, const double *__restrict__ tgt7,
-                       const double *__restrict__ gam, long nt, double k, double *__restrict__ part)
-{
-    __shared__ double tile[kTileD * 15];
-    const long si = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const double *q = srcd + (size_t)kRecD * (si < ns ? si : 0);
-    const double sp[3] = {q[0], q[1], q[2]};
-    SrcConst<double> sc;
-    for (int c = 0; c < 3; ++c) {
-        sc.n[c] = q[3 + c];
-        sc.J[c] = {q[6 + 2 * c], q[7 + 2 * c]};
-        sc.M[c] = {q[12 + 2 * c], q[13 + 2 * c]};
-    }
-    src_const_finish<double, true>(sc);
-    double acc[kAccAdj];
-    for (int a = 0; a < kAccAdj; ++a) acc[a] = 0.0;
-    for (long base = 0; base < nt; base += kTileD) {
-        const int cnt = (int)min((long)kTileD, nt - base);
-        __syncthreads();
-        for (int w = threadIdx.x; w < cnt * 15; w += blockDim.x) {
-            const int s = w / 15, c = w % 15;
-            const long ti = base + s;
-            double v;
-            if (c < 3) {
-                if (KIND == kKindFF) {
-                    const double th = tgt7[ti], ph = tgt7[nt + ti];
-                    v = c == 0 ? cos(ph) * sin(th) : (c == 1 ? sin(ph) * sin(th) : cos(th));
-                } else {
-                    v = tgt7[c * nt + ti];
-                }
-            } else {
-                v = gam[(long)(c - 3) * nt + ti];
-            }
-            tile[s * 15 + c] = v;
-        }
-        __syncthreads();
-        if (si >= ns) continue;
-        for (int s = 0; s < cnt; ++s) adj_src_pair_fp64<KIND, T>(sp, sc, tile + s * 15, k, acc);
-    }
-    if (si < ns)
-        for (int a = 0; a < kAccAdj; ++a) part[(long)a * ns + si] = acc[a];
-}
-
-// The constants of a target for the FP64 target-side adjoint: its point and
-// normal, a = conj(gE), b = conj(gH), n x a, n x b, a.n and b.n.
-struct TgtConst {
-    double p[3], n[3];
-    cx<double> a[3], b[3], nxa[3], nxb[3], an, bn;
-};
-
-__device__ __forceinline__ void tgt_const(const double *tgt7, const double *gam, long nt, long ti, TgtConst &tc)
-{
-    for (int c = 0; c < 3; ++c) {
-        tc.p[c] = tgt7[c * nt + ti];
-        tc.n[c] = tgt7[(3 + c) * nt + ti];
-        tc.a[c] = {gam[c * nt + ti], -gam[(3 + c) * nt + ti]};
-        tc.b[c] = {gam[(6 + c) * nt + ti], -gam[(9 + c) * nt + ti]};
-    }
-    cx<double> t3[3];
-    ccross_r(tc.a, tc.n[0], tc.n[1], tc.n[2], t3);
-    for (int c = 0; c < 3; ++c) tc.nxa[c] = {-t3[c].r, -t3[c].i};
-    ccross_r(tc.b, tc.n[0], tc.n[1], tc.n[2], t3);
-    for (int c = 0; c < 3; ++c) tc.nxb[c] = {-t3[c].r, -t3[c].i};
-    tc.an = cdot_r(tc.a, tc.n[0], tc.n[1], tc.n[2]);
-    tc.bn = cdot_r(tc.b, tc.n[0], tc.n[1], tc.n[2]);
-}
-
-// One (source, target) pair of the plain FP64 target-side adjoint: n_t .
-// grad_d phi for the source record r (kRecD). Unlit pairs give 0.
-template <int KIND, int T>
-__device__ __forceinline__ double adj_tgt_pair_fp64(const TgtConst &tc, const double *r, double k)
-{
-    const double dx = tc.p[0] - r[0], dy = tc.p[1] - r[1], dz = tc.p[2] - r[2];
-    if (KIND == kKindScalar) {
-        const double R = sqrt(dx * dx + dy * dy + dz * dz), rinv = 1.0 / R;
-        double sn, cs;
-        sincos(k * R, &sn, &cs);
-        const cx<double> c = {cs * rinv, -T * sn * rinv};
-        const cx<double> y = cmul(cmul(tc.a[0], cx<double>{r[6], r[7]}), c);   // a = conj(g)
-        return (-y.r * rinv + T * k * y.i) * rinv * (tc.n[0] * dx + tc.n[1] * dy + tc.n[2] * dz);
-    }
-    const double R = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
-    const double rinv = __ddiv_rn(1.0, R);
-    if (!lit_fp64(r + 3, dx, dy, dz, rinv)) return 0.0;
-    double sn, cs;
-    sincos(k * R, &sn, &cs);
-    const cx<double> J[3] = {{r[6], r[7]}, {r[8], r[9]}, {r[10], r[11]}};
-    const cx<double> M[3] = {{r[12], r[13]}, {r[14], r[15]}, {r[16], r[17]}};
-    const double ndn = tc.n[0] * dx + tc.n[1] * dy + tc.n[2] * dz;
-    return nf_adj_tgt_algebra<double, T, true>(dx, dy, dz, rinv, rinv / k, cs, T * sn, ndn, tc.a, tc.b, tc.nxa,
-                                               tc.nxb, tc.an, tc.bn, tc.n, J, M);
-}
-
-// Plain FP64 target-side displacement adjoint (near field, scalar).
-template <int KIND, int T>
-__global__ void __launch_bounds__(kThreadsD)
-po_adj_tgt_fp64_kernel(const double *__restrict__ srcd, long ns, const double *__restrict__ tgt7,
-                       const double *__restrict__ gam, long nt, double k, double *__restrict__ part)
-{
-    __shared__ double tile[kTileD * kRecD];
-    const long ti = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    TgtConst tc;
-    tgt_const(tgt7, gam, nt, ti < nt ? ti : 0, tc);
-    double acc = 0.0;
-    for (long base = 0; base < ns; base += kTileD) {
-        const int cnt = (int)min((long)kTileD, ns - base);
-        __syncthreads();
-        for (int w = threadIdx.x; w < cnt * kRecD; w += blockDim.x) tile[w] = srcd[base * kRecD + w];
-        __syncthreads();
-        if (ti >= nt) continue;
-        for (int s = 0; s < cnt; ++s) acc += adj_tgt_pair_fp64<KIND, T>(tc, tile + s * kRecD, k);
-    }
-    if (ti < nt) part[ti] = acc;
-}
-
-// The pairs the mixed adjoint left out as inside the tangent band: each is
-// decided by the reference's FP64 rounding and, if lit, its FP64 terms go
-// into the first source chunk's partials (currents; the source displacement
-// and the target displacement in the mixed kernel's units, per turn:
-// inv_kappa = 2 pi / k), before the epilogues. Order of the additions varies
-// between runs for a point with several such pairs (last bits there only).
-template <int KIND, int T, bool WANT_T>
-__global__ void __launch_bounds__(256)
-po_adj_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, const double *__restrict__ cur,
-                         int gmode, int ncx, int ncy, double fac_re, double fac_im, long nt,
-                         const double *__restrict__ tgt7, const double *__restrict__ gam, double k,
-                         double inv_kappa, double *__restrict__ part, double *__restrict__ gt, int *__restrict__ err)
-{
-    const unsigned total = *bl.count;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && total > bl.cap) atomicExch(err, kErrBandOverflow);
-    const unsigned n = min(total, bl.cap);
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int2 pr = bl.pairs[i];
-        const long si = pr.x, ti = pr.y;
-        double rec[kRecD];
-        src_record_d(si, ns, src7, cur, gmode, ncx, ncy, fac_re, fac_im, 0, rec);
-        SrcConst<double> sc;
-        for (int c = 0; c < 3; ++c) {
-            sc.n[c] = rec[3 + c];
-            sc.J[c] = {rec[6 + 2 * c], rec[7 + 2 * c]};
-            sc.M[c] = {rec[12 + 2 * c], rec[13 + 2 * c]};
-        }
-        src_const_finish<double, true>(sc);
-        double r[15];
-        if (KIND == kKindFF) ff_direction_d(tgt7, nt, ti, r);
-        else
-            for (int c = 0; c < 3; ++c) r[c] = tgt7[c * nt + ti];
-        for (int q = 0; q < 12; ++q) r[3 + q] = gam[(long)q * nt + ti];
-        double acc[kAccAdj];
-        for (int a = 0; a < kAccAdj; ++a) acc[a] = 0.0;
-        adj_src_pair_fp64<KIND, T>(rec, sc, r, k, acc);
-        for (int a = 0; a < kAccAdj; ++a) {
-            const double v = a < 12 ? acc[a] : acc[a] * inv_kappa;
-            if (v != 0.0) atomicAdd(&part[(long)a * ns + si], v);
-        }
-        if (WANT_T) {
-            TgtConst tc;
-            tgt_const(tgt7, gam, nt, ti, tc);
-            const double v = adj_tgt_pair_fp64<KIND, T>(tc, rec, k) * inv_kappa;
-            if (v != 0.0) atomicAdd(&gt[ti], v);
-        }
-    }
-}
-
 // ---------------------------------------------------------------- epilogues
 
 // Sums the chunks of the source-side partials; unfolds the currents by
@@ -601,40 +173,6 @@ __global__ void po_adj_tgt_epilogue_kernel(int nsplit, long nt, const double *__
 }
 
 // ----------------------------------------------------------- instantiations
-
-void *adj_src_fp64_kernel(int kind, int t_sign)
-{
-    if (kind == kKindScalar)
-        return t_sign < 0 ? reinterpret_cast<void *>(&po_adj_src_fp64_kernel<kKindScalar, -1>)
-                          : reinterpret_cast<void *>(&po_adj_src_fp64_kernel<kKindScalar, 1>);
-    if (kind == kKindNF)
-        return t_sign < 0 ? reinterpret_cast<void *>(&po_adj_src_fp64_kernel<kKindNF, -1>)
-                          : reinterpret_cast<void *>(&po_adj_src_fp64_kernel<kKindNF, 1>);
-    return t_sign < 0 ? reinterpret_cast<void *>(&po_adj_src_fp64_kernel<kKindFF, -1>)
-                      : reinterpret_cast<void *>(&po_adj_src_fp64_kernel<kKindFF, 1>);
-}
-
-void *adj_tgt_fp64_kernel(int kind, int t_sign)
-{
-    if (kind == kKindScalar)
-        return t_sign < 0 ? reinterpret_cast<void *>(&po_adj_tgt_fp64_kernel<kKindScalar, -1>)
-                          : reinterpret_cast<void *>(&po_adj_tgt_fp64_kernel<kKindScalar, 1>);
-    return t_sign < 0 ? reinterpret_cast<void *>(&po_adj_tgt_fp64_kernel<kKindNF, -1>)
-                      : reinterpret_cast<void *>(&po_adj_tgt_fp64_kernel<kKindNF, 1>);
-}
-
-void *adj_band_fixup_kernel(int kind, int t_sign, bool want_d, bool want_t)
-{
-    (void)want_d;   // the source displacement term is always kept (it is one partial row)
-    if (kind == kKindFF)
-        return t_sign < 0 ? reinterpret_cast<void *>(&po_adj_band_fixup_kernel<kKindFF, -1, false>)
-                          : reinterpret_cast<void *>(&po_adj_band_fixup_kernel<kKindFF, 1, false>);
-    if (want_t)
-        return t_sign < 0 ? reinterpret_cast<void *>(&po_adj_band_fixup_kernel<kKindNF, -1, true>)
-                          : reinterpret_cast<void *>(&po_adj_band_fixup_kernel<kKindNF, 1, true>);
-    return t_sign < 0 ? reinterpret_cast<void *>(&po_adj_band_fixup_kernel<kKindNF, -1, false>)
-                      : reinterpret_cast<void *>(&po_adj_band_fixup_kernel<kKindNF, 1, false>);
-}
 
 void *adj_cot_kernel() { return reinterpret_cast<void *>(&po_adj_cot_kernel); }
 void *adj_ehp_cot_kernel() { return reinterpret_cast<void *>(&po_adj_ehp_cot_kernel); }

@@ -225,11 +225,13 @@ __device__ __forceinline__ void band_defer(const BandList &bl, long si, long ti)
     if (i < bl.cap) bl.pairs[i] = make_int2((int)si, (int)ti);
 }
 
-// One source's FP64 record (kRecD doubles: x y z nx ny nz, J' (re, im) x y z,
-// M' likewise; scalar: S' in the J'x slot): the currents times the trapezoid
-// weight, the area and the complex factor (fac_re, fac_im).
+// One source's FP64 record (rec doubles: x y z nx ny nz, J' (re, im) x y z
+// and, with rec == kRecD, M' likewise; scalar: S' in the J'x slot): the
+// currents times the trapezoid weight, the area and the complex factor
+// (fac_re, fac_im).
 __device__ __forceinline__ void src_record_d(long i, long ns, const double *src7, const double *cur, int gmode,
-                                             int ncx, int ncy, double fac_re, double fac_im, int scalar, double *o)
+                                             int ncx, int ncy, double fac_re, double fac_im, int scalar, int rec,
+                                             double *o)
 {
     for (int c = 0; c < 6; ++c) o[c] = src7[c * ns + i];
     const double w = trap_weight(i, gmode, ncx, ncy) * src7[6 * ns + i];
@@ -238,10 +240,9 @@ __device__ __forceinline__ void src_record_d(long i, long ns, const double *src7
         const double re = cur[i], im = cur[ns + i];
         o[6] = fr_ * re - fi_ * im;
         o[7] = fr_ * im + fi_ * re;
-        for (int q = 8; q < kRecD; ++q) o[q] = 0.0;
         return;
     }
-    for (int q = 0; q < 6; ++q) {
+    for (int q = 0; q < (rec - 6) / 2; ++q) {
         const int grp = q / 3, ax = q % 3;
         const double re = cur[(grp * 6 + ax) * ns + i];
         const double im = cur[(grp * 6 + 3 + ax) * ns + i];

@@ -4,7 +4,8 @@
 //   bbox -> frame -> pack sources / targets -> main N-body kernel over a
 //   (target block, source chunk) grid -> FP64 epilogue summing the chunks.
 // Plain FP64 (precision 1):
-//   pack sources (double) -> one-thread-per-target FP64 direct sum -> epilogue.
+//   pack sources (double) -> FP64 direct sum over a (target block, source
+//   chunk) grid -> epilogue.
 // Scratch is stream-ordered on the caller's stream, from the library's own
 // memory pool (scratch_alloc / scratch_free); nothing here synchronises the
 // device.
@@ -35,7 +36,7 @@ struct DeviceInfo {
     cudaMemPool_t pool = nullptr;   // the library's own scratch pool
     int occ2[3][2][2] = {};  // pair-packed kernels, [kind][t>0][has_m]
     int occ_ff[2][2] = {};   // far-field tile kernels, [t>0][has_m]
-    std::map<void *, int> occ_adj;   // adjoint kernels: resident CTAs, attribute set
+    std::map<void *, int> occ_adj;   // adjoint and FP64 kernels: resident CTAs, attribute set
 };
 
 std::mutex g_mu;
@@ -124,6 +125,23 @@ static int device_info(DeviceInfo *&out)
         di.ready = true;
     }
     out = &di;
+    return 0;
+}
+
+// Resident CTAs per SM of a kernel (and its shared-memory attribute), looked
+// up once per device and kernel.
+static int kernel_occupancy(DeviceInfo *di, void *fk, int threads, int smem, int &occ)
+{
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = di->occ_adj.find(fk);
+    if (it != di->occ_adj.end()) {
+        occ = it->second;
+        return 0;
+    }
+    int nb = 0;
+    if (smem > 0) PO_CK(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    PO_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fk, threads, smem));
+    occ = di->occ_adj[fk] = std::max(nb, 1);
     return 0;
 }
 
@@ -354,7 +372,7 @@ int run_device(const RunArgs &a)
         return run_mixed(a, pool, err);
     }
 
-    // ---- plain FP64: one thread per target, the comparison path
+    // ---- plain FP64
     const int kind = a.mode == kFF ? kKindFF : (a.mode == kScalar ? kKindScalar : kKindNF);
     const int nacc = kind == kKindScalar ? 2 : kAcc;
     const double pif = (double)3.14159265359f;   // the reference's float-literal pi
@@ -375,21 +393,31 @@ int run_device(const RunArgs &a)
     const int scalar = kind == kKindScalar;
     const double *src7 = a.src7, *cur = a.cur, *tgt7 = a.tgt7;
     double *out = a.out;
+    const bool has_m = !scalar && !a.m_zero;
+    int rec = fp64_rec(kind, has_m);
+    void *fk = fp64_kernel(kind, has_m);
+    DeviceInfo *di = nullptr;
+    int occ = 1;
+    if ((rc = device_info(di)) || (rc = kernel_occupancy(di, fk, kThreadsD, 0, occ))) return rc;
+    const long ntb = (nt + kThreadsD - 1) / kThreadsD;
+    const long nsplit = choose_split(ntb, ns, (long)di->sms * occ, partial_cap(nt, nacc), kChunkD);
+    const long tiles = std::max(1L, (ns + kChunkD - 1) / kChunkD);
+    long chunk = (tiles + nsplit - 1) / nsplit * kChunkD;
     double *srcd = nullptr, *part = nullptr;
-    if ((rc = salloc(&srcd, (size_t)std::max(ns, 1L) * kRecD, s, owned)) ||
-        (rc = salloc(&part, (size_t)nacc * nt, s, owned))) {
+    if ((rc = salloc(&srcd, (size_t)std::max(ns, 1L) * rec, s, owned)) ||
+        (rc = salloc(&part, (size_t)nsplit * nacc * nt, s, owned))) {
         sfree(owned, s);
         return rc;
     }
-    void *pargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, (void *)&scalar, &srcd};
+    Wave64 w = wave64(k, t);
+    void *pargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, (void *)&scalar, &rec, &srcd};
     if (ns > 0) rc = launch(pack_src_d_kernel(), dim3(nblk_s), dim3(256), pargs, 0, s);
-    void *fargs[] = {&srcd, &ns, &tgt7, &nt, &k, &t, &part};
+    void *fargs[] = {&srcd, &ns, &chunk, &tgt7, &nt, &w, &part};
     timing_mark(s, true);
-    if (!rc) rc = launch(fp64_kernel(kind), dim3((unsigned)((nt + kThreadsD - 1) / kThreadsD)), dim3(kThreadsD),
-                         fargs, 0, s);
+    if (!rc) rc = launch(fk, dim3((unsigned)ntb, (unsigned)nsplit), dim3(kThreadsD), fargs, 0, s);
     timing_mark(s, false);
-    int one = 1;
-    void *eargs[] = {&mode, &one, &nt, &part, &tgt7, &t, &zeta_inv, &out};
+    int nspl = (int)nsplit;
+    void *eargs[] = {&mode, &nspl, &nt, &part, &tgt7, &t, &zeta_inv, &out};
     if (!rc) rc = launch(epilogue_kernel(), dim3(nblk_t), dim3(256), eargs, 0, s);
     sfree(owned, s);
     return rc;
@@ -516,8 +544,8 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
     timing_mark(s, false);
     if (!rc && p.band.count && ns > 0) {
         // the near-tangent pairs, decided and summed in FP64 into chunk 0
-        double k = a.k;
-        void *xargs[] = {&p.band, &ns, &src7, &cur, &gmode, &ncx, &ncy, &p.fac_re, &p.fac_im, &nt, &tgt7, &k, &t,
+        Wave64 w = wave64(a.k, t);
+        void *xargs[] = {&p.band, &ns, &src7, &cur, &gmode, &ncx, &ncy, &p.fac_re, &p.fac_im, &nt, &tgt7, &w,
                          &p.part, &err};
         rc = launch(band_fixup_kernel(p.kind), dim3(kFixupBlocks), dim3(256), xargs, 0, s);
     }
@@ -611,34 +639,41 @@ int run_adjoint(const AdjArgs &a)
     const int fp64_scalar = kind == kKindScalar ? 1 : 0, mixed_scalar = kind == kKindScalar ? 2 : 0;
 
     if (a.precision == 1) {
-        double *srcd = nullptr, *part = nullptr, *partt = nullptr;
-        if (!rc && ((rc = salloc(&srcd, (size_t)ns * kRecD, s, owned)) ||
-                    (rc = salloc(&part, (size_t)kAccAdj * ns, s, owned)) ||
-                    (rc = salloc(&partt, (size_t)std::max(nt, 1L), s, owned)))) {
+        const bool want_t = grad_dt != nullptr;
+        int rec = fp64_rec(kind, has_m);
+        void *fk = adj_fp64_kernel(kind, has_m, want_d, want_t);
+        int occ = 1;
+        if (!rc) rc = kernel_occupancy(di, fk, kThreadsD, 0, occ);
+        const long nsb = (ns + kThreadsD - 1) / kThreadsD;
+        const long nsplit = choose_split(nsb, nt, (long)di->sms * occ, partial_cap(ns, kAccAdj), kChunkD);
+        const long tiles = (nt + kChunkD - 1) / kChunkD;
+        long chunk = (tiles + nsplit - 1) / nsplit * kChunkD;
+        double *srcd = nullptr, *trec = nullptr, *part = nullptr, *gt = nullptr;
+        if (!rc && ((rc = salloc(&srcd, (size_t)ns * rec, s, owned)) ||
+                    (rc = salloc(&trec, (size_t)nt * adj64_rec(kind), s, owned)) ||
+                    (rc = salloc(&part, (size_t)nsplit * kAccAdj * ns, s, owned)) ||
+                    (want_t && (rc = salloc(&gt, (size_t)nt, s, owned))))) {
             sfree(owned, s);
             return rc;
         }
-        void *pargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, (void *)&fp64_scalar, &srcd};
+        Wave64 w = wave64(k, t);
+        void *pargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, (void *)&fp64_scalar, &rec, &srcd};
         if (!rc) rc = launch(pack_src_d_kernel(), dim3(nblk_s), dim3(256), pargs, 0, s);
-        void *sargs[] = {&srcd, &ns, &tgt7, &gam, &nt, &k, &part};
+        void *tpargs[] = {&nt, &tgt7, &gam, &trec};
+        if (!rc) rc = launch(adj_pack_tgt_d_kernel(kind), dim3(nblk_t), dim3(256), tpargs, 0, s);
+        if (want_t) PO_CK_RC(cudaMemsetAsync(gt, 0, sizeof(double) * nt, s));
+        void *sargs[] = {&srcd, &ns, &trec, &nt, &chunk, &w, &part, &gt};
         timing_mark(s, true);
-        if (!rc) rc = launch(adj_src_fp64_kernel(kind, ts), dim3((unsigned)((ns + kThreadsD - 1) / kThreadsD)),
-                             dim3(kThreadsD), sargs, 0, s);
+        if (!rc) rc = launch(fk, dim3((unsigned)nsb, (unsigned)nsplit), dim3(kThreadsD), sargs, 0, s);
         timing_mark(s, false);
-        int one = 1;
-        double dsc = far ? 1.0 : -1.0;
-        void *eargs[] = {(void *)&kind, &one, &ns, &part, &src7, &gmode, &ncx, &ncy, &fac_re, &fac_im, &dsc,
+        int nspl = (int)nsplit, one = 1;
+        double dsc = far ? 1.0 : -1.0, one_d = 1.0;
+        void *eargs[] = {(void *)&kind, &nspl, &ns, &part, &src7, &gmode, &ncx, &ncy, &fac_re, &fac_im, &dsc,
                          &grad_cur, &grad_ds};
         if (!rc) rc = launch(adj_src_epilogue_kernel(), dim3(nblk_s), dim3(256), eargs, 0, s);
-        if (!rc && grad_dt) {
-            void *targs[] = {&srcd, &ns, &tgt7, &gam, &nt, &k, &partt};
-            timing_mark(s, true);
-            rc = launch(adj_tgt_fp64_kernel(kind, ts), dim3((unsigned)((nt + kThreadsD - 1) / kThreadsD)), dim3(kThreadsD),
-                        targs, 0, s);
-            timing_mark(s, false);
-            double one_d = 1.0;
-            void *teargs[] = {&one, &nt, &partt, &one_d, &grad_dt};
-            if (!rc) rc = launch(adj_tgt_epilogue_kernel(), dim3(nblk_t), dim3(256), teargs, 0, s);
+        if (!rc && want_t) {
+            void *teargs[] = {&one, &nt, &gt, &one_d, &grad_dt};
+            rc = launch(adj_tgt_epilogue_kernel(), dim3(nblk_t), dim3(256), teargs, 0, s);
         }
         sfree(owned, s);
         return rc;
@@ -732,19 +767,7 @@ int run_adjoint(const AdjArgs &a)
     void *fk = adj_pk_kernel(kind, ts, has_m, want_d, want_t);
     const int smem2 = adj_pk_smem_bytes(kind, has_m, want_t);
     int occ2 = 1;
-    {
-        // once per device and kernel: the shared-memory attribute and the occupancy
-        std::lock_guard<std::mutex> lk(g_mu);
-        auto it = di->occ_adj.find(fk);
-        if (it != di->occ_adj.end()) {
-            occ2 = it->second;
-        } else {
-            PO_CK_RC(cudaFuncSetAttribute(fk, cudaFuncAttributeMaxDynamicSharedMemorySize, smem2));
-            PO_CK_RC(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ2, fk, kThreadsA, smem2));
-            occ2 = std::max(occ2, 1);
-            if (!rc) di->occ_adj[fk] = occ2;
-        }
-    }
+    if (!rc) rc = kernel_occupancy(di, fk, kThreadsA, smem2, occ2);
     const long tile_t = 2L * adj_pk_pairs_per_tile();
     const long nsb = (ns + kThreadsA - 1) / kThreadsA;
     const long split = choose_split(nsb, nt, (long)di->sms * occ2, partial_cap(ns, kAccAdj), tile_t);
@@ -760,9 +783,10 @@ int run_adjoint(const AdjArgs &a)
     if (!rc && band.count) {
         // the near-tangent pairs, decided and summed in FP64 into chunk 0 (and gt)
         double inv_kappa = 1.0 / kappa;
-        void *xargs[] = {&band, &ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, &nt, &tgt7, &gam, &k,
+        Wave64 w = wave64(k, t);
+        void *xargs[] = {&band, &ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, &nt, &tgt7, &gam, &w,
                          &inv_kappa, &part, &gt, &err};
-        rc = launch(adj_band_fixup_kernel(kind, ts, want_d, want_t), dim3(kFixupBlocks), dim3(256), xargs, 0, s);
+        rc = launch(adj_band_fixup_kernel(kind, want_t), dim3(kFixupBlocks), dim3(256), xargs, 0, s);
     }
     int nspl = (int)split;
     double dsc = far ? kappa : -kappa;

@@ -32,9 +32,8 @@
 //     kernel adds the chunks in a fixed order and applies the mode's physics
 //     (PEC current, EHP reflection, far-field projection) in FP64.
 //
-// The plain FP64 direct sum (po_fp64_kernel) is the comparison path: same
-// formulas, double everywhere, no splitting. The far field's forward kernel
-// is in po_farfield.cu.
+// The far field's forward kernel is in po_farfield.cu, the plain FP64 sums
+// (and the fixups above) in po_fp64.cu.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <cstdint>
@@ -683,141 +682,6 @@ __global__ void po_pack_tgt_kernel(long nt, const double *__restrict__ tgt7, con
     out[2 * i + 1] = make_float4(l[1], l[2], 0.f, 0.f);
 }
 
-// ---------------------------------------------------------------- FP64 path
-
-// Double record (kRecD doubles): x y z nx ny nz, J'(re,im)x3, M'(re,im)x3.
-__global__ void po_pack_src_d_kernel(long ns, const double *__restrict__ src7, const double *__restrict__ cur,
-                                     int gmode, int ncx, int ncy, double fac_re, double fac_im, int scalar,
-                                     double *__restrict__ out)
-{
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ns) return;
-    src_record_d(i, ns, src7, cur, gmode, ncx, ncy, fac_re, fac_im, scalar, out + (size_t)kRecD * i);
-}
-
-// One pair of the plain FP64 sum, added into acc (kAcc accumulators, or 2 for
-// the scalar kind): p the target point (mm) or, far field, its direction; r
-// the source's kRecD record. A pair the reference does not illuminate adds
-// nothing; the decision repeats its operation order and rounding (R_hat =
-// d * (1/R), then n . R_hat summed left to right, no FMA), so tangent pairs
-// are decided as it decides them.
-template <int KIND>
-__device__ __forceinline__ void fp64_pair(const double *p, const double *r, double k, double t, double *acc)
-{
-    if (KIND == kKindNF) {
-        const double dx = p[0] - r[0], dy = p[1] - r[1], dz = p[2] - r[2];
-        const double R = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
-        const double rinv = __ddiv_rn(1.0, R);
-        if (!lit_fp64(r + 3, dx, dy, dz, rinv)) return;
-        double sn, cs;
-        sincos(k * R, &sn, &cs);
-        const double gc = cs, gs = t * sn;
-        const double u = rinv / k, u2 = u * u;
-        const double s1r = t * u2, s1i = u2 * u - u;
-        const double c1r = gc * s1r - gs * s1i, c1i = gc * s1i + gs * s1r;
-        const double rinv2 = rinv * rinv;
-        const double c2r = (-3.0 * c1r + 2.0 * u * gs) * rinv2;
-        const double c2i = (-3.0 * c1i - 2.0 * u * gc) * rinv2;
-        const double s3r = -u2 * rinv, s3i = t * u * rinv;
-        const double c3r = gc * s3r - gs * s3i, c3i = gc * s3i + gs * s3r;
-        const double d[3] = {dx, dy, dz};
-        const double *J = r + 6, *M = r + 12;
-        const double jdr = J[0] * dx + J[2] * dy + J[4] * dz, jdi = J[1] * dx + J[3] * dy + J[5] * dz;
-        const double mdr = M[0] * dx + M[2] * dy + M[4] * dz, mdi = M[1] * dx + M[3] * dy + M[5] * dz;
-        const double Pr = c2r * jdr - c2i * jdi, Pi = c2r * jdi + c2i * jdr;
-        const double Qr = c2r * mdr - c2i * mdi, Qi = c2r * mdi + c2i * mdr;
-        for (int c = 0; c < 3; ++c) {
-            const int a1 = (c + 1) % 3, a2 = (c + 2) % 3;
-            // (J x d)_c and (M x d)_c
-            const double jxr = J[2 * a1] * d[a2] - J[2 * a2] * d[a1];
-            const double jxi = J[2 * a1 + 1] * d[a2] - J[2 * a2 + 1] * d[a1];
-            const double mxr = M[2 * a1] * d[a2] - M[2 * a2] * d[a1];
-            const double mxi = M[2 * a1 + 1] * d[a2] - M[2 * a2 + 1] * d[a1];
-            acc[c] += c1r * J[2 * c] - c1i * J[2 * c + 1] + Pr * d[c] + c3r * mxr - c3i * mxi;
-            acc[3 + c] += c1r * J[2 * c + 1] + c1i * J[2 * c] + Pi * d[c] + c3r * mxi + c3i * mxr;
-            acc[6 + c] += c1r * M[2 * c] - c1i * M[2 * c + 1] + Qr * d[c] - (c3r * jxr - c3i * jxi);
-            acc[9 + c] += c1r * M[2 * c + 1] + c1i * M[2 * c] + Qi * d[c] - (c3r * jxi + c3i * jxr);
-        }
-    } else if (KIND == kKindFF) {
-        if (__dadd_rn(__dadd_rn(__dmul_rn(r[3], p[0]), __dmul_rn(r[4], p[1])), __dmul_rn(r[5], p[2])) < 0.0) return;
-        double sn, cs;
-        sincos(k * (r[0] * p[0] + r[1] * p[1] + r[2] * p[2]), &sn, &cs);
-        const double gc = cs, gs = -t * sn;
-        for (int c = 0; c < 6; ++c) {
-            const double cr = r[6 + 2 * c], ci = r[7 + 2 * c];
-            const int slot = (c < 3) ? c : 6 + (c - 3);
-            acc[slot] += gc * cr - gs * ci;
-            acc[slot + 3] += gc * ci + gs * cr;
-        }
-    } else {
-        const double dx = p[0] - r[0], dy = p[1] - r[1], dz = p[2] - r[2];
-        const double R = sqrt(dx * dx + dy * dy + dz * dz);
-        double sn, cs;
-        sincos(k * R, &sn, &cs);
-        const double gr = cs / R, gi = -t * sn / R;
-        acc[0] += gr * r[6] - gi * r[7];
-        acc[1] += gr * r[7] + gi * r[6];
-    }
-}
-
-template <int KIND>
-__global__ void __launch_bounds__(kThreadsD)
-po_fp64_kernel(const double *__restrict__ src, long ns, const double *__restrict__ tgt7, long nt, double k,
-               double t, double *__restrict__ part)
-{
-    __shared__ double tile[kTileD * kRecD];
-    const long ti = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    double p[3] = {0, 0, 0};
-    if (ti < nt) {
-        if (KIND == kKindFF) ff_direction_d(tgt7, nt, ti, p);
-        else
-            for (int c = 0; c < 3; ++c) p[c] = tgt7[c * nt + ti];
-    }
-    double acc[kAcc];
-    for (int a = 0; a < kAcc; ++a) acc[a] = 0.0;
-    for (long base = 0; base < ns; base += kTileD) {
-        const int cnt = (int)min((long)kTileD, ns - base);
-        __syncthreads();
-        for (int q = threadIdx.x; q < cnt * kRecD; q += blockDim.x) tile[q] = src[base * kRecD + q];
-        __syncthreads();
-        if (ti >= nt) continue;
-        for (int s = 0; s < cnt; ++s) fp64_pair<KIND>(p, tile + s * kRecD, k, t, acc);
-    }
-    if (ti < nt) {
-        const int nacc = (KIND == kKindScalar) ? 2 : kAcc;
-        for (int a = 0; a < nacc; ++a) part[(long)a * nt + ti] = acc[a];
-    }
-}
-
-// The pairs a mixed kernel left out as inside the tangent band: each is
-// decided by the reference's FP64 rounding and, if lit, its FP64 term is
-// added into the first source chunk's partial sums (the epilogue adds the
-// chunks afterwards). The order of those additions varies between runs for
-// a target with several such pairs (last-bit differences there only).
-template <int KIND>
-__global__ void __launch_bounds__(256)
-po_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, const double *__restrict__ cur,
-                     int gmode, int ncx, int ncy, double fac_re, double fac_im, long nt,
-                     const double *__restrict__ tgt7, double k, double t, double *__restrict__ part,
-                     int *__restrict__ err)
-{
-    const unsigned total = *bl.count;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && total > bl.cap) atomicExch(err, kErrBandOverflow);
-    const unsigned n = min(total, bl.cap);
-    for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int2 pr = bl.pairs[i];
-        double rec[kRecD], p[3], acc[kAcc];
-        src_record_d(pr.x, ns, src7, cur, gmode, ncx, ncy, fac_re, fac_im, 0, rec);
-        if (KIND == kKindFF) ff_direction_d(tgt7, nt, pr.y, p);
-        else
-            for (int c = 0; c < 3; ++c) p[c] = tgt7[c * nt + pr.y];
-        for (int a = 0; a < kAcc; ++a) acc[a] = 0.0;
-        fp64_pair<KIND>(p, rec, k, t, acc);
-        for (int a = 0; a < kAcc; ++a)
-            if (acc[a] != 0.0) atomicAdd(&part[(long)a * nt + pr.y], acc[a]);
-    }
-}
-
 // ------------------------------------------------------------------ epilogue
 
 __device__ __forceinline__ void cross_d(const double a[3], const double b[3], double o[3])
@@ -931,13 +795,6 @@ __global__ void __launch_bounds__(256) po_fp32_probe_kernel(int iters, float see
 
 // ----------------------------------------------------------- instantiations
 
-void *fp64_kernel(int kind)
-{
-    if (kind == kKindNF) return reinterpret_cast<void *>(&po_fp64_kernel<kKindNF>);
-    if (kind == kKindFF) return reinterpret_cast<void *>(&po_fp64_kernel<kKindFF>);
-    return reinterpret_cast<void *>(&po_fp64_kernel<kKindScalar>);
-}
-
 template <int KIND, int T, bool HAS_M>
 static void *pk_ptr()
 {
@@ -959,7 +816,6 @@ void *bbox_kernel() { return reinterpret_cast<void *>(&po_bbox_kernel); }
 void *frame_kernel() { return reinterpret_cast<void *>(&po_frame_kernel); }
 void *pack_src_kernel() { return reinterpret_cast<void *>(&po_pack_src_kernel); }
 void *pack_tgt_kernel() { return reinterpret_cast<void *>(&po_pack_tgt_kernel); }
-void *pack_src_d_kernel() { return reinterpret_cast<void *>(&po_pack_src_d_kernel); }
 // Precision conversions of the float drop-in ABI's buffers (n elements).
 __global__ void po_f2d_kernel(const float *__restrict__ in, double *__restrict__ out, long n)
 {
@@ -978,10 +834,5 @@ void *f2d_kernel() { return reinterpret_cast<void *>(&po_f2d_kernel); }
 void *d2f_kernel() { return reinterpret_cast<void *>(&po_d2f_kernel); }
 void *fp32_probe_kernel() { return reinterpret_cast<void *>(&po_fp32_probe_kernel); }
 void *wait_selftest_kernel() { return reinterpret_cast<void *>(&po_wait_selftest_kernel); }
-void *band_fixup_kernel(int kind)
-{
-    return kind == kKindFF ? reinterpret_cast<void *>(&po_band_fixup_kernel<kKindFF>)
-                           : reinterpret_cast<void *>(&po_band_fixup_kernel<kKindNF>);
-}
 
 }  // namespace po

@@ -89,10 +89,25 @@ constexpr int kUnrollF = PO_UNROLL_F;
 constexpr int kUnrollA = PO_UNROLL_A;   // target pairs per iteration of the adjoint pair loop
 constexpr int kAccAdj = 13;
 
-// FP64 comparison kernel.
+// Plain FP64 kernels (po_fp64.cu).
 constexpr int kThreadsD = 128;
 constexpr int kTileD = 64;
+// Granularity of a chunk of the streamed axis: 16 lets a few hundred points
+// fill the GPU and evens the last wave (101 x 99 -> 41 x 43 forward and
+// adjoint: 13.3 ms; 14.9 with 64, 12.8 with 32, but 13 x 13 -> 5 x 5: 0.45,
+// 0.78 and 0.61 ms).
+constexpr int kChunkD = 16;
 constexpr int kRecD = 18;       // x y z nx ny nz, J' 6, M' 6 (doubles)
+// Doubles per source record (scalar: point, normal, S'; M = 0: no M') and
+// per target record of the adjoint.
+__host__ __device__ constexpr int fp64_rec(int kind, bool has_m) { return kind == kKindScalar ? 8 : (has_m ? kRecD : 12); }
+__host__ __device__ constexpr int adj64_rec(int kind) { return kind == kKindScalar ? 8 : (kind == kKindFF ? 18 : 22); }
+// The wave as the FP64 kernels take it: k, 1/k and the sign bit of t.
+struct Wave64 {
+    double k, inv_k;
+    unsigned neg;
+};
+Wave64 wave64(double k, double t);
 
 constexpr int kBboxThreads = 256;
 constexpr int kBboxBlocks = 152;
@@ -175,7 +190,7 @@ inline int pk_smem_bytes(int kind)
 void *pk_kernel(int kind, int t_sign, bool has_m);
 void *pack_src2_kernel();
 void *src_box_kernel();
-void *fp64_kernel(int kind);
+void *fp64_kernel(int kind, bool has_m);
 void *bbox_kernel();
 void *frame_kernel();
 void *pack_src_kernel();
@@ -186,10 +201,10 @@ void *f2d_kernel();   // float -> double, grid-stride over n
 void *d2f_kernel();   // double -> float
 void *fp32_probe_kernel();
 void *band_fixup_kernel(int kind);
-void *adj_band_fixup_kernel(int kind, int t_sign, bool want_d, bool want_t);
+void *adj_band_fixup_kernel(int kind, bool want_t);
 void *wait_selftest_kernel();
-void *adj_src_fp64_kernel(int kind, int t_sign);
-void *adj_tgt_fp64_kernel(int kind, int t_sign);
+void *adj_fp64_kernel(int kind, bool has_m, bool want_d, bool want_t);
+void *adj_pack_tgt_d_kernel(int kind);
 void *adj_cot_kernel();
 void *adj_ehp_cot_kernel();
 void *adj_src_epilogue_kernel();
