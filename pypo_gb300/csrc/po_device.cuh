@@ -56,6 +56,19 @@ __device__ __forceinline__ void fence_proxy_async()
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Programmatic dependent launch. A kernel launched after another one with
+// programmatic stream serialisation may start while that one runs: it begins
+// with pdl_wait(), which returns when every earlier kernel's writes are
+// visible. pdl_trigger() lets the next kernel's blocks be scheduled once every
+// block of this one has called it or ended; without a dependent both do
+// nothing. It stands at a kernel's end: called at the start of a kernel of
+// many blocks, it has the next kernel's few blocks placed on whichever SMs
+// are free at that moment instead of one to an SM (161,202 sources -> 25
+// targets: the 158 blocks of the pair kernel took 142 us alone and the call
+// 380 us).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 __device__ __forceinline__ void tma_load_1d(void *dst, const void *src, uint32_t bytes, uint64_t *bar)
 {
     asm volatile(

@@ -1,8 +1,9 @@
 // po_engine.cu -- host orchestration of one propagation on device buffers.
 //
 // Mixed precision (precision 0):
-//   bbox -> frame -> pack sources / targets -> main N-body kernel over a
-//   (target block, source chunk) grid -> FP64 epilogue summing the chunks.
+//   frame -> pack sources and targets -> main N-body kernel over a (target
+//   block, source chunk) grid -> near-tangent pairs -> FP64 epilogue summing
+//   the chunks.
 // Plain FP64 (precision 1):
 //   pack sources (double) -> FP64 direct sum over a (target block, source
 //   chunk) grid -> epilogue.
@@ -122,6 +123,7 @@ static int device_info(DeviceInfo *&out)
                 PO_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kThreads, smem));
                 di.occ_ff[ts][hm] = std::max(nb, 1);
             }
+        PO_CK(cudaFuncSetAttribute(frame_kernel(), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
         di.ready = true;
     }
     out = &di;
@@ -148,6 +150,9 @@ static int kernel_occupancy(DeviceInfo *di, void *fk, int threads, int smem, int
 long choose_split(long nb, long ns, long slots, long max_chunks, long tile)
 {
     const long tiles = std::max(1L, (ns + tile - 1) / tile);
+    // a chunk's partials cost the epilogue about 0.05 of a full wave's tile,
+    // less where the owning blocks fill only part of a wave
+    const double per_chunk = 0.002 + 0.048 * std::min(1.0, (double)nb / (double)slots);
     long best = 1;
     double best_cost = 1e300;
     for (long s = 1; s <= std::min(tiles, std::min(std::max(1L, max_chunks), 1024L)); ++s) {
@@ -155,7 +160,7 @@ long choose_split(long nb, long ns, long slots, long max_chunks, long tile)
         const long real = (tiles + chunk - 1) / chunk;
         if (real != s) continue;
         const long waves = (nb * real + slots - 1) / slots;
-        const double cost = (double)waves * chunk + 0.05 * real;
+        const double cost = (double)waves * chunk + per_chunk * real;
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = real;
@@ -240,24 +245,54 @@ static void sfree(std::vector<void *> &owned, cudaStream_t s)
     owned.clear();
 }
 
-// Stream-ordered scratch from the library's pool, freed (in stream order)
-// when the call's work is queued.
+// Stream-ordered scratch from the library's pool: one allocation per call
+// (each costs the stream about 2 us), carved up at commit() and freed (in
+// stream order) when the call's work is queued.
 class PoolScratch : public Scratch {
 public:
     explicit PoolScratch(cudaStream_t s) : s_(s) {}
-    ~PoolScratch() override { sfree(owned_, s_); }
+    ~PoolScratch() override { scratch_free(base_, s_); }
     int take(void **p, size_t bytes) override
     {
-        const int rc = scratch_alloc(p, bytes, s_);
-        if (!rc) owned_.push_back(*p);
-        return rc;
+        want_.push_back({p, used_});
+        used_ += (std::max<size_t>(bytes, 16) + 255) / 256 * 256;
+        return 0;
+    }
+    int commit() override
+    {
+        if (int rc = scratch_alloc(&base_, used_, s_)) return rc;
+        for (const auto &w : want_) *w.first = static_cast<char *>(base_) + w.second;
+        return 0;
     }
     size_t room() const override { return ~(size_t)0; }
 
 private:
     cudaStream_t s_;
-    std::vector<void *> owned_;
+    void *base_ = nullptr;
+    size_t used_ = 0;
+    std::vector<std::pair<void **, size_t>> want_;
 };
+
+// For a kernel that begins with pdl_wait(): it may start while the kernel
+// before it in the stream ends (programmatic stream serialisation; a chain
+// of small kernels takes 1.5 instead of 2.1 us a launch).
+static int launch_pdl(void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t s)
+{
+    if (grid.x == 0 || grid.y == 0) return 0;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    PO_CK(cudaLaunchKernelExC(&c, fn, args));
+    note_launches(1);
+    return 0;
+}
 
 static int launch(void *fn, dim3 grid, dim3 block, void **args, size_t smem, cudaStream_t s)
 {
@@ -360,6 +395,21 @@ int validate(const RunArgs &a)
     return 0;
 }
 
+// The epilogue of nsplit chunks: one thread a target, eight from eight chunks
+// on, and more where few targets (fewer blocks than SMs, each bound by its
+// SM's FP64 additions) have many chunks: 25 targets, 630 chunks: 30 us with
+// 32 threads, 18 us with 64.
+static int launch_epilogue(int mode, int nacc, int nsplit, long nt, const double *part, const double *tgt7, double t,
+                           double zeta_inv, double *out, cudaStream_t s)
+{
+    int groups = nsplit < 8 ? 1 : 8;
+    if (nsplit >= 32 && nt <= 152L * (kEpiThreads / 32)) groups = 32;
+    if (nsplit >= 64 && nt <= 152L * (kEpiThreads / 64)) groups = 64;
+    const long per = kEpiThreads / groups;
+    void *args[] = {&mode, &nacc, &nsplit, &nt, &part, &tgt7, &t, &zeta_inv, &out};
+    return launch_pdl(epilogue_kernel(groups), dim3((unsigned)((nt + per - 1) / per)), dim3(kEpiThreads), args, 0, s);
+}
+
 int run_device(const RunArgs &a)
 {
     if (int rc = validate(a)) return rc;
@@ -386,7 +436,7 @@ int run_device(const RunArgs &a)
     if (kind == kKindScalar) fac_re = -pref;
     std::vector<void *> owned;
     int rc = 0;
-    const unsigned nblk_s = (unsigned)((a.ns + 255) / 256), nblk_t = (unsigned)((a.nt + 255) / 256);
+    const unsigned nblk_s = (unsigned)((a.ns + 255) / 256);
     long nt = a.nt, ns = a.ns;
     int mode = a.mode, gmode = a.gmode, ncx = a.ncx, ncy = a.ncy;
     double t = a.t_dir, k = a.k;
@@ -417,8 +467,7 @@ int run_device(const RunArgs &a)
     if (!rc) rc = launch(fk, dim3((unsigned)ntb, (unsigned)nsplit), dim3(kThreadsD), fargs, 0, s);
     timing_mark(s, false);
     int nspl = (int)nsplit;
-    void *eargs[] = {&mode, &nspl, &nt, &part, &tgt7, &t, &zeta_inv, &out};
-    if (!rc) rc = launch(epilogue_kernel(), dim3(nblk_t), dim3(256), eargs, 0, s);
+    if (!rc) rc = launch_epilogue(mode, nacc, nspl, nt, part, tgt7, t, zeta_inv, out, s);
     sfree(owned, s);
     return rc;
 }
@@ -444,12 +493,11 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
     const bool scalar = p.kind == kKindScalar;
     p.far = p.kind == kKindFF;
     p.has_m = !scalar && !a.m_zero;
+    if (p.far && !p.has_m) p.nacc = 6;   // S_J alone
     const long ns = a.ns, nt = a.nt;
     p.tiles = std::max(1L, (ns + kTile - 1) / kTile);
     int rc = 0;
-    if ((rc = sc.get(&p.bbox, (size_t)kBboxBlocks * 6)) || (rc = sc.get(&p.frame, 1)) ||
-        (rc = sc.get(&p.tgtpk, (size_t)nt * 2)))
-        return rc;
+    if ((rc = sc.get(&p.frame, 1)) || (rc = sc.get(&p.tgtpk, (size_t)nt * 2))) return rc;
     if (!scalar) {
         p.band.cap = sc.band_cap(ns, nt);
         if ((rc = sc.get(&p.band.pairs, p.band.cap)) || (rc = sc.get(&p.band.count, 1))) return rc;
@@ -471,12 +519,12 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
     p.ntb = (nt + (long)kThreads * tpt - 1) / ((long)kThreads * tpt);
     const int occ = p.far ? di->occ_ff[p.ts > 0][p.has_m ? 1 : 0] : di->occ2[p.kind][p.ts > 0][p.has_m ? 1 : 0];
     const size_t room = std::min(sc.room(), (size_t)1 << 30);
-    const long max_chunks = (long)(room / ((size_t)p.nacc * nt * sizeof(double)));
-    if (max_chunks < 1) return sc.get(&p.part, (size_t)p.nacc * nt);   // fails with the source's message
+    const long max_chunks = std::max(1L, (long)(room / ((size_t)p.nacc * nt * sizeof(double))));
     p.nsplit = choose_split(p.ntb, ns, (long)di->sms * occ, max_chunks, kTile);
     const long chunk_tiles = (p.tiles + p.nsplit - 1) / p.nsplit;
     p.chunk = chunk_tiles * (p.far ? 1 : kTile);   // tiles (far field) or sources per chunk
-    return sc.get(&p.part, (size_t)p.nsplit * p.nacc * nt);
+    if ((rc = sc.get(&p.part, (size_t)p.nsplit * p.nacc * nt))) return rc;
+    return sc.commit();
 }
 
 int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
@@ -488,57 +536,48 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
     const int scalar = p.kind == kKindScalar;
     const double *src7 = a.src7, *cur = a.cur, *tgt7 = a.tgt7;
     double *out = a.out;
-    const unsigned nblk_s = (unsigned)((ns + 255) / 256), nblk_t = (unsigned)((nt + 255) / 256);
+    const unsigned nblk_s = (unsigned)((ns + 255) / 256);
     int rc = 0;
-    // ---- frame: far field keeps the coordinate origin (its phase reference)
-    long nb = p.far ? 0 : nt;   // the box covers the sources, plus the targets in the near field
-    void *bargs[] = {&src7, &ns, &tgt7, &nb, &p.bbox};
-    rc = launch(bbox_kernel(), dim3(kBboxBlocks), dim3(kBboxThreads), bargs, 0, s);
-    int nbb = kBboxBlocks;
-    int centred = p.far ? 0 : 1;
-    void *frargs[] = {&p.bbox, &nbb, &p.kappa, &centred, &p.frame};
-    if (!rc) rc = launch(frame_kernel(), dim3(1), dim3(32), frargs, 0, s);
+    // ---- frame: the box covers the sources, plus the targets in the near
+    // field; the far field keeps the coordinate origin (its phase reference)
+    long nb = p.far ? 0 : nt;
+    int centred = p.far ? 0 : 1, farflag = p.far ? 1 : 0;
+    void *frargs[] = {&src7, &ns, &tgt7, &nb, &p.kappa, &centred, &p.frame, &p.band.count};
+    rc = launch(frame_kernel(), dim3(kFrameCtas), dim3(kFrameThreads), frargs, 0, s);
     int boxes = !scalar && !p.has_m && ns > 0;   // the lit-tile proof serves the M = 0 kernels
-    if (p.far) {
-        // sources in Hilbert order, packed tile by tile with their centres
-        const long n1 = std::max(ns, 1L);
-        unsigned long long *k_in = p.keys, *k_out = p.keys + n1;
-        int *i_in = p.order, *i_out = p.order + n1;
+    // ---- sources (near field, scalar) and targets
+    long stiles = p.far || ns == 0 ? 0 : p.tiles;
+    void *pkargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &p.frame, &p.fac_re, &p.fac_im, &stiles,
+                      &p.srcpk, &nt, &tgt7, &farflag, &p.tgtpk};
+    if (!rc) rc = launch_pdl(pack_kernel(scalar, p.has_m), dim3((unsigned)(stiles + (nt + kTile - 1) / kTile)), dim3(kTile),
+                             pkargs, 0, s);
+    if (p.far && ns > 0) {
+        // far-field sources in Hilbert order, packed tile by tile with their centres
+        unsigned long long *k_in = p.keys, *k_out = p.keys + ns;
+        int *i_in = p.order, *i_out = p.order + ns;
         void *kargs[] = {&ns, &src7, &p.frame, &k_in, &i_in};
-        if (!rc && ns > 0) rc = launch(ff_key_kernel(), dim3(nblk_s), dim3(256), kargs, 0, s);
-        if (!rc && ns > 0) {
+        if (!rc) rc = launch_pdl(ff_key_kernel(), dim3(nblk_s), dim3(256), kargs, 0, s);
+        if (!rc) {
             cudaError_t e = ff_sort(p.sort_tmp, &p.sort_bytes, k_in, k_out, i_in, i_out, ns, s);
             if (e != cudaSuccess) rc = fail(2, std::string("source sort: ") + err_str(e));
             else note_launches(1);
         }
         const int *ord = i_out;
         void *pargs[] = {&ns, &ord, &src7, &cur, &gmode, &ncx, &ncy, &p.frame, &p.fac_re, &p.fac_im, &p.srcpk};
-        if (!rc && ns > 0) rc = launch(ff_pack_kernel(p.has_m), dim3((unsigned)p.tiles), dim3(32), pargs, 0, s);
-    } else {
-        float *srcf = reinterpret_cast<float *>(p.srcpk);
-        void *psargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &p.frame, &p.fac_re, &p.fac_im, (void *)&scalar, &srcf};
-        const unsigned nblk_p = (unsigned)((2 * ((ns + 1) / 2) + 255) / 256);
-        if (!rc && ns > 0) rc = launch(pack_src2_kernel(), dim3(nblk_p), dim3(256), psargs, 0, s);
-        float2 *rec2 = reinterpret_cast<float2 *>(p.srcpk);
-        void *sbargs[] = {&rec2, &ns};
-        if (!rc && boxes) rc = launch(src_box_kernel(), dim3((unsigned)p.tiles), dim3(32), sbargs, 0, s);
+        if (!rc) rc = launch(ff_pack_kernel(p.has_m), dim3((unsigned)p.tiles), dim3(32), pargs, 0, s);
     }
-    int farflag = p.far ? 1 : 0;
-    void *ptargs[] = {&nt, &tgt7, &p.frame, &farflag, &p.tgtpk};
-    if (!rc) rc = launch(pack_tgt_kernel(), dim3(nblk_t), dim3(256), ptargs, 0, s);
     const float4 *srcc = p.srcpk, *tgtc = p.tgtpk;
     long ntiles = ns > 0 ? p.tiles : 0;
     const int *sorted = p.order ? p.order + std::max(ns, 1L) : nullptr;   // far field: curve position -> source
-    if (!rc && p.band.count) PO_CK_RC(cudaMemsetAsync(p.band.count, 0, sizeof(unsigned), s));
     void *margs[] = {&srcc, p.far ? (void *)&ntiles : (void *)&ns, &p.chunk, &tgtc, &nt, &p.part, &err, &boxes,
                      &p.band, &ns, &sorted};
     timing_mark(s, true);
     if (!rc) {
         if (p.far)
-            rc = launch(ff_kernel(p.ts, p.has_m), dim3((unsigned)p.ntb, (unsigned)p.nsplit), dim3(kThreads), margs,
+            rc = launch_pdl(ff_kernel(p.ts, p.has_m), dim3((unsigned)p.ntb, (unsigned)p.nsplit), dim3(kThreads), margs,
                         ff_smem_bytes(p.has_m), s);
         else
-            rc = launch(pk_kernel(p.kind, p.ts, p.has_m), dim3((unsigned)p.ntb, (unsigned)p.nsplit), dim3(kThreads),
+            rc = launch_pdl(pk_kernel(p.kind, p.ts, p.has_m), dim3((unsigned)p.ntb, (unsigned)p.nsplit), dim3(kThreads),
                         margs, pk_smem_bytes(p.kind), s);
     }
     timing_mark(s, false);
@@ -547,11 +586,10 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
         Wave64 w = wave64(a.k, t);
         void *xargs[] = {&p.band, &ns, &src7, &cur, &gmode, &ncx, &ncy, &p.fac_re, &p.fac_im, &nt, &tgt7, &w,
                          &p.part, &err};
-        rc = launch(band_fixup_kernel(p.kind), dim3(kFixupBlocks), dim3(256), xargs, 0, s);
+        rc = launch_pdl(band_fixup_kernel(p.kind, p.has_m), dim3(kFixupBlocks), dim3(256), xargs, 0, s);
     }
     int nspl = (int)p.nsplit;
-    void *eargs[] = {&mode, &nspl, &nt, &p.part, &tgt7, &t, &p.zeta_inv, &out};
-    if (!rc) rc = launch(epilogue_kernel(), dim3(nblk_t), dim3(256), eargs, 0, s);
+    if (!rc) rc = launch_epilogue(mode, p.nacc, nspl, nt, p.part, tgt7, t, p.zeta_inv, out, s);
     if (!rc && a.extent_host) PO_CK_RC(cudaMemcpyAsync(a.extent_host, &p.frame->m, sizeof(double),
                                                        cudaMemcpyDeviceToHost, s));
     if (!rc && a.band_host && p.band.count)
@@ -680,22 +718,19 @@ int run_adjoint(const AdjArgs &a)
     }
 
     // ---- mixed precision
-    double *bbox = nullptr;
     Frame *frame = nullptr;
     float4 *srcpk = nullptr;
-    if (!rc && ((rc = salloc(&bbox, (size_t)kBboxBlocks * 6, s, owned)) || (rc = salloc(&frame, 1, s, owned)) ||
+    if (!rc && ((rc = salloc(&frame, 1, s, owned)) ||
                 (!far && (rc = salloc(&srcpk, (size_t)ns * kRec, s, owned))))) {
         sfree(owned, s);
         return rc;
     }
     long nb = far ? 0 : nt;
-    void *bargs[] = {&src7, &ns, &tgt7, &nb, &bbox};
-    if (!rc) rc = launch(bbox_kernel(), dim3(kBboxBlocks), dim3(kBboxThreads), bargs, 0, s);
-    int nbb = kBboxBlocks;
     double kap = kappa;
     int centred = far ? 0 : 1;
-    void *frargs[] = {&bbox, &nbb, &kap, &centred, &frame};
-    if (!rc) rc = launch(frame_kernel(), dim3(1), dim3(32), frargs, 0, s);
+    unsigned *none = nullptr;
+    void *frargs[] = {&src7, &ns, &tgt7, &nb, &kap, &centred, &frame, &none};
+    if (!rc) rc = launch(frame_kernel(), dim3(kFrameCtas), dim3(kFrameThreads), frargs, 0, s);
     const int *ff_order = nullptr;   // far field: curve position -> source
     if (far) {
         // sources in Hilbert order, in the forward's tile records: one adjoint

@@ -74,6 +74,7 @@ __device__ __forceinline__ unsigned long long hilbert_index(uint32_t x, uint32_t
 __global__ void po_ff_key_kernel(long ns, const double *__restrict__ src7, const Frame *__restrict__ frp,
                                  unsigned long long *__restrict__ key, int *__restrict__ idx)
 {
+    pdl_wait();
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= ns) return;
     const Frame fr = *frp;
@@ -259,6 +260,7 @@ po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const floa
     __shared__ __align__(8) uint64_t full[kStages];
     __shared__ float tbox_w[kThreads / 32][6];
     __shared__ float tbox[6];
+    pdl_wait();
 
     const long tbase = (long)blockIdx.x * kThreads * TP + threadIdx.x;
     float2 rf[TP][3];          // direction in FP32, duplicated into both lanes
@@ -496,14 +498,15 @@ po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const floa
         return;
     }
 
+    pdl_trigger();
 #pragma unroll
     for (int j = 0; j < TP; ++j) {
         const long ti = tbase + (long)j * kThreads;
         if (ti >= nt) continue;
 #pragma unroll
-        for (int a = 0; a < kAcc; ++a)
-            part[((long)blockIdx.y * kAcc + a) * nt + ti] =
-                a < NA ? (double)hi[j][a] + (double)lo[(a * TP + j) * kThreads + threadIdx.x] : 0.0;
+        for (int a = 0; a < NA; ++a)
+            part[((long)blockIdx.y * NA + a) * nt + ti] =
+                (double)hi[j][a] + (double)lo[(a * TP + j) * kThreads + threadIdx.x];
     }
 }
 

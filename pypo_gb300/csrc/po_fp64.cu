@@ -243,7 +243,7 @@ po_fp64_kernel(const double *__restrict__ src, long ns, long chunk, const double
     const long ti = (long)blockIdx.x * blockDim.x + threadIdx.x;
     double p[3] = {0, 0, 0};
     if (ti < nt) {
-        if (KIND == kKindFF) ff_direction_d(tgt7, nt, ti, p);
+        if constexpr (KIND == kKindFF) ff_direction_d(tgt7, nt, ti, p);
         else
             for (int c = 0; c < 3; ++c) p[c] = tgt7[c * nt + ti];
     }
@@ -280,25 +280,28 @@ __global__ void po_pack_src_d_kernel(long ns, const double *__restrict__ src7, c
 // added into the first source chunk's partial sums (the epilogue adds the
 // chunks afterwards). The order of those additions varies between runs for
 // a target with several such pairs (last-bit differences there only).
-template <int KIND>
+template <int KIND, bool HAS_M>
 __global__ void __launch_bounds__(256)
 po_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, const double *__restrict__ cur,
                      int gmode, int ncx, int ncy, double fac_re, double fac_im, long nt,
                      const double *__restrict__ tgt7, Wave64 w, double *__restrict__ part, int *__restrict__ err)
 {
+    constexpr int REC = fp64_rec(KIND, HAS_M), NACC = KIND == kKindFF && !HAS_M ? 6 : kAcc;
+    pdl_trigger();
+    pdl_wait();
     const unsigned total = *bl.count;
     if (blockIdx.x == 0 && threadIdx.x == 0 && total > bl.cap) atomicExch(err, kErrBandOverflow);
     const unsigned n = min(total, bl.cap);
     for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int2 pr = bl.pairs[i];
-        double rec[kRecD], p[3], acc[kAcc];
-        src_record_d(pr.x, ns, src7, cur, gmode, ncx, ncy, fac_re, fac_im, 0, kRecD, rec);
-        if (KIND == kKindFF) ff_direction_d(tgt7, nt, pr.y, p);
+        double rec[REC], p[3], acc[kAcc];
+        src_record_d(pr.x, ns, src7, cur, gmode, ncx, ncy, fac_re, fac_im, 0, REC, rec);
+        if constexpr (KIND == kKindFF) ff_direction_d(tgt7, nt, pr.y, p);
         else
             for (int c = 0; c < 3; ++c) p[c] = tgt7[c * nt + pr.y];
         for (int a = 0; a < kAcc; ++a) acc[a] = 0.0;
-        fwd_pair64<KIND, true>(p, rec, w, acc);
-        for (int a = 0; a < kAcc; ++a)
+        fwd_pair64<KIND, HAS_M>(p, rec, w, acc);
+        for (int a = 0; a < NACC; ++a)
             if (acc[a] != 0.0) atomicAdd(&part[(long)a * nt + pr.y], acc[a]);
     }
 }
@@ -314,13 +317,13 @@ namespace {
 template <int KIND>
 __device__ __forceinline__ void adj_record64(long i, long nt, const double *tgt7, const double *gam, double *o)
 {
-    if (KIND == kKindFF) {
+    if constexpr (KIND == kKindFF) {
         ff_direction_d(tgt7, nt, i, o);
         o[3] = o[4] = o[5] = 0.0;
     } else {
         for (int c = 0; c < 6; ++c) o[c] = tgt7[c * nt + i];
     }
-    if (KIND == kKindScalar) {
+    if constexpr (KIND == kKindScalar) {
         o[6] = gam[i];
         o[7] = gam[3 * nt + i];
         return;
@@ -666,11 +669,14 @@ void *adj_pack_tgt_d_kernel(int kind)
                            : reinterpret_cast<void *>(&po_adj_pack_tgt_d_kernel<kKindFF>);
 }
 
-void *band_fixup_kernel(int kind)
+template <bool HAS_M>
+static void *band_fixup_sel(int kind)
 {
-    return kind == kKindFF ? reinterpret_cast<void *>(&po_band_fixup_kernel<kKindFF>)
-                           : reinterpret_cast<void *>(&po_band_fixup_kernel<kKindNF>);
+    return kind == kKindFF ? reinterpret_cast<void *>(&po_band_fixup_kernel<kKindFF, HAS_M>)
+                           : reinterpret_cast<void *>(&po_band_fixup_kernel<kKindNF, HAS_M>);
 }
+
+void *band_fixup_kernel(int kind, bool has_m) { return has_m ? band_fixup_sel<true>(kind) : band_fixup_sel<false>(kind); }
 
 void *adj_band_fixup_kernel(int kind, bool want_t)
 {

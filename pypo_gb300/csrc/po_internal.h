@@ -75,23 +75,23 @@ void scratch_free(void *p, cudaStream_t s);
 // has not been freed (0 before the pool exists).
 int scratch_used(unsigned long long *bytes);
 
-// Where one mixed-precision propagation takes its scratch. Every buffer is
-// taken before the first launch, so a source that runs out fails before any
-// device work. take() gives 256-byte aligned memory; room() is what is left.
+// Where one call takes its scratch. Every buffer is asked for with take() or
+// get() before the first launch, and commit() then gives each its memory
+// (256-byte aligned), so a source that runs out fails before any device
+// work. The pointers asked for must stay where they are until commit().
+// room() is what is left.
 class Scratch {
 public:
     virtual ~Scratch() = default;
     virtual int take(void **p, size_t bytes) = 0;
+    virtual int commit() = 0;
     virtual size_t room() const = 0;
     // entries of the list of near-tangent pairs a call of ns x nt pairs takes (BandList)
     virtual unsigned band_cap(long ns, long nt) const { return band_cap_for(ns, nt); }
     template <typename T>
     int get(T **p, size_t count)
     {
-        void *q = nullptr;
-        const int rc = take(&q, count * sizeof(T));
-        *p = static_cast<T *>(q);
-        return rc;
+        return take(reinterpret_cast<void **>(p), count * sizeof(T));
     }
 };
 
@@ -106,7 +106,7 @@ struct MixedPlan {
     bool far = false, has_m = false;
     double kappa = 0, fac_re = 0, fac_im = 0, zeta_inv = 0;
     long tiles = 0, ntb = 0, nsplit = 1, chunk = 0;
-    double *bbox = nullptr, *part = nullptr;
+    double *part = nullptr;
     Frame *frame = nullptr;
     float4 *srcpk = nullptr, *tgtpk = nullptr;
     unsigned long long *keys = nullptr;

@@ -4,7 +4,7 @@
 // (near field), :1656-1781 (far field) and :1279-1331 (scalar), written as an
 // N-body kernel:
 //
-//   * sources are packed once, two per record (po_pack_src2): positions in
+//   * sources are packed once, two per record (po_pack_kernel, po_prep.cu): positions in
 //     "turn" units (mm * k / 2 pi) relative to a frame origin, split into a
 //     hi part on a power-of-two quantum q (few significant bits, so that
 //     differences and squares of hi parts are exact in FP32) and a small lo
@@ -219,7 +219,7 @@ __device__ __forceinline__ void sc_pair2(float2 *acc, const float2 *tc, const fl
 
 // Whether every (source, target) pair of a tile passes the illumination
 // test, proven from the tile's box and the CTA's target box tb (lo xyz,
-// hi xyz, a bound on |t|_1). The tile's box (po_src_box_kernel: lowest and
+// hi xyz, a bound on |t|_1). The tile's box (po_pack_kernel: lowest and
 // highest normal xyz, largest n.s, largest |s|_1) travels with the tile in
 // the unused slot 21 of its first four pair records, so it arrives in
 // shared memory with the tile's copy: n.(t - s) >= min over the boxes of
@@ -247,8 +247,7 @@ __device__ __forceinline__ bool tile_lit(const float4 *tile, const float *tb)
 // chunks): blockIdx.y picks a chunk of sources (a multiple of kTile, so
 // chunks start on a pair boundary), whose tiles of kTile/2 pair records
 // stream through kStages TMA stages. The thread's target (hi xyz, lo xyz)
-// is duplicated into both lanes once. With `boxes` (po_src_box_kernel has
-// run on the records), a near-field tile proven lit for the CTA skips the
+// is duplicated into both lanes once. With `boxes` (the records carry them), a near-field tile proven lit for the CTA skips the
 // per-pair illumination test (M = 0 kernels). The far field has its own
 // kernel (po_farfield.cu).
 template <int KIND, int T, bool HAS_M, int TP>
@@ -262,6 +261,7 @@ po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *
     constexpr int NACC = KIND == kKindScalar ? 2 : kAcc;
     extern __shared__ __align__(128) float4 stage[];   // kStages * PT * REC, then the compensation words
     __shared__ __align__(8) uint64_t full[kStages];
+    pdl_wait();
 
     const long tbase = (long)blockIdx.x * kThreads * TP + threadIdx.x;
     float2 tc[TP][9];
@@ -428,6 +428,7 @@ po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *
         return;
     }
 
+    pdl_trigger();
 #pragma unroll
     for (int j = 0; j < TP; ++j) {
         const long ti = tbase + (long)j * kThreads;
@@ -457,77 +458,7 @@ __global__ void po_wait_selftest_kernel(uint32_t limit, int *__restrict__ err)
     if (__syncthreads_or(!ok) && threadIdx.x == 0) atomicExch(err, kErrWaitTimeout);
 }
 
-// ----------------------------------------------------------- frame & packing
-
-__global__ void po_bbox_kernel(const double *__restrict__ a, long na, const double *__restrict__ b, long nb,
-                               double *__restrict__ partial)
-{
-    __shared__ double sm[6][kBboxThreads];
-    double v[6] = {CUDART_INF, CUDART_INF, CUDART_INF, -CUDART_INF, -CUDART_INF, -CUDART_INF};
-    const long stride = (long)gridDim.x * blockDim.x;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < na + nb; i += stride) {
-        const double *p = i < na ? a : b;
-        const long n = i < na ? na : nb;
-        const long k = i < na ? i : i - na;
-        for (int c = 0; c < 3; ++c) {
-            const double x = p[c * n + k];
-            v[c] = fmin(v[c], x);
-            v[3 + c] = fmax(v[3 + c], x);
-        }
-    }
-    for (int c = 0; c < 6; ++c) sm[c][threadIdx.x] = v[c];
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int c = 0; c < 6; ++c)
-                sm[c][threadIdx.x] = c < 3 ? fmin(sm[c][threadIdx.x], sm[c][threadIdx.x + w])
-                                           : fmax(sm[c][threadIdx.x], sm[c][threadIdx.x + w]);
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int c = 0; c < 6; ++c) partial[blockIdx.x * 6 + c] = sm[c][0];
-}
-
-// One warp: reduce the block partials (lane l takes blocks l, l + 32, ...;
-// min and max are exact in any order) and fix origin, scale and quantum.
-// centred: origin at the bbox centre (near field, scalar); otherwise origin 0
-// (far field: the phase reference is the coordinate origin).
-__global__ void po_frame_kernel(const double *__restrict__ partial, int nblk, double kappa, int centred,
-                                Frame *__restrict__ fr)
-{
-    double lo[3] = {CUDART_INF, CUDART_INF, CUDART_INF}, hi[3] = {-CUDART_INF, -CUDART_INF, -CUDART_INF};
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x)
-        for (int c = 0; c < 3; ++c) {
-            lo[c] = fmin(lo[c], partial[b * 6 + c]);
-            hi[c] = fmax(hi[c], partial[b * 6 + 3 + c]);
-        }
-    for (int o = 16; o > 0; o >>= 1)
-        for (int c = 0; c < 3; ++c) {
-            lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-            hi[c] = fmax(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
-        }
-    if (threadIdx.x != 0) return;
-    double m = 0.0;
-    for (int c = 0; c < 3; ++c) {
-        double o = 0.0;
-        if (centred && lo[c] <= hi[c]) o = 0.5 * (lo[c] + hi[c]);
-        fr->o[c] = o;
-        if (lo[c] <= hi[c]) m = fmax(m, fmax(fabs(hi[c] - o), fabs(lo[c] - o)));
-    }
-    m *= kappa;
-    // Smallest power of two q with 2 m / q <= 2048, so |hi/q| <= 1024.5.
-    double need = 2.0 * m / 2048.0;
-    double q = 0x1p-40;
-    while (q < need) q *= 2.0;
-    fr->kappa = kappa;
-    fr->q = q;
-    fr->inv_q = 1.0 / q;
-    fr->m = m;
-    for (int c = 0; c < 3; ++c) {
-        fr->lo[c] = lo[c];
-        fr->hi[c] = hi[c];
-    }
-}
+// ------------------------------------------------------- packing (adjoint)
 
 // One-source records for the adjoint kernels (a thread owns one source),
 // 6 float4 (kRec):
@@ -576,112 +507,6 @@ __global__ void po_pack_src_kernel(long ns, const double *__restrict__ src7, con
     o[5] = make_float4((float)src7[5 * ns + i], 0.f, 0.f, 0.f);
 }
 
-// Pair-packed source records (layouts above ff_pair2 / sc_pair2; rec4 float4
-// per pair: kRec2, or kRec2Scalar for the scalar kind). One thread per lane;
-// an odd source count pads the last pair with a copy of the last source
-// carrying zero currents.
-__global__ void po_pack_src2_kernel(long ns, const double *__restrict__ src7, const double *__restrict__ cur,
-                                    int gmode, int ncx, int ncy, const Frame *__restrict__ frp, double fac_re,
-                                    double fac_im, int scalar, float *__restrict__ out)
-{
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long np = (ns + 1) / 2;
-    if (i >= 2 * np) return;
-    const long k = i < ns ? i : ns - 1;
-    const Frame fr = *frp;
-    float v[2 * kRec2];
-    for (int c = 0; c < 3; ++c) split_hi_lo((src7[c * ns + k] - fr.o[c]) * fr.kappa, fr, v[c], v[3 + c]);
-    const double w = i < ns ? trap_weight(k, gmode, ncx, ncy) * src7[6 * ns + k] : 0.0;
-    const double fr_ = fac_re * w, fi_ = fac_im * w;
-    const int rec4 = scalar ? kRec2Scalar : kRec2;
-    if (scalar) {
-        const double re = cur[k], im = cur[ns + k];
-        v[6] = (float)(fr_ * re - fi_ * im);
-        v[7] = (float)(fr_ * im + fi_ * re);
-    } else {
-        for (int c = 0; c < 3; ++c) v[6 + c] = (float)src7[(3 + c) * ns + k];
-        for (int q = 0; q < 6; ++q) {
-            const int grp = q / 3, ax = q % 3;
-            const double re = cur[(grp * 6 + ax) * ns + k];
-            const double im = cur[(grp * 6 + 3 + ax) * ns + k];
-            v[9 + 2 * q] = (float)(fr_ * re - fi_ * im);
-            v[10 + 2 * q] = (float)(fr_ * im + fi_ * re);
-        }
-        v[21] = 0.f;
-    }
-    float *o = out + (i >> 1) * (rec4 * 4) + (i & 1);
-    for (int q = 0; q < 2 * rec4; ++q) o[2 * q] = v[q];
-}
-
-// Box of each source tile (kTile sources = kTile / 2 pair records) for the
-// lit-tile proof of po_pk_kernel: lowest normal xyz, highest normal xyz,
-// largest n.s and largest |s|_1 (s = hi + lo, turns), kBoxF floats written
-// into the unused slot 21 of the tile's first four pair records. One warp
-// per tile; the padding source of an odd count repeats the last source, so
-// it changes nothing.
-__global__ void po_src_box_kernel(float2 *__restrict__ rec, long ns)
-{
-    constexpr int PT = kTile / 2;
-    constexpr int R2 = 2 * kRec2;   // float2 slots per pair record
-    float v[kBoxF] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F,
-                      -CUDART_INF_F, 0.0f};
-    const long np = (ns + 1) / 2;
-    for (int p = threadIdx.x; p < PT; p += 32) {
-        const long pair = (long)blockIdx.x * PT + p;
-        if (pair >= np) break;
-        const float2 *r = rec + pair * R2;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            float sv[3], nv[3];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                sv[c] = (h ? r[c].y : r[c].x) + (h ? r[3 + c].y : r[3 + c].x);
-                nv[c] = h ? r[6 + c].y : r[6 + c].x;
-                v[c] = fminf(v[c], nv[c]);
-                v[3 + c] = fmaxf(v[3 + c], nv[c]);
-            }
-            v[6] = fmaxf(v[6], fmaf(nv[2], sv[2], fmaf(nv[1], sv[1], nv[0] * sv[0])));
-            v[7] = fmaxf(v[7], fabsf(sv[0]) + fabsf(sv[1]) + fabsf(sv[2]));
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int q = 0; q < kBoxF; ++q) {
-            const float u = __shfl_xor_sync(0xffffffffu, v[q], o);
-            v[q] = q < 3 ? fminf(v[q], u) : fmaxf(v[q], u);
-        }
-    if (threadIdx.x < kBoxF) {
-        const long pair = (long)blockIdx.x * PT + (threadIdx.x >> 1);
-        float *slot = reinterpret_cast<float *>(rec + pair * R2 + 21);
-        if (pair < np) slot[threadIdx.x & 1] = v[threadIdx.x];
-    }
-}
-
-// Near-field / scalar targets: hi/lo split positions in the same frame.
-// Far-field targets: direction r_hat from (polar, azimuth), hi part on 2^-11.
-__global__ void po_pack_tgt_kernel(long nt, const double *__restrict__ tgt7, const Frame *__restrict__ frp,
-                                   int far, float4 *__restrict__ out)
-{
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nt) return;
-    float h[3], l[3];
-    if (far) {
-        const double th = tgt7[i], ph = tgt7[nt + i];
-        const double r[3] = {cos(ph) * sin(th), sin(ph) * sin(th), cos(th)};
-        for (int c = 0; c < 3; ++c) {
-            const double hd = rint(r[c] * 2048.0) / 2048.0;
-            h[c] = (float)hd;
-            l[c] = (float)(r[c] - hd);
-        }
-    } else {
-        const Frame fr = *frp;
-        for (int c = 0; c < 3; ++c) split_hi_lo((tgt7[c * nt + i] - fr.o[c]) * fr.kappa, fr, h[c], l[c]);
-    }
-    out[2 * i] = make_float4(h[0], h[1], h[2], l[0]);
-    out[2 * i + 1] = make_float4(l[1], l[2], 0.f, 0.f);
-}
-
 // ------------------------------------------------------------------ epilogue
 
 __device__ __forceinline__ void cross_d(const double a[3], const double b[3], double o[3])
@@ -691,28 +516,57 @@ __device__ __forceinline__ void cross_d(const double a[3], const double b[3], do
     o[2] = a[0] * b[1] - a[1] * b[0];
 }
 
-// Sums the source chunks in order and writes the mode's outputs (FP64).
-// Output rows follow the reference's bundle order.
-__global__ void po_epilogue_kernel(int mode, int nsplit, long nt, const double *__restrict__ part,
-                                   const double *__restrict__ tgt7, double t, double zeta_inv,
-                                   double *__restrict__ out)
+// Sums the source chunks in a fixed order and writes the mode's outputs
+// (FP64). Output rows follow the reference's bundle order. nacc: rows per
+// chunk (2 scalar; 6 where the far field has no M; else 12). G threads share
+// a target: thread g adds chunks g, g + G, ..., then the G sums are added in
+// a tree, so that many chunks of few targets are not one thread's chain of
+// loads and one SM's FP64 additions.
+template <int G>
+__global__ void __launch_bounds__(kEpiThreads)
+po_epilogue_kernel(int mode, int nacc, int nsplit, long nt, const double *__restrict__ part,
+                   const double *__restrict__ tgt7, double t, double zeta_inv, double *__restrict__ out)
 {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int TB = kEpiThreads / G;   // targets per block
+    __shared__ double sh[G > 1 ? G / 2 : 1][G > 1 ? kAcc : 1][G > 1 ? TB : 1];
+    pdl_wait();
+    const int tl = threadIdx.x % TB, g = threadIdx.x / TB;
+    const long i = (long)blockIdx.x * TB + tl;
+    double a[kAcc];
+#pragma unroll
+    for (int q = 0; q < kAcc; ++q) a[q] = 0.0;
+    auto sum = [&](auto n_c) {
+        constexpr int N = decltype(n_c)::value;
+#pragma unroll 4
+        for (int s = g; s < nsplit; s += G)
+#pragma unroll
+            for (int q = 0; q < N; ++q) a[q] += part[((long)s * N + q) * nt + i];
+    };
+    if (i < nt) {
+        if (nacc == 2) sum(std::integral_constant<int, 2>{});
+        else if (nacc == 6) sum(std::integral_constant<int, 6>{});
+        else sum(std::integral_constant<int, kAcc>{});
+    }
+    if constexpr (G > 1) {
+#pragma unroll
+        for (int w = G / 2; w > 0; w >>= 1) {
+            if (g >= w && g < 2 * w)
+#pragma unroll
+                for (int q = 0; q < kAcc; ++q) sh[g - w][q][tl] = a[q];
+            __syncthreads();
+            if (g < w)
+#pragma unroll
+                for (int q = 0; q < kAcc; ++q) a[q] += sh[g][q][tl];
+            __syncthreads();
+        }
+        if (g > 0) return;
+    }
     if (i >= nt) return;
     if (mode == kScalar) {
-        double re = 0, im = 0;
-        for (int s = 0; s < nsplit; ++s) {
-            re += part[((long)s * 2 + 0) * nt + i];
-            im += part[((long)s * 2 + 1) * nt + i];
-        }
-        out[i] = re;
-        out[nt + i] = im;
+        out[i] = a[0];
+        out[nt + i] = a[1];
         return;
     }
-    double a[kAcc];
-    for (int q = 0; q < kAcc; ++q) a[q] = 0.0;
-    for (int s = 0; s < nsplit; ++s)
-        for (int q = 0; q < kAcc; ++q) a[q] += part[((long)s * kAcc + q) * nt + i];
     // a: E.re[3] E.im[3] H.re[3] H.im[3]
     double er[3] = {a[0], a[1], a[2]}, ei[3] = {a[3], a[4], a[5]};
     double hr[3] = {a[6], a[7], a[8]}, hi[3] = {a[9], a[10], a[11]};
@@ -810,12 +664,7 @@ void *pk_kernel(int kind, int t_sign, bool has_m)
     return t_sign < 0 ? pk_ptr<kKindScalar, -1, false>() : pk_ptr<kKindScalar, 1, false>();
 }
 
-void *pack_src2_kernel() { return reinterpret_cast<void *>(&po_pack_src2_kernel); }
-void *src_box_kernel() { return reinterpret_cast<void *>(&po_src_box_kernel); }
-void *bbox_kernel() { return reinterpret_cast<void *>(&po_bbox_kernel); }
-void *frame_kernel() { return reinterpret_cast<void *>(&po_frame_kernel); }
 void *pack_src_kernel() { return reinterpret_cast<void *>(&po_pack_src_kernel); }
-void *pack_tgt_kernel() { return reinterpret_cast<void *>(&po_pack_tgt_kernel); }
 // Precision conversions of the float drop-in ABI's buffers (n elements).
 __global__ void po_f2d_kernel(const float *__restrict__ in, double *__restrict__ out, long n)
 {
@@ -829,7 +678,13 @@ __global__ void po_d2f_kernel(const double *__restrict__ in, float *__restrict__
         out[i] = (float)in[i];
 }
 
-void *epilogue_kernel() { return reinterpret_cast<void *>(&po_epilogue_kernel); }
+void *epilogue_kernel(int groups)
+{
+    if (groups == 64) return reinterpret_cast<void *>(&po_epilogue_kernel<64>);
+    if (groups == 32) return reinterpret_cast<void *>(&po_epilogue_kernel<32>);
+    return groups == 8 ? reinterpret_cast<void *>(&po_epilogue_kernel<8>)
+                       : reinterpret_cast<void *>(&po_epilogue_kernel<1>);
+}
 void *f2d_kernel() { return reinterpret_cast<void *>(&po_f2d_kernel); }
 void *d2f_kernel() { return reinterpret_cast<void *>(&po_d2f_kernel); }
 void *fp32_probe_kernel() { return reinterpret_cast<void *>(&po_fp32_probe_kernel); }

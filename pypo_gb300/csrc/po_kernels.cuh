@@ -109,8 +109,10 @@ struct Wave64 {
 };
 Wave64 wave64(double k, double t);
 
-constexpr int kBboxThreads = 256;
-constexpr int kBboxBlocks = 152;
+// The frame kernel: one thread-block cluster (16 is the most a cluster may
+// have, past the portable 8).
+constexpr int kFrameThreads = 512;
+constexpr int kFrameCtas = 16;
 
 // Illumination test of the mixed-precision kernels: a pair with
 // n . R_hat >= kTangentBand is lit, one below -kTangentBand is not (the FP32
@@ -188,19 +190,17 @@ inline int pk_smem_bytes(int kind)
 }
 
 void *pk_kernel(int kind, int t_sign, bool has_m);
-void *pack_src2_kernel();
-void *src_box_kernel();
+void *pack_kernel(bool scalar, bool has_m);   // source tiles (near field, scalar) and targets
 void *fp64_kernel(int kind, bool has_m);
-void *bbox_kernel();
 void *frame_kernel();
 void *pack_src_kernel();
-void *pack_tgt_kernel();
 void *pack_src_d_kernel();
-void *epilogue_kernel();
+constexpr int kEpiThreads = 256;
+void *epilogue_kernel(int groups);   // 1, 8, 32 or 64 threads share a target's chunks
 void *f2d_kernel();   // float -> double, grid-stride over n
 void *d2f_kernel();   // double -> float
 void *fp32_probe_kernel();
-void *band_fixup_kernel(int kind);
+void *band_fixup_kernel(int kind, bool has_m);
 void *adj_band_fixup_kernel(int kind, bool want_t);
 void *wait_selftest_kernel();
 void *adj_fp64_kernel(int kind, bool has_m, bool want_d, bool want_t);

@@ -87,6 +87,7 @@ public:
         used_ += need;
         return 0;
     }
+    int commit() override { return 0; }   // take() has given the memory already
     size_t room() const override { return kStaticScratchBytes - kOffScratch - used_; }
     unsigned band_cap(long, long) const override { return po::kBandCapStatic; }
 

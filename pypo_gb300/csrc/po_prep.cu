@@ -1,0 +1,263 @@
+// po_prep.cu -- set-up kernels of the mixed-precision paths: the frame of the
+// split representation, and the packed records of sources and targets.
+//
+// A small propagation is bound by its launches (2.1 us each on the device,
+// and as much per stream-ordered allocation), so the set-up is two kernels:
+// the frame in one thread-block cluster (no partial buffer, no second
+// launch), and one pack kernel for the source records, their tile boxes and
+// the targets. Each later kernel of a call is launched with programmatic
+// stream serialisation and begins with pdl_wait().
+#include <cuda_runtime.h>
+#include <math_constants.h>
+
+#include <cstdint>
+
+#include "po_device.cuh"
+#include "po_kernels.cuh"
+
+namespace po {
+
+namespace {
+
+__device__ __forceinline__ uint32_t cluster_rank()
+{
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// Store into the shared memory of cluster rank `rank` at this CTA's address p.
+__device__ __forceinline__ void st_cluster(long long *p, uint32_t rank, long long v)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+    asm volatile("st.shared::cluster.s64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+}
+
+// Doubles as integers of the same order, and back (its own inverse): the
+// comparisons of a box run on the integer pipe, the FP64 pipe being 32 times
+// slower (161,227 points on 8 SMs: about 30 us of FP64 comparisons).
+__device__ __forceinline__ long long order_key(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffll); }
+constexpr long long kKeyInf = 0x7ff0000000000000ll;   // order_key of +infinity; of -infinity: ~kKeyInf
+
+// Smallest power of two q >= need, at least 2^-40 (need NaN: 2^-40; need
+// infinite or past the largest power of two: infinity).
+__device__ __forceinline__ double quantum(double need)
+{
+    const double least = 0x1p-40;
+    if (!(need > least)) return least;
+    const long long bits = __double_as_longlong(need);
+    const long long e = bits >> 52;   // need > 2^-40: positive and normal
+    return __longlong_as_double(((bits & 0xfffffffffffffll) ? e + 1 : e) << 52);
+}
+
+}  // namespace
+
+// Box of the points of a (na) and b (nb; rows x, y, z first), and from it the
+// frame: origin, scale and quantum. One cluster of kFrameCtas CTAs: minima and
+// maxima are exact in any order, so the split does not show in the result
+// (NaN coordinates are left out). centred: origin at the box centre (near
+// field, scalar); otherwise origin 0 (far field: the phase reference is the
+// coordinate origin). zero: a word cleared for the call's later kernels (the
+// band list's count), or null.
+__global__ void __launch_bounds__(kFrameThreads) __cluster_dims__(kFrameCtas, 1, 1)
+po_frame_kernel(const double *__restrict__ a, long na, const double *__restrict__ b, long nb, double kappa,
+                int centred, Frame *__restrict__ fr, unsigned *__restrict__ zero)
+{
+    __shared__ long long box[6][kFrameCtas];   // rank 0's copy gathers the cluster's
+    __shared__ long long wbox[6][kFrameThreads / 32];
+    pdl_trigger();
+    cluster_arrive();   // completed below: every CTA has started before one writes into rank 0's memory
+    const uint32_t rank = cluster_rank();
+    if (rank == 0 && threadIdx.x == 0 && zero) *zero = 0u;
+    long long v[6] = {kKeyInf, kKeyInf, kKeyInf, ~kKeyInf, ~kKeyInf, ~kKeyInf};
+    auto scan = [&](const double *__restrict__ p, long n) {
+#pragma unroll 4
+        for (long i = (long)rank * kFrameThreads + threadIdx.x; i < n; i += (long)kFrameCtas * kFrameThreads)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const long long x = __double_as_longlong(p[c * n + i]), y = order_key(x);
+                const bool nan = (x & 0x7fffffffffffffffll) > kKeyInf;
+                v[c] = nan ? v[c] : min(v[c], y);
+                v[3 + c] = nan ? v[3 + c] : max(v[3 + c], y);
+            }
+    };
+    scan(a, na);
+    scan(b, nb);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const long long u = __shfl_xor_sync(0xffffffffu, v[q], o);
+            v[q] = q < 3 ? min(v[q], u) : max(v[q], u);
+        }
+        if ((threadIdx.x & 31) == 0) wbox[q][threadIdx.x >> 5] = v[q];
+    }
+    __syncthreads();
+    cluster_wait();
+    if (threadIdx.x < 6) {
+        const int q = threadIdx.x;
+        long long r = wbox[q][0];
+        for (int w = 1; w < kFrameThreads / 32; ++w) r = q < 3 ? min(r, wbox[q][w]) : max(r, wbox[q][w]);
+        st_cluster(&box[q][rank], 0, r);
+    }
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (rank != 0 || threadIdx.x != 0) return;
+    double lo[3], hi[3], m = 0.0;
+    for (int c = 0; c < 3; ++c) {
+        long long l = box[c][0], h = box[3 + c][0];
+        for (int r = 1; r < kFrameCtas; ++r) {
+            l = min(l, box[c][r]);
+            h = max(h, box[3 + c][r]);
+        }
+        lo[c] = __longlong_as_double(order_key(l));
+        hi[c] = __longlong_as_double(order_key(h));
+        double o = 0.0;
+        if (centred && lo[c] <= hi[c]) o = 0.5 * (lo[c] + hi[c]);
+        fr->o[c] = o;
+        if (lo[c] <= hi[c]) m = fmax(m, fmax(fabs(hi[c] - o), fabs(lo[c] - o)));
+    }
+    m *= kappa;
+    // 2 m / q <= 2048, so |hi/q| <= 1024.5
+    const double q = quantum(2.0 * m / 2048.0);
+    fr->kappa = kappa;
+    fr->q = q;
+    fr->inv_q = 1.0 / q;
+    fr->m = m;
+    for (int c = 0; c < 3; ++c) {
+        fr->lo[c] = lo[c];
+        fr->hi[c] = hi[c];
+    }
+}
+
+// Packed target i. Near field / scalar: hi/lo split position in the frame.
+// Far field: direction r_hat from (polar, azimuth), hi part on 2^-11.
+__device__ __forceinline__ void pack_target(long i, long nt, const double *tgt7, const Frame &fr, int far, float4 *out)
+{
+    float h[3], l[3];
+    if (far) {
+        const double th = tgt7[i], ph = tgt7[nt + i];
+        const double r[3] = {cos(ph) * sin(th), sin(ph) * sin(th), cos(th)};
+        for (int c = 0; c < 3; ++c) {
+            const double hd = rint(r[c] * 2048.0) / 2048.0;
+            h[c] = (float)hd;
+            l[c] = (float)(r[c] - hd);
+        }
+    } else {
+        for (int c = 0; c < 3; ++c) split_hi_lo((tgt7[c * nt + i] - fr.o[c]) * fr.kappa, fr, h[c], l[c]);
+    }
+    out[2 * i] = make_float4(h[0], h[1], h[2], l[0]);
+    out[2 * i + 1] = make_float4(l[1], l[2], 0.f, 0.f);
+}
+
+// Blocks 0 .. tiles-1: one tile of kTile sources each, as pair-packed records
+// (layouts in po_kernels.cu; SCALAR: kRec2Scalar float4 per pair, else kRec2),
+// assembled in shared memory and written out in coalesced float4. An odd
+// source count pads the last pair with a copy of the last source carrying
+// zero currents. Near field, M = 0 (near field, M = 0) the tile's box for the
+// lit-tile proof goes into the unused slot 21 of its first four pair
+// records: lowest normal xyz, highest normal xyz, largest n.s, largest |s|_1
+// (s = hi + lo, turns); the padding source changes nothing there.
+// The remaining blocks: kTile targets each. far: no source tiles here (the
+// far field packs them in curve order), and the targets are directions.
+template <bool SCALAR, bool HAS_M>
+__global__ void __launch_bounds__(kTile)
+po_pack_kernel(long ns, const double *__restrict__ src7, const double *__restrict__ cur, int gmode, int ncx, int ncy,
+               const Frame *__restrict__ frp, double fac_re, double fac_im, long tiles,
+               float4 *__restrict__ src, long nt, const double *__restrict__ tgt7, int far, float4 *__restrict__ tgt)
+{
+    constexpr int R4 = SCALAR ? kRec2Scalar : kRec2;
+    __shared__ __align__(16) float4 buf[kTile / 2 * R4];
+    __shared__ float wbox[kTile / 32][kBoxF];
+    pdl_wait();
+    const Frame fr = *frp;
+    if ((long)blockIdx.x >= tiles) {
+        const long i = ((long)blockIdx.x - tiles) * kTile + threadIdx.x;
+        if (i < nt) pack_target(i, nt, tgt7, fr, far, tgt);
+        pdl_trigger();
+        return;
+    }
+    const long first = (long)blockIdx.x * kTile, i = first + threadIdx.x;
+    const int np = (int)(min((long)kTile, ns - first) + 1) / 2;   // pairs of this tile
+    float v[2 * R4];
+    if ((int)threadIdx.x < 2 * np) {
+        const long k = i < ns ? i : ns - 1;
+        for (int c = 0; c < 3; ++c) split_hi_lo((src7[c * ns + k] - fr.o[c]) * fr.kappa, fr, v[c], v[3 + c]);
+        const double w = i < ns ? trap_weight(k, gmode, ncx, ncy) * src7[6 * ns + k] : 0.0;
+        const double fr_ = fac_re * w, fi_ = fac_im * w;
+        if (SCALAR) {
+            const double re = cur[k], im = cur[ns + k];
+            v[6] = (float)(fr_ * re - fi_ * im);
+            v[7] = (float)(fr_ * im + fi_ * re);
+        } else {
+            for (int c = 0; c < 3; ++c) v[6 + c] = (float)src7[(3 + c) * ns + k];
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                if (!HAS_M && q >= 3) {   // the M = 0 kernels do not read M'
+                    v[9 + 2 * q] = v[10 + 2 * q] = 0.f;
+                    continue;
+                }
+                const int grp = q / 3, ax = q % 3;
+                const double re = cur[(grp * 6 + ax) * ns + k];
+                const double im = cur[(grp * 6 + 3 + ax) * ns + k];
+                v[9 + 2 * q] = (float)(fr_ * re - fi_ * im);
+                v[10 + 2 * q] = (float)(fr_ * im + fi_ * re);
+            }
+            v[2 * R4 - 1] = 0.f;
+        }
+        float *o = reinterpret_cast<float *>(buf) + (threadIdx.x >> 1) * (R4 * 4) + (threadIdx.x & 1);
+#pragma unroll
+        for (int q = 0; q < 2 * R4; ++q) o[2 * q] = v[q];
+    }
+    if (!SCALAR && !HAS_M) {
+        float x[kBoxF] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F,
+                          -CUDART_INF_F, 0.0f};
+        if ((int)threadIdx.x < 2 * np) {
+            float s[3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                s[c] = v[c] + v[3 + c];
+                x[c] = x[3 + c] = v[6 + c];
+            }
+            x[6] = fmaf(v[8], s[2], fmaf(v[7], s[1], v[6] * s[0]));
+            x[7] = fabsf(s[0]) + fabsf(s[1]) + fabsf(s[2]);
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < kBoxF; ++q) {
+                const float u = __shfl_xor_sync(0xffffffffu, x[q], o);
+                x[q] = q < 3 ? fminf(x[q], u) : fmaxf(x[q], u);
+            }
+        if ((threadIdx.x & 31) == 0)
+#pragma unroll
+            for (int q = 0; q < kBoxF; ++q) wbox[threadIdx.x >> 5][q] = x[q];
+        __syncthreads();
+        if (threadIdx.x < kBoxF) {
+            const int q = threadIdx.x;
+            float r = wbox[0][q];
+            for (int w = 1; w < kTile / 32; ++w) r = q < 3 ? fminf(r, wbox[w][q]) : fmaxf(r, wbox[w][q]);
+            if (q / 2 < np) reinterpret_cast<float *>(buf)[(q / 2) * (R4 * 4) + 42 + (q & 1)] = r;
+        }
+    }
+    __syncthreads();
+    float4 *dst = src + (size_t)blockIdx.x * (kTile / 2) * R4;
+    for (int q = threadIdx.x; q < np * R4; q += kTile) dst[q] = buf[q];
+    pdl_trigger();
+}
+
+void *frame_kernel() { return reinterpret_cast<void *>(&po_frame_kernel); }
+
+void *pack_kernel(bool scalar, bool has_m)
+{
+    if (scalar) return reinterpret_cast<void *>(&po_pack_kernel<true, false>);
+    return has_m ? reinterpret_cast<void *>(&po_pack_kernel<false, true>)
+                 : reinterpret_cast<void *>(&po_pack_kernel<false, false>);
+}
+
+}  // namespace po
