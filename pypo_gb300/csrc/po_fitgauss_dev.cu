@@ -22,17 +22,25 @@
 //
 // The grid is the surface's own (generateGrid without transform; x, y rows
 // of the 7-row device layout). Every pass over the points is one kernel with
-// FP64 per-thread sums, a block tree, and the block partials added in block
-// order by whichever block finishes last (a fixed grid, so each sum is
-// deterministic). The host does the window's run lengths, the moment
+// FP64 per-thread sums, a block tree, and the block partials added by
+// whichever block finishes last (a fixed grid and a fixed order, so each sum
+// is deterministic). The host does the window's run lengths, the moment
 // algebra and the simplex (po_nm.h, the code of po_fmin): its few hundred
 // dependent FP64 operations per step run far faster on the host than on one
 // GPU thread (GB300's FP64 units are few, and a lone thread waits out each
 // latency). The fit region's points are compacted once per minimisation;
 // each launch then evaluates every point the current simplex step may ask
-// for (reflection with its expansion and both contractions; all of a
-// shrink's vertices; the whole initial simplex), so a step costs one round
-// trip. A point's sums do not depend on the batch it is in.
+// for (a point's sums do not depend on what else is in its launch).
+//
+// A fit is a chain of a few hundred such launches, each waited for, so a
+// launch's round trip is what counts. The last block writes the sums straight
+// into a page-locked block of the host and then a sequence number, for which
+// the host watches: an empty kernel's round trip is 7.6 us that way, 12.6 with
+// a copy and a stream synchronise (14.5 into pageable memory). The region's
+// points are spread over the SMs, one warp per 32 points and Gaussian: with
+// 256 consecutive points to a block a region of 1500 sat on six SMs and their
+// FP64 pipes (2 a clock). Measured, a 201 x 201 beam's figures (two fits, LIN):
+// 13.3 -> 5.3 ms, 15 us a simplex step.
 //
 // Kept from the reference on purpose, with their effects:
 //   * the window's corners are read as x[min(cols), i0], x[max(cols), i0],
@@ -51,7 +59,9 @@
 #include <cuda_runtime.h>
 #include <math_constants.h>
 
+#include <algorithm>
 #include <cmath>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -98,9 +108,53 @@ __device__ __forceinline__ double gauss_at(const Gauss &g, int scale, double x, 
     return scale == kScaleDb ? __dmul_rn(20.0, log10(e)) : e;
 }
 
-// The last block to finish adds the block partials (in block order) into res.
+// Where a kernel's results go on the host: `data` in page-locked memory, then
+// `seq` into *flag once they are there. flag null: nowhere (the host copies
+// the device words).
+struct Mail {
+    double *data;
+    unsigned *flag;
+    unsigned seq;
+};
+
+// The calling thread's v as word q, for the threads that have one, then the
+// sequence number. Called by every thread of one block.
+__device__ void post(const Mail &mail, bool mine, int q, double v)
+{
+    if (!mail.flag) return;
+    if (mine) {
+        mail.data[q] = v;
+        __threadfence_system();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence_system();
+        *reinterpret_cast<volatile unsigned *>(mail.flag) = mail.seq;
+    }
+}
+
+// The nrow rows of nq partials (stride words apart) added in row order, word
+// q in thread q: the rows are fetched by all threads (buf: kFgThreads words)
+// and only the additions are serial.
+__device__ double add_rows(const double *part, int nrow, int stride, int nq, double *buf)
+{
+    const int per = kFgThreads / nq;   // rows a fetch
+    double v = 0.0;
+    for (int b = 0; b < nrow; b += per) {
+        const int rows = min(per, nrow - b);
+        const int r = threadIdx.x / nq, q = threadIdx.x - r * nq;
+        __syncthreads();
+        if (r < rows) buf[threadIdx.x] = __ldcg(&part[(long)(b + r) * stride + q]);
+        __syncthreads();
+        if ((int)threadIdx.x < nq)
+            for (int k = 0; k < rows; ++k) v += buf[k * nq + threadIdx.x];
+    }
+    return v;
+}
+
+// The last block to finish adds the block partials into res and posts them.
 template <int NS>
-__device__ void finish_sums(const double (&s)[NS], double *part, double *res, unsigned *count)
+__device__ void finish_sums(const double (&s)[NS], double *part, double *res, unsigned *count, const Mail &mail)
 {
     __shared__ double sh[NS][kFgThreads];
     __shared__ bool last;
@@ -118,12 +172,11 @@ __device__ void finish_sums(const double (&s)[NS], double *part, double *res, un
     }
     __syncthreads();
     if (!last) return;
-    if (threadIdx.x < NS) {
-        double v = 0.0;
-        for (unsigned b = 0; b < gridDim.x; ++b) v += __ldcg(&part[(long)b * NS + threadIdx.x]);
-        res[threadIdx.x] = v;
-    }
+    __threadfence();
+    const double v = add_rows(part, gridDim.x, NS, NS, sh[0]);
+    if (threadIdx.x < NS) res[threadIdx.x] = v;
     if (threadIdx.x == 0) *count = 0u;
+    post(mail, threadIdx.x < NS, threadIdx.x, v);
 }
 
 // (value, index) maximum, first index on ties, NaN above every number (as
@@ -136,14 +189,9 @@ __device__ __forceinline__ bool beats(double v, long i, double w, long j)
     return i < j;
 }
 
-__device__ void finish_argmax(double v, long i, double sum, double *part, double *res, unsigned *count)
+// Maximum with its index, and a sum, over the block's threads into slot 0.
+__device__ void argmax_tree(double *sv, long *si, double *ss)
 {
-    __shared__ double sv[kFgThreads], ss[kFgThreads];
-    __shared__ long si[kFgThreads];
-    __shared__ bool last;
-    sv[threadIdx.x] = v;
-    si[threadIdx.x] = i;
-    ss[threadIdx.x] = sum;
     __syncthreads();
     for (int w = kFgThreads / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) {
@@ -156,6 +204,20 @@ __device__ void finish_argmax(double v, long i, double sum, double *part, double
         }
         __syncthreads();
     }
+}
+
+// res[0..2] = maximum, its first index, sum; posted at mail.data[0..2].
+__device__ void finish_argmax(double v, long i, double sum, double *part, double *res, unsigned *count,
+                              const Mail &mail)
+{
+    static_assert(kFgBlocks <= kFgThreads, "one thread per block partial");
+    __shared__ double sv[kFgThreads], ss[kFgThreads];
+    __shared__ long si[kFgThreads];
+    __shared__ bool last;
+    sv[threadIdx.x] = v;
+    si[threadIdx.x] = i;
+    ss[threadIdx.x] = sum;
+    argmax_tree(sv, si, ss);
     if (threadIdx.x == 0) {
         part[3L * blockIdx.x] = sv[0];
         part[3L * blockIdx.x + 1] = (double)si[0];
@@ -164,22 +226,26 @@ __device__ void finish_argmax(double v, long i, double sum, double *part, double
         last = atomicAdd(count, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last || threadIdx.x != 0) return;
-    double bv = __ldcg(&part[0]), bs = 0.0;
-    long bi = (long)__ldcg(&part[1]);
-    for (unsigned b = 0; b < gridDim.x; ++b) {
-        const double w = __ldcg(&part[3L * b]);
-        const long j = (long)__ldcg(&part[3L * b + 1]);
-        if (beats(w, j, bv, bi)) {
-            bv = w;
-            bi = j;
-        }
-        bs += __ldcg(&part[3L * b + 2]);
+    if (!last) return;
+    __threadfence();
+    const unsigned b = threadIdx.x < gridDim.x ? threadIdx.x : 0u;   // a repeated block changes no maximum
+    sv[threadIdx.x] = __ldcg(&part[3L * b]);
+    si[threadIdx.x] = (long)__ldcg(&part[3L * b + 1]);
+    ss[threadIdx.x] = threadIdx.x < gridDim.x ? __ldcg(&part[3L * b + 2]) : 0.0;
+    const double sum_b = ss[threadIdx.x];
+    argmax_tree(sv, si, ss);
+    // the sum in block order
+    ss[threadIdx.x] = sum_b;
+    __syncthreads();
+    if (threadIdx.x == 2) {
+        double t = 0.0;
+        for (unsigned k = 0; k < gridDim.x; ++k) t += ss[k];
+        ss[0] = t;
     }
-    res[0] = bv;
-    res[1] = (double)bi;
-    res[2] = bs;
-    *count = 0u;
+    const double r = threadIdx.x == 0 ? sv[0] : (threadIdx.x == 1 ? (double)si[0] : ss[0]);
+    if (threadIdx.x < 3) res[threadIdx.x] = r;
+    if (threadIdx.x == 0) *count = 0u;
+    post(mail, threadIdx.x < 3, threadIdx.x, r);
 }
 
 // |E_c| into a; res[0] = max |E_c| (NaN if any is NaN).
@@ -197,16 +263,21 @@ fg_abs_kernel(long n, const double *__restrict__ fr, const double *__restrict__ 
             mi = i;
         }
     }
-    finish_argmax(m, mi, 0.0, part, res, count);
+    finish_argmax(m, mi, 0.0, part, res, count, Mail{});
 }
 
 // Normalised pattern: nf = a / amax, fit = nf (LIN) or 20 log10 nf (dB).
-// res[0] = max fit, res[1] = its first index, res[2] = sum nf^2.
+// res[0] = max fit, res[1] = its first index, res[2] = sum nf^2; posted with
+// amax as a fourth word.
 __global__ void __launch_bounds__(kFgThreads)
 fg_pattern_kernel(long n, const double *__restrict__ a, const double *__restrict__ amax, int scale,
-                  double *__restrict__ fit, double *part, double *res, unsigned *count)
+                  double *__restrict__ fit, double *part, double *res, unsigned *count, Mail mail)
 {
     const double m = *amax;
+    if (mail.flag && blockIdx.x == 0 && threadIdx.x == 0) {
+        mail.data[3] = m;
+        __threadfence_system();
+    }
     double best = -CUDART_INF;
     long bi = n;
     double s = 0.0;
@@ -220,24 +291,46 @@ fg_pattern_kernel(long n, const double *__restrict__ a, const double *__restrict
             bi = i;
         }
     }
-    finish_argmax(best, bi, s, part, res, count);
+    finish_argmax(best, bi, s, part, res, count, mail);
 }
 
 // Selection of the points the sums run over:
 //   mode 0: fit >= thr;
-//   mode 1: fit >= thr and xlo < x < xhi and ylo < y < yhi;
+//   mode 1: fit >= thr and xlo < x < xhi and ylo < y < yhi, the bounds read
+//     at the grid points w;
 //   mode 2: grid row 1 (i / ncy == 1).
-// res[0] = number of points selected.
+// Block b takes the b-th contiguous share of the points (block_share) and
+// writes how many it selected into bcount[b]; res[0] = their sum.
 struct Window {
-    double xlo, xhi, ylo, yhi;
+    long xlo, xhi, ylo, yhi;   // grid points whose x, x, y, y bound the window
 };
+
+__device__ __forceinline__ void block_share(long n, long &b, long &e)
+{
+    const long per = (n + gridDim.x - 1) / gridDim.x;
+    b = min(n, (long)blockIdx.x * per);
+    e = min(n, b + per);
+}
 
 __global__ void __launch_bounds__(kFgThreads)
 fg_select_kernel(long n, int ncy, const double *__restrict__ g7, const double *__restrict__ fit, double thr,
-                 int mode, Window w, unsigned char *__restrict__ sel, double *part, double *res, unsigned *count)
+                 int mode, Window w, unsigned char *__restrict__ sel, int *__restrict__ bcount, double *part,
+                 double *res, unsigned *count, Mail mail)
 {
-    double c[1] = {0.0};
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
+    __shared__ int on_block;
+    if (threadIdx.x == 0) on_block = 0;
+    __syncthreads();
+    double xlo = 0, xhi = 0, ylo = 0, yhi = 0;
+    if (mode == 1) {
+        xlo = g7[w.xlo];
+        xhi = g7[w.xhi];
+        ylo = g7[n + w.ylo];
+        yhi = g7[n + w.yhi];
+    }
+    long b, e;
+    block_share(n, b, e);
+    int c = 0;
+    for (long i = b + threadIdx.x; i < e; i += kFgThreads) {
         bool on;
         if (mode == 2) {
             on = i / ncy == 1;
@@ -245,13 +338,17 @@ fg_select_kernel(long n, int ncy, const double *__restrict__ g7, const double *_
             on = fit[i] >= thr;
             if (mode == 1) {
                 const double x = g7[i], y = g7[n + i];
-                on = on && x > w.xlo && x < w.xhi && y > w.ylo && y < w.yhi;
+                on = on && x > xlo && x < xhi && y > ylo && y < yhi;
             }
         }
         sel[i] = on ? 1 : 0;
-        c[0] += on ? 1.0 : 0.0;
+        c += on ? 1 : 0;
     }
-    finish_sums<1>(c, part, res, count);
+    atomicAdd(&on_block, c);
+    __syncthreads();
+    if (threadIdx.x == 0) bcount[blockIdx.x] = on_block;
+    double s[1] = {(double)c};
+    finish_sums<1>(s, part, res, count, mail);
 }
 
 // Mask values along the peak's row (ncy bytes) and column (ncx bytes).
@@ -266,7 +363,7 @@ __global__ void fg_lines_kernel(int ncx, int ncy, long i0, long j0, const double
 // Image moments of the selection: sum f, x f, y f, x^2 f, y^2 f, x y f.
 __global__ void __launch_bounds__(kFgThreads)
 fg_moments_kernel(long n, const double *__restrict__ g7, const double *__restrict__ fit,
-                  const unsigned char *__restrict__ sel, double *part, double *res, unsigned *count)
+                  const unsigned char *__restrict__ sel, double *part, double *res, unsigned *count, Mail mail)
 {
     double s[6] = {0, 0, 0, 0, 0, 0};
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
@@ -279,63 +376,72 @@ fg_moments_kernel(long n, const double *__restrict__ g7, const double *__restric
         s[4] += __dmul_rn(__dmul_rn(y, y), f);
         s[5] += __dmul_rn(__dmul_rn(x, y), f);
     }
-    finish_sums<6>(s, part, res, count);
+    finish_sums<6>(s, part, res, count, mail);
 }
 
 // Power of the linear Gaussian over every point: sum Psi^2.
 __global__ void __launch_bounds__(kFgThreads)
-fg_power_kernel(long n, const double *__restrict__ g7, Gauss g, double *part, double *res, unsigned *count)
+fg_power_kernel(long n, const double *__restrict__ g7, Gauss g, double *part, double *res, unsigned *count,
+                Mail mail)
 {
     double s[1] = {0.0};
     for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
         const double p = gauss_at(g, kScaleLin, g7[i], g7[n + i]);
         s[0] += __dmul_rn(p, p);
     }
-    finish_sums<1>(s, part, res, count);
+    finish_sums<1>(s, part, res, count, mail);
 }
 
 // Order-preserving compaction of the selected points into (x, y, pattern)
-// arrays; *count = how many. One CTA; thread t takes a contiguous chunk.
-constexpr int kCompactThreads = 1024;
-
-__global__ void __launch_bounds__(kCompactThreads)
-fg_compact_kernel(long n, const unsigned char *__restrict__ sel, const double *__restrict__ g7,
-                  const double *__restrict__ fit, double *__restrict__ cx, double *__restrict__ cy,
-                  double *__restrict__ cf, long *__restrict__ count)
+// arrays: each block places its share (fg_select_kernel's) behind the earlier
+// blocks' counts, 256 points at a time with a ballot scan.
+__global__ void __launch_bounds__(kFgThreads)
+fg_compact_kernel(long n, const unsigned char *__restrict__ sel, const int *__restrict__ bcount,
+                  const double *__restrict__ g7, const double *__restrict__ fit, double *__restrict__ cx,
+                  double *__restrict__ cy, double *__restrict__ cf)
 {
-    __shared__ long offs[kCompactThreads];
-    const long per = (n + kCompactThreads - 1) / kCompactThreads;
-    const long b = min(n, (long)threadIdx.x * per), e = min(n, b + per);
-    long c = 0;
-    for (long i = b; i < e; ++i) c += sel[i] ? 1 : 0;
-    offs[threadIdx.x] = c;
+    constexpr int kWarps = kFgThreads / 32;
+    __shared__ int wc[kWarps];
+    __shared__ long base;
+    if (threadIdx.x == 0) base = 0;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        long acc = 0;
-        for (int t = 0; t < kCompactThreads; ++t) {
-            const long v = offs[t];
-            offs[t] = acc;
-            acc += v;
+    if (threadIdx.x < blockIdx.x) atomicAdd(reinterpret_cast<unsigned long long *>(&base),
+                                            (unsigned long long)bcount[threadIdx.x]);
+    __syncthreads();
+    long o = base, b, e;
+    block_share(n, b, e);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    for (long t = b; t < e; t += kFgThreads) {
+        const long i = t + threadIdx.x;
+        const bool on = i < e && sel[i];
+        const unsigned ball = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) wc[wid] = __popc(ball);
+        __syncthreads();
+        int before = __popc(ball & ((1u << lane) - 1u)), all = 0;
+        for (int k = 0; k < kWarps; ++k) {
+            before += k < wid ? wc[k] : 0;
+            all += wc[k];
         }
-        *count = acc;
+        if (on) {
+            cx[o + before] = g7[i];
+            cy[o + before] = g7[n + i];
+            cf[o + before] = fit[i];
+        }
+        o += all;
+        __syncthreads();
     }
-    __syncthreads();
-    long o = offs[threadIdx.x];
-    for (long i = b; i < e; ++i)
-        if (sel[i]) {
-            cx[o] = g7[i];
-            cy[o] = g7[n + i];
-            cf[o] = fit[i];
-            ++o;
-        }
 }
 
-// Overlap sums of up to kBatch Gaussians over the m compacted points: rows
-// (sum f Psi, sum Psi^2, sum f^2) per Gaussian, the block that finishes last
-// adding the block partials in block order. Each Gaussian's sums follow the
-// same per-thread, per-block and cross-block order whatever else is in the
-// batch.
+// Overlap sums of up to kBatch Gaussians over the m compacted points: (sum f
+// Psi, sum Psi^2, sum f^2) per Gaussian. A unit is 32 consecutive points (and
+// those kUnits units further on); block u takes unit u, its warp k Gaussian k,
+// so that a region of a few thousand points spreads over the SMs. The block
+// that finishes last adds the units in order, by eights and then the eights,
+// so that each Gaussian's sums follow one order whatever the grid and
+// whatever else is in the batch.
 constexpr int kBatch = 8;
+constexpr int kUnits = 152 * 8;
+static_assert(kBatch == kFgThreads / 32, "one warp per Gaussian");
 
 struct GaussBatch {
     Gauss g[kBatch];
@@ -343,56 +449,52 @@ struct GaussBatch {
 };
 
 __global__ void __launch_bounds__(kFgThreads)
-fg_overlap_kernel(const long *__restrict__ count, const double *__restrict__ cx, const double *__restrict__ cy,
+fg_overlap_kernel(long m, const double *__restrict__ cx, const double *__restrict__ cy,
                   const double *__restrict__ cf, int scale, GaussBatch b, double *part, double *res,
-                  unsigned *done)
+                  unsigned *done, Mail mail)
 {
-    constexpr int kWarps = kFgThreads / 32;
-    __shared__ double ws[3 * kBatch][kWarps];
+    constexpr int NQ = 3 * kBatch;
+    __shared__ double eights[kUnits / 8][NQ];
     __shared__ bool last;
-    const long m = *count;
-    const int nq = 3 * b.k, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double s[3 * kBatch];
-#pragma unroll
-    for (int q = 0; q < 3 * kBatch; ++q) s[q] = 0.0;
-    for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < m; i += (long)gridDim.x * blockDim.x) {
-        const double f = cf[i], x = cx[i], y = cy[i];
-#pragma unroll
-        for (int k = 0; k < kBatch; ++k) {
-            if (k < b.k) {
-                const double p = gauss_at(b.g[k], scale, x, y);
-                s[3 * k] += __dmul_rn(f, p);
-                s[3 * k + 1] += __dmul_rn(p, p);
-                s[3 * k + 2] += __dmul_rn(f, f);
-            }
+    const int nq = 3 * b.k, lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    if (k < b.k) {
+        const Gauss g = b.g[k];
+        double s[3] = {0.0, 0.0, 0.0};
+        for (long i = (long)blockIdx.x * 32 + lane; i < m; i += 32L * kUnits) {
+            const double f = cf[i];
+            const double p = gauss_at(g, scale, cx[i], cy[i]);
+            s[0] += __dmul_rn(f, p);
+            s[1] += __dmul_rn(p, p);
+            s[2] += __dmul_rn(f, f);
         }
-    }
-    // per warp: a fixed shuffle tree; per block: warps in order
 #pragma unroll
-    for (int q = 0; q < 3 * kBatch; ++q) {
-        if (q < nq) {
-            double v = s[q];
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-            if (lane == 0) ws[q][wid] = v;
+        for (int q = 0; q < 3; ++q) {
+            for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], o);
+            if (lane == 0) part[(long)blockIdx.x * NQ + 3 * k + q] = s[q];
         }
-    }
-    __syncthreads();
-    if (threadIdx.x < nq) {
-        double v = 0.0;
-        for (int w = 0; w < kWarps; ++w) v += ws[threadIdx.x][w];
-        part[(long)blockIdx.x * 3 * kBatch + threadIdx.x] = v;
-        __threadfence();
+        if (lane == 0) __threadfence();
     }
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
     __syncthreads();
     if (!last) return;
-    if (threadIdx.x < nq) {
+    __threadfence();
+    const int units = gridDim.x, n8 = (units + 7) / 8;
+    for (int t = threadIdx.x; t < n8 * nq; t += kFgThreads) {
+        const int e = t / nq, q = t - e * nq;
         double v = 0.0;
-        for (unsigned bb = 0; bb < gridDim.x; ++bb) v += __ldcg(&part[(long)bb * 3 * kBatch + threadIdx.x]);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v += 8 * e + u < units ? __ldcg(&part[(long)(8 * e + u) * NQ + q]) : 0.0;
+        eights[e][q] = v;
+    }
+    __syncthreads();
+    double v = 0.0;
+    if ((int)threadIdx.x < nq) {
+        for (int e = 0; e < n8; ++e) v += eights[e][threadIdx.x];
         res[threadIdx.x] = v;
     }
     if (threadIdx.x == 0) *done = 0u;
+    post(mail, (int)threadIdx.x < nq, threadIdx.x, v);
 }
 
 __global__ void fg_generate_kernel(long n, const double *__restrict__ g7, Gauss g, int scale, double *__restrict__ out)
@@ -409,11 +511,54 @@ bool np_index(long r, long dim, long &out)
     return true;
 }
 
+// A page-locked block that the kernels post results into: borrowed by one fit
+// at a time, kept for later ones (at most kMailKeep of them, one per fit that
+// ran at the same time).
+struct MailBox {
+    double data[3 * kBatch];
+    unsigned flag;
+};
+constexpr size_t kMailKeep = 16;
+std::mutex g_mail_mu;
+std::vector<MailBox *> g_mail_free;
+
+MailBox *mailbox_borrow()
+{
+    {
+        std::lock_guard<std::mutex> lk(g_mail_mu);
+        if (!g_mail_free.empty()) {
+            MailBox *m = g_mail_free.back();
+            g_mail_free.pop_back();
+            return m;
+        }
+    }
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, sizeof(MailBox), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;   // the fit copies its results instead
+    }
+    static_cast<MailBox *>(p)->flag = 0u;
+    return static_cast<MailBox *>(p);
+}
+
+void mailbox_return(MailBox *m)
+{
+    if (!m) return;
+    {
+        std::lock_guard<std::mutex> lk(g_mail_mu);
+        if (g_mail_free.size() < kMailKeep) {
+            g_mail_free.push_back(m);
+            return;
+        }
+    }
+    cudaFreeHost(m);
+}
+
 // Scratch of one fit, one allocation.
 struct FitScratch {
     double *a = nullptr, *fit = nullptr, *part = nullptr, *res = nullptr;
     double *cx = nullptr, *cy = nullptr, *cf = nullptr, *opart = nullptr, *ores = nullptr;
-    long *ncomp = nullptr;
+    int *bcount = nullptr;
     unsigned char *sel = nullptr, *lines = nullptr;
     unsigned *count = nullptr;
     void *base = nullptr;
@@ -421,18 +566,26 @@ struct FitScratch {
 
 class Fit {
 public:
-    Fit(int ncx, int ncy, const double *g7, cudaStream_t s) : ncx_(ncx), ncy_(ncy), n_((long)ncx * ncy), g7_(g7), s_(s) {}
+    Fit(int ncx, int ncy, const double *g7, cudaStream_t s)
+        : ncx_(ncx), ncy_(ncy), n_((long)ncx * ncy), g7_(g7), s_(s), box_(mailbox_borrow())
+    {
+        if (box_) seq_ = box_->flag;
+    }
     ~Fit()
     {
         if (sc_.base) cudaFreeAsync(sc_.base, s_);
+        if (waiting_) cudaStreamSynchronize(s_);   // a failed wait: nothing may write into the box any more
+        mailbox_return(box_);
     }
+    Fit(const Fit &) = delete;
+    Fit &operator=(const Fit &) = delete;
 
     int alloc()
     {
         const size_t nd = (size_t)n_ * sizeof(double);
         const size_t parts = sizeof(double) * kFgBlocks * kFgMaxSums;
-        const size_t bytes = 5 * (nd + 256) + parts + sizeof(double) * (kFgBlocks + 1) * 3 * kBatch + 8 * 256 +
-                             2 * ((size_t)n_ + 256) + (size_t)ncx_ + ncy_ + 256;
+        const size_t bytes = 5 * (nd + 256) + parts + sizeof(double) * (kUnits + 1) * 3 * kBatch + 8 * 256 +
+                             sizeof(int) * kFgBlocks + 2 * ((size_t)n_ + 256) + (size_t)ncx_ + ncy_ + 256;
         if (int rc = po::scratch_alloc(reinterpret_cast<void **>(&sc_.base), bytes, s_)) return rc;
         char *p = static_cast<char *>(sc_.base);
         auto take = [&](size_t b) {
@@ -448,8 +601,8 @@ public:
         sc_.cx = reinterpret_cast<double *>(take(nd));
         sc_.cy = reinterpret_cast<double *>(take(nd));
         sc_.cf = reinterpret_cast<double *>(take(nd));
-        sc_.ncomp = reinterpret_cast<long *>(take(sizeof(long)));
-        sc_.opart = reinterpret_cast<double *>(take(sizeof(double) * kFgBlocks * 3 * kBatch));
+        sc_.bcount = reinterpret_cast<int *>(take(sizeof(int) * kFgBlocks));
+        sc_.opart = reinterpret_cast<double *>(take(sizeof(double) * kUnits * 3 * kBatch));
         sc_.ores = reinterpret_cast<double *>(take(sizeof(double) * 3 * kBatch));
         sc_.sel = reinterpret_cast<unsigned char *>(take((size_t)n_));
         sc_.lines = reinterpret_cast<unsigned char *>(take((size_t)ncx_ + ncy_));
@@ -458,11 +611,33 @@ public:
         return 0;
     }
 
-    // Launch status, then the first k result words on the host.
-    int read(double *h, int k, const char *what)
+    // The destination of the next kernel's results.
+    Mail mail()
+    {
+        if (!box_) return Mail{};
+        waiting_ = true;
+        return Mail{box_->data, &box_->flag, ++seq_};
+    }
+
+    // Launch status, then the first k result words (posted, or res on the device) on the host.
+    int read(double *h, int k, const double *res, const char *what)
     {
         cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h, sc_.res, sizeof(double) * k, cudaMemcpyDeviceToHost, s_);
+        if (e == cudaSuccess && box_) {
+            // every so often the stream itself is asked, so that an error ends the wait
+            for (unsigned spin = 1;; ++spin) {
+                if (__atomic_load_n(&box_->flag, __ATOMIC_ACQUIRE) == seq_) break;
+                if (spin % 65536u) continue;
+                e = cudaStreamQuery(s_);
+                if (e == cudaErrorNotReady) continue;
+                if (e == cudaSuccess && __atomic_load_n(&box_->flag, __ATOMIC_ACQUIRE) == seq_) break;
+                return fail(2, std::string(what) + ": " + (e == cudaSuccess ? "no result" : cudaGetErrorString(e)));
+            }
+            waiting_ = false;
+            for (int q = 0; q < k; ++q) h[q] = box_->data[q];
+            return 0;
+        }
+        if (e == cudaSuccess) e = cudaMemcpyAsync(h, res, sizeof(double) * k, cudaMemcpyDeviceToHost, s_);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
         if (e != cudaSuccess) return fail(2, std::string(what) + ": " + cudaGetErrorString(e));
         return 0;
@@ -470,20 +645,15 @@ public:
 
     int pattern(const double *fr, const double *fi, int scale, double &fit_max, long &imax, double &nf2)
     {
-        double h[3];
-        fg_abs_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, fr, fi, sc_.a, sc_.part, sc_.res, sc_.count);
-        note_launches(1);
-        if (int rc = read(h, 1, "field magnitude")) return rc;
-        if (!(h[0] > 0.0) || std::isinf(h[0]))
+        // res[3] = max |E_c|, kept there for the pattern kernel and as its fourth word
+        double h[4];
+        fg_abs_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, fr, fi, sc_.a, sc_.part, sc_.res + 3, sc_.count);
+        fg_pattern_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, sc_.a, sc_.res + 3, scale, sc_.fit, sc_.part, sc_.res,
+                                                             sc_.count, mail());
+        note_launches(2);
+        if (int rc = read(h, 4, sc_.res, "pattern")) return rc;
+        if (!(h[3] > 0.0) || std::isinf(h[3]))
             return fail(1, "the field component is zero, NaN or infinite: its normalisation is undefined");
-        // the maximum stays on the device (res[0]); copy it aside before res is reused
-        double *amax = sc_.res + 4;
-        cudaError_t e = cudaMemcpyAsync(amax, sc_.res, sizeof(double), cudaMemcpyDeviceToDevice, s_);
-        if (e != cudaSuccess) return fail(2, std::string("field maximum: ") + cudaGetErrorString(e));
-        fg_pattern_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, sc_.a, amax, scale, sc_.fit, sc_.part, sc_.res,
-                                                             sc_.count);
-        note_launches(1);
-        if (int rc = read(h, 3, "pattern")) return rc;
         fit_max = h[0];
         imax = (long)h[1];
         nf2 = h[2];
@@ -492,10 +662,12 @@ public:
 
     int select(double thr, int mode, const Window &w, double &count)
     {
-        fg_select_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, ncy_, g7_, sc_.fit, thr, mode, w, sc_.sel, sc_.part,
-                                                            sc_.res, sc_.count);
+        fg_select_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, ncy_, g7_, sc_.fit, thr, mode, w, sc_.sel, sc_.bcount,
+                                                            sc_.part, sc_.res, sc_.count, mail());
         note_launches(1);
-        return read(&count, 1, "fit region");
+        const int rc = read(&count, 1, sc_.res, "fit region");
+        m_ = rc ? 0 : (long)count;
+        return rc;
     }
 
     int lines(long i0, long j0, double thr, std::vector<unsigned char> &row, std::vector<unsigned char> &col)
@@ -513,25 +685,19 @@ public:
         return 0;
     }
 
-    int grid_value(int r, long flat, double &v)
-    {
-        cudaError_t e = cudaMemcpyAsync(&v, g7_ + (long)r * n_ + flat, sizeof(double), cudaMemcpyDeviceToHost, s_);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
-        if (e != cudaSuccess) return fail(2, std::string("grid value: ") + cudaGetErrorString(e));
-        return 0;
-    }
-
     int moments(double *m6)
     {
-        fg_moments_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, g7_, sc_.fit, sc_.sel, sc_.part, sc_.res, sc_.count);
+        fg_moments_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, g7_, sc_.fit, sc_.sel, sc_.part, sc_.res, sc_.count,
+                                                             mail());
         note_launches(1);
-        return read(m6, 6, "moments");
+        return read(m6, 6, sc_.res, "moments");
     }
 
     // The simplex from p0 over the current selection (fmin(GaussAbs, p0)).
     int fmin(const double *p0, int scale, double *popt)
     {
-        fg_compact_kernel<<<1, kCompactThreads, 0, s_>>>(n_, sc_.sel, g7_, sc_.fit, sc_.cx, sc_.cy, sc_.cf, sc_.ncomp);
+        fg_compact_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, sc_.sel, sc_.bcount, g7_, sc_.fit, sc_.cx, sc_.cy,
+                                                             sc_.cf);
         note_launches(1);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return fail(2, std::string("fit region compaction: ") + cudaGetErrorString(e));
@@ -588,14 +754,12 @@ public:
         GaussBatch b{};
         b.k = k;
         for (int q = 0; q < k; ++q) b.g[q] = gauss_of(pts[q]);
-        fg_overlap_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(sc_.ncomp, sc_.cx, sc_.cy, sc_.cf, scale, b, sc_.opart,
-                                                             sc_.ores, sc_.count);
+        const unsigned nblk = (unsigned)std::min<long>(kUnits, std::max(1L, (m_ + 31) / 32));
+        fg_overlap_kernel<<<nblk, kFgThreads, 0, s_>>>(m_, sc_.cx, sc_.cy, sc_.cf, scale, b, sc_.opart, sc_.ores,
+                                                        sc_.count, mail());
         note_launches(1);
         double h[3 * kBatch];
-        cudaError_t e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(h, sc_.ores, sizeof(double) * 3 * k, cudaMemcpyDeviceToHost, s_);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s_);
-        if (e != cudaSuccess) return fail(2, std::string("overlap sums: ") + cudaGetErrorString(e));
+        if (int rc = read(h, 3 * k, sc_.ores, "overlap sums")) return rc;
         for (int q = 0; q < k; ++q) {
             const double c00 = h[3 * q] * h[3 * q] / h[3 * q + 2] / h[3 * q + 1];
             val[q] = std::fabs(1 - std::fabs(c00));
@@ -605,9 +769,10 @@ public:
 
     int power(const double *p, double &pw)
     {
-        fg_power_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, g7_, gauss_of(p), sc_.part, sc_.res, sc_.count);
+        fg_power_kernel<<<kFgBlocks, kFgThreads, 0, s_>>>(n_, g7_, gauss_of(p), sc_.part, sc_.res, sc_.count,
+                                                           mail());
         note_launches(1);
-        return read(&pw, 1, "Gaussian power");
+        return read(&pw, 1, sc_.res, "Gaussian power");
     }
 
 private:
@@ -615,6 +780,10 @@ private:
     long n_;
     const double *g7_;
     cudaStream_t s_;
+    MailBox *box_;
+    unsigned seq_ = 0;
+    bool waiting_ = false;
+    long m_ = 0;   // points of the current selection
     FitScratch sc_;
 };
 
@@ -688,11 +857,7 @@ int fit_gauss_abs_dev(int ncx, int ncy, const double *g7, const double *fr, cons
         return fail(1, "fit: the window corners index past the grid (the reference raises IndexError here)");
     c1 = c0;
     q1 = q0;
-    Window w{};
-    if (int rc = F.grid_value(0, r0 * ncy + c0, w.xlo)) return rc;
-    if (int rc = F.grid_value(0, r1 * ncy + c1, w.xhi)) return rc;
-    if (int rc = F.grid_value(1, q0 * ncy + s0, w.ylo)) return rc;
-    if (int rc = F.grid_value(1, q1 * ncy + s1, w.yhi)) return rc;
+    const Window w{r0 * ncy + c0, r1 * ncy + c1, q0 * ncy + s0, q1 * ncy + s1};
 
     double count;
     if (int rc = F.select(thr_of(thres), 1, w, count)) return rc;
