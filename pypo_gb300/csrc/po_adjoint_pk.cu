@@ -19,16 +19,7 @@
 //
 // The three projections of W (on R_hat, n_s, n_t) come from one complex
 // vector per pair, Z = b x J - a x M: W.v = -v.Z (scalar triple product).
-//
-// Far field: the same kernel with the far-field pair (currents and source
-// displacement; far-field targets are directions and do not move). A CTA
-// owns one tile of 128 sources in Hilbert order (the forward's tile records,
-// po_farfield.cu): e^{-t j k r.s} = e^{-t j k r.c} e^{-t j k r.(s - c)}, so
-// each stage's cotangents are multiplied once by conj(e^{-t j k r.c}) for
-// the CTA's centre c (ff_rotate_cot), and the pair loop takes only the
-// offset's phase: FP32 for a narrow tile, split for a wide one. With M = 0,
-// a cotangent tile whose direction box proves every pair lit for the CTA's
-// source normals skips the illumination mask.
+// The far field's adjoint is in po_ff_adjoint.cu.
 #include <cuda_runtime.h>
 #include <math_constants.h>
 #include <cstdint>
@@ -44,12 +35,8 @@ namespace po {
 //   with the target displacement: 18-20 n_t, 21-22 a.n_t; with M as well:
 //   23-24 b.n_t (a = conj(gE), b = conj(gH)). A padding target has zero
 //   cotangent.
-// Far field: 0-2 r_hat hi (on 2^-11), 3-5 r_hat lo, 6-11 gS_J, 12-17 gS_M,
-//   18-20 r_hat = hi + lo (11 float4).
-__host__ __device__ constexpr int adj2_rec(int kind, bool has_m, bool want_t)
-{
-    return kind == kKindFF ? 11 : (want_t ? (has_m ? 13 : 12) : 9);   // scalar: the near-field layout
-}
+// The scalar kind has the near-field layout.
+__host__ __device__ constexpr int adj2_rec(bool has_m, bool want_t) { return want_t ? (has_m ? 13 : 12) : 9; }
 
 constexpr int kPairsA2 = PO_PAIRS_A;   // target pairs per shared-memory stage
 #ifndef PO_FLUSH_A
@@ -61,7 +48,7 @@ static_assert(kThreadsA == 128 && (kFlush == 16 || kFlush == 32),
               "the transpose maps 128 threads onto 16 pairs x 8 segments or 32 pairs x 4");
 
 __global__ void po_adj_pack_tgt2_kernel(long nt, const double *__restrict__ tgt7, const double *__restrict__ gam,
-                                        const Frame *__restrict__ frp, int far, int rec4, float *__restrict__ out)
+                                        const Frame *__restrict__ frp, int rec4, float *__restrict__ out)
 {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     const long np = (nt + 1) / 2;
@@ -70,29 +57,14 @@ __global__ void po_adj_pack_tgt2_kernel(long nt, const double *__restrict__ tgt7
     const bool real = i < nt;
     const Frame fr = *frp;
     float v[26];
-    if (far) {
-        const double th = tgt7[k], ph = tgt7[nt + k];
-        const double rd[3] = {cos(ph) * sin(th), sin(ph) * sin(th), cos(th)};
-        for (int c = 0; c < 3; ++c) {
-            const double hd = rint(rd[c] * 2048.0) / 2048.0;
-            v[c] = (float)hd;
-            v[3 + c] = (float)(rd[c] - hd);
-        }
-    } else {
-        for (int c = 0; c < 3; ++c) {
-            const double x = (tgt7[c * nt + k] - fr.o[c]) * fr.kappa;
-            const double hd = rint(x * fr.inv_q) * fr.q;
-            v[c] = (float)hd;
-            v[3 + c] = (float)(x - hd);
-        }
-    }
+    for (int c = 0; c < 3; ++c) split_hi_lo((tgt7[c * nt + k] - fr.o[c]) * fr.kappa, fr, v[c], v[3 + c]);
     double ge[6], gh[6], n[3];   // (re, im) x y z
     for (int c = 0; c < 3; ++c) {
         ge[2 * c] = real ? gam[c * nt + k] : 0.0;
         ge[2 * c + 1] = real ? gam[(3 + c) * nt + k] : 0.0;
         gh[2 * c] = real ? gam[(6 + c) * nt + k] : 0.0;
         gh[2 * c + 1] = real ? gam[(9 + c) * nt + k] : 0.0;
-        n[c] = real && !far ? tgt7[(3 + c) * nt + k] : 0.0;
+        n[c] = real ? tgt7[(3 + c) * nt + k] : 0.0;
     }
     for (int q = 0; q < 6; ++q) {
         v[6 + q] = (float)ge[q];
@@ -107,7 +79,7 @@ __global__ void po_adj_pack_tgt2_kernel(long nt, const double *__restrict__ tgt7
         v[dot_at] = (float)dr;
         v[dot_at + 1] = (float)di;
     }
-    for (int c = 0; c < 3; ++c) v[18 + c] = far ? v[c] + v[3 + c] : (float)n[c];
+    for (int c = 0; c < 3; ++c) v[18 + c] = (float)n[c];
     v[25] = 0.f;
     float *o = out + (i >> 1) * (long)(rec4 * 4) + (i & 1);
     for (int q = 0; q < 2 * rec4; ++q) o[2 * q] = v[q];
@@ -344,167 +316,28 @@ __device__ __forceinline__ void adj_sc_pair2(float2 *acc, float2 &vt, const floa
     if (WANT_T) vt = mul2(g, fma2(r[20], dz, fma2(r[19], dy, mul2(r[18], dx))));
 }
 
-// Far-field pair of targets against the thread's source:
-//   Jbar' += conj(G) gS_J, Mbar' += conj(G) gS_M (G = e^{-t j k r'.r_hat}),
-//   source displacement: Re[-t j k G (conj(gS_J).J' + conj(gS_M).M')] (n_s . r_hat),
-// k in turns is 2 pi.
-// LIT: the tile is proven lit for the CTA's sources (every pair passes the
-// illumination test), so the sign (-1)^q is set on the bits and the mask is
-// left out; the result is the same bits.
-__device__ __forceinline__ float2 adj_ff_ndr2(const float2 *r, const SrcC &s)
-{
-    return fma2(dup2(s.n[2]), r[20], fma2(dup2(s.n[1]), r[19], mul2(dup2(s.n[0]), r[18])));
-}
-
-template <int T, bool HAS_M, bool WANT_D, bool LIT, bool WIDE>
-__device__ __forceinline__ void adj_ff_pair2(float2 *acc, const float2 *r, const SrcC &s, bool &band)
-{
-    // the phase of the source's offset w from its tile centre (the centre's
-    // phase is already in the cotangents): narrow tiles p = r.w in FP32
-    // (|w| <= kFFNarrow turns), reduced exactly to the nearest turn; wide
-    // tiles from the split offset, reduced in half turns with a parity
-    float2 sn, cs, tq = dup2(0.0f);
-    if (WIDE) {
-        const float2 Ph = fma2(dup2(s.sh[2]), r[2], fma2(dup2(s.sh[1]), r[1], mul2(dup2(s.sh[0]), r[0])));
-        const float2 Pl = fma2(dup2(s.sl[2]), r[20], fma2(dup2(s.sl[1]), r[19], fma2(dup2(s.sl[0]), r[18],
-                          fma2(dup2(s.sh[2]), r[5], fma2(dup2(s.sh[1]), r[4], mul2(dup2(s.sh[0]), r[3]))))));
-        ff_phase_sincos2(Ph, Pl, sn, cs, tq);
-    } else {
-        const float2 magic = dup2(12582912.0f), twopi = dup2(6.28318530717958648f);
-        const float2 P = fma2(dup2(s.sh[2]), r[20], fma2(dup2(s.sh[1]), r[19], mul2(dup2(s.sh[0]), r[18])));
-        const float2 ang = mul2(sub2(P, sub2(add2(P, magic), magic)), twopi);
-        __sincosf(ang.x, &sn.x, &cs.x);
-        __sincosf(ang.y, &sn.y, &cs.y);
-    }
-    const float2 ndr = adj_ff_ndr2(r, s);
-    float2 gc, gs;                                          // G = (gc, gs)
-    if (LIT) {
-        gc = WIDE ? flip_parity(cs, tq) : cs;
-        gs = WIDE ? flip_parity(T > 0 ? neg2(sn) : sn, tq) : (T > 0 ? neg2(sn) : sn);
-    } else {
-        const float2 one = WIDE ? flip_parity(dup2(1.0f), tq) : dup2(1.0f);
-        band = band || (fabsf(ndr.x) < kTangentBand) || (fabsf(ndr.y) < kTangentBand);
-        const float2 m = make_float2(ndr.x >= kTangentBand ? one.x : 0.0f, ndr.y >= kTangentBand ? one.y : 0.0f);
-        gc = mul2(cs, m);
-        gs = mul2(T > 0 ? neg2(sn) : sn, m);
-    }
-    // conj(G) g = (gc g.re + gs g.im, gc g.im - gs g.re)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        acc[c] = fma2(gs, r[7 + 2 * c], fma2(gc, r[6 + 2 * c], acc[c]));
-        acc[3 + c] = fma2(neg2(gs), r[6 + 2 * c], fma2(gc, r[7 + 2 * c], acc[3 + c]));
-        acc[6 + c] = fma2(gs, r[13 + 2 * c], fma2(gc, r[12 + 2 * c], acc[6 + c]));
-        acc[9 + c] = fma2(neg2(gs), r[12 + 2 * c], fma2(gc, r[13 + 2 * c], acc[9 + c]));
-    }
-    if (WANT_D) {
-        // X = conj(gS_J).J' (+ conj(gS_M).M'); Z = G X, Im Z = gc X.im + gs X.re
-        float2 xr = dup2(0.f), xi = dup2(0.f);
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const float2 jr = dup2(s.J[2 * c]), ji = dup2(s.J[2 * c + 1]);
-            xr = fma2(r[6 + 2 * c], jr, fma2(r[7 + 2 * c], ji, xr));
-            xi = fma2(r[6 + 2 * c], ji, fma2(neg2(r[7 + 2 * c]), jr, xi));
-            if (HAS_M) {
-                const float2 mr = dup2(s.M[2 * c]), mi = dup2(s.M[2 * c + 1]);
-                xr = fma2(r[12 + 2 * c], mr, fma2(r[13 + 2 * c], mi, xr));
-                xi = fma2(r[12 + 2 * c], mi, fma2(neg2(r[13 + 2 * c]), mr, xi));
-            }
-        }
-        const float2 zi = fma2(gc, xi, mul2(gs, xr));
-        acc[12] = fma2(mul2(zi, ndr), dup2(T > 0 ? 6.28318530717958647f : -6.28318530717958647f), acc[12]);
-    }
-}
-
-// Direction box of each far-field cotangent tile (kPairsA2 pair records) for
-// the lit-tile proof of the far-field adjoint: lowest and highest r_hat per
-// axis, written into the unused slot 21 of the tile's first three pair
-// records. One warp per tile; the padding target of an odd count repeats
-// the last target, so it changes nothing.
-__global__ void po_adj_tgt_box_kernel(float2 *__restrict__ rec, long nt)
-{
-    constexpr int R2 = 2 * adj2_rec(kKindFF, false, false);   // float2 slots per pair record
-    float v[6] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-    const long np = (nt + 1) / 2;
-    for (int p = threadIdx.x; p < kPairsA2; p += 32) {
-        const long pair = (long)blockIdx.x * kPairsA2 + p;
-        if (pair >= np) break;
-        const float2 *r = rec + pair * R2;
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            v[c] = fminf(v[c], fminf(r[18 + c].x, r[18 + c].y));
-            v[3 + c] = fmaxf(v[3 + c], fmaxf(r[18 + c].x, r[18 + c].y));
-        }
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const float u = __shfl_xor_sync(0xffffffffu, v[q], o);
-            v[q] = q < 3 ? fminf(v[q], u) : fmaxf(v[q], u);
-        }
-    if (threadIdx.x < 6) {
-        const long pair = (long)blockIdx.x * kPairsA2 + (threadIdx.x >> 1);
-        float *slot = reinterpret_cast<float *>(rec + pair * R2 + 21);
-        if (pair < np) slot[threadIdx.x & 1] = v[threadIdx.x];
-    }
-}
-
-// Far field: one stage's pair record of two directions (lanes), its
-// cotangents gS_J, gS_M (slots 6-17, (re, im) per axis) multiplied in place by
-// conj(e^{-t j k r.c}) for the CTA's tile centre c (hi xyz, lo xyz, turns).
-// One thread per record: spreading a record over four threads (each forming
-// the phase and rotating its share) measured 279.6 -> 297.0 ms on dish_ff.
-// With s = c + w, conj(G) g = conj(G_w) (conj(G_c) g), so the pair loop needs
-// only the offset's phase. r.c in split form: hi products exact (r hi on
-// 2^-11, c hi on the frame's quantum), the rest in one FP32 sum, reduced
-// exactly to half turns, as the forward's tile phase.
-template <int T>
-__device__ __forceinline__ void ff_rotate_cot(float4 *rec4, const float *c)
-{
-    float2 *r = reinterpret_cast<float2 *>(rec4);
-    const float2 Ph = fma2(dup2(c[2]), r[2], fma2(dup2(c[1]), r[1], mul2(dup2(c[0]), r[0])));
-    const float2 Pl = fma2(dup2(c[5]), r[20], fma2(dup2(c[4]), r[19], fma2(dup2(c[3]), r[18],
-                      fma2(dup2(c[2]), r[5], fma2(dup2(c[1]), r[4], mul2(dup2(c[0]), r[3]))))));
-    float2 sn, cs, tq;
-    ff_phase_sincos2(Ph, Pl, sn, cs, tq);
-    const float2 gc = flip_parity(cs, tq), gs = flip_parity(T > 0 ? neg2(sn) : sn, tq);
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        const float2 re = r[6 + 2 * q], im = r[7 + 2 * q];
-        r[6 + 2 * q] = fma2(gc, re, mul2(gs, im));
-        r[7 + 2 * q] = fma2(gc, im, mul2(neg2(gs), re));
-    }
-}
-
 // The rare path of a tile in which some pair fell inside the tangent band:
 // the thread's source is tested again against the tile's targets, with the
 // pair loop's operations, and each pair inside the band is listed for the
 // FP64 fixup (an idle source or padding target is only left out). tile:
 // cnt target pair records (RT float4 each), the first with target index
 // 2 * pfirst.
-template <int KIND, int RT>
+template <int RT>
 __device__ __forceinline__ void adj_band_scan(const float4 *tile, int cnt, long pfirst, const SrcC &s, long si,
                                               long ns, long nt, BandList bl)
 {
     if (si >= ns) return;
 #pragma unroll 1
     for (int p = 0; p < cnt; ++p) {
-        float2 r[22];
-        if (KIND == kKindFF) {
-            const float4 v0 = tile[p * RT + 9], v1 = tile[p * RT + 10];   // float2 slots 18-21
-            r[18] = make_float2(v0.x, v0.y);
-            r[19] = make_float2(v0.z, v0.w);
-            r[20] = make_float2(v1.x, v1.y);
-        } else {
+        float2 r[6];
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float4 v = tile[p * RT + c];
-                r[2 * c] = make_float2(v.x, v.y);
-                r[2 * c + 1] = make_float2(v.z, v.w);
-            }
+        for (int c = 0; c < 3; ++c) {
+            const float4 v = tile[p * RT + c];
+            r[2 * c] = make_float2(v.x, v.y);
+            r[2 * c + 1] = make_float2(v.z, v.w);
         }
-        const float2 nd = KIND == kKindFF ? adj_ff_ndr2(r, s) : adj_geo2(r, s).ndd;
-        const float2 bw = KIND == kKindFF ? dup2(kTangentBand) : mul2(dup2(kTangentBand), adj_geo2(r, s).Rh);
+        const AdjGeo2 g = adj_geo2(r, s);
+        const float2 nd = g.ndd, bw = mul2(dup2(kTangentBand), g.Rh);
         const long t0 = 2 * (pfirst + p);
         if (fabsf(nd.x) < bw.x && t0 < nt) band_defer(bl, si, t0);
         if (fabsf(nd.y) < bw.y && t0 + 1 < nt) band_defer(bl, si, t0 + 1);
@@ -512,13 +345,11 @@ __device__ __forceinline__ void adj_band_scan(const float4 *tile, int cnt, long 
 }
 
 template <int KIND, int T, bool HAS_M, bool WANT_D, bool WANT_T>
-__global__ void __launch_bounds__(kThreadsA, KIND == kKindFF ? kMinBlocksFF : (HAS_M ? kMinBlocksA2M : kMinBlocksA2))
+__global__ void __launch_bounds__(kThreadsA, HAS_M ? kMinBlocksA2M : kMinBlocksA2)
 po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__restrict__ trec, long nt, long chunk,
-                 double *__restrict__ part, double *__restrict__ gt, int *__restrict__ err, int boxes, BandList bl,
-                 const int *__restrict__ order)
+                 double *__restrict__ part, double *__restrict__ gt, int *__restrict__ err, BandList bl)
 {
-    static_assert(KIND != kKindFF || !WANT_T, "far-field targets do not move");
-    constexpr int RT = adj2_rec(KIND, HAS_M, WANT_T);
+    constexpr int RT = adj2_rec(HAS_M, WANT_T);
     constexpr int NL = 2 * RT;                    // float2 slots read per pair
     extern __shared__ __align__(128) float4 stage[];   // kStages * kPairsA2 * RT, lo, transpose buffer
     __shared__ __align__(8) uint64_t full[kStages];
@@ -526,33 +357,8 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
     float2 *vbuf = reinterpret_cast<float2 *>(lo + kAccAdj * kThreadsA);   // [kFlush][kThreadsA]
 
     SrcC s;
-    long si;                 // the thread's source (its index in the caller's arrays)
-    [[maybe_unused]] bool wide = false;     // far field: the CTA's tile stores split offsets
-    [[maybe_unused]] float cen[6] = {};     // far field: the tile centre, hi xyz and lo xyz (turns)
-    if constexpr (KIND == kKindFF) {
-        // one CTA per far-field source tile (po_ff_pack_kernel's records, in
-        // Hilbert order): the offset from the tile centre, J', the normal, M'
-        constexpr int R4 = ff_rec4(HAS_M), T4 = ff_tile4(HAS_M);
-        static_assert(kThreadsA == kTile, "one far-field source tile per adjoint CTA");
-        const float *tf = reinterpret_cast<const float *>(srcpk + (size_t)blockIdx.x * T4);
-#pragma unroll
-        for (int c = 0; c < 6; ++c) cen[c] = tf[c];
-        wide = tf[12] != 0.0f;
-        const float *rec = tf + kFFHead * 4 + (threadIdx.x >> 1) * R4 * 4 + (threadIdx.x & 1);   // slot k: rec[2k]
-        const long pos = (long)blockIdx.x * kThreadsA + threadIdx.x;
-        si = pos < ns ? (long)order[pos] : ns;   // padding: past the end, never written
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            s.sh[c] = rec[2 * c];
-            s.sl[c] = rec[2 * (12 + c)];
-            s.n[c] = rec[2 * (9 + c)];
-            s.J[2 * c] = rec[2 * (3 + c)];
-            s.J[2 * c + 1] = rec[2 * (6 + c)];
-            s.M[2 * c] = HAS_M ? rec[2 * (16 + c)] : 0.0f;
-            s.M[2 * c + 1] = HAS_M ? rec[2 * (19 + c)] : 0.0f;
-        }
-    } else {
-        si = (long)blockIdx.x * kThreadsA + threadIdx.x;
+    const long si = (long)blockIdx.x * kThreadsA + threadIdx.x;
+    {
         float4 q[kRec];
 #pragma unroll
         for (int c = 0; c < kRec; ++c) q[c] = si < ns ? srcpk[(size_t)kRec * si + c] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -581,41 +387,6 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
     for (int a = 0; a < kAccAdj; ++a) {
         hi[a] = 0.f;
         lo[a * kThreadsA + threadIdx.x] = 0.f;
-    }
-
-    // Far field, M = 0: the CTA's box of source normals for the lit-tile
-    // proof (a tile's directions r_hat against it: min n.r_hat >= 1e-5, the
-    // least of n.r over the two boxes being the sum of the least corner
-    // products per axis; the per-pair test: lit when n.r_hat >= 1e-6). Only there: the
-    // near-field adjoint needs n_s.R for its displacement gradient anyway,
-    // and a second copy of the loop is not worth its cost with M.
-    constexpr bool kLitA = KIND == kKindFF && !HAS_M;
-    __shared__ float nbox_w[kThreadsA / 32][6];
-    __shared__ float nbox[6];
-    if (kLitA) {
-        float v[6];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            v[c] = si < ns ? s.n[c] : CUDART_INF_F;
-            v[3 + c] = si < ns ? s.n[c] : -CUDART_INF_F;
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                const float u = __shfl_xor_sync(0xffffffffu, v[q], o);
-                v[q] = q < 3 ? fminf(v[q], u) : fmaxf(v[q], u);
-            }
-        if ((threadIdx.x & 31) == 0)
-#pragma unroll
-            for (int q = 0; q < 6; ++q) nbox_w[threadIdx.x >> 5][q] = v[q];
-        __syncthreads();
-        if (threadIdx.x < 6) {
-            const int q = threadIdx.x;
-            float r = nbox_w[0][q];
-            for (int w = 1; w < kThreadsA / 32; ++w) r = q < 3 ? fminf(r, nbox_w[w][q]) : fmaxf(r, nbox_w[w][q]);
-            nbox[q] = r;
-        }
     }
 
     const long t0 = (long)blockIdx.y * chunk;     // chunk: a multiple of 2 * kPairsA2 targets
@@ -651,74 +422,26 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
         const float4 *tile = stage + (size_t)(it % kStages) * kPairsA2 * RT;
         const long pfirst = p0 + (long)it * kPairsA2;
         const int cnt = (int)min((long)kPairsA2, p1 - pfirst);
-        if constexpr (KIND == kKindFF) {
-            // the stage's cotangents times conj(e^{-t j k r.c}) for this CTA's tile centre c
-            if (threadIdx.x < cnt)
-                ff_rotate_cot<T>(stage + (size_t)(it % kStages) * kPairsA2 * RT + threadIdx.x * RT, cen);
-            __syncthreads();
-        }
         float2 acc[kAccAdj];
 #pragma unroll
         for (int a = 0; a < kAccAdj; ++a) acc[a] = make_float2(0.f, 0.f);
         bool band = false;   // a pair of this tile fell inside the tangent band
-        // block-uniform: the tile's direction box (in the first three pair
-        // records, as po_adj_tgt_box_kernel wrote it) against the CTA's normals
-        [[maybe_unused]] bool lit = false;
-        if constexpr (kLitA) {
-            if (boxes && cnt >= 3) {
-                const float *f = reinterpret_cast<const float *>(tile);
-                float L = 0.0f;
-#pragma unroll
-                for (int c = 0; c < 3; ++c) {
-                    const float tl = f[(c >> 1) * RT * 4 + 42 + (c & 1)];
-                    const float th = f[((3 + c) >> 1) * RT * 4 + 42 + ((3 + c) & 1)];
-                    L += fminf(fminf(nbox[c] * tl, nbox[c] * th), fminf(nbox[3 + c] * tl, nbox[3 + c] * th));
-                }
-                lit = L >= 1e-5f;
-            }
-        }
         for (int fb = 0; fb < cnt; fb += kFlush) {
             const int fend = min(cnt, fb + kFlush);
-            if constexpr (KIND == kKindFF) {
-                // far field: one copy of the pair loop per case, all block-uniform.
-                // LIT: the tile is proven lit (M = 0), so the mask is left out.
-                // WIDE: the CTA's offsets are split, so the phase is too.
-                auto pairs = [&](auto lit_c, auto wide_c) {
-                    constexpr bool LIT = decltype(lit_c)::value, WIDE = decltype(wide_c)::value;
 #pragma unroll kUnrollA
-                    for (int p = fb; p < fend; ++p) {
-                        float2 rec[NL];
+            for (int p = fb; p < fend; ++p) {
+                float2 rec[NL];
 #pragma unroll
-                        for (int c = 0; c < RT; ++c) {
-                            const float4 v = tile[p * RT + c];
-                            rec[2 * c] = make_float2(v.x, v.y);
-                            rec[2 * c + 1] = make_float2(v.z, v.w);
-                        }
-                        adj_ff_pair2<T, HAS_M, WANT_D, LIT, WIDE>(acc, rec, s, band);
-                    }
-                };
-                if (wide)
-                    pairs(std::false_type{}, std::true_type{});
-                else if (lit)
-                    pairs(std::bool_constant<kLitA>{}, std::false_type{});
-                else
-                    pairs(std::false_type{}, std::false_type{});
-            } else {
-#pragma unroll kUnrollA
-                for (int p = fb; p < fend; ++p) {
-                    float2 rec[NL];
-#pragma unroll
-                    for (int c = 0; c < RT; ++c) {
-                        const float4 v = tile[p * RT + c];
-                        rec[2 * c] = make_float2(v.x, v.y);
-                        rec[2 * c + 1] = make_float2(v.z, v.w);
-                    }
-                    float2 vt = make_float2(0.f, 0.f);
-                    if (KIND == kKindNF)
-                        adj_nf_pair2<T, HAS_M, WANT_D, WANT_T>(acc, vt, rec, s, band);
-                    else adj_sc_pair2<T, WANT_D, WANT_T>(acc, vt, rec, s);
-                    if (WANT_T) vbuf[(p - fb) * kThreadsA + threadIdx.x] = vt;
+                for (int c = 0; c < RT; ++c) {
+                    const float4 v = tile[p * RT + c];
+                    rec[2 * c] = make_float2(v.x, v.y);
+                    rec[2 * c + 1] = make_float2(v.z, v.w);
                 }
+                float2 vt = make_float2(0.f, 0.f);
+                if (KIND == kKindNF)
+                    adj_nf_pair2<T, HAS_M, WANT_D, WANT_T>(acc, vt, rec, s, band);
+                else adj_sc_pair2<T, WANT_D, WANT_T>(acc, vt, rec, s);
+                if (WANT_T) vbuf[(p - fb) * kThreadsA + threadIdx.x] = vt;
             }
             if (WANT_T) {
                 // Sum the CTA's sources for each target pair of this flush: thread
@@ -759,7 +482,7 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
             float &l = lo[a * kThreadsA + threadIdx.x];
             l = __fadd_rn(l, e);
         }
-        if (KIND != kKindScalar && band) adj_band_scan<KIND, RT>(tile, cnt, pfirst, s, si, ns, nt, bl);
+        if (KIND != kKindScalar && band) adj_band_scan<RT>(tile, cnt, pfirst, s, si, ns, nt, bl);
         __syncthreads();
         if (threadIdx.x == 0 && it + kStages < ntiles) issue(it + kStages);
     }
@@ -769,17 +492,15 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
         part[((long)blockIdx.y * kAccAdj + a) * ns + si] = (double)hi[a] + (double)lo[a * kThreadsA + threadIdx.x];
 }
 
-int adj_pk_smem_bytes(int kind, bool has_m, bool want_t)
+int adj_pk_smem_bytes(bool has_m, bool want_t)
 {
-    return kStages * kPairsA2 * adj2_rec(kind, has_m, want_t) * 16 + kAccAdj * kThreadsA * 4 +
+    return kStages * kPairsA2 * adj2_rec(has_m, want_t) * 16 + kAccAdj * kThreadsA * 4 +
            (want_t ? kFlush * kThreadsA * 8 : 0);
 }
 
 int adj_pk_pairs_per_tile() { return kPairsA2; }
 
-int adj_pk_rec4(int kind, bool has_m, bool want_t) { return adj2_rec(kind, has_m, want_t); }
-
-void *adj_tgt_box_kernel() { return reinterpret_cast<void *>(&po_adj_tgt_box_kernel); }
+int adj_pk_rec4(bool has_m, bool want_t) { return adj2_rec(has_m, want_t); }
 
 template <int KIND, int T, bool HAS_M, bool WANT_D, bool WANT_T>
 static void *adj_pk_ptr()
@@ -790,8 +511,6 @@ static void *adj_pk_ptr()
 template <int T, bool HAS_M>
 static void *adj_pk_sel(int kind, bool want_d, bool want_t)
 {
-    if (kind == kKindFF) return want_d ? adj_pk_ptr<kKindFF, T, HAS_M, true, false>()
-                                       : adj_pk_ptr<kKindFF, T, HAS_M, false, false>();
     if (kind == kKindScalar) {
         if (want_d) return want_t ? adj_pk_ptr<kKindScalar, T, false, true, true>()
                                   : adj_pk_ptr<kKindScalar, T, false, true, false>();

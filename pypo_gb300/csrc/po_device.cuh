@@ -99,6 +99,14 @@ __device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a
 __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a, b); }
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
 
+// two_sum on both lanes.
+__device__ __forceinline__ void two_sum2(float2 a, float2 b, float2 &s, float2 &e)
+{
+    s = add2(a, b);
+    const float2 bb = sub2(s, a);
+    e = add2(sub2(a, sub2(s, bb)), sub2(b, bb));
+}
+
 // 1/sqrt(x), flush-to-zero form (x = R^2 in turns^2 is never subnormal for
 // distinct points).
 __device__ __forceinline__ float rsqrt_ftz(float x)

@@ -768,27 +768,28 @@ int run_adjoint(const AdjArgs &a)
                           &srcpk};
         if (!rc) rc = launch(pack_src_kernel(), dim3(nblk_s), dim3(256), psargs, 0, s);
     }
-    // Pair-packed adjoint: sources in registers, pairs of targets streamed.
-    // Near field fused (currents, source and target displacement in one pass).
+    // Near field and scalar: a source per thread, pairs of targets streamed,
+    // fused (currents, source and target displacement in one pass). Far field:
+    // two sources per thread, stages of kFFDirs directions streamed.
     const bool want_t = grad_dt != nullptr;
-    const int rec4 = adj_pk_rec4(kind, has_m, want_t);
+    const int rec4 = far ? 0 : adj_pk_rec4(has_m, want_t);
     const long npair = (nt + 1) / 2;
+    long nstage = (nt + kFFDirs - 1) / kFFDirs;
     float *trec2 = nullptr;
     double *gt = nullptr;
-    if (!rc && ((rc = salloc(&trec2, (size_t)npair * rec4 * 4, s, owned)) ||
-                (want_t && (rc = salloc(&gt, (size_t)nt, s, owned))))) {
+    const size_t trec4 = far ? (size_t)nstage * ff_adj_stage4() : (size_t)npair * rec4;
+    if (!rc && ((rc = salloc(&trec2, trec4 * 4, s, owned)) || (want_t && (rc = salloc(&gt, (size_t)nt, s, owned))))) {
         sfree(owned, s);
         return rc;
     }
-    int farflag = far ? 1 : 0;
-    void *p2args[] = {&nt, &tgt7, &gam, &frame, &farflag, (void *)&rec4, &trec2};
-    const unsigned nblk_p = (unsigned)((2 * npair + 255) / 256);
-    if (!rc) rc = launch(adj_pack_tgt2_kernel(), dim3(nblk_p), dim3(256), p2args, 0, s);
-    // direction boxes of the far-field tiles for the lit-tile proof (M = 0 kernels)
-    int boxes = far && !has_m && nt > 0;
-    void *tbargs[] = {&trec2, &nt};
-    const unsigned ntile_a = (unsigned)((npair + adj_pk_pairs_per_tile() - 1) / adj_pk_pairs_per_tile());
-    if (!rc && boxes) rc = launch(adj_tgt_box_kernel(), dim3(ntile_a), dim3(32), tbargs, 0, s);
+    if (far) {
+        void *p2args[] = {&nt, &tgt7, &gam, &trec2};
+        if (!rc) rc = launch(ff_pack_cot_kernel(), dim3((unsigned)nstage), dim3(kFFDirs), p2args, 0, s);
+    } else {
+        void *p2args[] = {&nt, &tgt7, &gam, &frame, (void *)&rec4, &trec2};
+        const unsigned nblk_p = (unsigned)((2 * npair + 255) / 256);
+        if (!rc) rc = launch(adj_pack_tgt2_kernel(), dim3(nblk_p), dim3(256), p2args, 0, s);
+    }
     if (want_t) PO_CK_RC(cudaMemsetAsync(gt, 0, sizeof(double) * nt, s));
     BandList band{nullptr, nullptr, 0};   // near-tangent pairs (not the scalar kind)
     if (!rc && kind != kKindScalar) {
@@ -799,21 +800,24 @@ int run_adjoint(const AdjArgs &a)
         }
         PO_CK_RC(cudaMemsetAsync(band.count, 0, sizeof(unsigned), s));
     }
-    void *fk = adj_pk_kernel(kind, ts, has_m, want_d, want_t);
-    const int smem2 = adj_pk_smem_bytes(kind, has_m, want_t);
+    void *fk = far ? ff_adj_kernel(ts, has_m, want_d) : adj_pk_kernel(kind, ts, has_m, want_d, want_t);
+    const int smem2 = far ? ff_adj_smem_bytes(want_d) : adj_pk_smem_bytes(has_m, want_t);
+    const int threads = far ? ff_adj_threads() : kThreadsA;
     int occ2 = 1;
-    if (!rc) rc = kernel_occupancy(di, fk, kThreadsA, smem2, occ2);
-    const long tile_t = 2L * adj_pk_pairs_per_tile();
-    const long nsb = (ns + kThreadsA - 1) / kThreadsA;
+    if (!rc) rc = kernel_occupancy(di, fk, threads, smem2, occ2);
+    const long tile_t = far ? kFFDirs : 2L * adj_pk_pairs_per_tile();
+    const long nsb = far ? (ns + kTile - 1) / kTile : (ns + kThreadsA - 1) / kThreadsA;
     const long split = choose_split(nsb, nt, (long)di->sms * occ2, partial_cap(ns, kAccAdj), tile_t);
     const long tiles = std::max(1L, (nt + tile_t - 1) / tile_t);
-    long chunk = ((tiles + split - 1) / split) * tile_t;
+    long chunk = (tiles + split - 1) / split * (far ? 1 : tile_t);   // stages (far field) or targets
     double *part = nullptr;
     if (!rc && (rc = salloc(&part, (size_t)split * kAccAdj * ns, s, owned))) { sfree(owned, s); return rc; }
     const float4 *srcc = srcpk, *trc2 = reinterpret_cast<const float4 *>(trec2);
-    void *fargs[] = {&srcc, &ns, &trc2, &nt, &chunk, &part, &gt, &err, &boxes, &band, &ff_order};
+    void *nfargs[] = {&srcc, &ns, &trc2, &nt, &chunk, &part, &gt, &err, &band};
+    void *ffargs[] = {&srcc, &ns, &trc2, &nstage, &chunk, &nt, &part, &err, &band, &ff_order};
     timing_mark(s, true);
-    if (!rc) rc = launch(fk, dim3((unsigned)nsb, (unsigned)split), dim3(kThreadsA), fargs, smem2, s);
+    if (!rc) rc = launch(fk, dim3((unsigned)nsb, (unsigned)split), dim3((unsigned)threads), far ? ffargs : nfargs,
+                         smem2, s);
     timing_mark(s, false);
     if (!rc && band.count) {
         // the near-tangent pairs, decided and summed in FP64 into chunk 0 (and gt)

@@ -81,10 +81,9 @@ constexpr int kMinBlocksA2 = PO_MINB_A2;
 #define PO_MINB_A2M 2
 #endif
 constexpr int kMinBlocksA2M = PO_MINB_A2M;
-#ifndef PO_MINB_FF
-#define PO_MINB_FF 5             // the far-field adjoint: 5 CTAs/SM hold it under 96 registers
-#endif
-constexpr int kMinBlocksFF = PO_MINB_FF;
+constexpr int kMinBlocksFA = 6, kMinBlocksFAM = 4;   // resident CTAs per SM asked of ptxas (M = 0, with M)
+constexpr int kStagesFA = 2;
+constexpr int kFFDirs = 64;   // directions per stage of the far-field adjoint
 constexpr int kUnrollF = PO_UNROLL_F;
 constexpr int kUnrollA = PO_UNROLL_A;   // target pairs per iteration of the adjoint pair loop
 constexpr int kAccAdj = 13;
@@ -208,14 +207,19 @@ void *adj_pack_tgt_d_kernel(int kind);
 void *adj_cot_kernel();
 void *adj_ehp_cot_kernel();
 void *adj_src_epilogue_kernel();
-// Pair-packed adjoint: near field fused (currents, source and target
-// displacement), far field (currents, source displacement).
+// Far-field adjoint (po_ff_adjoint.cu): stages of kFFDirs packed directions.
+void *ff_pack_cot_kernel();
+void *ff_adj_kernel(int t_sign, bool has_m, bool want_d);
+int ff_adj_smem_bytes(bool want_d);
+int ff_adj_threads();
+int ff_adj_stage4();   // float4 per stage
+// Pair-packed adjoint, near field and scalar, fused: currents, source and
+// target displacement.
 void *adj_pk_kernel(int kind, int t_sign, bool has_m, bool want_d, bool want_t);
 void *adj_pack_tgt2_kernel();
-int adj_pk_smem_bytes(int kind, bool has_m, bool want_t);
+int adj_pk_smem_bytes(bool has_m, bool want_t);
 int adj_pk_pairs_per_tile();
-int adj_pk_rec4(int kind, bool has_m, bool want_t);   // float4 per pair-packed cotangent record
-void *adj_tgt_box_kernel();   // far-field cotangent tiles: direction boxes for the lit-tile proof
+int adj_pk_rec4(bool has_m, bool want_t);   // float4 per pair-packed cotangent record
 void *adj_tgt_epilogue_kernel();
 
 }  // namespace po
