@@ -40,66 +40,18 @@ namespace po {
 
 // ------------------------------------------------------- cotangent mapping
 
-// Cotangents of the mode's output rows -> (gE, gH) per target (near field)
-// or (gS_J, gS_M) (far field), as 12 double rows (re xyz, im xyz, ...).
+// The mapping itself is cot_map (po_device.cuh); this kernel serves the FP64
+// path, the mixed paths map while they pack (po_adj_pack_kernel below,
+// po_ff_pack_cot_kernel).
 __global__ void po_adj_cot_kernel(int mode, long nt, const double *__restrict__ cot, const double *__restrict__ tgt7,
                                   double t, double *__restrict__ gam)
 {
     const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nt) return;
-    double ge[6] = {0, 0, 0, 0, 0, 0}, gh[6] = {0, 0, 0, 0, 0, 0};
-    auto row = [&](int r) { return cot[(long)r * nt + i]; };
-    if (mode == kEH || mode == kFF) {
-        for (int c = 0; c < 6; ++c) {
-            ge[c] = row(c);
-            gh[c] = row(6 + c);
-        }
-    }
-    if (mode == kScalar) {   // (re, im) of the one complex output, in the E.x slot
-        ge[0] = row(0);
-        ge[3] = row(1);
-    }
-    if (mode == kJMEH) {
-        for (int c = 0; c < 6; ++c) {
-            ge[c] = row(12 + c);
-            gh[c] = row(18 + c);
-        }
-    }
-    if (mode == kJM || mode == kJMEH) {
-        // J = 2 n x H  ->  gH += 2 gJ x n
-        const double n[3] = {tgt7[3 * nt + i], tgt7[4 * nt + i], tgt7[5 * nt + i]};
-        for (int part_ = 0; part_ < 2; ++part_) {
-            const double g[3] = {row(3 * part_ + 0), row(3 * part_ + 1), row(3 * part_ + 2)};
-            gh[3 * part_ + 0] += 2.0 * (g[1] * n[2] - g[2] * n[1]);
-            gh[3 * part_ + 1] += 2.0 * (g[2] * n[0] - g[0] * n[2]);
-            gh[3 * part_ + 2] += 2.0 * (g[0] * n[1] - g[1] * n[0]);
-        }
-    }
-    if (mode == kFF) {
-        // gS_J = P gE + t r x gH ; gS_M = P gH - t r x gE
-        const double th = tgt7[i], ph = tgt7[nt + i];
-        const double r[3] = {cos(ph) * sin(th), sin(ph) * sin(th), cos(th)};
-        double sj[6], sm[6];
-        for (int part_ = 0; part_ < 2; ++part_) {
-            const double *e = ge + 3 * part_, *h = gh + 3 * part_;
-            const double ed = e[0] * r[0] + e[1] * r[1] + e[2] * r[2];
-            const double hd = h[0] * r[0] + h[1] * r[1] + h[2] * r[2];
-            const double rxh[3] = {r[1] * h[2] - r[2] * h[1], r[2] * h[0] - r[0] * h[2], r[0] * h[1] - r[1] * h[0]};
-            const double rxe[3] = {r[1] * e[2] - r[2] * e[1], r[2] * e[0] - r[0] * e[2], r[0] * e[1] - r[1] * e[0]};
-            for (int c = 0; c < 3; ++c) {
-                sj[3 * part_ + c] = e[c] - ed * r[c] + t * rxh[c];
-                sm[3 * part_ + c] = h[c] - hd * r[c] - t * rxe[c];
-            }
-        }
-        for (int c = 0; c < 6; ++c) {
-            ge[c] = sj[c];
-            gh[c] = sm[c];
-        }
-    }
-    for (int c = 0; c < 6; ++c) {
-        gam[(long)c * nt + i] = ge[c];
-        gam[(long)(6 + c) * nt + i] = gh[c];
-    }
+    double g[12], r[3] = {0, 0, 0};
+    if (mode == kFF) ff_direction_d(tgt7, nt, i, r);
+    cot_map(mode, i, nt, cot, tgt7, r, t, g);
+    for (int q = 0; q < 12; ++q) gam[(long)q * nt + i] = g[q];
 }
 
 // EHP: the outputs are a pointwise nonlinear function of the incident E, H at
@@ -128,55 +80,172 @@ __global__ void po_adj_ehp_cot_kernel(long nt, const double *__restrict__ cot, c
 // ---------------------------------------------------------------- epilogues
 
 // Sums the chunks of the source-side partials; unfolds the currents by
-// conj(fac * weight * area); scales the displacement term to mm.
-__global__ void po_adj_src_epilogue_kernel(int kind, int nsplit, long ns, const double *__restrict__ part,
-                                           const double *__restrict__ src7, int gmode, int ncx, int ncy,
-                                           double fac_re, double fac_im, double dscale,
-                                           double *__restrict__ grad_cur, double *__restrict__ grad_ds)
+// conj(fac * weight * area); scales the displacement term to mm. G threads
+// share a source (thread g adds chunks g, g + G, ..., then a tree), as in the
+// forward's epilogue. The blocks past the sources scale the target sums gt
+// into grad_dt.
+template <int G>
+__global__ void __launch_bounds__(kEpiThreads)
+po_adj_epilogue_kernel(int kind, int nsplit, long ns, const double *__restrict__ part,
+                       const double *__restrict__ src7, int gmode, int ncx, int ncy, double fac_re, double fac_im,
+                       double dscale, double *__restrict__ grad_cur, double *__restrict__ grad_ds, long nt,
+                       const double *__restrict__ gt, double tscale, double *__restrict__ grad_dt)
 {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ns) return;
-    double a[kAccAdj];
-    for (int q = 0; q < kAccAdj; ++q) a[q] = 0.0;
-    for (int s = 0; s < nsplit; ++s)
-        for (int q = 0; q < kAccAdj; ++q) a[q] += part[((long)s * kAccAdj + q) * ns + i];
-    double w = src7[6 * ns + i];
-    if (gmode >= 0) {
-        const long xu = i / ncy, yv = i - xu * ncy;
-        if (xu == 0 || xu == ncx - 1) w *= 0.5;
-        if (gmode != 1 && (yv == 0 || yv == ncy - 1)) w *= 0.5;
+    constexpr int SB = kEpiThreads / G;   // sources per block
+    __shared__ double sh[G > 1 ? G / 2 : 1][G > 1 ? kAccAdj : 1][G > 1 ? SB : 1];
+    pdl_wait();
+    const long nblk_s = (ns + SB - 1) / SB;
+    if ((long)blockIdx.x >= nblk_s) {
+        const long j = ((long)blockIdx.x - nblk_s) * kEpiThreads + threadIdx.x;
+        if (j < nt) grad_dt[j] = tscale * gt[j];
+        return;
     }
+    const int sl = threadIdx.x % SB, g = threadIdx.x / SB;
+    const long i = (long)blockIdx.x * SB + sl;
+    double a[kAccAdj];
+#pragma unroll
+    for (int q = 0; q < kAccAdj; ++q) a[q] = 0.0;
+    if (i < ns) {
+#pragma unroll 2
+        for (int s = g; s < nsplit; s += G)
+#pragma unroll
+            for (int q = 0; q < kAccAdj; ++q) a[q] += part[((long)s * kAccAdj + q) * ns + i];
+    }
+    if constexpr (G > 1) {
+#pragma unroll
+        for (int w = G / 2; w > 0; w >>= 1) {
+            if (g >= w && g < 2 * w)
+#pragma unroll
+                for (int q = 0; q < kAccAdj; ++q) sh[g - w][q][sl] = a[q];
+            __syncthreads();
+            if (g < w)
+#pragma unroll
+                for (int q = 0; q < kAccAdj; ++q) a[q] += sh[g][q][sl];
+            __syncthreads();
+        }
+        if (g > 0) return;
+    }
+    if (i >= ns) return;
+    const double w = trap_weight(i, gmode, ncx, ncy) * src7[6 * ns + i];
     const double fr = fac_re * w, fi = fac_im * w;
     if (grad_cur && kind == kKindScalar) {
         // conj(f) * (re + j im), two rows
         grad_cur[i] = fr * a[0] + fi * a[3];
         grad_cur[ns + i] = fr * a[3] - fi * a[0];
     } else if (grad_cur)
-        for (int g = 0; g < 2; ++g)
+        for (int h = 0; h < 2; ++h)
             for (int c = 0; c < 3; ++c) {
-                const double re = a[6 * g + c], im = a[6 * g + 3 + c];
+                const double re = a[6 * h + c], im = a[6 * h + 3 + c];
                 // conj(f) * (re + j im)
-                grad_cur[(long)(6 * g + c) * ns + i] = fr * re + fi * im;
-                grad_cur[(long)(6 * g + 3 + c) * ns + i] = fr * im - fi * re;
+                grad_cur[(long)(6 * h + c) * ns + i] = fr * re + fi * im;
+                grad_cur[(long)(6 * h + 3 + c) * ns + i] = fr * im - fi * re;
             }
     if (grad_ds) grad_ds[i] = dscale * a[12];
 }
 
-__global__ void po_adj_tgt_epilogue_kernel(int nsplit, long nt, const double *__restrict__ part, double dscale,
-                                           double *__restrict__ grad_dt)
+// -------------------------------------------------------------------- packing
+
+// Set-up of the near-field and scalar adjoint. Blocks 0 .. sblk-1: one source
+// a thread, as the one-source records of the pair kernel, 6 float4 (kRec):
+//   r0 = (sh.x, sh.y, sh.z, n.x)     hi position (turns), normal x
+//   r1 = (sl.x, sl.y, sl.z, n.y)     lo position (turns), normal y
+//   r2 = (Jx.re, Jx.im, Jy.re, Jy.im)
+//   r3 = (Jz.re, Jz.im, Mx.re, Mx.im)
+//   r4 = (My.re, My.im, Mz.re, Mz.im)
+//   r5 = (n.z, 0, 0, 0)
+// (scalar: S' in the J.x slot, the rest zero); fac: complex factor folded into
+// the currents (times weight * area). The remaining blocks: a target each
+// thread (an odd count's last pair padded with the last target carrying no
+// cotangent): its cotangents mapped onto E and H, written to gam (unless null)
+// for the near-tangent pairs and into the pair-packed records (layout in
+// po_adjoint_pk.cu, rec4 float4 per pair); its sum gt cleared.
+__global__ void __launch_bounds__(128)
+po_adj_pack_kernel(long ns, const double *__restrict__ src7, const double *__restrict__ cur, int gmode, int ncx,
+                   int ncy, const Frame *__restrict__ frp, double fac_re, double fac_im, int scalar, long sblk,
+                   float4 *__restrict__ src, int mode, long nt, const double *__restrict__ tgt7,
+                   const double *__restrict__ cot, double t, double *__restrict__ gam, int rec4,
+                   float *__restrict__ tgt, double *__restrict__ gt)
 {
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nt) return;
-    double s = 0.0;
-    for (int c = 0; c < nsplit; ++c) s += part[(long)c * nt + i];
-    grad_dt[i] = dscale * s;
+    pdl_wait();
+    const Frame fr = *frp;
+    if ((long)blockIdx.x < sblk) {
+        const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+        if (i >= ns) return;
+        float h[3], l[3];
+        for (int c = 0; c < 3; ++c) split_hi_lo((src7[c * ns + i] - fr.o[c]) * fr.kappa, fr, h[c], l[c]);
+        const double w = trap_weight(i, gmode, ncx, ncy) * src7[6 * ns + i];
+        const double fr_ = fac_re * w, fi_ = fac_im * w;
+        float c[12];   // J.re/im x y z interleaved, then M
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const int grp = q / 3, ax = q % 3;
+            if (scalar && q > 0) {
+                c[2 * q] = c[2 * q + 1] = 0.f;
+                continue;
+            }
+            const double re = cur[scalar ? i : (grp * 6 + ax) * ns + i];
+            const double im = cur[scalar ? ns + i : (grp * 6 + 3 + ax) * ns + i];
+            c[2 * q] = (float)(fr_ * re - fi_ * im);
+            c[2 * q + 1] = (float)(fr_ * im + fi_ * re);
+        }
+        float4 *o = src + (size_t)kRec * i;
+        o[0] = make_float4(h[0], h[1], h[2], (float)src7[3 * ns + i]);
+        o[1] = make_float4(l[0], l[1], l[2], (float)src7[4 * ns + i]);
+        o[2] = make_float4(c[0], c[1], c[2], c[3]);
+        o[3] = make_float4(c[4], c[5], c[6], c[7]);
+        o[4] = make_float4(c[8], c[9], c[10], c[11]);
+        o[5] = make_float4((float)src7[5 * ns + i], 0.f, 0.f, 0.f);
+        pdl_trigger();
+        return;
+    }
+    const long i = ((long)blockIdx.x - sblk) * blockDim.x + threadIdx.x;
+    if (i >= 2 * ((nt + 1) / 2)) return;
+    const bool real = i < nt;
+    const long k = real ? i : nt - 1;
+    float v[26];
+    for (int c = 0; c < 3; ++c) split_hi_lo((tgt7[c * nt + k] - fr.o[c]) * fr.kappa, fr, v[c], v[3 + c]);
+    double g[12], n[3];   // gE re xyz, im xyz, gH likewise
+    for (int q = 0; q < 12; ++q) g[q] = 0.0;
+    for (int c = 0; c < 3; ++c) n[c] = 0.0;
+    if (real) {
+        cot_map(mode, k, nt, cot, tgt7, n, t, g);
+        if (gam)
+            for (int q = 0; q < 12; ++q) gam[(long)q * nt + k] = g[q];
+        for (int c = 0; c < 3; ++c) n[c] = tgt7[(3 + c) * nt + k];
+        if (gt) gt[k] = 0.0;
+    }
+#pragma unroll
+    for (int w = 0; w < 2; ++w) {
+        const double *gw = g + 6 * w;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            v[6 + 6 * w + 2 * c] = (float)gw[c];
+            v[7 + 6 * w + 2 * c] = (float)gw[3 + c];
+        }
+        // a = conj(gE), b = conj(gH): a.n | b.n
+        const double dr = gw[0] * n[0] + gw[1] * n[1] + gw[2] * n[2];
+        const double di = -(gw[3] * n[0] + gw[4] * n[1] + gw[5] * n[2]);
+        v[21 + 2 * w] = (float)dr;
+        v[22 + 2 * w] = (float)di;
+    }
+    for (int c = 0; c < 3; ++c) v[18 + c] = (float)n[c];
+    v[25] = 0.f;
+    float *o = tgt + (i >> 1) * (long)(rec4 * 4) + (i & 1);
+#pragma unroll
+    for (int q = 0; q < 26; ++q)
+        if (q < 2 * rec4) o[2 * q] = v[q];
+    pdl_trigger();
 }
 
 // ----------------------------------------------------------- instantiations
 
 void *adj_cot_kernel() { return reinterpret_cast<void *>(&po_adj_cot_kernel); }
 void *adj_ehp_cot_kernel() { return reinterpret_cast<void *>(&po_adj_ehp_cot_kernel); }
-void *adj_src_epilogue_kernel() { return reinterpret_cast<void *>(&po_adj_src_epilogue_kernel); }
-void *adj_tgt_epilogue_kernel() { return reinterpret_cast<void *>(&po_adj_tgt_epilogue_kernel); }
+void *adj_pack_kernel() { return reinterpret_cast<void *>(&po_adj_pack_kernel); }
+void *adj_epilogue_kernel(int groups)
+{
+    return groups == 8 ? reinterpret_cast<void *>(&po_adj_epilogue_kernel<8>)
+                       : reinterpret_cast<void *>(&po_adj_epilogue_kernel<1>);
+}
 
 }  // namespace po

@@ -47,44 +47,6 @@ constexpr int kSegs = kThreadsA / kFlush;   // threads summing one target pair
 static_assert(kThreadsA == 128 && (kFlush == 16 || kFlush == 32),
               "the transpose maps 128 threads onto 16 pairs x 8 segments or 32 pairs x 4");
 
-__global__ void po_adj_pack_tgt2_kernel(long nt, const double *__restrict__ tgt7, const double *__restrict__ gam,
-                                        const Frame *__restrict__ frp, int rec4, float *__restrict__ out)
-{
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long np = (nt + 1) / 2;
-    if (i >= 2 * np) return;
-    const long k = i < nt ? i : nt - 1;
-    const bool real = i < nt;
-    const Frame fr = *frp;
-    float v[26];
-    for (int c = 0; c < 3; ++c) split_hi_lo((tgt7[c * nt + k] - fr.o[c]) * fr.kappa, fr, v[c], v[3 + c]);
-    double ge[6], gh[6], n[3];   // (re, im) x y z
-    for (int c = 0; c < 3; ++c) {
-        ge[2 * c] = real ? gam[c * nt + k] : 0.0;
-        ge[2 * c + 1] = real ? gam[(3 + c) * nt + k] : 0.0;
-        gh[2 * c] = real ? gam[(6 + c) * nt + k] : 0.0;
-        gh[2 * c + 1] = real ? gam[(9 + c) * nt + k] : 0.0;
-        n[c] = real ? tgt7[(3 + c) * nt + k] : 0.0;
-    }
-    for (int q = 0; q < 6; ++q) {
-        v[6 + q] = (float)ge[q];
-        v[12 + q] = (float)gh[q];
-    }
-    // a = conj(gE), b = conj(gH): a.n and b.n
-    for (int w = 0; w < 2; ++w) {
-        const double *g = w == 0 ? ge : gh;
-        const double dr = g[0] * n[0] + g[2] * n[1] + g[4] * n[2];
-        const double di = -(g[1] * n[0] + g[3] * n[1] + g[5] * n[2]);
-        const int dot_at = w == 0 ? 21 : 23;   // a.n | b.n
-        v[dot_at] = (float)dr;
-        v[dot_at + 1] = (float)di;
-    }
-    for (int c = 0; c < 3; ++c) v[18 + c] = (float)n[c];
-    v[25] = 0.f;
-    float *o = out + (i >> 1) * (long)(rec4 * 4) + (i & 1);
-    for (int q = 0; q < 2 * rec4; ++q) o[2 * q] = v[q];
-}
-
 // Per-thread constants of the thread's source (forward-packed record).
 struct SrcC {
     float sh[3], sl[3], n[3];
@@ -353,6 +315,7 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
     constexpr int NL = 2 * RT;                    // float2 slots read per pair
     extern __shared__ __align__(128) float4 stage[];   // kStages * kPairsA2 * RT, lo, transpose buffer
     __shared__ __align__(8) uint64_t full[kStages];
+    pdl_wait();
     float *lo = reinterpret_cast<float *>(stage + (size_t)kStages * kPairsA2 * RT);
     float2 *vbuf = reinterpret_cast<float2 *>(lo + kAccAdj * kThreadsA);   // [kFlush][kThreadsA]
 
@@ -486,6 +449,7 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
         __syncthreads();
         if (threadIdx.x == 0 && it + kStages < ntiles) issue(it + kStages);
     }
+    pdl_trigger();
     if (si >= ns) return;
 #pragma unroll
     for (int a = 0; a < kAccAdj; ++a)
@@ -525,7 +489,5 @@ void *adj_pk_kernel(int kind, int t_sign, bool has_m, bool want_d, bool want_t)
     if (t_sign < 0) return has_m ? adj_pk_sel<-1, true>(kind, want_d, want_t) : adj_pk_sel<-1, false>(kind, want_d, want_t);
     return has_m ? adj_pk_sel<1, true>(kind, want_d, want_t) : adj_pk_sel<1, false>(kind, want_d, want_t);
 }
-
-void *adj_pack_tgt2_kernel() { return reinterpret_cast<void *>(&po_adj_pack_tgt2_kernel); }
 
 }  // namespace po

@@ -65,7 +65,7 @@ __device__ __forceinline__ void fence_proxy_async()
 // many blocks, it has the next kernel's few blocks placed on whichever SMs
 // are free at that moment instead of one to an SM (161,202 sources -> 25
 // targets: the 158 blocks of the pair kernel took 142 us alone and the call
-// 380 us).
+// 380 us; an epilogue of 333 blocks that reads 570 MB took 0.25 ms longer).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
@@ -280,6 +280,50 @@ __device__ __forceinline__ void ff_direction_d(const double *tgt7, long nt, long
     p[0] = cos(ph) * sin(th);
     p[1] = sin(ph) * sin(th);
     p[2] = cos(th);
+}
+
+// Cotangents of the mode's output rows of target i -> g: (gE, gH) (near
+// field) or (gS_J, gS_M) (far field, r its direction) as re xyz, im xyz of
+// each; the scalar kind's (re, im) in the E.x slot.
+__device__ __forceinline__ void cot_map(int mode, long i, long nt, const double *cot, const double *tgt7,
+                                        const double *r, double t, double *g)
+{
+    auto row = [&](int q) { return cot[(long)q * nt + i]; };
+    double *ge = g, *gh = g + 6;
+    for (int c = 0; c < 12; ++c) g[c] = 0.0;
+    if (mode == kEH || mode == kFF)
+        for (int c = 0; c < 12; ++c) g[c] = row(c);
+    if (mode == kScalar) {
+        ge[0] = row(0);
+        ge[3] = row(1);
+    }
+    if (mode == kJMEH)
+        for (int c = 0; c < 12; ++c) g[c] = row(12 + c);
+    if (mode == kJM || mode == kJMEH) {
+        // J = 2 n x H  ->  gH += 2 gJ x n
+        const double n[3] = {tgt7[3 * nt + i], tgt7[4 * nt + i], tgt7[5 * nt + i]};
+        for (int p = 0; p < 2; ++p) {
+            const double j[3] = {row(3 * p + 0), row(3 * p + 1), row(3 * p + 2)};
+            gh[3 * p + 0] += 2.0 * (j[1] * n[2] - j[2] * n[1]);
+            gh[3 * p + 1] += 2.0 * (j[2] * n[0] - j[0] * n[2]);
+            gh[3 * p + 2] += 2.0 * (j[0] * n[1] - j[1] * n[0]);
+        }
+    }
+    if (mode == kFF) {
+        // gS_J = P gE + t r x gH ; gS_M = P gH - t r x gE
+        for (int p = 0; p < 2; ++p) {
+            double *e = ge + 3 * p, *h = gh + 3 * p;
+            const double ed = e[0] * r[0] + e[1] * r[1] + e[2] * r[2];
+            const double hd = h[0] * r[0] + h[1] * r[1] + h[2] * r[2];
+            const double rxh[3] = {r[1] * h[2] - r[2] * h[1], r[2] * h[0] - r[0] * h[2], r[0] * h[1] - r[1] * h[0]};
+            const double rxe[3] = {r[1] * e[2] - r[2] * e[1], r[2] * e[0] - r[0] * e[2], r[0] * e[1] - r[1] * e[0]};
+            for (int c = 0; c < 3; ++c) {
+                const double sj = e[c] - ed * r[c] + t * rxh[c], sm = h[c] - hd * r[c] - t * rxe[c];
+                e[c] = sj;
+                h[c] = sm;
+            }
+        }
+    }
 }
 
 // --------------------------------------------------- EHP reflection, generic

@@ -229,22 +229,6 @@ int scratch_used(unsigned long long *bytes)
     return 0;
 }
 
-template <typename T>
-static int salloc(T **p, size_t count, cudaStream_t s, std::vector<void *> &owned)
-{
-    void *q = nullptr;
-    if (int rc = scratch_alloc(&q, count * sizeof(T), s)) return rc;
-    owned.push_back(q);
-    *p = static_cast<T *>(q);
-    return 0;
-}
-
-static void sfree(std::vector<void *> &owned, cudaStream_t s)
-{
-    for (void *q : owned) scratch_free(q, s);
-    owned.clear();
-}
-
 // Stream-ordered scratch from the library's pool: one allocation per call
 // (each costs the stream about 2 us), carved up at commit() and freed (in
 // stream order) when the call's work is queued.
@@ -434,7 +418,6 @@ int run_device(const RunArgs &a)
     double fac_re = pref, fac_im = 0.0;
     if (kind == kKindFF) { fac_re = 0.0; fac_im = -pref; }
     if (kind == kKindScalar) fac_re = -pref;
-    std::vector<void *> owned;
     int rc = 0;
     const unsigned nblk_s = (unsigned)((a.ns + 255) / 256);
     long nt = a.nt, ns = a.ns;
@@ -454,11 +437,10 @@ int run_device(const RunArgs &a)
     const long tiles = std::max(1L, (ns + kChunkD - 1) / kChunkD);
     long chunk = (tiles + nsplit - 1) / nsplit * kChunkD;
     double *srcd = nullptr, *part = nullptr;
-    if ((rc = salloc(&srcd, (size_t)std::max(ns, 1L) * rec, s, owned)) ||
-        (rc = salloc(&part, (size_t)nsplit * nacc * nt, s, owned))) {
-        sfree(owned, s);
-        return rc;
-    }
+    PoolScratch sc(s);
+    sc.get(&srcd, (size_t)std::max(ns, 1L) * rec);
+    sc.get(&part, (size_t)nsplit * nacc * nt);
+    if ((rc = sc.commit())) return rc;
     Wave64 w = wave64(k, t);
     void *pargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, (void *)&scalar, &rec, &srcd};
     if (ns > 0) rc = launch(pack_src_d_kernel(), dim3(nblk_s), dim3(256), pargs, 0, s);
@@ -468,7 +450,6 @@ int run_device(const RunArgs &a)
     timing_mark(s, false);
     int nspl = (int)nsplit;
     if (!rc) rc = launch_epilogue(mode, nacc, nspl, nt, part, tgt7, t, zeta_inv, out, s);
-    sfree(owned, s);
     return rc;
 }
 
@@ -648,16 +629,75 @@ int run_adjoint(const AdjArgs &a)
     const double *src7 = a.src7, *cur = a.cur, *tgt7 = a.tgt7, *cot = a.cot;
     double *grad_cur = a.grad_cur, *grad_ds = a.grad_ds, *grad_dt = a.grad_dt;
     const unsigned nblk_s = (unsigned)((ns + 255) / 256), nblk_t = (unsigned)((nt + 255) / 256);
-    std::vector<void *> owned;
-    int rc = 0;
-    double *gam = nullptr;
-    if ((rc = salloc(&gam, (size_t)12 * nt, s, owned))) { sfree(owned, s); return rc; }
+    const bool want_t = grad_dt != nullptr, fp64 = a.precision == 1;
+    // scalar sources: 2-row currents, S' in the record's J.x slot
+    const int scalar = kind == kKindScalar ? 1 : 0;
+
+    // ---- launch shape and scratch (one allocation)
+    // FP64: a source per thread, targets streamed. Mixed near field and scalar:
+    // the same on pairs of targets. Mixed far field: two sources per thread,
+    // stages of kFFDirs directions. All fused: currents and displacements in
+    // one pass.
+    void *fk = fp64 ? adj_fp64_kernel(kind, has_m, want_d, want_t)
+                    : (far ? ff_adj_kernel(ts, has_m, want_d) : adj_pk_kernel(kind, ts, has_m, want_d, want_t));
+    const int smem = fp64 ? 0 : (far ? ff_adj_smem_bytes(want_d) : adj_pk_smem_bytes(has_m, want_t));
+    const int threads = fp64 ? kThreadsD : (far ? ff_adj_threads() : kThreadsA);
+    const int per_block = !fp64 && far ? kTile : threads;   // sources per block
+    const long tile_t = fp64 ? kChunkD : (far ? kFFDirs : 2L * adj_pk_pairs_per_tile());
+    int occ = 1, rc = 0;
+    if ((rc = kernel_occupancy(di, fk, threads, smem, occ))) return rc;
+    const long nsb = (ns + per_block - 1) / per_block;
+    const long split = choose_split(nsb, nt, (long)di->sms * occ, partial_cap(ns, kAccAdj), tile_t);
+    const long tiles_t = std::max(1L, (nt + tile_t - 1) / tile_t);
+    const long per_chunk = (tiles_t + split - 1) / split;
+    long chunk = !fp64 && far ? per_chunk : per_chunk * tile_t;   // stages (mixed far field) or targets
+
+    PoolScratch sc(s);
+    double *gam = nullptr, *eh = nullptr, *part = nullptr, *gt = nullptr, *srcd = nullptr, *trecd = nullptr;
+    Frame *frame = nullptr;
+    float4 *srcpk = nullptr;
+    float *trec = nullptr;
+    unsigned long long *keys = nullptr;
+    int *ord = nullptr;
+    void *sort_tmp = nullptr;
+    size_t sort_bytes = 0;
+    BandList band{nullptr, nullptr, 0};   // near-tangent pairs (mixed, not the scalar kind)
+    const long npair = (nt + 1) / 2, ntile_s = (ns + kTile - 1) / kTile;
+    long nstage = (nt + kFFDirs - 1) / kFFDirs;
+    int rec = fp64_rec(kind, has_m), rec4 = far ? 0 : adj_pk_rec4(has_m, want_t);
+    sc.get(&gam, (size_t)12 * nt);
+    if (a.mode == kEHP) sc.get(&eh, (size_t)12 * nt);
+    sc.get(&part, (size_t)split * kAccAdj * ns);
+    if (want_t) sc.get(&gt, (size_t)nt);
+    if (fp64) {
+        sc.get(&srcd, (size_t)ns * rec);
+        sc.get(&trecd, (size_t)nt * adj64_rec(kind));
+    } else {
+        sc.get(&frame, 1);
+        if (kind != kKindScalar) {
+            band.cap = band_cap_for(ns, nt);
+            sc.get(&band.pairs, band.cap);
+            sc.get(&band.count, 1);
+        }
+        if (far) {
+            cudaError_t e = ff_sort(nullptr, &sort_bytes, nullptr, nullptr, nullptr, nullptr, ns, s);
+            if (e != cudaSuccess) return fail(2, std::string("sort size query: ") + err_str(e));
+            sc.get(&keys, 2 * (size_t)ns);
+            sc.get(&ord, 2 * (size_t)ns);
+            sc.take(&sort_tmp, sort_bytes);
+            sc.get(&srcpk, (size_t)ntile_s * ff_tile4(has_m));
+            sc.get(&trec, (size_t)nstage * ff_adj_stage4() * 4);
+        } else {
+            sc.get(&srcpk, (size_t)ns * kRec);
+            sc.get(&trec, (size_t)npair * rec4 * 4);
+        }
+    }
+    if ((rc = sc.commit())) return rc;
+
     if (a.mode == kEHP) {
         // EHP is nonlinear in the target's fields: the EH forward at the same
         // inputs and precision, then the EHP map's vector-Jacobian product
         // there (po_adj_ehp_cot_kernel) gives the EH adjoint's cotangents
-        double *eh = nullptr;
-        if ((rc = salloc(&eh, (size_t)12 * nt, s, owned))) { sfree(owned, s); return rc; }
         RunArgs fa = a;
         fa.mode = kEH;
         fa.out = eh;
@@ -668,181 +708,90 @@ int run_adjoint(const AdjArgs &a)
         double zi = 1.0 / std::sqrt(mu0 / (a.epsilon * (1.0 / (mu0 * c_l * c_l))));
         void *eargs[] = {&nt, &cot, &eh, &tgt7, &zi, &gam};
         if (!rc) rc = launch(adj_ehp_cot_kernel(), dim3((unsigned)((nt + 127) / 128)), dim3(128), eargs, 0, s);
-    } else {
-        void *cargs[] = {&mode, &nt, &cot, &tgt7, &t, &gam};
-        rc = launch(adj_cot_kernel(), dim3(nblk_t), dim3(256), cargs, 0, s);
-    }
-    // scalar sources: 2-row currents (FP64 record: S' in its J.x slot; mixed
-    // one-source record: the same, the other currents zero)
-    const int fp64_scalar = kind == kKindScalar ? 1 : 0, mixed_scalar = kind == kKindScalar ? 2 : 0;
-
-    if (a.precision == 1) {
-        const bool want_t = grad_dt != nullptr;
-        int rec = fp64_rec(kind, has_m);
-        void *fk = adj_fp64_kernel(kind, has_m, want_d, want_t);
-        int occ = 1;
-        if (!rc) rc = kernel_occupancy(di, fk, kThreadsD, 0, occ);
-        const long nsb = (ns + kThreadsD - 1) / kThreadsD;
-        const long nsplit = choose_split(nsb, nt, (long)di->sms * occ, partial_cap(ns, kAccAdj), kChunkD);
-        const long tiles = (nt + kChunkD - 1) / kChunkD;
-        long chunk = (tiles + nsplit - 1) / nsplit * kChunkD;
-        double *srcd = nullptr, *trec = nullptr, *part = nullptr, *gt = nullptr;
-        if (!rc && ((rc = salloc(&srcd, (size_t)ns * rec, s, owned)) ||
-                    (rc = salloc(&trec, (size_t)nt * adj64_rec(kind), s, owned)) ||
-                    (rc = salloc(&part, (size_t)nsplit * kAccAdj * ns, s, owned)) ||
-                    (want_t && (rc = salloc(&gt, (size_t)nt, s, owned))))) {
-            sfree(owned, s);
-            return rc;
-        }
-        Wave64 w = wave64(k, t);
-        void *pargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, (void *)&fp64_scalar, &rec, &srcd};
-        if (!rc) rc = launch(pack_src_d_kernel(), dim3(nblk_s), dim3(256), pargs, 0, s);
-        void *tpargs[] = {&nt, &tgt7, &gam, &trec};
-        if (!rc) rc = launch(adj_pack_tgt_d_kernel(kind), dim3(nblk_t), dim3(256), tpargs, 0, s);
-        if (want_t) PO_CK_RC(cudaMemsetAsync(gt, 0, sizeof(double) * nt, s));
-        void *sargs[] = {&srcd, &ns, &trec, &nt, &chunk, &w, &part, &gt};
-        timing_mark(s, true);
-        if (!rc) rc = launch(fk, dim3((unsigned)nsb, (unsigned)nsplit), dim3(kThreadsD), sargs, 0, s);
-        timing_mark(s, false);
-        int nspl = (int)nsplit, one = 1;
-        double dsc = far ? 1.0 : -1.0, one_d = 1.0;
-        void *eargs[] = {(void *)&kind, &nspl, &ns, &part, &src7, &gmode, &ncx, &ncy, &fac_re, &fac_im, &dsc,
-                         &grad_cur, &grad_ds};
-        if (!rc) rc = launch(adj_src_epilogue_kernel(), dim3(nblk_s), dim3(256), eargs, 0, s);
-        if (!rc && want_t) {
-            void *teargs[] = {&one, &nt, &gt, &one_d, &grad_dt};
-            rc = launch(adj_tgt_epilogue_kernel(), dim3(nblk_t), dim3(256), teargs, 0, s);
-        }
-        sfree(owned, s);
-        return rc;
-    }
-
-    // ---- mixed precision
-    Frame *frame = nullptr;
-    float4 *srcpk = nullptr;
-    if (!rc && ((rc = salloc(&frame, 1, s, owned)) ||
-                (!far && (rc = salloc(&srcpk, (size_t)ns * kRec, s, owned))))) {
-        sfree(owned, s);
-        return rc;
-    }
-    long nb = far ? 0 : nt;
-    double kap = kappa;
-    int centred = far ? 0 : 1;
-    unsigned *none = nullptr;
-    void *frargs[] = {&src7, &ns, &tgt7, &nb, &kap, &centred, &frame, &none};
-    if (!rc) rc = launch(frame_kernel(), dim3(kFrameCtas), dim3(kFrameThreads), frargs, 0, s);
-    const int *ff_order = nullptr;   // far field: curve position -> source
-    if (far) {
-        // sources in Hilbert order, in the forward's tile records: one adjoint
-        // CTA per tile, whose centre's phase goes into the cotangents
-        const long n1 = std::max(ns, 1L);
-        const long ntile = (ns + kTile - 1) / kTile;
-        size_t sort_bytes = 0;
-        unsigned long long *keys = nullptr;
-        int *ord = nullptr;
-        unsigned char *sort_tmp = nullptr;
-        float4 *tiles = nullptr;
-        cudaError_t e = ff_sort(nullptr, &sort_bytes, nullptr, nullptr, nullptr, nullptr, n1, s);
-        if (e != cudaSuccess) rc = fail(2, std::string("sort size query: ") + err_str(e));
-        if (!rc && ((rc = salloc(&keys, 2 * (size_t)n1, s, owned)) || (rc = salloc(&ord, 2 * (size_t)n1, s, owned)) ||
-                    (rc = salloc(&sort_tmp, std::max<size_t>(sort_bytes, 16), s, owned)) ||
-                    (rc = salloc(&tiles, (size_t)ntile * ff_tile4(has_m), s, owned)))) {
-            sfree(owned, s);
-            return rc;
-        }
-        unsigned long long *k_in = keys, *k_out = keys + n1;
-        int *i_in = ord, *i_out = ord + n1;
-        void *kargs[] = {&ns, &src7, &frame, &k_in, &i_in};
-        if (!rc) rc = launch(ff_key_kernel(), dim3(nblk_s), dim3(256), kargs, 0, s);
-        if (!rc) {
-            e = ff_sort(sort_tmp, &sort_bytes, k_in, k_out, i_in, i_out, ns, s);
-            if (e != cudaSuccess) rc = fail(2, std::string("source sort: ") + err_str(e));
-            else note_launches(1);
-        }
-        ff_order = i_out;
-        void *fpargs[] = {&ns, &ff_order, &src7, &cur, &gmode, &ncx, &ncy, &frame, &fac_re, &fac_im, &tiles};
-        if (!rc) rc = launch(ff_pack_kernel(has_m), dim3((unsigned)ntile), dim3(32), fpargs, 0, s);
-        srcpk = tiles;
-    } else {
-        void *psargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &frame, &fac_re, &fac_im, (void *)&mixed_scalar,
-                          &srcpk};
-        if (!rc) rc = launch(pack_src_kernel(), dim3(nblk_s), dim3(256), psargs, 0, s);
-    }
-    // Near field and scalar: a source per thread, pairs of targets streamed,
-    // fused (currents, source and target displacement in one pass). Far field:
-    // two sources per thread, stages of kFFDirs directions streamed.
-    const bool want_t = grad_dt != nullptr;
-    const int rec4 = far ? 0 : adj_pk_rec4(has_m, want_t);
-    const long npair = (nt + 1) / 2;
-    long nstage = (nt + kFFDirs - 1) / kFFDirs;
-    float *trec2 = nullptr;
-    double *gt = nullptr;
-    const size_t trec4 = far ? (size_t)nstage * ff_adj_stage4() : (size_t)npair * rec4;
-    if (!rc && ((rc = salloc(&trec2, trec4 * 4, s, owned)) || (want_t && (rc = salloc(&gt, (size_t)nt, s, owned))))) {
-        sfree(owned, s);
-        return rc;
-    }
-    if (far) {
-        void *p2args[] = {&nt, &tgt7, &gam, &trec2};
-        if (!rc) rc = launch(ff_pack_cot_kernel(), dim3((unsigned)nstage), dim3(kFFDirs), p2args, 0, s);
-    } else {
-        void *p2args[] = {&nt, &tgt7, &gam, &frame, (void *)&rec4, &trec2};
-        const unsigned nblk_p = (unsigned)((2 * npair + 255) / 256);
-        if (!rc) rc = launch(adj_pack_tgt2_kernel(), dim3(nblk_p), dim3(256), p2args, 0, s);
-    }
-    if (want_t) PO_CK_RC(cudaMemsetAsync(gt, 0, sizeof(double) * nt, s));
-    BandList band{nullptr, nullptr, 0};   // near-tangent pairs (not the scalar kind)
-    if (!rc && kind != kKindScalar) {
-        band.cap = band_cap_for(ns, nt);
-        if ((rc = salloc(&band.pairs, band.cap, s, owned)) || (rc = salloc(&band.count, 1, s, owned))) {
-            sfree(owned, s);
-            return rc;
-        }
-        PO_CK_RC(cudaMemsetAsync(band.count, 0, sizeof(unsigned), s));
-    }
-    void *fk = far ? ff_adj_kernel(ts, has_m, want_d) : adj_pk_kernel(kind, ts, has_m, want_d, want_t);
-    const int smem2 = far ? ff_adj_smem_bytes(want_d) : adj_pk_smem_bytes(has_m, want_t);
-    const int threads = far ? ff_adj_threads() : kThreadsA;
-    int occ2 = 1;
-    if (!rc) rc = kernel_occupancy(di, fk, threads, smem2, occ2);
-    const long tile_t = far ? kFFDirs : 2L * adj_pk_pairs_per_tile();
-    const long nsb = far ? (ns + kTile - 1) / kTile : (ns + kThreadsA - 1) / kThreadsA;
-    const long split = choose_split(nsb, nt, (long)di->sms * occ2, partial_cap(ns, kAccAdj), tile_t);
-    const long tiles = std::max(1L, (nt + tile_t - 1) / tile_t);
-    long chunk = (tiles + split - 1) / split * (far ? 1 : tile_t);   // stages (far field) or targets
-    double *part = nullptr;
-    if (!rc && (rc = salloc(&part, (size_t)split * kAccAdj * ns, s, owned))) { sfree(owned, s); return rc; }
-    const float4 *srcc = srcpk, *trc2 = reinterpret_cast<const float4 *>(trec2);
-    void *nfargs[] = {&srcc, &ns, &trc2, &nt, &chunk, &part, &gt, &err, &band};
-    void *ffargs[] = {&srcc, &ns, &trc2, &nstage, &chunk, &nt, &part, &err, &band, &ff_order};
-    timing_mark(s, true);
-    if (!rc) rc = launch(fk, dim3((unsigned)nsb, (unsigned)split), dim3((unsigned)threads), far ? ffargs : nfargs,
-                         smem2, s);
-    timing_mark(s, false);
-    if (!rc && band.count) {
-        // the near-tangent pairs, decided and summed in FP64 into chunk 0 (and gt)
-        double inv_kappa = 1.0 / kappa;
-        Wave64 w = wave64(k, t);
-        void *xargs[] = {&band, &ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, &nt, &tgt7, &gam, &w,
-                         &inv_kappa, &part, &gt, &err};
-        rc = launch(adj_band_fixup_kernel(kind, want_t), dim3(kFixupBlocks), dim3(256), xargs, 0, s);
+        mode = kEH;
+        cot = gam;
     }
     int nspl = (int)split;
-    double dsc = far ? kappa : -kappa;
-    void *eargs[] = {(void *)&kind, &nspl, &ns, &part, &src7, &gmode, &ncx, &ncy, &fac_re, &fac_im, &dsc,
-                     &grad_cur, &grad_ds};
-    if (!rc) rc = launch(adj_src_epilogue_kernel(), dim3(nblk_s), dim3(256), eargs, 0, s);
-    if (!rc && want_t) {
-        int one = 1;
-        double dsct = kappa;
-        void *teargs[] = {&one, &nt, &gt, &dsct, &grad_dt};
-        rc = launch(adj_tgt_epilogue_kernel(), dim3(nblk_t), dim3(256), teargs, 0, s);
+    double dsc = 1.0, tsc = 1.0;   // gradient per mm from the kernels' units
+    const int *ff_order = nullptr;   // far field: curve position -> source
+
+    if (fp64) {
+        dsc = far ? 1.0 : -1.0;
+        if (a.mode != kEHP) {
+            void *cargs[] = {&mode, &nt, &cot, &tgt7, &t, &gam};
+            if (!rc) rc = launch(adj_cot_kernel(), dim3(nblk_t), dim3(256), cargs, 0, s);
+        }
+        Wave64 w = wave64(k, t);
+        void *pargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, (void *)&scalar, &rec, &srcd};
+        if (!rc) rc = launch(pack_src_d_kernel(), dim3(nblk_s), dim3(256), pargs, 0, s);
+        void *tpargs[] = {&nt, &tgt7, &gam, &trecd};
+        if (!rc) rc = launch(adj_pack_tgt_d_kernel(kind), dim3(nblk_t), dim3(256), tpargs, 0, s);
+        if (want_t) PO_CK_RC(cudaMemsetAsync(gt, 0, sizeof(double) * nt, s));
+        void *sargs[] = {&srcd, &ns, &trecd, &nt, &chunk, &w, &part, &gt};
+        timing_mark(s, true);
+        if (!rc) rc = launch(fk, dim3((unsigned)nsb, (unsigned)split), dim3((unsigned)threads), sargs, 0, s);
+        timing_mark(s, false);
+    } else {
+        dsc = far ? kappa : -kappa;
+        tsc = kappa;
+        long nb = far ? 0 : nt;
+        double kap = kappa;
+        int centred = far ? 0 : 1;
+        void *frargs[] = {&src7, &ns, &tgt7, &nb, &kap, &centred, &frame, &band.count};
+        if (!rc) rc = launch(frame_kernel(), dim3(kFrameCtas), dim3(kFrameThreads), frargs, 0, s);
+        if (far) {
+            // sources in Hilbert order, in the forward's tile records: one adjoint
+            // CTA per tile, whose centre's phase goes into the cotangents
+            void *p2args[] = {&nt, &tgt7, &cot, &t, &gam, &trec};
+            if (!rc) rc = launch_pdl(ff_pack_cot_kernel(), dim3((unsigned)nstage), dim3(kFFDirs), p2args, 0, s);
+            unsigned long long *k_in = keys, *k_out = keys + ns;
+            int *i_in = ord, *i_out = ord + ns;
+            void *kargs[] = {&ns, &src7, &frame, &k_in, &i_in};
+            if (!rc) rc = launch_pdl(ff_key_kernel(), dim3(nblk_s), dim3(256), kargs, 0, s);
+            if (!rc) {
+                cudaError_t e = ff_sort(sort_tmp, &sort_bytes, k_in, k_out, i_in, i_out, ns, s);
+                if (e != cudaSuccess) rc = fail(2, std::string("source sort: ") + err_str(e));
+                else note_launches(1);
+            }
+            ff_order = i_out;
+            void *fpargs[] = {&ns, &ff_order, &src7, &cur, &gmode, &ncx, &ncy, &frame, &fac_re, &fac_im, &srcpk};
+            if (!rc) rc = launch(ff_pack_kernel(has_m), dim3((unsigned)ntile_s), dim3(32), fpargs, 0, s);
+        } else {
+            long sblk = (ns + 127) / 128;
+            double *gam_out = a.mode == kEHP ? nullptr : gam;   // EHP: the cotangents are gam already
+            void *pargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &frame, &fac_re, &fac_im, (void *)&scalar, &sblk,
+                             &srcpk, &mode, &nt, &tgt7, &cot, &t, &gam_out, &rec4, &trec, &gt};
+            if (!rc) rc = launch_pdl(adj_pack_kernel(), dim3((unsigned)(sblk + (2 * npair + 127) / 128)), dim3(128),
+                                     pargs, 0, s);
+        }
+        const float4 *srcc = srcpk, *trc = reinterpret_cast<const float4 *>(trec);
+        void *nfargs[] = {&srcc, &ns, &trc, &nt, &chunk, &part, &gt, &err, &band};
+        void *ffargs[] = {&srcc, &ns, &trc, &nstage, &chunk, &nt, &part, &err, &band, &ff_order};
+        timing_mark(s, true);
+        if (!rc) rc = launch_pdl(fk, dim3((unsigned)nsb, (unsigned)split), dim3((unsigned)threads),
+                                 far ? ffargs : nfargs, smem, s);
+        timing_mark(s, false);
+        if (!rc && band.count) {
+            // the near-tangent pairs, decided and summed in FP64 into chunk 0 (and gt)
+            double inv_kappa = 1.0 / kappa;
+            Wave64 w = wave64(k, t);
+            void *xargs[] = {&band, &ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, &nt, &tgt7, &gam, &w,
+                             &inv_kappa, &part, &gt, &err};
+            rc = launch_pdl(adj_band_fixup_kernel(kind, want_t), dim3(kFixupBlocks), dim3(256), xargs, 0, s);
+        }
     }
-    if (!rc && a.extent_host) PO_CK_RC(cudaMemcpyAsync(a.extent_host, &frame->m, sizeof(double),
-                                                       cudaMemcpyDeviceToHost, s));
+    long nt_e = want_t ? nt : 0;
+    const int groups = nspl >= 8 && ns <= 152L * kEpiThreads ? 8 : 1;   // fewer blocks than SMs: share the chunks
+    const long per = kEpiThreads / groups;
+    void *eargs[] = {(void *)&kind, &nspl, &ns, &part, &src7, &gmode, &ncx, &ncy, &fac_re, &fac_im, &dsc,
+                     &grad_cur, &grad_ds, &nt_e, &gt, &tsc, &grad_dt};
+    if (!rc) rc = launch_pdl(adj_epilogue_kernel(groups),
+                             dim3((unsigned)((ns + per - 1) / per + (nt_e + kEpiThreads - 1) / kEpiThreads)),
+                             dim3(kEpiThreads), eargs, 0, s);
+    if (!rc && a.extent_host && frame) PO_CK_RC(cudaMemcpyAsync(a.extent_host, &frame->m, sizeof(double),
+                                                                cudaMemcpyDeviceToHost, s));
     if (!rc && a.band_host && band.count)
         PO_CK_RC(cudaMemcpyAsync(a.band_host, band.count, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
-    sfree(owned, s);
     return rc;
 }
 

@@ -53,18 +53,23 @@ __host__ __device__ constexpr int dir_slot(int d) { return (d & 1) * kHalf + (d 
 
 }  // namespace
 
-// One CTA per stage. The last stage is filled up with copies of the last
-// direction carrying no cotangent.
+// One CTA per stage: the directions, and their cotangents mapped onto S_J and
+// S_M (also written to gam for the near-tangent pairs). The last stage is
+// filled up with copies of the last direction carrying no cotangent.
 __global__ void __launch_bounds__(kFFDirs)
-po_ff_pack_cot_kernel(long nt, const double *__restrict__ tgt7, const double *__restrict__ gam,
-                      float4 *__restrict__ out)
+po_ff_pack_cot_kernel(long nt, const double *__restrict__ tgt7, const double *__restrict__ cot, double t,
+                      double *__restrict__ gam, float4 *__restrict__ out)
 {
     __shared__ __align__(16) float buf[kStage4 * 4];
     __shared__ float wbox[kFFDirs / 32][6];
     const long i = (long)blockIdx.x * kFFDirs + threadIdx.x;
     const long k = i < nt ? i : nt - 1;
-    const double th = tgt7[k], ph = tgt7[nt + k];
-    const double rd[3] = {cos(ph) * sin(th), sin(ph) * sin(th), cos(th)};
+    pdl_wait();
+    double rd[3], gk[12];
+    ff_direction_d(tgt7, nt, k, rd);
+    cot_map(kFF, k, nt, cot, tgt7, rd, t, gk);
+    if (i < nt)
+        for (int q = 0; q < 12; ++q) gam[(long)q * nt + i] = gk[q];
     float *o = buf + (kDirHead + dir_slot(threadIdx.x) * kDirRec4) * 4;
     float v[6];
 #pragma unroll
@@ -77,8 +82,8 @@ po_ff_pack_cot_kernel(long nt, const double *__restrict__ tgt7, const double *__
         v[c] = v[3 + c] = o[c];
 #pragma unroll
         for (int g = 0; g < 2; ++g) {
-            o[3 + 6 * g + 2 * c] = i < nt ? (float)gam[(6 * g + c) * nt + k] : 0.f;
-            o[4 + 6 * g + 2 * c] = i < nt ? (float)gam[(6 * g + 3 + c) * nt + k] : 0.f;
+            o[3 + 6 * g + 2 * c] = i < nt ? (float)gk[6 * g + c] : 0.f;
+            o[4 + 6 * g + 2 * c] = i < nt ? (float)gk[6 * g + 3 + c] : 0.f;
         }
     }
     o[15] = o[22] = o[23] = 0.f;
@@ -105,6 +110,7 @@ po_ff_pack_cot_kernel(long nt, const double *__restrict__ tgt7, const double *__
     __syncthreads();
     float4 *dst = out + (size_t)blockIdx.x * kStage4;
     for (int q = threadIdx.x; q < kStage4; q += kFFDirs) dst[q] = reinterpret_cast<const float4 *>(buf)[q];
+    pdl_trigger();
 }
 
 namespace {
@@ -219,6 +225,7 @@ po_ff_adj_kernel(const float4 *__restrict__ tiles, long ns, const float4 *__rest
     constexpr bool kLit = !HAS_M;
     extern __shared__ __align__(128) float4 stage[];   // kStagesFA stages, then per thread: totals' lo, the even sums
     __shared__ __align__(8) uint64_t full[kStagesFA];
+    pdl_wait();
     float2 *keep = reinterpret_cast<float2 *>(stage + (size_t)kStagesFA * kStage4) + threadIdx.x;
     auto lo = [&](int a) -> float2 & { return keep[a * kThreadsFA]; };
     auto even = [&](int a) -> float2 & { return keep[(NA + a) * kThreadsFA]; };
@@ -358,6 +365,7 @@ po_ff_adj_kernel(const float4 *__restrict__ tiles, long ns, const float4 *__rest
         __syncthreads();
         if (threadIdx.x == 0 && it + kStagesFA < nst) issue(it + kStagesFA);
     }
+    pdl_trigger();
 #pragma unroll
     for (int l = 0; l < 2; ++l) {
         if (pos + l >= ns) continue;

@@ -287,7 +287,6 @@ po_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, cons
                      const double *__restrict__ tgt7, Wave64 w, double *__restrict__ part, int *__restrict__ err)
 {
     constexpr int REC = fp64_rec(KIND, HAS_M), NACC = KIND == kKindFF && !HAS_M ? 6 : kAcc;
-    pdl_trigger();
     pdl_wait();
     const unsigned total = *bl.count;
     if (blockIdx.x == 0 && threadIdx.x == 0 && total > bl.cap) atomicExch(err, kErrBandOverflow);
@@ -304,6 +303,7 @@ po_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, cons
         for (int a = 0; a < NACC; ++a)
             if (acc[a] != 0.0) atomicAdd(&part[(long)a * nt + pr.y], acc[a]);
     }
+    pdl_trigger();
 }
 
 // ------------------------------------------------------------------ adjoint
@@ -602,6 +602,7 @@ po_adj_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, 
                          const double *__restrict__ tgt7, const double *__restrict__ gam, Wave64 w,
                          double inv_kappa, double *__restrict__ part, double *__restrict__ gt, int *__restrict__ err)
 {
+    pdl_wait();
     const unsigned total = *bl.count;
     if (blockIdx.x == 0 && threadIdx.x == 0 && total > bl.cap) atomicExch(err, kErrBandOverflow);
     const unsigned n = min(total, bl.cap);
@@ -618,6 +619,7 @@ po_adj_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, 
         }
         if (WANT_T && v != 0.0) atomicAdd(&gt[pr.y], v);
     }
+    pdl_trigger();
 }
 
 // ---------------------------------------------------------------- host side

@@ -458,55 +458,6 @@ __global__ void po_wait_selftest_kernel(uint32_t limit, int *__restrict__ err)
     if (__syncthreads_or(!ok) && threadIdx.x == 0) atomicExch(err, kErrWaitTimeout);
 }
 
-// ------------------------------------------------------- packing (adjoint)
-
-// One-source records for the adjoint kernels (a thread owns one source),
-// 6 float4 (kRec):
-//   r0 = (sh.x, sh.y, sh.z, n.x)     hi position (turns), normal x
-//   r1 = (sl.x, sl.y, sl.z, n.y)     lo position (turns), normal y
-//   r2 = (Jx.re, Jx.im, Jy.re, Jy.im)
-//   r3 = (Jz.re, Jz.im, Mx.re, Mx.im)
-//   r4 = (My.re, My.im, Mz.re, Mz.im)
-//   r5 = (n.z, 0, 0, 0)
-// Scalar record, 2 float4 (kRecScalar): (sh, S'.re), (sl, S'.im), with
-// scalar == 1; scalar == 2 puts S' in the J.x slot of the 6-float4 record
-// (the scalar adjoint).
-// fac: complex factor folded into the currents (times weight * area).
-__global__ void po_pack_src_kernel(long ns, const double *__restrict__ src7, const double *__restrict__ cur,
-                                   int gmode, int ncx, int ncy, const Frame *__restrict__ frp, double fac_re,
-                                   double fac_im, int scalar, float4 *__restrict__ out)
-{
-    const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= ns) return;
-    const Frame fr = *frp;
-    float h[3], l[3];
-    for (int c = 0; c < 3; ++c) split_hi_lo((src7[c * ns + i] - fr.o[c]) * fr.kappa, fr, h[c], l[c]);
-    const double w = trap_weight(i, gmode, ncx, ncy) * src7[6 * ns + i];
-    const double fr_ = fac_re * w, fi_ = fac_im * w;
-    if (scalar == 1) {
-        const double re = cur[i], im = cur[ns + i];
-        out[2 * i] = make_float4(h[0], h[1], h[2], (float)(fr_ * re - fi_ * im));
-        out[2 * i + 1] = make_float4(l[0], l[1], l[2], (float)(fr_ * im + fi_ * re));
-        return;
-    }
-    float c[12];   // J.re/im x y z interleaved, then M
-    for (int q = 0; q < 6; ++q) {
-        const int grp = q / 3, ax = q % 3;
-        // scalar == 2: the 2-row scalar field S in the J.x slot, the rest zero
-        const double re = scalar ? (q == 0 ? cur[i] : 0.0) : cur[(grp * 6 + ax) * ns + i];
-        const double im = scalar ? (q == 0 ? cur[ns + i] : 0.0) : cur[(grp * 6 + 3 + ax) * ns + i];
-        c[2 * q] = (float)(fr_ * re - fi_ * im);
-        c[2 * q + 1] = (float)(fr_ * im + fi_ * re);
-    }
-    float4 *o = out + (size_t)kRec * i;
-    o[0] = make_float4(h[0], h[1], h[2], (float)src7[3 * ns + i]);
-    o[1] = make_float4(l[0], l[1], l[2], (float)src7[4 * ns + i]);
-    o[2] = make_float4(c[0], c[1], c[2], c[3]);
-    o[3] = make_float4(c[4], c[5], c[6], c[7]);
-    o[4] = make_float4(c[8], c[9], c[10], c[11]);
-    o[5] = make_float4((float)src7[5 * ns + i], 0.f, 0.f, 0.f);
-}
-
 // ------------------------------------------------------------------ epilogue
 
 __device__ __forceinline__ void cross_d(const double a[3], const double b[3], double o[3])
@@ -664,7 +615,6 @@ void *pk_kernel(int kind, int t_sign, bool has_m)
     return t_sign < 0 ? pk_ptr<kKindScalar, -1, false>() : pk_ptr<kKindScalar, 1, false>();
 }
 
-void *pack_src_kernel() { return reinterpret_cast<void *>(&po_pack_src_kernel); }
 // Precision conversions of the float drop-in ABI's buffers (n elements).
 __global__ void po_f2d_kernel(const float *__restrict__ in, double *__restrict__ out, long n)
 {

@@ -192,7 +192,6 @@ void *pk_kernel(int kind, int t_sign, bool has_m);
 void *pack_kernel(bool scalar, bool has_m);   // source tiles (near field, scalar) and targets
 void *fp64_kernel(int kind, bool has_m);
 void *frame_kernel();
-void *pack_src_kernel();
 void *pack_src_d_kernel();
 constexpr int kEpiThreads = 256;
 void *epilogue_kernel(int groups);   // 1, 8, 32 or 64 threads share a target's chunks
@@ -205,8 +204,9 @@ void *wait_selftest_kernel();
 void *adj_fp64_kernel(int kind, bool has_m, bool want_d, bool want_t);
 void *adj_pack_tgt_d_kernel(int kind);
 void *adj_cot_kernel();
+void *adj_pack_kernel();                 // near field, scalar: sources, targets and cotangents
+void *adj_epilogue_kernel(int groups);   // 1 or 8 threads share a source's chunks
 void *adj_ehp_cot_kernel();
-void *adj_src_epilogue_kernel();
 // Far-field adjoint (po_ff_adjoint.cu): stages of kFFDirs packed directions.
 void *ff_pack_cot_kernel();
 void *ff_adj_kernel(int t_sign, bool has_m, bool want_d);
@@ -216,10 +216,8 @@ int ff_adj_stage4();   // float4 per stage
 // Pair-packed adjoint, near field and scalar, fused: currents, source and
 // target displacement.
 void *adj_pk_kernel(int kind, int t_sign, bool has_m, bool want_d, bool want_t);
-void *adj_pack_tgt2_kernel();
 int adj_pk_smem_bytes(bool has_m, bool want_t);
 int adj_pk_pairs_per_tile();
 int adj_pk_rec4(bool has_m, bool want_t);   // float4 per pair-packed cotangent record
-void *adj_tgt_epilogue_kernel();
 
 }  // namespace po
