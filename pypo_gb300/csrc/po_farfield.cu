@@ -242,24 +242,20 @@ __device__ __forceinline__ void ff_band_scan(const float4 *recs, long pos0, cons
     }
 }
 
-// Grid = (direction blocks of 2 * kThreads, tile chunks). Every thread owns
-// two directions (lanes of the per-tile phase); each pair record's two
-// sources are the two lanes of every packed operation of the pair loop.
-// `boxes`: the tiles' normal boxes may prove a tile lit for the CTA's
-// directions (M = 0 kernels), which skips the per-pair illumination test.
-template <int T, bool HAS_M>
+// The kernel with magnetic currents. Grid = (direction blocks of 2 * kThreads,
+// tile chunks). Every thread owns two directions (lanes of the per-tile
+// phase); each pair record's two sources are the two lanes of every packed
+// operation of the pair loop.
+template <int T>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
 po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const float4 *__restrict__ tgt, long nt,
-             double *__restrict__ part, int *__restrict__ err, int boxes, BandList bl, long ns,
+             double *__restrict__ part, int *__restrict__ err, int, BandList bl, long ns,
              const int *__restrict__ order)
 {
-    constexpr int R4 = ff_rec4(HAS_M), T4 = ff_tile4(HAS_M), TP = 2;
-    constexpr int NA = HAS_M ? 12 : 6;   // accumulators in use: S_J (re xyz, im xyz), then S_M
-    constexpr bool kLitPath = !HAS_M;
+    constexpr int R4 = ff_rec4(true), T4 = ff_tile4(true), TP = 2;
+    constexpr int NA = 12;   // S_J (re xyz, im xyz), then S_M
     extern __shared__ __align__(128) float4 stage[];   // kStages tiles, then the compensation words
     __shared__ __align__(8) uint64_t full[kStages];
-    __shared__ float tbox_w[kThreads / 32][6];
-    __shared__ float tbox[6];
     pdl_wait();
 
     const long tbase = (long)blockIdx.x * kThreads * TP + threadIdx.x;
@@ -287,37 +283,6 @@ po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const floa
                 rl[q].y = l[q];
                 rw[q].y = f;
             }
-        }
-    }
-
-    // The CTA's box of directions (the lit-tile proof, M = 0 kernels).
-    if (kLitPath) {
-        float v[6] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
-#pragma unroll
-        for (int j = 0; j < TP; ++j) {
-            if (tbase + (long)j * kThreads >= nt) continue;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                v[c] = fminf(v[c], rf[j][c].x);
-                v[3 + c] = fmaxf(v[3 + c], rf[j][c].x);
-            }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                const float u = __shfl_xor_sync(0xffffffffu, v[q], o);
-                v[q] = q < 3 ? fminf(v[q], u) : fmaxf(v[q], u);
-            }
-        if ((threadIdx.x & 31) == 0)
-#pragma unroll
-            for (int q = 0; q < 6; ++q) tbox_w[threadIdx.x >> 5][q] = v[q];
-        __syncthreads();
-        if (threadIdx.x < 6) {
-            const int q = threadIdx.x;
-            float r = tbox_w[0][q];
-            for (int w = 1; w < kThreads / 32; ++w) r = q < 3 ? fminf(r, tbox_w[w][q]) : fmaxf(r, tbox_w[w][q]);
-            tbox[q] = r;
         }
     }
 
@@ -367,13 +332,9 @@ po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const floa
             for (int a = 0; a < NA; ++a) acc[j][a] = make_float2(0.f, 0.f);
 
         bool band = false;   // a pair of this tile fell inside the tangent band
-        // VAR 0: narrow tile proven lit (M = 0); 1: narrow tile; 2: wide tile
-        auto pairs = [&](auto var_c) {
-            constexpr int VAR = decltype(var_c)::value;
-            // float4 read per pair record: offsets and J' (and the normal
-            // unless the tile is proven lit; the lo offsets in a wide tile;
-            // M')
-            constexpr int NLD = HAS_M ? R4 : (VAR == 0 ? 5 : (VAR == 1 ? 6 : 8));
+        auto pairs = [&](auto wide_c) {
+            constexpr bool WIDE = decltype(wide_c)::value;
+            constexpr int NLD = R4;   // float4 read per pair record
             const float4 *recs = tile + kFFHead;
 #pragma unroll 2
             for (int s = 0; s < kTile / 2; ++s) {
@@ -387,7 +348,7 @@ po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const floa
 #pragma unroll
                 for (int j = 0; j < TP; ++j) {
                     float2 gc, gs;
-                    if (VAR < 2) {
+                    if (!WIDE) {
                         // p = r . (s - c) in turns; y = p - rint(p), exact, |y| <= 1/2
                         const float2 P = fma2(r[2], rf[j][2], fma2(r[1], rf[j][1], mul2(r[0], rf[j][0])));
                         const float2 y = sub2(P, sub2(add2(P, magic), magic));
@@ -412,48 +373,25 @@ po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const floa
                         gc = flip_parity(cs, tq);
                         gs = flip_parity(T > 0 ? neg2(sn) : sn, tq);
                     }
-                    if (VAR != 0) {
-                        // lit when n . r >= the band, not when below minus it; a pair
-                        // inside it is left out here and listed afterwards (ff_band_scan)
-                        const float2 ndr = ff_ndr2(r, rf[j]);
-                        band = band || (fabsf(ndr.x) < kTangentBand) || (fabsf(ndr.y) < kTangentBand);
-                        const float2 m = make_float2(ndr.x >= kTangentBand ? 1.0f : 0.0f, ndr.y >= kTangentBand ? 1.0f : 0.0f);
-                        gc = mul2(gc, m);
-                        gs = mul2(gs, m);
-                    }
+                    // lit when n . r >= the band, not when below minus it; a pair
+                    // inside it is left out here and listed afterwards (ff_band_scan)
+                    const float2 ndr = ff_ndr2(r, rf[j]);
+                    band = band || (fabsf(ndr.x) < kTangentBand) || (fabsf(ndr.y) < kTangentBand);
+                    const float2 m = make_float2(ndr.x >= kTangentBand ? 1.0f : 0.0f, ndr.y >= kTangentBand ? 1.0f : 0.0f);
+                    gc = mul2(gc, m);
+                    gs = mul2(gs, m);
 #pragma unroll
                     for (int c = 0; c < 3; ++c) {
                         acc[j][c] = fma2(neg2(gs), r[6 + c], fma2(gc, r[3 + c], acc[j][c]));
                         acc[j][3 + c] = fma2(gs, r[3 + c], fma2(gc, r[6 + c], acc[j][3 + c]));
-                        if (HAS_M) {
-                            acc[j][6 + c] = fma2(neg2(gs), r[19 + c], fma2(gc, r[16 + c], acc[j][6 + c]));
-                            acc[j][9 + c] = fma2(gs, r[16 + c], fma2(gc, r[19 + c], acc[j][9 + c]));
-                        }
+                        acc[j][6 + c] = fma2(neg2(gs), r[19 + c], fma2(gc, r[16 + c], acc[j][6 + c]));
+                        acc[j][9 + c] = fma2(gs, r[16 + c], fma2(gc, r[19 + c], acc[j][9 + c]));
                     }
                 }
             }
         };
-        bool lit = false;
-        if (kLitPath && boxes) {
-            // every pair lit when the least n . r over the tile's box of
-            // normals and the CTA's box of directions is at least 1e-5 (the
-            // per-pair test is lit when n . r >= 1e-6): the least of n r over n in
-            // [a, b], r in [c, d] is the least of the four corner products
-            float L = 0.0f;
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float a = hdr[6 + c], b = hdr[9 + c];
-                L += fminf(fminf(a * tbox[c], a * tbox[3 + c]), fminf(b * tbox[c], b * tbox[3 + c]));
-            }
-            lit = L >= 1e-5f;   // block-uniform: every thread reads the same boxes
-        }
-        // block-uniform as well
-        if (hdr[12] != 0.0f)
-            pairs(std::integral_constant<int, 2>{});
-        else if (kLitPath && lit)
-            pairs(std::integral_constant<int, 0>{});
-        else
-            pairs(std::integral_constant<int, 1>{});
+        if (hdr[12] != 0.0f) pairs(std::true_type{});   // block-uniform
+        else pairs(std::false_type{});
 
         // The tile's phase r . c for both directions (lanes): hi products
         // exact, the rest in one FP32 sum; reduced exactly to half turns.
@@ -510,6 +448,271 @@ po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const floa
     }
 }
 
+// The kernel without magnetic currents: the same grid and the same bits, with
+// the thread's two directions in the lanes of every packed operation and a
+// pair record's two sources taken one after the other, each into its own sums.
+// A source's words are then 32-bit factors for both lanes: a packed operation
+// with three distinct register pairs takes 3.2 clocks of the FP32 pipe, with
+// such a factor 2.6 (1,002,001 sources x 160,801 directions: 114.2 -> 105.1 ms).
+// With M the sums of two sources are too many registers for it (14.4 -> 14.6
+// ms on 249,999 x 40,803), so po_ff_kernel stays for those.
+// `boxes`: the tiles' normal boxes may prove a tile lit for the CTA's
+// directions, which skips the per-pair illumination test.
+template <int T>
+__global__ void __launch_bounds__(kThreads, kMinBlocksFF0)
+po_ff0_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const float4 *__restrict__ tgt, long nt,
+             double *__restrict__ part, int *__restrict__ err, int boxes, BandList bl, long ns,
+             const int *__restrict__ order)
+{
+    constexpr int R4 = ff_rec4(false), T4 = ff_tile4(false), TP = 2;
+    constexpr int NA = 6;   // S_J (re xyz, im xyz)
+    extern __shared__ __align__(128) float4 stage[];   // kStages tiles, then the compensation words
+    __shared__ __align__(8) uint64_t full[kStages];
+    __shared__ float tbox_w[kThreads / 32][6];
+    __shared__ float tbox[6];
+    pdl_wait();
+
+    const long tbase = (long)blockIdx.x * kThreads * TP + threadIdx.x;
+    float2 rh[3], rl[3], rw[3];   // hi, lo and FP32 direction; lane j = direction j
+#pragma unroll
+    for (int j = 0; j < TP; ++j) {
+        const long ti = tbase + (long)j * kThreads;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), c = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (ti < nt) {
+            a = tgt[2 * ti];
+            c = tgt[2 * ti + 1];
+        }
+        const float h[3] = {a.x, a.y, a.z}, l[3] = {a.w, c.x, c.y};
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+            const float f = h[q] + l[q];
+            if (j == 0) {
+                rh[q].x = h[q];
+                rl[q].x = l[q];
+                rw[q].x = f;
+            } else {
+                rh[q].y = h[q];
+                rl[q].y = l[q];
+                rw[q].y = f;
+            }
+        }
+    }
+
+    // The CTA's box of directions (the lit-tile proof).
+    {
+        float v[6] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+#pragma unroll
+        for (int j = 0; j < TP; ++j) {
+            if (tbase + (long)j * kThreads >= nt) continue;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float f = j == 0 ? rw[c].x : rw[c].y;
+                v[c] = fminf(v[c], f);
+                v[3 + c] = fmaxf(v[3 + c], f);
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+            for (int q = 0; q < 6; ++q) {
+                const float u = __shfl_xor_sync(0xffffffffu, v[q], o);
+                v[q] = q < 3 ? fminf(v[q], u) : fmaxf(v[q], u);
+            }
+        if ((threadIdx.x & 31) == 0)
+#pragma unroll
+            for (int q = 0; q < 6; ++q) tbox_w[threadIdx.x >> 5][q] = v[q];
+        __syncthreads();
+        if (threadIdx.x < 6) {
+            const int q = threadIdx.x;
+            float r = tbox_w[0][q];
+            for (int w = 1; w < kThreads / 32; ++w) r = q < 3 ? fminf(r, tbox_w[w][q]) : fmaxf(r, tbox_w[w][q]);
+            tbox[q] = r;
+        }
+    }
+
+    float2 hi[NA];   // lanes: directions
+    float2 *lo = reinterpret_cast<float2 *>(stage + (size_t)kStages * T4);
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        hi[a] = make_float2(0.f, 0.f);
+        lo[a * kThreads + threadIdx.x] = make_float2(0.f, 0.f);
+    }
+
+    const long t0 = (long)blockIdx.y * chunk;
+    const int ntl = (int)max(0L, min(ntiles, t0 + chunk) - t0);
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+
+    auto issue = [&](int it) {
+        constexpr uint32_t bytes = (uint32_t)(T4 * sizeof(float4));
+        uint64_t *bar = &full[it % kStages];
+        fence_proxy_async();
+        mbar_expect_tx(bar, bytes);
+        tma_load_1d(stage + (size_t)(it % kStages) * T4, src + (t0 + it) * T4, bytes, bar);
+    };
+    if (threadIdx.x == 0)
+        for (int it = 0; it < ntl && it < kStages; ++it) issue(it);
+
+    const float2 magic = dup2(12582912.0f), twopi = dup2(6.28318530717958648f);
+    bool aborted = false;
+    for (int it = 0; it < ntl; ++it) {
+        const bool ok = mbar_wait_bounded(&full[it % kStages], (uint32_t)((it / kStages) & 1));
+        if (__syncthreads_or(!ok)) {
+            if (threadIdx.x == 0) atomicExch(err, kErrWaitTimeout);
+            aborted = true;
+            break;
+        }
+        const float4 *tile = stage + (size_t)(it % kStages) * T4;
+        const float *hdr = reinterpret_cast<const float *>(tile);
+        float2 acc[2][NA];   // even sources, odd sources
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int a = 0; a < NA; ++a) acc[j][a] = make_float2(0.f, 0.f);
+
+        bool band = false;   // a pair of this tile fell inside the tangent band
+        // VAR 0: narrow tile proven lit (M = 0); 1: narrow tile; 2: wide tile
+        auto pairs = [&](auto var_c) {
+            constexpr int VAR = decltype(var_c)::value;
+            // float4 read per pair record: offsets and J' (and the normal
+            // unless the tile is proven lit; the lo offsets in a wide tile)
+            constexpr int NLD = VAR == 0 ? 5 : (VAR == 1 ? 6 : 8);
+            const float4 *recs = tile + kFFHead;
+#pragma unroll kUnrollFF0
+            for (int s = 0; s < kTile / 2; ++s) {
+                float rec[2][2 * NLD];
+#pragma unroll
+                for (int q = 0; q < NLD; ++q) {
+                    const float4 v = recs[s * R4 + q];
+                    rec[0][2 * q] = v.x;
+                    rec[1][2 * q] = v.y;
+                    rec[0][2 * q + 1] = v.z;
+                    rec[1][2 * q + 1] = v.w;
+                }
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    const float *r = rec[j];
+                    float2 gc, gs;
+                    if (VAR < 2) {
+                        // p = r . (s - c) in turns; y = p - rint(p), exact, |y| <= 1/2
+                        const float2 P = fma2(dup2(r[2]), rw[2], fma2(dup2(r[1]), rw[1], mul2(dup2(r[0]), rw[0])));
+                        const float2 y = sub2(P, sub2(add2(P, magic), magic));
+                        const float2 ang = mul2(y, twopi);
+                        float2 sn, cs;
+                        __sincosf(ang.x, &sn.x, &cs.x);
+                        __sincosf(ang.y, &sn.y, &cs.y);
+                        // G = e^{-t j 2 pi p} = cos - t j sin
+                        gc = cs;
+                        gs = T > 0 ? neg2(sn) : sn;
+                    } else {
+                        // p = r_hi . s_hi (exact) + (r . s_lo + r_lo . s_hi), reduced in half turns
+                        const float2 Ph = fma2(dup2(r[2]), rh[2], fma2(dup2(r[1]), rh[1], mul2(dup2(r[0]), rh[0])));
+                        const float2 Pl = fma2(dup2(r[14]), rw[2], fma2(dup2(r[13]), rw[1], fma2(dup2(r[12]), rw[0],
+                                          fma2(dup2(r[2]), rl[2], fma2(dup2(r[1]), rl[1], mul2(dup2(r[0]), rl[0]))))));
+                        float2 sn, cs, tq;
+                        ff_phase_sincos2(Ph, Pl, sn, cs, tq);
+                        gc = flip_parity(cs, tq);
+                        gs = flip_parity(T > 0 ? neg2(sn) : sn, tq);
+                    }
+                    if (VAR != 0) {
+                        // lit when n . r >= the band, not when below minus it; a pair
+                        // inside it is left out here and listed afterwards (ff_band_scan)
+                        const float2 ndr = fma2(dup2(r[11]), rw[2], fma2(dup2(r[10]), rw[1], mul2(dup2(r[9]), rw[0])));
+                        band = band || (fabsf(ndr.x) < kTangentBand) || (fabsf(ndr.y) < kTangentBand);
+                        const float2 m = make_float2(ndr.x >= kTangentBand ? 1.0f : 0.0f, ndr.y >= kTangentBand ? 1.0f : 0.0f);
+                        gc = mul2(gc, m);
+                        gs = mul2(gs, m);
+                    }
+                    float2 *A = acc[j];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) A[c] = fma2(gc, dup2(r[3 + c]), A[c]);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) A[3 + c] = fma2(gc, dup2(r[6 + c]), A[3 + c]);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) A[c] = fma2(neg2(gs), dup2(r[6 + c]), A[c]);
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) A[3 + c] = fma2(gs, dup2(r[3 + c]), A[3 + c]);
+                }
+            }
+        };
+        bool lit = false;
+        if (boxes) {
+            // every pair lit when the least n . r over the tile's box of
+            // normals and the CTA's box of directions is at least 1e-5 (the
+            // per-pair test is lit when n . r >= 1e-6): the least of n r over n in
+            // [a, b], r in [c, d] is the least of the four corner products
+            float L = 0.0f;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const float a = hdr[6 + c], b = hdr[9 + c];
+                L += fminf(fminf(a * tbox[c], a * tbox[3 + c]), fminf(b * tbox[c], b * tbox[3 + c]));
+            }
+            lit = L >= 1e-5f;   // block-uniform: every thread reads the same boxes
+        }
+        // block-uniform as well
+        if (hdr[12] != 0.0f)
+            pairs(std::integral_constant<int, 2>{});
+        else if (lit)
+            pairs(std::integral_constant<int, 0>{});
+        else
+            pairs(std::integral_constant<int, 1>{});
+
+        // The tile's phase r . c for both directions (lanes): hi products
+        // exact, the rest in one FP32 sum; reduced exactly to half turns.
+        const float ch[3] = {hdr[0], hdr[1], hdr[2]}, cl[3] = {hdr[3], hdr[4], hdr[5]};
+        const float2 Ph = fma2(dup2(ch[2]), rh[2], fma2(dup2(ch[1]), rh[1], mul2(dup2(ch[0]), rh[0])));
+        const float2 Pl = fma2(dup2(cl[2]), rw[2], fma2(dup2(cl[1]), rw[1], fma2(dup2(cl[0]), rw[0],
+                          fma2(dup2(ch[2]), rl[2], fma2(dup2(ch[1]), rl[1], mul2(dup2(ch[0]), rl[0]))))));
+        float2 sn, cs, tq;
+        ff_phase_sincos2(Ph, Pl, sn, cs, tq);
+        const float2 gc = flip_parity(cs, tq), gs = flip_parity(T > 0 ? neg2(sn) : sn, tq);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const float2 Sr = add2(acc[0][c], acc[1][c]);
+            const float2 Si = add2(acc[0][3 + c], acc[1][3 + c]);
+            const float2 v[2] = {fma2(gc, Sr, mul2(neg2(gs), Si)), fma2(gc, Si, mul2(gs, Sr))};
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int a = c + 3 * q;
+                float2 sum, e;
+                two_sum2(hi[a], v[q], sum, e);
+                hi[a] = sum;
+                float2 &l = lo[a * kThreads + threadIdx.x];
+                l = add2(l, e);
+            }
+        }
+        if (band) {
+            const float2 rf[TP][3] = {{dup2(rw[0].x), dup2(rw[1].x), dup2(rw[2].x)},
+                                      {dup2(rw[0].y), dup2(rw[1].y), dup2(rw[2].y)}};
+            ff_band_scan<TP, R4>(tile + kFFHead, (t0 + it) * kTile, rf, tbase, ns, nt, order, bl);
+        }
+        __syncthreads();
+        if (threadIdx.x == 0 && it + kStages < ntl) issue(it + kStages);
+    }
+
+    if (aborted) {
+        if (threadIdx.x == 0)
+            for (int s = 0; s < kStages; ++s) (void)mbar_wait_bounded(&full[s], 0);
+        return;
+    }
+
+    pdl_trigger();
+#pragma unroll
+    for (int j = 0; j < TP; ++j) {
+        const long ti = tbase + (long)j * kThreads;
+        if (ti >= nt) continue;
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const float2 l = lo[a * kThreads + threadIdx.x];
+            part[((long)blockIdx.y * NA + a) * nt + ti] =
+                j == 0 ? (double)hi[a].x + (double)l.x : (double)hi[a].y + (double)l.y;
+        }
+    }
+}
+
 // ------------------------------------------------------------------ host side
 
 int ff_smem_bytes(bool has_m) { return kStages * ff_tile4(has_m) * 16 + (has_m ? 12 : 6) * 2 * kThreads * 4; }
@@ -525,10 +728,8 @@ void *ff_pack_kernel(bool has_m)
 void *ff_kernel(int t_sign, bool has_m)
 {
     if (t_sign < 0)
-        return has_m ? reinterpret_cast<void *>(&po_ff_kernel<-1, true>)
-                     : reinterpret_cast<void *>(&po_ff_kernel<-1, false>);
-    return has_m ? reinterpret_cast<void *>(&po_ff_kernel<1, true>)
-                 : reinterpret_cast<void *>(&po_ff_kernel<1, false>);
+        return has_m ? reinterpret_cast<void *>(&po_ff_kernel<-1>) : reinterpret_cast<void *>(&po_ff0_kernel<-1>);
+    return has_m ? reinterpret_cast<void *>(&po_ff_kernel<1>) : reinterpret_cast<void *>(&po_ff0_kernel<1>);
 }
 
 // Radix sort of (key, index) pairs on `s`; with temp == nullptr only sets

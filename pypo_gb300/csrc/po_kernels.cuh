@@ -84,6 +84,10 @@ constexpr int kMinBlocksA2M = PO_MINB_A2M;
 constexpr int kMinBlocksFA = 6, kMinBlocksFAM = 4;   // resident CTAs per SM asked of ptxas (M = 0, with M)
 constexpr int kStagesFA = 2;
 constexpr int kFFDirs = 64;   // directions per stage of the far-field adjoint
+// The far-field forward without magnetic currents, two pair records an
+// iteration at 5 CTAs/SM: 105.1 ms on 1,002,001 x 160,801 (one record 112.3;
+// at 4 CTAs/SM 109.7 with one, 111.7 with two, 109.4 with four).
+constexpr int kMinBlocksFF0 = 5, kUnrollFF0 = 2;
 constexpr int kUnrollF = PO_UNROLL_F;
 constexpr int kUnrollA = PO_UNROLL_A;   // target pairs per iteration of the adjoint pair loop
 constexpr int kAccAdj = 13;
