@@ -130,6 +130,14 @@ static int device_info(DeviceInfo *&out)
     return 0;
 }
 
+// Share of a chunk that the last wave is expected to idle (choose_split). Near
+// field and scalar: 0.3 (scalar 10,403 -> 14,399 0.197 -> 0.185 ms, feed ->
+// dish step 2.00 -> 1.97 against 0). The far-field forward's tiles differ
+// more in cost (narrow, wide, lit): 0.5 (122,500 -> 22,650 2.74 -> 2.58 ms).
+// Its adjoint, whose stages are alike, is best left at 0 (17.59 against 17.78
+// ms on 251,001 x 40,803 with 0.3).
+constexpr double kTailNF = 0.3, kTailFF = 0.5;
+
 // Resident CTAs per SM of a kernel (and its shared-memory attribute), looked
 // up once per device and kernel.
 static int kernel_occupancy(DeviceInfo *di, void *fk, int threads, int smem, int &occ)
@@ -147,12 +155,16 @@ static int kernel_occupancy(DeviceInfo *di, void *fk, int threads, int smem, int
     return 0;
 }
 
-long choose_split(long nb, long ns, long slots, long max_chunks, long tile)
+long choose_split(long nb, long ns, long slots, long max_chunks, long tile, double tail)
 {
     const long tiles = std::max(1L, (ns + tile - 1) / tile);
     // a chunk's partials cost the epilogue about 0.05 of a full wave's tile,
     // less where the owning blocks fill only part of a wave
     const double per_chunk = 0.002 + 0.048 * std::min(1.0, (double)nb / (double)slots);
+    // a CTA's start (barriers, its first copies) costs about 0.3 of a tile:
+    // without it, 10,201 sources -> 40,401 targets went to 40 chunks of 2 tiles
+    // (2.10 ms; 2.06 with 12 of 7)
+    const double start = 0.3;
     long best = 1;
     double best_cost = 1e300;
     for (long s = 1; s <= std::min(tiles, std::min(std::max(1L, max_chunks), 1024L)); ++s) {
@@ -160,7 +172,7 @@ long choose_split(long nb, long ns, long slots, long max_chunks, long tile)
         const long real = (tiles + chunk - 1) / chunk;
         if (real != s) continue;
         const long waves = (nb * real + slots - 1) / slots;
-        const double cost = (double)waves * chunk + per_chunk * real;
+        const double cost = (double)waves * (chunk + start) + tail * chunk + per_chunk * real;
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = real;
@@ -433,7 +445,7 @@ int run_device(const RunArgs &a)
     int occ = 1;
     if ((rc = device_info(di)) || (rc = kernel_occupancy(di, fk, kThreadsD, 0, occ))) return rc;
     const long ntb = (nt + kThreadsD - 1) / kThreadsD;
-    const long nsplit = choose_split(ntb, ns, (long)di->sms * occ, partial_cap(nt, nacc), kChunkD);
+    const long nsplit = choose_split(ntb, ns, (long)di->sms * occ, partial_cap(nt, nacc), kChunkD, 0.0);
     const long tiles = std::max(1L, (ns + kChunkD - 1) / kChunkD);
     long chunk = (tiles + nsplit - 1) / nsplit * kChunkD;
     double *srcd = nullptr, *part = nullptr;
@@ -501,7 +513,7 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
     const int occ = p.far ? di->occ_ff[p.ts > 0][p.has_m ? 1 : 0] : di->occ2[p.kind][p.ts > 0][p.has_m ? 1 : 0];
     const size_t room = std::min(sc.room(), (size_t)1 << 30);
     const long max_chunks = std::max(1L, (long)(room / ((size_t)p.nacc * nt * sizeof(double))));
-    p.nsplit = choose_split(p.ntb, ns, (long)di->sms * occ, max_chunks, kTile);
+    p.nsplit = choose_split(p.ntb, ns, (long)di->sms * occ, max_chunks, kTile, p.far ? kTailFF : kTailNF);
     const long chunk_tiles = (p.tiles + p.nsplit - 1) / p.nsplit;
     p.chunk = chunk_tiles * (p.far ? 1 : kTile);   // tiles (far field) or sources per chunk
     if ((rc = sc.get(&p.part, (size_t)p.nsplit * p.nacc * nt))) return rc;
@@ -647,7 +659,7 @@ int run_adjoint(const AdjArgs &a)
     int occ = 1, rc = 0;
     if ((rc = kernel_occupancy(di, fk, threads, smem, occ))) return rc;
     const long nsb = (ns + per_block - 1) / per_block;
-    const long split = choose_split(nsb, nt, (long)di->sms * occ, partial_cap(ns, kAccAdj), tile_t);
+    const long split = choose_split(nsb, nt, (long)di->sms * occ, partial_cap(ns, kAccAdj), tile_t, far ? 0.0 : kTailNF);
     const long tiles_t = std::max(1L, (nt + tile_t - 1) / tile_t);
     const long per_chunk = (tiles_t + split - 1) / split;
     long chunk = !fp64 && far ? per_chunk : per_chunk * tile_t;   // stages (mixed far field) or targets
