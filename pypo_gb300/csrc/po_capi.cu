@@ -224,6 +224,63 @@ done:
     return rc;
 }
 
+// Page-locked staging of the drop-in calls: blocks of kStageBytes, borrowed by
+// one call at a time and kept for later ones (at most kStageKeep).
+constexpr size_t kStageBytes = size_t(8) << 20;
+constexpr size_t kStageKeep = 4;
+std::mutex g_stage_mu;
+std::vector<void *> g_stage_free;
+
+class Staging {
+public:
+    ~Staging()
+    {
+        if (!p_) return;
+        {
+            std::lock_guard<std::mutex> lk(g_stage_mu);
+            if (g_stage_free.size() < kStageKeep) {
+                g_stage_free.push_back(p_);
+                return;
+            }
+        }
+        cudaFreeHost(p_);
+    }
+    // A block for `bytes`, or null (too many, or no page-locked memory).
+    float *borrow(size_t bytes)
+    {
+        if (bytes > kStageBytes) return nullptr;
+        {
+            std::lock_guard<std::mutex> lk(g_stage_mu);
+            if (!g_stage_free.empty()) {
+                p_ = g_stage_free.back();
+                g_stage_free.pop_back();
+            }
+        }
+        if (!p_ && cudaHostAlloc(&p_, kStageBytes, cudaHostAllocPortable) != cudaSuccess) {
+            p_ = nullptr;
+            (void)cudaGetLastError();
+        }
+        return static_cast<float *>(p_);
+    }
+
+private:
+    void *p_ = nullptr;
+};
+
+// n floats copied; whether any of them is non-zero (-0.0 counts as zero, NaN
+// as non-zero).
+bool copy_any(float *dst, const float *src, long n)
+{
+    unsigned any = 0;
+    for (long i = 0; i < n; ++i) {
+        unsigned b;
+        std::memcpy(&b, src + i, sizeof b);
+        any |= b & 0x7fffffffu;
+        std::memcpy(dst + i, &b, sizeof b);
+    }
+    return any != 0;
+}
+
 // reflparamsf -> reflparams with owned double arrays.
 struct Widened {
     double coeffs[3], lxu[2], lyv[2], gcenter[2], transf[16];
@@ -257,10 +314,12 @@ void widen(const reflparamsf &f, Widened &w)
 // Shared body of the callKernelf_* drop-ins. Both grids are generated in
 // FP64 on the device from the widened reflparams (the reference generates
 // them on the host); the float currents are copied as they are and widened
-// on the device; after the mixed-precision run and the call's one
-// synchronisation of its kernels, the outputs and the two grids are narrowed
-// to float on the device and copied into the caller's bundle rows and
-// containers cs / ct, as the reference leaves them.
+// on the device; after the mixed-precision run, the outputs and the two grids
+// are narrowed to float on the device and copied into the caller's bundle
+// rows and containers cs / ct, as the reference leaves them. Up to
+// kStageBytes the caller's rows go through page-locked staging, one copy each
+// way and one synchronisation (31 x 33 -> 31 x 31: 38 copies of pageable rows
+// took 0.4 of the call's 0.64 ms); larger calls copy row by row.
 int drop_in(int mode, float *const *res, reflparamsf source, reflparamsf target, reflcontainerf *cs,
             reflcontainerf *ct, float *const *inp, float k, float epsilon, float t)
 {
@@ -284,26 +343,43 @@ int drop_in(int mode, float *const *res, reflparamsf source, reflparamsf target,
     widen(target, wt);
     cudaStream_t s = nullptr;
     if (int rc = lib_stream(&s)) return rc;
-    double *d_src = nullptr, *d_cur = nullptr, *d_tgt = nullptr, *d_out = nullptr;
-    float *d_f = nullptr;   // float staging: the currents in, then the outputs and grids out
-    const long nf = std::max({(long)ncur * ns, (long)nout * nt, 7L * std::max(ns, nt)});
+    // one scratch block: outputs, source grid, target grid (in this order: they
+    // are narrowed in one pass), currents, then the floats
+    const bool want_s = cs && cs->x, want_t = ct && ct->x;
+    const long n_in = (long)ncur * ns, n_res = (long)nout * nt;
+    const long n_back = n_res + (want_s || want_t ? 7 * (ns + nt) : 0);
+    const long nf = std::max(n_in, n_back);
+    double *d_out = nullptr;
     int rc = 0, code = 0;
     HostSlots local{};
     HostSlots *hs = host_slots(&local);
     po::RunArgs a;
     const unsigned cblk = 608;   // 152 SMs x 4, grid-stride
-    PO_SCRATCH(d_src, sizeof(double) * 7 * ns);
-    PO_SCRATCH(d_cur, sizeof(double) * ncur * ns);
-    PO_SCRATCH(d_tgt, sizeof(double) * 7 * nt);
-    PO_SCRATCH(d_out, sizeof(double) * nout * nt);
-    PO_SCRATCH(d_f, sizeof(float) * nf);
+    double *d_src = nullptr, *d_tgt = nullptr, *d_cur = nullptr;
+    float *d_f = nullptr;
+    Staging staging;
+    float *const h = staging.borrow(sizeof(float) * nf);
+    bool any_m = false;
+    PO_SCRATCH(d_out, sizeof(double) * (n_res + 7 * (ns + nt) + n_in) + sizeof(float) * nf);
+    d_src = d_out + n_res;
+    d_tgt = d_src + 7 * ns;
+    d_cur = d_tgt + 7 * nt;
+    d_f = reinterpret_cast<float *>(d_cur + n_in);
     if ((rc = po::generate_grid_dev(ws.r, d_src, true, true, s)) ||
         (rc = po::generate_grid_dev(wt.r, d_tgt, true, true, s)))
         goto done;
-    for (int r = 0; r < ncur; ++r)
-        CK(cudaMemcpyAsync(d_f + (size_t)r * ns, inp[r], sizeof(float) * ns, cudaMemcpyHostToDevice, s));
+    if (h) {
+        for (int r = 0; r < ncur; ++r) {
+            const bool any = copy_any(h + (size_t)r * ns, inp[r], ns);
+            any_m = any_m || (r >= 6 && any);
+        }
+        CK(cudaMemcpyAsync(d_f, h, sizeof(float) * n_in, cudaMemcpyHostToDevice, s));
+    } else {
+        for (int r = 0; r < ncur; ++r)
+            CK(cudaMemcpyAsync(d_f + (size_t)r * ns, inp[r], sizeof(float) * ns, cudaMemcpyHostToDevice, s));
+    }
     {
-        long n = (long)ncur * ns;
+        long n = n_in;
         void *args[] = {&d_f, &d_cur, &n};
         CK(cudaLaunchKernel(po::f2d_kernel(), dim3(cblk), dim3(256), args, 0, s));
     }
@@ -322,8 +398,8 @@ int drop_in(int mode, float *const *res, reflparamsf source, reflparamsf target,
     a.precision = 0;
     a.m_zero = false;
     if (mode != po::kScalar) {
-        bool mz = false;
-        if ((rc = device_m_is_zero(d_cur, ns, s, mz))) goto done;
+        bool mz = !any_m;
+        if (!h && (rc = device_m_is_zero(d_cur, ns, s, mz))) goto done;
         a.m_zero = mz;
     }
     a.extent_host = &hs->extent;
@@ -333,38 +409,38 @@ int drop_in(int mode, float *const *res, reflparamsf source, reflparamsf target,
     rc = po::run_device(a);
     if (rc) goto done;
     {
-        long n = (long)nout * nt;
+        long n = n_back;
         void *args[] = {&d_out, &d_f, &n};
         CK(cudaLaunchKernel(po::d2f_kernel(), dim3(cblk), dim3(256), args, 0, s));
     }
-    for (int r = 0; r < nout; ++r)
-        CK(cudaMemcpyAsync(res[r], d_f + (size_t)r * nt, sizeof(float) * nt, cudaMemcpyDeviceToHost, s));
+    if (h) CK(cudaMemcpyAsync(h, d_f, sizeof(float) * n_back, cudaMemcpyDeviceToHost, s));
+    else
+        for (int r = 0; r < nout; ++r)
+            CK(cudaMemcpyAsync(res[r], d_f + (size_t)r * nt, sizeof(float) * nt, cudaMemcpyDeviceToHost, s));
     rc = po::read_device_error(s, &code);   // the kernels' one synchronisation
     if (!rc && code) rc = fail(4, device_error_text(code));
     if (rc) goto done;
     t_extent = hs->extent;
     t_band = hs->band;
+    if (h)
+        for (int r = 0; r < nout; ++r) std::memcpy(res[r], h + (size_t)r * nt, sizeof(float) * nt);
     // the grids, as the reference leaves them in cs and ct
     for (int w = 0; w < 2; ++w) {
+        if (!(w == 0 ? want_s : want_t)) continue;
         reflcontainerf *cf = w == 0 ? cs : ct;
-        if (!cf || !cf->x) continue;
-        long n = 7L * (w == 0 ? ns : nt);
-        double *g = w == 0 ? d_src : d_tgt;
-        void *args[] = {&g, &d_f, &n};
-        CK(cudaLaunchKernel(po::d2f_kernel(), dim3(cblk), dim3(256), args, 0, s));
+        const long np = w == 0 ? ns : nt;
+        const long at = n_res + (w == 0 ? 0 : 7 * ns);
         float *dst[7] = {cf->x, cf->y, cf->z, cf->nx, cf->ny, cf->nz, cf->area};
-        const long np = n / 7;
-        for (int r = 0; r < 7; ++r)
-            if (dst[r]) CK(cudaMemcpyAsync(dst[r], d_f + (size_t)r * np, sizeof(float) * np, cudaMemcpyDeviceToHost, s));
+        for (int r = 0; r < 7; ++r) {
+            if (!dst[r]) continue;
+            if (h) std::memcpy(dst[r], h + at + r * np, sizeof(float) * np);
+            else CK(cudaMemcpyAsync(dst[r], d_f + at + r * np, sizeof(float) * np, cudaMemcpyDeviceToHost, s));
+        }
     }
-    CK(cudaStreamSynchronize(s));
+    if (!h) CK(cudaStreamSynchronize(s));
 done:
-    if (d_src) cudaFreeAsync(d_src, s);
-    if (d_cur) cudaFreeAsync(d_cur, s);
-    if (d_tgt) cudaFreeAsync(d_tgt, s);
     if (d_out) cudaFreeAsync(d_out, s);
-    if (d_f) cudaFreeAsync(d_f, s);
-    if (s && rc) cudaStreamSynchronize(s);
+    if (s && rc) cudaStreamSynchronize(s);   // copies from or into host memory may still be in flight
     return rc;
 }
 

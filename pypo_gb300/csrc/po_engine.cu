@@ -362,16 +362,35 @@ int read_device_error(cudaStream_t s, int *code)
 {
     // Both words: the allocating paths' (if it exists yet) and the
     // allocation-free entry's (if it has set up on this device). Nothing is
-    // allocated here, so callers of the allocation-free entry can use it.
-    int *w[2] = {error_word_impl(false), static_status_word()};
-    int got[2] = {0, 0};
-    for (int i = 0; i < 2; ++i) {
-        if (!w[i]) continue;
-        PO_CK(cudaMemcpyAsync(&got[i], w[i], sizeof(int), cudaMemcpyDeviceToHost, s));
-        PO_CK(cudaMemsetAsync(w[i], 0, sizeof(int), s));
+    // allocated on the device here, so callers of the allocation-free entry
+    // can use it. The words are read into page-locked memory (one small block
+    // per calling thread, kept; the stack where that fails: a copy into
+    // pageable memory waits for the stream and costs 10 us more), and cleared
+    // only where one is set.
+    thread_local int *pinned = nullptr;
+    thread_local bool tried = false;
+    if (!tried) {
+        tried = true;
+        if (cudaMallocHost(&pinned, 2 * sizeof(int)) != cudaSuccess) {
+            pinned = nullptr;
+            (void)cudaGetLastError();
+        }
     }
+    int local[2];
+    int *got = pinned ? pinned : local;
+    int *w[2] = {error_word_impl(false), static_status_word()};
+    got[0] = got[1] = 0;
+    for (int i = 0; i < 2; ++i)
+        if (w[i]) PO_CK(cudaMemcpyAsync(&got[i], w[i], sizeof(int), cudaMemcpyDeviceToHost, s));
     PO_CK(cudaStreamSynchronize(s));
     *code = got[0] ? got[0] : got[1];
+    bool cleared = false;
+    for (int i = 0; i < 2; ++i)
+        if (w[i] && got[i]) {
+            PO_CK(cudaMemsetAsync(w[i], 0, sizeof(int), s));
+            cleared = true;
+        }
+    if (cleared) PO_CK(cudaStreamSynchronize(s));
     return 0;
 }
 

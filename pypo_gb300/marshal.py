@@ -56,13 +56,21 @@ def fill_reflparams(refl, ctype=ctypes.c_double):
     return st, keep
 
 
+def _point_rows(st, first, block):
+    """Point the struct's consecutive pointer members, from the one named
+    `first` on, at the rows of `block` (one write of all the addresses: a
+    ctypes pointer object per member takes 4 us each)."""
+    at = getattr(type(st), first).offset
+    n = block.shape[0]
+    np.ndarray((n,), np.uintp, buffer=st, offset=at)[:] = block.ctypes.data + block.strides[0] * np.arange(n)
+
+
 def alloc_container(n, ctype=ctypes.c_double):
     """reflcontainer(f) whose 7 arrays are one (7, n) numpy block."""
     st = S.reflcontainer() if ctype is ctypes.c_double else S.reflcontainerf()
     block = np.zeros((7, n), dtype=_NP[ctype])
     st.size = n
-    for i, name in enumerate(("x", "y", "z", "nx", "ny", "nz", "area")):
-        setattr(st, name, _ptr(block[i], ctype))
+    _point_rows(st, "x", block)
     st._block = block
     return st, block
 
@@ -72,8 +80,7 @@ def fill_container(block, ctype=ctypes.c_double):
     block = np.ascontiguousarray(block, dtype=_NP[ctype])
     st = S.reflcontainer() if ctype is ctypes.c_double else S.reflcontainerf()
     st.size = block.shape[1]
-    for i, name in enumerate(("x", "y", "z", "nx", "ny", "nz", "area")):
-        setattr(st, name, _ptr(block[i], ctype))
+    _point_rows(st, "x", block)
     st._block = block
     return st, block
 
@@ -83,10 +90,8 @@ def bundle(cls, block, ctype):
     The struct holds a reference to `block`, so a temporary block stays
     alive as long as the struct does."""
     st = cls()
-    names = [f[0] for f in cls._fields_]
-    assert block.shape[0] == len(names)
-    for i, name in enumerate(names):
-        setattr(st, name, _ptr(block[i], ctype))
+    assert block.shape[0] == len(cls._fields_)
+    _point_rows(st, cls._fields_[0][0], block)
     st._block = block
     return st
 
@@ -106,12 +111,8 @@ def currents_block(cur, ctype=ctypes.c_double):
 
 def block_to_complex(block, n_complex):
     """Rows in bundle order (r1x r1y r1z i1x i1y i1z ...) to (3*n_complex, n) complex."""
-    out = []
+    out = np.empty((3 * n_complex, block.shape[1]), dtype=np.complex128)
     for b in range(n_complex):
-        re = block[6 * b:6 * b + 3]
-        im = block[6 * b + 3:6 * b + 6]
-        z = np.empty(re.shape, dtype=np.complex128)
-        z.real = re
-        z.imag = im
-        out.append(z)
-    return np.concatenate(out, axis=0)
+        out.real[3 * b:3 * b + 3] = block[6 * b:6 * b + 3]
+        out.imag[3 * b:3 * b + 3] = block[6 * b + 3:6 * b + 6]
+    return out
