@@ -79,22 +79,22 @@ __global__ void po_adj_ehp_cot_kernel(long nt, const double *__restrict__ cot, c
 
 // ---------------------------------------------------------------- epilogues
 
-// Sums the chunks of the source-side partials; unfolds the currents by
-// conj(fac * weight * area); scales the displacement term to mm. G threads
-// share a source (thread g adds chunks g, g + G, ..., then a tree), as in the
-// forward's epilogue. The blocks past the sources scale the target sums gt
-// into grad_dt.
-template <int G>
+// Sums the chunks of the source-side partials (N rows: adj_rows); unfolds the
+// currents by conj(fac * weight * area); scales the displacement term to mm.
+// G threads share a source (thread g adds chunks g, g + G, ..., then a tree),
+// as in the forward's epilogue. The blocks past the nblk_s of the sources
+// scale the target sums gt into grad_dt; where the call has no rows, nblk_s
+// is 0 (of the N = 1 instance).
+template <int G, int N>
 __global__ void __launch_bounds__(kEpiThreads)
 po_adj_epilogue_kernel(int kind, int nsplit, long ns, const double *__restrict__ part,
                        const double *__restrict__ src7, int gmode, int ncx, int ncy, double fac_re, double fac_im,
-                       double dscale, double *__restrict__ grad_cur, double *__restrict__ grad_ds, long nt,
+                       double dscale, double *__restrict__ grad_cur, double *__restrict__ grad_ds, long nblk_s, long nt,
                        const double *__restrict__ gt, double tscale, double *__restrict__ grad_dt)
 {
     constexpr int SB = kEpiThreads / G;   // sources per block
-    __shared__ double sh[G > 1 ? G / 2 : 1][G > 1 ? kAccAdj : 1][G > 1 ? SB : 1];
+    __shared__ double sh[G > 1 ? G / 2 : 1][G > 1 ? N : 1][G > 1 ? SB : 1];
     pdl_wait();
-    const long nblk_s = (ns + SB - 1) / SB;
     if ((long)blockIdx.x >= nblk_s) {
         const long j = ((long)blockIdx.x - nblk_s) * kEpiThreads + threadIdx.x;
         if (j < nt) grad_dt[j] = tscale * gt[j];
@@ -102,25 +102,25 @@ po_adj_epilogue_kernel(int kind, int nsplit, long ns, const double *__restrict__
     }
     const int sl = threadIdx.x % SB, g = threadIdx.x / SB;
     const long i = (long)blockIdx.x * SB + sl;
-    double a[kAccAdj];
+    double a[N];
 #pragma unroll
-    for (int q = 0; q < kAccAdj; ++q) a[q] = 0.0;
+    for (int q = 0; q < N; ++q) a[q] = 0.0;
     if (i < ns) {
 #pragma unroll 2
         for (int s = g; s < nsplit; s += G)
 #pragma unroll
-            for (int q = 0; q < kAccAdj; ++q) a[q] += part[((long)s * kAccAdj + q) * ns + i];
+            for (int q = 0; q < N; ++q) a[q] += part[((long)s * N + q) * ns + i];
     }
     if constexpr (G > 1) {
 #pragma unroll
         for (int w = G / 2; w > 0; w >>= 1) {
             if (g >= w && g < 2 * w)
 #pragma unroll
-                for (int q = 0; q < kAccAdj; ++q) sh[g - w][q][sl] = a[q];
+                for (int q = 0; q < N; ++q) sh[g - w][q][sl] = a[q];
             __syncthreads();
             if (g < w)
 #pragma unroll
-                for (int q = 0; q < kAccAdj; ++q) a[q] += sh[g][q][sl];
+                for (int q = 0; q < N; ++q) a[q] += sh[g][q][sl];
             __syncthreads();
         }
         if (g > 0) return;
@@ -130,17 +130,17 @@ po_adj_epilogue_kernel(int kind, int nsplit, long ns, const double *__restrict__
     const double fr = fac_re * w, fi = fac_im * w;
     if (grad_cur && kind == kKindScalar) {
         // conj(f) * (re + j im), two rows
-        grad_cur[i] = fr * a[0] + fi * a[3];
-        grad_cur[ns + i] = fr * a[3] - fi * a[0];
-    } else if (grad_cur)
+        grad_cur[i] = fr * a[0] + fi * a[N > 1 ? 1 : 0];
+        grad_cur[ns + i] = fr * a[N > 1 ? 1 : 0] - fi * a[0];
+    } else if (N >= 12 && grad_cur)
         for (int h = 0; h < 2; ++h)
             for (int c = 0; c < 3; ++c) {
-                const double re = a[6 * h + c], im = a[6 * h + 3 + c];
+                const double re = a[N >= 12 ? 6 * h + c : 0], im = a[N >= 12 ? 6 * h + 3 + c : 0];
                 // conj(f) * (re + j im)
                 grad_cur[(long)(6 * h + c) * ns + i] = fr * re + fi * im;
                 grad_cur[(long)(6 * h + 3 + c) * ns + i] = fr * im - fi * re;
             }
-    if (grad_ds) grad_ds[i] = dscale * a[12];
+    if (grad_ds) grad_ds[i] = dscale * a[N - 1];   // the last row
 }
 
 // -------------------------------------------------------------------- packing
@@ -242,10 +242,22 @@ po_adj_pack_kernel(long ns, const double *__restrict__ src7, const double *__res
 void *adj_cot_kernel() { return reinterpret_cast<void *>(&po_adj_cot_kernel); }
 void *adj_ehp_cot_kernel() { return reinterpret_cast<void *>(&po_adj_ehp_cot_kernel); }
 void *adj_pack_kernel() { return reinterpret_cast<void *>(&po_adj_pack_kernel); }
-void *adj_epilogue_kernel(int groups)
+template <int N>
+static void *adj_epilogue_sel(int groups)
 {
-    return groups == 8 ? reinterpret_cast<void *>(&po_adj_epilogue_kernel<8>)
-                       : reinterpret_cast<void *>(&po_adj_epilogue_kernel<1>);
+    return groups == 8 ? reinterpret_cast<void *>(&po_adj_epilogue_kernel<8, N>)
+                       : reinterpret_cast<void *>(&po_adj_epilogue_kernel<1, N>);
+}
+
+void *adj_epilogue_kernel(int groups, int rows)
+{
+    switch (rows) {
+    case 2: return adj_epilogue_sel<2>(groups);
+    case 3: return adj_epilogue_sel<3>(groups);
+    case 12: return adj_epilogue_sel<12>(groups);
+    case 13: return adj_epilogue_sel<13>(groups);
+    default: return adj_epilogue_sel<1>(groups);
+    }
 }
 
 }  // namespace po

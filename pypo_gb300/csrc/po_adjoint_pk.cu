@@ -85,7 +85,7 @@ __device__ __forceinline__ AdjGeo2 adj_geo2(const float2 *r, const SrcC &s)
 // accumulators + the source displacement term; vt: the two targets' terms.
 // band: set when a pair lies inside the tangent band (left out here; the
 // kernel lists it afterwards with adj_band_scan).
-template <int T, bool HAS_M, bool WANT_D, bool WANT_T>
+template <int T, bool HAS_M, bool WANT_C, bool WANT_D, bool WANT_T>
 __device__ __forceinline__ void adj_nf_pair2(float2 *acc, float2 &vt, const float2 *r, const SrcC &s, bool &band)
 {
     const AdjGeo2 g = adj_geo2(r, s);
@@ -116,30 +116,32 @@ __device__ __forceinline__ void adj_nf_pair2(float2 *acc, float2 &vt, const floa
     // gE.R_hat, gH.R_hat
     const float2 ger = fma2(Ezr, ez, fma2(Eyr, ey, mul2(Exr, ex))), gei = fma2(Ezi, ez, fma2(Eyi, ey, mul2(Exi, ex)));
     const float2 ghr = fma2(Hzr, ez, fma2(Hyr, ey, mul2(Hxr, ex))), ghi = fma2(Hzi, ez, fma2(Hyi, ey, mul2(Hxi, ex)));
-    // P = conj(C2) (gE.R_hat), Q = conj(C2) (gH.R_hat)
-    const float2 Pr = fma2(C2r, ger, mul2(C2i, gei)), Pi = fma2(C2r, gei, mul2(neg2(C2i), ger));
-    const float2 Qr = fma2(C2r, ghr, mul2(C2i, ghi)), Qi = fma2(C2r, ghi, mul2(neg2(C2i), ghr));
-    // K = conj(C3) gH, L = conj(C3) gE
-    const float2 Kxr = fma2(C3r, Hxr, mul2(C3i, Hxi)), Kxi = fma2(C3r, Hxi, mul2(neg2(C3i), Hxr));
-    const float2 Kyr = fma2(C3r, Hyr, mul2(C3i, Hyi)), Kyi = fma2(C3r, Hyi, mul2(neg2(C3i), Hyr));
-    const float2 Kzr = fma2(C3r, Hzr, mul2(C3i, Hzi)), Kzi = fma2(C3r, Hzi, mul2(neg2(C3i), Hzr));
-    const float2 Lxr = fma2(C3r, Exr, mul2(C3i, Exi)), Lxi = fma2(C3r, Exi, mul2(neg2(C3i), Exr));
-    const float2 Lyr = fma2(C3r, Eyr, mul2(C3i, Eyi)), Lyi = fma2(C3r, Eyi, mul2(neg2(C3i), Eyr));
-    const float2 Lzr = fma2(C3r, Ezr, mul2(C3i, Ezi)), Lzi = fma2(C3r, Ezi, mul2(neg2(C3i), Ezr));
-    // Jbar' += conj(c1) gE + P R_hat + K x R_hat
-    acc[0] = fma2(c1r, Exr, fma2(c1i, Exi, fma2(Pr, ex, fma2(Kyr, ez, fma2(neg2(Kzr), ey, acc[0])))));
-    acc[1] = fma2(c1r, Eyr, fma2(c1i, Eyi, fma2(Pr, ey, fma2(Kzr, ex, fma2(neg2(Kxr), ez, acc[1])))));
-    acc[2] = fma2(c1r, Ezr, fma2(c1i, Ezi, fma2(Pr, ez, fma2(Kxr, ey, fma2(neg2(Kyr), ex, acc[2])))));
-    acc[3] = fma2(c1r, Exi, fma2(neg2(c1i), Exr, fma2(Pi, ex, fma2(Kyi, ez, fma2(neg2(Kzi), ey, acc[3])))));
-    acc[4] = fma2(c1r, Eyi, fma2(neg2(c1i), Eyr, fma2(Pi, ey, fma2(Kzi, ex, fma2(neg2(Kxi), ez, acc[4])))));
-    acc[5] = fma2(c1r, Ezi, fma2(neg2(c1i), Ezr, fma2(Pi, ez, fma2(Kxi, ey, fma2(neg2(Kyi), ex, acc[5])))));
-    // Mbar' += conj(c1) gH + Q R_hat - L x R_hat
-    acc[6] = fma2(c1r, Hxr, fma2(c1i, Hxi, fma2(Qr, ex, fma2(neg2(Lyr), ez, fma2(Lzr, ey, acc[6])))));
-    acc[7] = fma2(c1r, Hyr, fma2(c1i, Hyi, fma2(Qr, ey, fma2(neg2(Lzr), ex, fma2(Lxr, ez, acc[7])))));
-    acc[8] = fma2(c1r, Hzr, fma2(c1i, Hzi, fma2(Qr, ez, fma2(neg2(Lxr), ey, fma2(Lyr, ex, acc[8])))));
-    acc[9] = fma2(c1r, Hxi, fma2(neg2(c1i), Hxr, fma2(Qi, ex, fma2(neg2(Lyi), ez, fma2(Lzi, ey, acc[9])))));
-    acc[10] = fma2(c1r, Hyi, fma2(neg2(c1i), Hyr, fma2(Qi, ey, fma2(neg2(Lzi), ex, fma2(Lxi, ez, acc[10])))));
-    acc[11] = fma2(c1r, Hzi, fma2(neg2(c1i), Hzr, fma2(Qi, ez, fma2(neg2(Lxi), ey, fma2(Lyi, ex, acc[11])))));
+    if (WANT_C) {
+        // P = conj(C2) (gE.R_hat), Q = conj(C2) (gH.R_hat)
+        const float2 Pr = fma2(C2r, ger, mul2(C2i, gei)), Pi = fma2(C2r, gei, mul2(neg2(C2i), ger));
+        const float2 Qr = fma2(C2r, ghr, mul2(C2i, ghi)), Qi = fma2(C2r, ghi, mul2(neg2(C2i), ghr));
+        // K = conj(C3) gH, L = conj(C3) gE
+        const float2 Kxr = fma2(C3r, Hxr, mul2(C3i, Hxi)), Kxi = fma2(C3r, Hxi, mul2(neg2(C3i), Hxr));
+        const float2 Kyr = fma2(C3r, Hyr, mul2(C3i, Hyi)), Kyi = fma2(C3r, Hyi, mul2(neg2(C3i), Hyr));
+        const float2 Kzr = fma2(C3r, Hzr, mul2(C3i, Hzi)), Kzi = fma2(C3r, Hzi, mul2(neg2(C3i), Hzr));
+        const float2 Lxr = fma2(C3r, Exr, mul2(C3i, Exi)), Lxi = fma2(C3r, Exi, mul2(neg2(C3i), Exr));
+        const float2 Lyr = fma2(C3r, Eyr, mul2(C3i, Eyi)), Lyi = fma2(C3r, Eyi, mul2(neg2(C3i), Eyr));
+        const float2 Lzr = fma2(C3r, Ezr, mul2(C3i, Ezi)), Lzi = fma2(C3r, Ezi, mul2(neg2(C3i), Ezr));
+        // Jbar' += conj(c1) gE + P R_hat + K x R_hat
+        acc[0] = fma2(c1r, Exr, fma2(c1i, Exi, fma2(Pr, ex, fma2(Kyr, ez, fma2(neg2(Kzr), ey, acc[0])))));
+        acc[1] = fma2(c1r, Eyr, fma2(c1i, Eyi, fma2(Pr, ey, fma2(Kzr, ex, fma2(neg2(Kxr), ez, acc[1])))));
+        acc[2] = fma2(c1r, Ezr, fma2(c1i, Ezi, fma2(Pr, ez, fma2(Kxr, ey, fma2(neg2(Kyr), ex, acc[2])))));
+        acc[3] = fma2(c1r, Exi, fma2(neg2(c1i), Exr, fma2(Pi, ex, fma2(Kyi, ez, fma2(neg2(Kzi), ey, acc[3])))));
+        acc[4] = fma2(c1r, Eyi, fma2(neg2(c1i), Eyr, fma2(Pi, ey, fma2(Kzi, ex, fma2(neg2(Kxi), ez, acc[4])))));
+        acc[5] = fma2(c1r, Ezi, fma2(neg2(c1i), Ezr, fma2(Pi, ez, fma2(Kxi, ey, fma2(neg2(Kyi), ex, acc[5])))));
+        // Mbar' += conj(c1) gH + Q R_hat - L x R_hat
+        acc[6] = fma2(c1r, Hxr, fma2(c1i, Hxi, fma2(Qr, ex, fma2(neg2(Lyr), ez, fma2(Lzr, ey, acc[6])))));
+        acc[7] = fma2(c1r, Hyr, fma2(c1i, Hyi, fma2(Qr, ey, fma2(neg2(Lzr), ex, fma2(Lxr, ez, acc[7])))));
+        acc[8] = fma2(c1r, Hzr, fma2(c1i, Hzi, fma2(Qr, ez, fma2(neg2(Lxr), ey, fma2(Lyr, ex, acc[8])))));
+        acc[9] = fma2(c1r, Hxi, fma2(neg2(c1i), Hxr, fma2(Qi, ex, fma2(neg2(Lyi), ez, fma2(Lzi, ey, acc[9])))));
+        acc[10] = fma2(c1r, Hyi, fma2(neg2(c1i), Hyr, fma2(Qi, ey, fma2(neg2(Lzi), ex, fma2(Lxi, ez, acc[10])))));
+        acc[11] = fma2(c1r, Hzi, fma2(neg2(c1i), Hzr, fma2(Qi, ez, fma2(neg2(Lxi), ey, fma2(Lyi, ex, acc[11])))));
+    }
     if (!WANT_D && !WANT_T) return;
 
     // a = conj(gE), b = conj(gH): alpha = a.J (+ b.M), beta = (J.R_hat)(a.R_hat) (+ (M.R_hat)(b.R_hat)),
@@ -244,7 +246,7 @@ __device__ __forceinline__ void adj_nf_pair2(float2 *acc, float2 &vt, const floa
 //   n . grad_d phi = (dphi/dR) (n . d) / R with phi = Re[conj(g) S' c] and
 //   dc/dR = c (-t j k - 1 / R)   (k = 2 pi in turns);
 // no illumination test (the reference's scalar sum has none).
-template <int T, bool WANT_D, bool WANT_T>
+template <int T, bool WANT_C, bool WANT_D, bool WANT_T>
 __device__ __forceinline__ void adj_sc_pair2(float2 *acc, float2 &vt, const float2 *r, const SrcC &s)
 {
     const float2 dhx = sub2(r[0], dup2(s.sh[0])), dhy = sub2(r[1], dup2(s.sh[1])), dhz = sub2(r[2], dup2(s.sh[2]));
@@ -261,8 +263,10 @@ __device__ __forceinline__ void adj_sc_pair2(float2 *acc, float2 &vt, const floa
     const float2 rs = flip_parity(rinv, tq);
     const float2 cr = mul2(cs, rs), ci = mul2(T > 0 ? neg2(sn) : sn, rs);
     const float2 gr = r[6], gi = r[7];
-    acc[0] = fma2(cr, gr, fma2(ci, gi, acc[0]));
-    acc[3] = fma2(cr, gi, fma2(neg2(ci), gr, acc[3]));
+    if (WANT_C) {
+        acc[0] = fma2(cr, gr, fma2(ci, gi, acc[0]));
+        acc[3] = fma2(cr, gi, fma2(neg2(ci), gr, acc[3]));
+    }
     if (!WANT_D && !WANT_T) return;
     // X = conj(g) S', Y = X c, dphi/dR = Re[Y (-1/R - t j 2 pi)] = -Y.re / R + t 2 pi Y.im
     const float2 Sr = dup2(s.J[0]), Si = dup2(s.J[1]);
@@ -306,8 +310,17 @@ __device__ __forceinline__ void adj_band_scan(const float4 *tile, int cnt, long 
     }
 }
 
-template <int KIND, int T, bool HAS_M, bool WANT_D, bool WANT_T>
-__global__ void __launch_bounds__(kThreadsA, HAS_M ? kMinBlocksA2M : kMinBlocksA2)
+// WANT_C: the currents' gradient. Without it (a fixed feed, the gradient with
+// respect to a reflector's shape alone) the 12 current accumulators and the
+// projections that only they use, a third of the pair's work, are left out,
+// with their partials and epilogue rows; grad_dt alone has no partials. The
+// scalar kind keeps its 2 current rows instead of 12. Measured, 40,000 sources
+// x 20,000 targets, ms, with all accumulators / now: ds 6.58 / 3.86, dt 6.91 /
+// 4.15, ds and dt 7.45 / 4.73; with M 8.12 / 5.61, 8.38 / 5.72, 9.37 / 6.61;
+// scalar, all three gradients 1.69 / 1.49.
+template <int KIND, int T, bool HAS_M, bool WANT_C, bool WANT_D, bool WANT_T>
+__global__ void __launch_bounds__(kThreadsA, WANT_C ? (HAS_M ? kMinBlocksA2M : kMinBlocksA2)
+                                                    : (HAS_M ? kMinBlocksA2MN : kMinBlocksA2N))
 po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__restrict__ trec, long nt, long chunk,
                  double *__restrict__ part, double *__restrict__ gt, int *__restrict__ err, BandList bl)
 {
@@ -317,7 +330,8 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
     __shared__ __align__(8) uint64_t full[kStages];
     pdl_wait();
     float *lo = reinterpret_cast<float *>(stage + (size_t)kStages * kPairsA2 * RT);
-    float2 *vbuf = reinterpret_cast<float2 *>(lo + kAccAdj * kThreadsA);   // [kFlush][kThreadsA]
+    constexpr int NROW = adj_rows(KIND, WANT_C, WANT_D);
+    float2 *vbuf = reinterpret_cast<float2 *>(lo + NROW * kThreadsA);   // [kFlush][kThreadsA]
 
     SrcC s;
     const long si = (long)blockIdx.x * kThreadsA + threadIdx.x;
@@ -345,9 +359,9 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
         for (int ri = 0; ri < 2; ++ri) dn[ri] = fmaf(v[4 + ri], s.n[2], fmaf(v[2 + ri], s.n[1], v[ri] * s.n[0]));
     }
 
-    float hi[kAccAdj];
+    float hi[NROW > 0 ? NROW : 1];
 #pragma unroll
-    for (int a = 0; a < kAccAdj; ++a) {
+    for (int a = 0; a < NROW; ++a) {
         hi[a] = 0.f;
         lo[a * kThreadsA + threadIdx.x] = 0.f;
     }
@@ -402,8 +416,8 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
                 }
                 float2 vt = make_float2(0.f, 0.f);
                 if (KIND == kKindNF)
-                    adj_nf_pair2<T, HAS_M, WANT_D, WANT_T>(acc, vt, rec, s, band);
-                else adj_sc_pair2<T, WANT_D, WANT_T>(acc, vt, rec, s);
+                    adj_nf_pair2<T, HAS_M, WANT_C, WANT_D, WANT_T>(acc, vt, rec, s, band);
+                else adj_sc_pair2<T, WANT_C, WANT_D, WANT_T>(acc, vt, rec, s);
                 if (WANT_T) vbuf[(p - fb) * kThreadsA + threadIdx.x] = vt;
             }
             if (WANT_T) {
@@ -439,10 +453,12 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
         }
 #pragma unroll
         for (int a = 0; a < kAccAdj; ++a) {
+            const int r = adj_row(KIND, WANT_C, WANT_D, a);
+            if (r < 0) continue;
             float sm, e;
-            two_sum(hi[a], __fadd_rn(acc[a].x, acc[a].y), sm, e);
-            hi[a] = sm;
-            float &l = lo[a * kThreadsA + threadIdx.x];
+            two_sum(hi[r], __fadd_rn(acc[a].x, acc[a].y), sm, e);
+            hi[r] = sm;
+            float &l = lo[r * kThreadsA + threadIdx.x];
             l = __fadd_rn(l, e);
         }
         if (KIND != kKindScalar && band) adj_band_scan<RT>(tile, cnt, pfirst, s, si, ns, nt, bl);
@@ -452,13 +468,13 @@ po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__rest
     pdl_trigger();
     if (si >= ns) return;
 #pragma unroll
-    for (int a = 0; a < kAccAdj; ++a)
-        part[((long)blockIdx.y * kAccAdj + a) * ns + si] = (double)hi[a] + (double)lo[a * kThreadsA + threadIdx.x];
+    for (int a = 0; a < NROW; ++a)
+        part[((long)blockIdx.y * NROW + a) * ns + si] = (double)hi[a] + (double)lo[a * kThreadsA + threadIdx.x];
 }
 
-int adj_pk_smem_bytes(bool has_m, bool want_t)
+int adj_pk_smem_bytes(int kind, bool has_m, bool want_c, bool want_d, bool want_t)
 {
-    return kStages * kPairsA2 * adj2_rec(has_m, want_t) * 16 + kAccAdj * kThreadsA * 4 +
+    return kStages * kPairsA2 * adj2_rec(has_m, want_t) * 16 + adj_rows(kind, want_c, want_d) * kThreadsA * 4 +
            (want_t ? kFlush * kThreadsA * 8 : 0);
 }
 
@@ -466,28 +482,31 @@ int adj_pk_pairs_per_tile() { return kPairsA2; }
 
 int adj_pk_rec4(bool has_m, bool want_t) { return adj2_rec(has_m, want_t); }
 
-template <int KIND, int T, bool HAS_M, bool WANT_D, bool WANT_T>
-static void *adj_pk_ptr()
+template <int KIND, int T, bool HAS_M, bool WANT_C>
+static void *adj_pk_sel(bool want_d, bool want_t)
 {
-    return reinterpret_cast<void *>(&po_adj_pk_kernel<KIND, T, HAS_M, WANT_D, WANT_T>);
+    if (want_d) return want_t ? reinterpret_cast<void *>(&po_adj_pk_kernel<KIND, T, HAS_M, WANT_C, true, true>)
+                              : reinterpret_cast<void *>(&po_adj_pk_kernel<KIND, T, HAS_M, WANT_C, true, false>);
+    // at least one gradient is wanted
+    if (want_t || !WANT_C) return reinterpret_cast<void *>(&po_adj_pk_kernel<KIND, T, HAS_M, WANT_C, false, true>);
+    return reinterpret_cast<void *>(&po_adj_pk_kernel<KIND, T, HAS_M, true, false, false>);
 }
 
-template <int T, bool HAS_M>
-static void *adj_pk_sel(int kind, bool want_d, bool want_t)
+template <int T>
+static void *adj_pk_kind(int kind, bool has_m, bool want_c, bool want_d, bool want_t)
 {
-    if (kind == kKindScalar) {
-        if (want_d) return want_t ? adj_pk_ptr<kKindScalar, T, false, true, true>()
-                                  : adj_pk_ptr<kKindScalar, T, false, true, false>();
-        return want_t ? adj_pk_ptr<kKindScalar, T, false, false, true>() : adj_pk_ptr<kKindScalar, T, false, false, false>();
-    }
-    if (want_d) return want_t ? adj_pk_ptr<kKindNF, T, HAS_M, true, true>() : adj_pk_ptr<kKindNF, T, HAS_M, true, false>();
-    return want_t ? adj_pk_ptr<kKindNF, T, HAS_M, false, true>() : adj_pk_ptr<kKindNF, T, HAS_M, false, false>();
+    if (kind == kKindScalar) return want_c ? adj_pk_sel<kKindScalar, T, false, true>(want_d, want_t)
+                                           : adj_pk_sel<kKindScalar, T, false, false>(want_d, want_t);
+    if (has_m) return want_c ? adj_pk_sel<kKindNF, T, true, true>(want_d, want_t)
+                             : adj_pk_sel<kKindNF, T, true, false>(want_d, want_t);
+    return want_c ? adj_pk_sel<kKindNF, T, false, true>(want_d, want_t)
+                  : adj_pk_sel<kKindNF, T, false, false>(want_d, want_t);
 }
 
-void *adj_pk_kernel(int kind, int t_sign, bool has_m, bool want_d, bool want_t)
+void *adj_pk_kernel(int kind, int t_sign, bool has_m, bool want_c, bool want_d, bool want_t)
 {
-    if (t_sign < 0) return has_m ? adj_pk_sel<-1, true>(kind, want_d, want_t) : adj_pk_sel<-1, false>(kind, want_d, want_t);
-    return has_m ? adj_pk_sel<1, true>(kind, want_d, want_t) : adj_pk_sel<1, false>(kind, want_d, want_t);
+    return t_sign < 0 ? adj_pk_kind<-1>(kind, has_m, want_c, want_d, want_t)
+                      : adj_pk_kind<1>(kind, has_m, want_c, want_d, want_t);
 }
 
 }  // namespace po

@@ -660,7 +660,8 @@ int run_adjoint(const AdjArgs &a)
     const double *src7 = a.src7, *cur = a.cur, *tgt7 = a.tgt7, *cot = a.cot;
     double *grad_cur = a.grad_cur, *grad_ds = a.grad_ds, *grad_dt = a.grad_dt;
     const unsigned nblk_s = (unsigned)((ns + 255) / 256), nblk_t = (unsigned)((nt + 255) / 256);
-    const bool want_t = grad_dt != nullptr, fp64 = a.precision == 1;
+    const bool want_c = grad_cur != nullptr, want_t = grad_dt != nullptr, fp64 = a.precision == 1;
+    const int rows = adj_rows(kind, want_c, want_d);   // of the source-side partials
     // scalar sources: 2-row currents, S' in the record's J.x slot
     const int scalar = kind == kKindScalar ? 1 : 0;
 
@@ -669,16 +670,19 @@ int run_adjoint(const AdjArgs &a)
     // the same on pairs of targets. Mixed far field: two sources per thread,
     // stages of kFFDirs directions. All fused: currents and displacements in
     // one pass.
-    void *fk = fp64 ? adj_fp64_kernel(kind, has_m, want_d, want_t)
-                    : (far ? ff_adj_kernel(ts, has_m, want_d) : adj_pk_kernel(kind, ts, has_m, want_d, want_t));
-    const int smem = fp64 ? 0 : (far ? ff_adj_smem_bytes(want_d) : adj_pk_smem_bytes(has_m, want_t));
+    void *fk = fp64 ? adj_fp64_kernel(kind, has_m, want_c, want_d, want_t)
+                    : (far ? ff_adj_kernel(ts, has_m, want_c, want_d)
+                           : adj_pk_kernel(kind, ts, has_m, want_c, want_d, want_t));
+    const int smem = fp64 ? 0 : (far ? ff_adj_smem_bytes(want_c, want_d)
+                                     : adj_pk_smem_bytes(kind, has_m, want_c, want_d, want_t));
     const int threads = fp64 ? kThreadsD : (far ? ff_adj_threads() : kThreadsA);
     const int per_block = !fp64 && far ? kTile : threads;   // sources per block
     const long tile_t = fp64 ? kChunkD : (far ? kFFDirs : 2L * adj_pk_pairs_per_tile());
     int occ = 1, rc = 0;
     if ((rc = kernel_occupancy(di, fk, threads, smem, occ))) return rc;
     const long nsb = (ns + per_block - 1) / per_block;
-    const long split = choose_split(nsb, nt, (long)di->sms * occ, partial_cap(ns, kAccAdj), tile_t, far ? 0.0 : kTailNF);
+    const long split = choose_split(nsb, nt, (long)di->sms * occ, partial_cap(ns, std::max(rows, 1)), tile_t,
+                                    far ? 0.0 : kTailNF);
     const long tiles_t = std::max(1L, (nt + tile_t - 1) / tile_t);
     const long per_chunk = (tiles_t + split - 1) / split;
     long chunk = !fp64 && far ? per_chunk : per_chunk * tile_t;   // stages (mixed far field) or targets
@@ -698,7 +702,7 @@ int run_adjoint(const AdjArgs &a)
     int rec = fp64_rec(kind, has_m), rec4 = far ? 0 : adj_pk_rec4(has_m, want_t);
     sc.get(&gam, (size_t)12 * nt);
     if (a.mode == kEHP) sc.get(&eh, (size_t)12 * nt);
-    sc.get(&part, (size_t)split * kAccAdj * ns);
+    sc.get(&part, (size_t)split * rows * ns);
     if (want_t) sc.get(&gt, (size_t)nt);
     if (fp64) {
         sc.get(&srcd, (size_t)ns * rec);
@@ -806,19 +810,21 @@ int run_adjoint(const AdjArgs &a)
             // the near-tangent pairs, decided and summed in FP64 into chunk 0 (and gt)
             double inv_kappa = 1.0 / kappa;
             Wave64 w = wave64(k, t);
+            int wc = want_c, wd = want_d;
             void *xargs[] = {&band, &ns, &src7, &cur, &gmode, &ncx, &ncy, &fac_re, &fac_im, &nt, &tgt7, &gam, &w,
-                             &inv_kappa, &part, &gt, &err};
+                             &inv_kappa, &wc, &wd, &part, &gt, &err};
             rc = launch_pdl(adj_band_fixup_kernel(kind, want_t), dim3(kFixupBlocks), dim3(256), xargs, 0, s);
         }
     }
     long nt_e = want_t ? nt : 0;
     const int groups = nspl >= 8 && ns <= 152L * kEpiThreads ? 8 : 1;   // fewer blocks than SMs: share the chunks
     const long per = kEpiThreads / groups;
+    long nblk_e = rows > 0 ? (ns + per - 1) / per : 0;
     void *eargs[] = {(void *)&kind, &nspl, &ns, &part, &src7, &gmode, &ncx, &ncy, &fac_re, &fac_im, &dsc,
-                     &grad_cur, &grad_ds, &nt_e, &gt, &tsc, &grad_dt};
-    if (!rc) rc = launch_pdl(adj_epilogue_kernel(groups),
-                             dim3((unsigned)((ns + per - 1) / per + (nt_e + kEpiThreads - 1) / kEpiThreads)),
-                             dim3(kEpiThreads), eargs, 0, s);
+                     &grad_cur, &grad_ds, &nblk_e, &nt_e, &gt, &tsc, &grad_dt};
+    if (!rc) rc = launch_pdl(adj_epilogue_kernel(groups, rows),
+                             dim3((unsigned)(nblk_e + (nt_e + kEpiThreads - 1) / kEpiThreads)), dim3(kEpiThreads),
+                             eargs, 0, s);
     if (!rc && a.extent_host && frame) PO_CK_RC(cudaMemcpyAsync(a.extent_host, &frame->m, sizeof(double),
                                                                 cudaMemcpyDeviceToHost, s));
     if (!rc && a.band_host && band.count)

@@ -326,13 +326,13 @@ __device__ __forceinline__ void adj_record64(long i, long nt, const double *tgt7
     if constexpr (KIND == kKindScalar) {
         o[6] = gam[i];
         o[7] = gam[3 * nt + i];
-        return;
+    } else {
+        for (int g = 0; g < 2; ++g)
+            for (int c = 0; c < 3; ++c) {
+                o[6 + 6 * g + 2 * c] = gam[(6 * g + c) * nt + i];
+                o[7 + 6 * g + 2 * c] = gam[(6 * g + 3 + c) * nt + i];
+            }
     }
-    for (int g = 0; g < 2; ++g)
-        for (int c = 0; c < 3; ++c) {
-            o[6 + 6 * g + 2 * c] = gam[(6 * g + c) * nt + i];
-            o[7 + 6 * g + 2 * c] = gam[(6 * g + 3 + c) * nt + i];
-        }
     if (KIND == kKindNF)
         for (int g = 0; g < 2; ++g) {
             const double *v = o + 6 + 6 * g, *n = o + 3;
@@ -398,10 +398,10 @@ __device__ __forceinline__ double dot64(const double *v, const double *z)
 
 // One pair of the FP64 adjoint: the source's record s (kRecD or, without
 // magnetic terms, 12 doubles) against the target record r. acc: the 12
-// current accumulators and n_s . grad_d phi (WANT_D); returns n_t . grad_d
+// current accumulators (WANT_C) and n_s . grad_d phi (WANT_D); returns n_t . grad_d
 // phi (WANT_T). Unlit pairs add nothing. The formulas are those of the mixed
 // kernels (po_adjoint_pk.cu).
-template <int KIND, bool HAS_M, bool WANT_D, bool WANT_T>
+template <int KIND, bool HAS_M, bool WANT_C, bool WANT_D, bool WANT_T>
 __device__ __forceinline__ double adj_pair64(const double *s, const double *r, const Wave64 &w, double *acc)
 {
     if (KIND == kKindFF) {
@@ -411,7 +411,7 @@ __device__ __forceinline__ double adj_pair64(const double *s, const double *r, c
         sincos64(w.k * fma(s[2], r[2], fma(s[1], r[1], s[0] * r[0])), cs, sn);
         const double gs = flip64(sn, w.neg ^ 0x80000000u);   // G = (cs, gs)
 #pragma unroll
-        for (int c = 0; c < 6; ++c) {
+        for (int c = 0; c < (WANT_C ? 6 : 0); ++c) {
             const double gr = r[6 + 2 * c], gi = r[7 + 2 * c];
             const int slot = c < 3 ? c : 6 + (c - 3);
             acc[slot] = fma(gs, gi, fma(cs, gr, acc[slot]));
@@ -436,8 +436,10 @@ __device__ __forceinline__ double adj_pair64(const double *s, const double *r, c
         double cs, sn;
         sincos64(w.k * g.R, cs, sn);
         const double cr = cs * g.rinv, ci = flip64(sn, w.neg ^ 0x80000000u) * g.rinv;
-        acc[0] = fma(cr, r[6], fma(ci, r[7], acc[0]));
-        acc[3] = fma(cr, r[7], fma(-ci, r[6], acc[3]));
+        if (WANT_C) {
+            acc[0] = fma(cr, r[6], fma(ci, r[7], acc[0]));
+            acc[3] = fma(cr, r[7], fma(-ci, r[6], acc[3]));
+        }
         if (!WANT_D && !WANT_T) return 0.0;
         const double xr = fma(r[6], s[6], r[7] * s[7]), xi = fma(r[6], s[7], -(r[7] * s[6]));
         const double yr = fma(xr, cr, -(xi * ci)), yi = fma(xr, ci, xi * cr);
@@ -454,8 +456,10 @@ __device__ __forceinline__ double adj_pair64(const double *s, const double *r, c
     double ger, gei, ghr, ghi;
     dot_re(E, e, ger, gei);
     dot_re(H, e, ghr, ghi);
-    vjp64<1>(c, E, ger, gei, H, e, acc, acc + 3);
-    vjp64<-1>(c, H, ghr, ghi, E, e, acc + 6, acc + 9);
+    if (WANT_C) {
+        vjp64<1>(c, E, ger, gei, H, e, acc, acc + 3);
+        vjp64<-1>(c, H, ghr, ghi, E, e, acc + 6, acc + 9);
+    }
     if (!WANT_D && !WANT_T) return 0.0;
 
     // alpha = a.J + b.M, beta = (J.e)(a.e) + (M.e)(b.e), Z = b x J - a x M, W.v = -v.Z
@@ -539,8 +543,11 @@ __global__ void po_adj_pack_tgt_d_kernel(long nt, const double *__restrict__ tgt
 // shared memory kFlushD at a time. WANT_T: each target's
 // values are summed over the CTA's sources through shared memory and added
 // to gt with one atomicAdd (the order of those varies between runs: gt is
-// reproducible to ~1e-16, not bitwise).
-template <int KIND, bool HAS_M, bool WANT_D, bool WANT_T>
+// reproducible to ~1e-16, not bitwise). Only the accumulators of the
+// gradients asked for are kept (8,000 sources x 8,000 targets, near field, ms:
+// all three 33.0, the two displacements 22.2, the currents and grad_dt 29.7,
+// grad_dt alone 19.4).
+template <int KIND, bool HAS_M, bool WANT_C, bool WANT_D, bool WANT_T>
 __global__ void __launch_bounds__(kThreadsD)
 po_adj_fp64_kernel(const double *__restrict__ src, long ns, const double *__restrict__ trec, long nt, long chunk,
                    Wave64 w, double *__restrict__ part, double *__restrict__ gt)
@@ -564,7 +571,7 @@ po_adj_fp64_kernel(const double *__restrict__ src, long ns, const double *__rest
         if (si < ns) {
 #pragma unroll 1
             for (int q = 0; q < cnt; ++q) {
-                const double v = adj_pair64<KIND, HAS_M, WANT_D, WANT_T>(s, tile + q * TR, w, acc);
+                const double v = adj_pair64<KIND, HAS_M, WANT_C, WANT_D, WANT_T>(s, tile + q * TR, w, acc);
                 if (WANT_T) vbuf[q * (kThreadsD + 1) + threadIdx.x] = v;
             }
         } else if (WANT_T) {
@@ -586,7 +593,10 @@ po_adj_fp64_kernel(const double *__restrict__ src, long ns, const double *__rest
     }
     if (si >= ns) return;
 #pragma unroll
-    for (int a = 0; a < kAccAdj; ++a) part[((long)blockIdx.y * kAccAdj + a) * ns + si] = acc[a];
+    for (int a = 0; a < kAccAdj; ++a) {
+        const int r = adj_row(KIND, WANT_C, WANT_D, a);
+        if (r >= 0) part[((long)blockIdx.y * adj_rows(KIND, WANT_C, WANT_D) + r) * ns + si] = acc[a];
+    }
 }
 
 // The pairs the mixed adjoint left out as inside the tangent band: each is
@@ -600,7 +610,8 @@ __global__ void __launch_bounds__(256)
 po_adj_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, const double *__restrict__ cur,
                          int gmode, int ncx, int ncy, double fac_re, double fac_im, long nt,
                          const double *__restrict__ tgt7, const double *__restrict__ gam, Wave64 w,
-                         double inv_kappa, double *__restrict__ part, double *__restrict__ gt, int *__restrict__ err)
+                         double inv_kappa, int want_c, int want_d, double *__restrict__ part,
+                         double *__restrict__ gt, int *__restrict__ err)
 {
     pdl_wait();
     const unsigned total = *bl.count;
@@ -612,10 +623,11 @@ po_adj_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, 
         src_record_d(pr.x, ns, src7, cur, gmode, ncx, ncy, fac_re, fac_im, 0, kRecD, s);
         adj_record64<KIND>(pr.y, nt, tgt7, gam, r);
         for (int a = 0; a < kAccAdj; ++a) acc[a] = 0.0;
-        const double v = adj_pair64<KIND, true, true, WANT_T>(s, r, w, acc) * inv_kappa;
+        const double v = adj_pair64<KIND, true, true, true, WANT_T>(s, r, w, acc) * inv_kappa;
         for (int a = 0; a < kAccAdj; ++a) {
+            const int row = adj_row(KIND, want_c, want_d, a);
             const double x = a < 12 ? acc[a] : acc[a] * inv_kappa;
-            if (x != 0.0) atomicAdd(&part[(long)a * ns + pr.x], x);
+            if (row >= 0 && x != 0.0) atomicAdd(&part[(long)row * ns + pr.x], x);
         }
         if (WANT_T && v != 0.0) atomicAdd(&gt[pr.y], v);
     }
@@ -645,23 +657,33 @@ void *fp64_kernel(int kind, bool has_m)
                  : reinterpret_cast<void *>(&po_fp64_kernel<kKindFF, false>);
 }
 
-template <int KIND, bool HAS_M>
+template <int KIND, bool HAS_M, bool WANT_C>
 static void *adj_fp64_sel(bool want_d, bool want_t)
 {
-    if constexpr (KIND != kKindFF)
-        if (want_t)
-            return want_d ? reinterpret_cast<void *>(&po_adj_fp64_kernel<KIND, HAS_M, true, true>)
-                          : reinterpret_cast<void *>(&po_adj_fp64_kernel<KIND, HAS_M, false, true>);
-    return want_d ? reinterpret_cast<void *>(&po_adj_fp64_kernel<KIND, HAS_M, true, false>)
-                  : reinterpret_cast<void *>(&po_adj_fp64_kernel<KIND, HAS_M, false, false>);
+    if constexpr (KIND != kKindFF) {
+        if (want_t && want_d) return reinterpret_cast<void *>(&po_adj_fp64_kernel<KIND, HAS_M, WANT_C, true, true>);
+        if (want_t || (!WANT_C && !want_d))
+            return reinterpret_cast<void *>(&po_adj_fp64_kernel<KIND, HAS_M, WANT_C, false, true>);
+    }
+    // at least one gradient is wanted
+    if (want_d || !WANT_C) return reinterpret_cast<void *>(&po_adj_fp64_kernel<KIND, HAS_M, WANT_C, true, false>);
+    return reinterpret_cast<void *>(&po_adj_fp64_kernel<KIND, HAS_M, true, false, false>);
 }
 
-void *adj_fp64_kernel(int kind, bool has_m, bool want_d, bool want_t)
+template <int KIND, bool HAS_M>
+static void *adj_fp64_c(bool want_c, bool want_d, bool want_t)
 {
-    if (kind == kKindScalar) return adj_fp64_sel<kKindScalar, false>(want_d, want_t);
+    return want_c ? adj_fp64_sel<KIND, HAS_M, true>(want_d, want_t) : adj_fp64_sel<KIND, HAS_M, false>(want_d, want_t);
+}
+
+void *adj_fp64_kernel(int kind, bool has_m, bool want_c, bool want_d, bool want_t)
+{
+    if (kind == kKindScalar) return adj_fp64_c<kKindScalar, false>(want_c, want_d, want_t);
     if (kind == kKindNF)
-        return has_m ? adj_fp64_sel<kKindNF, true>(want_d, want_t) : adj_fp64_sel<kKindNF, false>(want_d, want_t);
-    return has_m ? adj_fp64_sel<kKindFF, true>(want_d, want_t) : adj_fp64_sel<kKindFF, false>(want_d, want_t);
+        return has_m ? adj_fp64_c<kKindNF, true>(want_c, want_d, want_t)
+                     : adj_fp64_c<kKindNF, false>(want_c, want_d, want_t);
+    return has_m ? adj_fp64_c<kKindFF, true>(want_c, want_d, want_t)
+                 : adj_fp64_c<kKindFF, false>(want_c, want_d, want_t);
 }
 
 void *adj_pack_tgt_d_kernel(int kind)

@@ -81,6 +81,10 @@ constexpr int kMinBlocksA2 = PO_MINB_A2;
 #define PO_MINB_A2M 2
 #endif
 constexpr int kMinBlocksA2M = PO_MINB_A2M;
+// Without the currents' gradient (120 and 140 registers needed). 40,000
+// sources x 20,000 targets, both displacement gradients, ms: 4.73 at 4 blocks
+// without M (4.83 at 3, 4.80 at 5), 6.61 at 3 with M (6.71 at 2 and at 4).
+constexpr int kMinBlocksA2N = 4, kMinBlocksA2MN = 3;
 constexpr int kMinBlocksFA = 6, kMinBlocksFAM = 4;   // resident CTAs per SM asked of ptxas (M = 0, with M)
 constexpr int kStagesFA = 2;
 constexpr int kFFDirs = 64;   // directions per stage of the far-field adjoint
@@ -90,7 +94,21 @@ constexpr int kFFDirs = 64;   // directions per stage of the far-field adjoint
 constexpr int kMinBlocksFF0 = 5, kUnrollFF0 = 2;
 constexpr int kUnrollF = PO_UNROLL_F;
 constexpr int kUnrollA = PO_UNROLL_A;   // target pairs per iteration of the adjoint pair loop
-constexpr int kAccAdj = 13;
+constexpr int kAccAdj = 13;   // the pair formulas' accumulators: 12 of the currents, 1 of the displacement
+// Of those, the ones that a call's kernels keep, as rows of the partials: the
+// currents' (c; the scalar kind has two, E.x re and im) where that gradient is
+// wanted, then the source displacement's (d). adj_row: accumulator a's row, or -1.
+__host__ __device__ constexpr int adj_rows(int kind, bool c, bool d)
+{
+    return (c ? (kind == kKindScalar ? 2 : 12) : 0) + (d ? 1 : 0);
+}
+__host__ __device__ constexpr int adj_row(int kind, bool c, bool d, int a)
+{
+    if (a == 12) return d ? adj_rows(kind, c, false) : -1;
+    if (!c) return -1;
+    if (kind != kKindScalar) return a;
+    return a == 0 ? 0 : (a == 3 ? 1 : -1);
+}
 
 // Plain FP64 kernels (po_fp64.cu).
 constexpr int kThreadsD = 128;
@@ -205,22 +223,22 @@ void *fp32_probe_kernel();
 void *band_fixup_kernel(int kind, bool has_m);
 void *adj_band_fixup_kernel(int kind, bool want_t);
 void *wait_selftest_kernel();
-void *adj_fp64_kernel(int kind, bool has_m, bool want_d, bool want_t);
+void *adj_fp64_kernel(int kind, bool has_m, bool want_c, bool want_d, bool want_t);
 void *adj_pack_tgt_d_kernel(int kind);
 void *adj_cot_kernel();
 void *adj_pack_kernel();                 // near field, scalar: sources, targets and cotangents
-void *adj_epilogue_kernel(int groups);   // 1 or 8 threads share a source's chunks
+void *adj_epilogue_kernel(int groups, int rows);   // 1 or 8 threads share a source's chunks of `rows` rows
 void *adj_ehp_cot_kernel();
 // Far-field adjoint (po_ff_adjoint.cu): stages of kFFDirs packed directions.
 void *ff_pack_cot_kernel();
-void *ff_adj_kernel(int t_sign, bool has_m, bool want_d);
-int ff_adj_smem_bytes(bool want_d);
+void *ff_adj_kernel(int t_sign, bool has_m, bool want_c, bool want_d);
+int ff_adj_smem_bytes(bool want_c, bool want_d);
 int ff_adj_threads();
 int ff_adj_stage4();   // float4 per stage
 // Pair-packed adjoint, near field and scalar, fused: currents, source and
 // target displacement.
-void *adj_pk_kernel(int kind, int t_sign, bool has_m, bool want_d, bool want_t);
-int adj_pk_smem_bytes(bool has_m, bool want_t);
+void *adj_pk_kernel(int kind, int t_sign, bool has_m, bool want_c, bool want_d, bool want_t);
+int adj_pk_smem_bytes(int kind, bool has_m, bool want_c, bool want_d, bool want_t);
 int adj_pk_pairs_per_tile();
 int adj_pk_rec4(bool has_m, bool want_t);   // float4 per pair-packed cotangent record
 
