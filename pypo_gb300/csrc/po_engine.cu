@@ -35,7 +35,7 @@ struct DeviceInfo {
     bool ready = false;
     int sms = 0;
     cudaMemPool_t pool = nullptr;   // the library's own scratch pool
-    int occ2[3][2][2] = {};  // pair-packed kernels, [kind][t>0][has_m]
+    int occ2[3][2][2] = {};  // near-field and scalar kernels, [kind][t>0][has_m]
     int occ_ff[2][2] = {};   // far-field tile kernels, [t>0][has_m]
     std::map<void *, int> occ_adj;   // adjoint and FP64 kernels: resident CTAs, attribute set
 };
@@ -108,7 +108,7 @@ static int device_info(DeviceInfo *&out)
                 for (int hm = 0; hm < 2; ++hm) {
                     if (kind == kKindFF || (kind == kKindScalar && hm)) continue;   // FF: occ_ff below
                     void *fn = pk_kernel(kind, ts ? 1 : -1, hm != 0);
-                    const int smem = pk_smem_bytes(kind);
+                    const int smem = pk_smem_bytes(kind, hm != 0);
                     PO_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
                     int nb = 0;
                     PO_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kThreads, smem));
@@ -523,12 +523,13 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
             (rc = sc.get(&p.order, 2 * (size_t)n1)) || (rc = sc.take(&p.sort_tmp, p.sort_bytes)))
             return rc;
     } else {
-        const size_t src_f4 = (size_t)((std::max(ns, 1L) + 1) / 2) * (scalar ? kRec2Scalar : kRec2);
+        // 11 float4 (scalar: 4) per two sources: no less than either layout's tiles take
+        const size_t src_f4 = (size_t)((std::max(ns, 1L) + 1) / 2) * (scalar ? 4 : 11);
         if ((rc = sc.get(&p.srcpk, src_f4))) return rc;
     }
     // source chunks: balance waves over the SMs; the partials must fit the scratch left
-    const int tpt = p.far ? 2 : pk_tpt(p.kind);   // targets per thread
-    p.ntb = (nt + (long)kThreads * tpt - 1) / ((long)kThreads * tpt);
+    const long per_block = p.far ? 2L * kThreads : kThreads;   // targets per CTA
+    p.ntb = (nt + per_block - 1) / per_block;
     const int occ = p.far ? di->occ_ff[p.ts > 0][p.has_m ? 1 : 0] : di->occ2[p.kind][p.ts > 0][p.has_m ? 1 : 0];
     const size_t room = std::min(sc.room(), (size_t)1 << 30);
     const long max_chunks = std::max(1L, (long)(room / ((size_t)p.nacc * nt * sizeof(double))));
@@ -590,7 +591,7 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
                         ff_smem_bytes(p.has_m), s);
         else
             rc = launch_pdl(pk_kernel(p.kind, p.ts, p.has_m), dim3((unsigned)p.ntb, (unsigned)p.nsplit), dim3(kThreads),
-                        margs, pk_smem_bytes(p.kind), s);
+                        margs, pk_smem_bytes(p.kind, p.has_m), s);
     }
     timing_mark(s, false);
     if (!rc && p.band.count && ns > 0) {

@@ -4,7 +4,7 @@
 // (near field), :1656-1781 (far field) and :1279-1331 (scalar), written as an
 // N-body kernel:
 //
-//   * sources are packed once, two per record (po_pack_kernel, po_prep.cu): positions in
+//   * sources are packed once, in tiles of 128 (po_pack_kernel, po_prep.cu): positions in
 //     "turn" units (mm * k / 2 pi) relative to a frame origin, split into a
 //     hi part on a power-of-two quantum q (few significant bits, so that
 //     differences and squares of hi parts are exact in FP32) and a small lo
@@ -13,8 +13,8 @@
 //   * a CTA owns 128 targets held in registers and walks its share of the
 //     sources tile by tile; tiles are staged into shared memory by 1-D TMA
 //     bulk copies (cp.async.bulk) completing on mbarriers, 3 stages deep;
-//   * every arithmetic step is a packed FP32x2 operation over the two
-//     sources of a record;
+//   * every arithmetic step is a packed FP32x2 operation over two targets of
+//     a thread; half of the threads take a tile's even sources, half the odd;
 //   * per pair: exact hi separation + lo correction, R^2 exact-plus-small,
 //     R = Rh + res / (2 Rh) by one Newton step, one exact half-turn phase
 //     reduction, sin/cos of the reduced angle only, everything else in FP32;
@@ -22,7 +22,7 @@
 //     so long oscillatory sums stay compensated;
 //   * (M = 0) a tile whose box of normals and positions proves every pair
 //     lit for the CTA's targets runs without the per-pair illumination test
-//     (tile_lit; the boxes travel in the records' spare slot 21);
+//     (tile_lit; the boxes travel ahead of the tile's records);
 //   * the per-pair test counts a pair lit when n . d >= 1e-6 R and unlit
 //     below -1e-6 R; a pair in between is left out, its tile flagged, and the
 //     rare path after the tile's fold lists it (nf_band_scan) for
@@ -48,18 +48,33 @@ namespace po {
 // field; for the far field the same slots hold S_J = sum G J' and S_M; the
 // scalar kind has 2 (re, im).
 
-// ------------------------------------------------ pair-packed kernels
+// -------------------------------------------------- near field and scalar
 //
-// Pair-packed source record (kRec2 float4 per pair of sources a = 2p and
-// b = 2p + 1; every float2 slot holds (value for a, value for b)):
-//   slots 0-2 hi position, 3-5 lo position, 6-8 unit normal,
-//   9-14 J' (re, im) for x, y, z, 15-20 M' likewise, 21 unused.
-// Lane x of every packed operation works on source a and lane y on source b;
-// the thread's target is duplicated into both lanes once. The algebra is the
-// one of nf_pair; the sign (-1)^q of the half-turn sin/cos reduction is folded
-// into u, and the illumination test is a per-lane select of 1/R.
+// Source tile of n <= kTile sources (pk_tile4 float4; po_pack_kernel): near
+// field without M, the tile's box (kBoxF floats); then the records of the
+// even sources and, behind them, of the odd ones, R4 float4 each:
+//   0-2 hi position, 3-5 lo position, 6-8 unit normal, 9-14 J' (re, im) for
+//   x, y, z, 15 unused; with M, 15-20 M' likewise, the last of them (which
+//   would need a sixth float4) in an array behind the records.
+// Scalar: 0-5 positions, 6-7 S'.
+// Lane x of every packed operation works on the thread's first target and
+// lane y on its second: a source's words are 32-bit registers that serve both
+// lanes. A packed fma reads its operands at one 64-bit register a cycle, and
+// such a factor counts half; the loop is bound by those reads, ahead of the
+// FMA pipe (two sources in the lanes, with 64-bit pairs in the record: 80 % of
+// the pipe), and a record is 4 float4 instead of 8. The even and odd sources'
+// sums of a tile stay apart until its end, as the two lanes of such records
+// kept them; by halves of the CTA, a thread needs one set of accumulators, not
+// two, and the CTA still has 128 targets and four warps. Sources in the lanes
+// / now, ms: dish to focal plane 68.24 / 66.98, 40,602 x 10,100 1.310 / 1.280,
+// with M 2.081 / 2.039, scalar 0.461 / 0.443, scalar 10,403 x 14,399 0.185 /
+// 0.173. Both sources in one thread (two sets of accumulators, 172 registers):
+// 66.98, 68.4 at 3 CTAs an SM.
+// The algebra is the one of nf_pair; the sign (-1)^q of the half-turn
+// sin/cos reduction is folded into u, and the illumination test is a per-lane
+// select of 1/R.
 
-// The geometry of a pair record (two sources) against a target, in the
+// The geometry of a source against the two targets, in the
 // split representation: S0 = |d_hi|^2 (exact), S1 the rest of |d|^2, 1/R
 // (approximate), R, d = t - s, and n_s . d. nf_pair2 and nf_band_scan both
 // use these, so the band decision of the scan is the pair loop's, bit for bit.
@@ -91,31 +106,28 @@ __device__ __forceinline__ float2 nf_nd2(const NfGeo2 &g, const float2 *r)
 
 // The rare path of a tile in which some pair fell inside the tangent band:
 // the thread's pairs are tested again, with the pair loop's operations, and
-// each one inside the band is listed for the FP64 fixup (an idle target or
-// a padding source is only left out). tile: the tile's pair records (rec
-// float4 each), cnt of them, the first with source index 2 * pfirst.
-template <int TP, int REC>
-__device__ __forceinline__ void nf_band_scan(const float4 *tile, int cnt, long pfirst, const float2 (*tc)[9],
-                                          long tbase, long ns, long nt, BandList bl)
+// each one inside the band is listed for the FP64 fixup (an idle target is
+// only left out). recs: the thread's half of the tile's records (R4 float4
+// each), cnt of them, record s being source first + 2 s.
+template <int R4>
+__device__ __forceinline__ void nf_band_scan(const float4 *recs, int cnt, long first, const float2 *tc, long t0,
+                                             long t1, long nt, BandList bl)
 {
 #pragma unroll 1
     for (int s = 0; s < cnt; ++s) {
-        float2 rec[10];
+        float2 rec[12];
 #pragma unroll
-        for (int q = 0; q < 5; ++q) {
-            const float4 v = tile[s * REC + q];
-            rec[2 * q] = make_float2(v.x, v.y);
-            rec[2 * q + 1] = make_float2(v.z, v.w);
+        for (int q = 0; q < 3; ++q) {
+            const float4 v = recs[s * R4 + q];
+            rec[4 * q] = dup2(v.x);
+            rec[4 * q + 1] = dup2(v.y);
+            rec[4 * q + 2] = dup2(v.z);
+            rec[4 * q + 3] = dup2(v.w);
         }
-        const long sp = 2 * (pfirst + s);
-#pragma unroll
-        for (int j = 0; j < TP; ++j) {
-            const long ti = tbase + (long)j * kThreads;
-            const NfGeo2 g = nf_geo2(tc[j], tc[j] + 3, rec);
-            const float2 nd = nf_nd2(g, rec), bw = mul2(dup2(kTangentBand), g.Rh);
-            if (fabsf(nd.x) < bw.x && ti < nt && sp < ns) band_defer(bl, sp, ti);
-            if (fabsf(nd.y) < bw.y && ti < nt && sp + 1 < ns) band_defer(bl, sp + 1, ti);
-        }
+        const NfGeo2 g = nf_geo2(tc, tc + 3, rec);
+        const float2 nd = nf_nd2(g, rec), bw = mul2(dup2(kTangentBand), g.Rh);
+        if (fabsf(nd.x) < bw.x && t0 < nt) band_defer(bl, first + 2 * s, t0);
+        if (fabsf(nd.y) < bw.y && t1 < nt) band_defer(bl, first + 2 * s, t1);
     }
 }
 
@@ -195,7 +207,7 @@ __device__ __forceinline__ void nf_pair2(float2 *acc, const float2 *th, const fl
     }
 }
 
-// Scalar, pair-packed: acc += S' e^{-t j k r} / r. Record slots: 0-2 hi,
+// Scalar: acc += S' e^{-t j k r} / r. Record: 0-2 hi,
 // 3-5 lo, 6-7 S' (re, im) with prefactor, weights and k/2pi folded in.
 template <int T>
 __device__ __forceinline__ void sc_pair2(float2 *acc, const float2 *tc, const float2 *r)
@@ -220,20 +232,16 @@ __device__ __forceinline__ void sc_pair2(float2 *acc, const float2 *tc, const fl
 // Whether every (source, target) pair of a tile passes the illumination
 // test, proven from the tile's box and the CTA's target box tb (lo xyz,
 // hi xyz, a bound on |t|_1). The tile's box (po_pack_kernel: lowest and
-// highest normal xyz, largest n.s, largest |s|_1) travels with the tile in
-// the unused slot 21 of its first four pair records, so it arrives in
-// shared memory with the tile's copy: n.(t - s) >= min over the boxes of
+// highest normal xyz, largest n.s, largest |s|_1) travels ahead of the
+// tile's records, so it arrives in shared memory with the tile's copy:
+// n.(t - s) >= min over the boxes of
 // n.t - max n.s, required above a margin of 1e-5 (|t|_1 + |s|_1) for the
 // FP32 rounding of both sides (a pair is lit for the per-pair test when
 // n.d >= 1e-6 R, kTangentBand). The least of
 // n t over n in [a, b], t in [c, d] is the least of the four corner products.
-template <int REC>
 __device__ __forceinline__ bool tile_lit(const float4 *tile, const float *tb)
 {
-    const float *f = reinterpret_cast<const float *>(tile);
-    float bx[kBoxF];
-#pragma unroll
-    for (int q = 0; q < kBoxF; ++q) bx[q] = f[(q >> 1) * REC * 4 + 42 + (q & 1)];
+    const float *bx = reinterpret_cast<const float *>(tile);
     float L = 0.0f;
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -243,50 +251,50 @@ __device__ __forceinline__ bool tile_lit(const float4 *tile, const float *tb)
     return L - bx[6] >= 1e-5f * (tb[6] + bx[7]);
 }
 
-// Pair-packed main kernel of all three kinds. Grid = (target blocks, source
-// chunks): blockIdx.y picks a chunk of sources (a multiple of kTile, so
-// chunks start on a pair boundary), whose tiles of kTile/2 pair records
-// stream through kStages TMA stages. The thread's target (hi xyz, lo xyz)
-// is duplicated into both lanes once. With `boxes` (the records carry them), a near-field tile proven lit for the CTA skips the
-// per-pair illumination test (M = 0 kernels). The far field has its own
-// kernel (po_farfield.cu).
-template <int KIND, int T, bool HAS_M, int TP>
-__global__ void __launch_bounds__(kThreads, HAS_M ? kMinBlocksM : kMinBlocks)
+// Main kernel of the near field and the scalar kind. Grid = (blocks of
+// kThreads targets, source chunks): blockIdx.y picks a chunk of sources (a
+// multiple of kTile), whose tiles stream through kStages TMA stages. The
+// first half of the CTA's threads works on the tiles' even sources, the
+// second on the odd ones; each thread has two targets, one per lane. At a
+// tile's end the halves exchange half of their FP32 partials each, add them
+// and fold the sums into their float-float totals. With `boxes`, a near-field
+// tile proven lit for the CTA skips the per-pair illumination test (M = 0
+// kernels). The far field has its own kernel (po_farfield.cu).
+template <int KIND, int T, bool HAS_M>
+__global__ void __launch_bounds__(kThreads, pk_min_blocks(KIND, HAS_M))
 po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *__restrict__ tgt, long nt,
              double *__restrict__ part, int *__restrict__ err, int boxes, BandList bl)
 {
-    constexpr int PT = kTile / 2;                                       // pairs per tile
-    constexpr int REC = KIND == kKindScalar ? kRec2Scalar : kRec2;      // float4 per pair record
-    constexpr int NLD = KIND == kKindScalar ? kRec2Scalar : (HAS_M ? kRec2 : 8);   // float4 read per pair
+    constexpr int HEAD = pk_head(KIND, HAS_M), R4 = pk_rec4(KIND, HAS_M), T4 = pk_tile4(KIND, HAS_M, kTile);
     constexpr int NACC = KIND == kKindScalar ? 2 : kAcc;
-    extern __shared__ __align__(128) float4 stage[];   // kStages * PT * REC, then the compensation words
+    constexpr int NF = NACC / 2;          // accumulators that a thread folds
+    constexpr int HT = kThreads / 2;      // threads of a half
+    constexpr int NR = 4 * R4 + (HAS_M ? 1 : 0);
+    constexpr int UNROLL = pk_unroll(KIND, HAS_M);
+    extern __shared__ __align__(128) float4 stage[];   // kStages tiles, the exchange, the compensation words
     __shared__ __align__(8) uint64_t full[kStages];
     pdl_wait();
 
-    const long tbase = (long)blockIdx.x * kThreads * TP + threadIdx.x;
-    float2 tc[TP][9];
+    const int half = threadIdx.x / HT, l = threadIdx.x % HT;
+    const long ti[2] = {(long)blockIdx.x * kThreads + l, (long)blockIdx.x * kThreads + HT + l};
+    float2 tc[6];   // hi xyz, lo xyz; lanes: the two targets
 #pragma unroll
-    for (int j = 0; j < TP; ++j) {
-        const long ti = tbase + (long)j * kThreads;
+    for (int j = 0; j < 2; ++j) {
         float4 a = make_float4(0.f, 0.f, 1.0f, 0.f);   // idle lanes: R > 0
         float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (ti < nt) {
-            a = tgt[2 * ti];
-            c = tgt[2 * ti + 1];
+        if (ti[j] < nt) {
+            a = tgt[2 * ti[j]];
+            c = tgt[2 * ti[j] + 1];
         }
-        tc[j][0] = dup2(a.x);
-        tc[j][1] = dup2(a.y);
-        tc[j][2] = dup2(a.z);
-        tc[j][3] = dup2(a.w);
-        tc[j][4] = dup2(c.x);
-        tc[j][5] = dup2(c.y);
-        tc[j][6] = dup2(a.x + a.w);
-        tc[j][7] = dup2(a.y + c.x);
-        tc[j][8] = dup2(a.z + c.y);
+        const float v[6] = {a.x, a.y, a.z, a.w, c.x, c.y};
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+            if (j == 0) tc[q].x = v[q];
+            else tc[q].y = v[q];
     }
 
     // The CTA's target box for the lit-tile proof: positions (hi + lo, turns)
-    // or directions, and a bound on |t|_1, over its real targets. The proof
+    // and a bound on |t|_1, over its real targets. The proof
     // and its second copy of the pair loop are built for M = 0 only: with the
     // magnetic terms the two-copy kernel measured slower in both copies
     // (feed 101^2 -> dish 101^2, JM: 0.566 ms with one copy, 0.592 lit and
@@ -297,11 +305,11 @@ po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *
     if (kLitPath) {
         float v[6] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
-        for (int j = 0; j < TP; ++j) {
-            if (tbase + (long)j * kThreads >= nt) continue;
+        for (int j = 0; j < 2; ++j) {
+            if (ti[j] >= nt) continue;
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                const float x = tc[j][c].x + tc[j][3 + c].x;
+                const float x = j == 0 ? tc[c].x + tc[3 + c].x : tc[c].y + tc[3 + c].y;
                 v[c] = fminf(v[c], x);
                 v[3 + c] = fmaxf(v[3 + c], x);
             }
@@ -329,20 +337,19 @@ po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *
         }
     }
 
-    float hi[TP][NACC];
-    float *lo = reinterpret_cast<float *>(stage + (size_t)kStages * PT * REC);
+    // Totals of accumulators half * NF + a; lanes: targets.
+    float2 hi[NF];
+    float2 *ex = reinterpret_cast<float2 *>(stage + (size_t)kStages * T4);   // [NF][kThreads]
+    float2 *lo = ex + NF * kThreads;
 #pragma unroll
-    for (int j = 0; j < TP; ++j)
-#pragma unroll
-        for (int a = 0; a < NACC; ++a) {
-            hi[j][a] = 0.f;
-            lo[(a * TP + j) * kThreads + threadIdx.x] = 0.f;
-        }
+    for (int a = 0; a < NF; ++a) {
+        hi[a] = make_float2(0.f, 0.f);
+        lo[a * kThreads + threadIdx.x] = make_float2(0.f, 0.f);
+    }
 
     const long s0 = (long)blockIdx.y * chunk;
     const long s1 = min(ns, s0 + chunk);
-    const long p0 = s0 / 2, p1 = (s1 + 1) / 2;
-    const int ntiles = p1 > p0 ? (int)((p1 - p0 + PT - 1) / PT) : 0;
+    const int ntiles = s1 > s0 ? (int)((s1 - s0 + kTile - 1) / kTile) : 0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) mbar_init(&full[s], 1);
@@ -351,13 +358,12 @@ po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *
     __syncthreads();
 
     auto issue = [&](int it) {
-        const long first = p0 + (long)it * PT;
-        const long cnt = min((long)PT, p1 - first);
-        const uint32_t bytes = (uint32_t)(cnt * REC * sizeof(float4));
+        const long first = s0 + (long)it * kTile;
+        const uint32_t bytes = (uint32_t)(pk_tile4(KIND, HAS_M, (int)min((long)kTile, s1 - first)) * sizeof(float4));
         uint64_t *bar = &full[it % kStages];
         fence_proxy_async();
         mbar_expect_tx(bar, bytes);
-        tma_load_1d(stage + (size_t)(it % kStages) * PT * REC, src + first * REC, bytes, bar);
+        tma_load_1d(stage + (size_t)(it % kStages) * T4, src + first / kTile * T4, bytes, bar);
     };
     if (threadIdx.x == 0)
         for (int it = 0; it < ntiles && it < kStages; ++it) issue(it);
@@ -370,56 +376,59 @@ po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *
             aborted = true;
             break;
         }
-        const float4 *tile = stage + (size_t)(it % kStages) * PT * REC;
-        const int cnt = (int)min((long)PT, p1 - (p0 + (long)it * PT));
-        float2 acc[TP][NACC];
+        const float4 *tile = stage + (size_t)(it % kStages) * T4;
+        const long first = s0 + (long)it * kTile;
+        const int n = (int)min((long)kTile, s1 - first);
+        const int ne = (n + 1) / 2, cnt = half ? n - ne : ne;   // the thread's records
+        const float4 *recs = tile + HEAD + (half ? ne * R4 : 0);
+        const float *last = reinterpret_cast<const float *>(tile + n * R4) + (half ? ne : 0);   // M'z im
+        float2 acc[NACC];
 #pragma unroll
-        for (int j = 0; j < TP; ++j)
-#pragma unroll
-            for (int a = 0; a < NACC; ++a) acc[j][a] = make_float2(0.f, 0.f);
+        for (int a = 0; a < NACC; ++a) acc[a] = make_float2(0.f, 0.f);
 
         bool band = false;   // a pair of this tile fell inside the tangent band
         auto pairs = [&](auto lit_c) {
             constexpr bool LIT = decltype(lit_c)::value;
-#pragma unroll kUnrollF
+#pragma unroll UNROLL
             for (int s = 0; s < cnt; ++s) {
-                float2 rec[2 * NLD];
+                float2 rec[NR];
 #pragma unroll
-                for (int q = 0; q < NLD; ++q) {
-                    const float4 v = tile[s * REC + q];
-                    rec[2 * q] = make_float2(v.x, v.y);
-                    rec[2 * q + 1] = make_float2(v.z, v.w);
+                for (int q = 0; q < R4; ++q) {
+                    const float4 v = recs[s * R4 + q];
+                    rec[4 * q] = dup2(v.x);
+                    rec[4 * q + 1] = dup2(v.y);
+                    rec[4 * q + 2] = dup2(v.z);
+                    rec[4 * q + 3] = dup2(v.w);
                 }
-#pragma unroll
-                for (int j = 0; j < TP; ++j) {
-                    if (KIND == kKindNF) nf_pair2<T, HAS_M, LIT>(acc[j], tc[j], tc[j] + 3, rec, band);
-                    else sc_pair2<T>(acc[j], tc[j], rec);
-                }
+                if (HAS_M) rec[NR - 1] = dup2(last[s]);
+                if (KIND == kKindNF) nf_pair2<T, HAS_M, LIT>(acc, tc, tc + 3, rec, band);
+                else sc_pair2<T>(acc, tc, rec);
             }
         };
         // block-uniform: every thread reads the same tile box and target box
-        // (a tile of fewer than 4 pair records carries no box)
         if constexpr (kLitPath) {
-            if (boxes && cnt >= 4 && tile_lit<REC>(tile, tbox))
+            if (boxes && tile_lit(tile, tbox))
                 pairs(std::true_type{});
             else
                 pairs(std::false_type{});
         } else {
             pairs(std::false_type{});
         }
+        // the partner (the other half's thread with the same targets) gets the
+        // accumulators that it folds
 #pragma unroll
-        for (int j = 0; j < TP; ++j)
-#pragma unroll
-            for (int a = 0; a < NACC; ++a) {
-                float s, e;
-                two_sum(hi[j][a], __fadd_rn(acc[j][a].x, acc[j][a].y), s, e);
-                hi[j][a] = s;
-                float &l = lo[(a * TP + j) * kThreads + threadIdx.x];
-                l = __fadd_rn(l, e);
-            }
-        if (KIND == kKindNF && band) nf_band_scan<TP, REC>(tile, cnt, p0 + (long)it * PT, tc, tbase, ns, nt, bl);
+        for (int a = 0; a < NF; ++a) ex[a * kThreads + threadIdx.x] = half ? acc[a] : acc[NF + a];
+        if (KIND == kKindNF && band) nf_band_scan<R4>(recs, cnt, first + half, tc, ti[0], ti[1], nt, bl);
         __syncthreads();
         if (threadIdx.x == 0 && it + kStages < ntiles) issue(it + kStages);
+#pragma unroll
+        for (int a = 0; a < NF; ++a) {
+            float2 s, e;
+            two_sum2(hi[a], add2(half ? acc[NF + a] : acc[a], ex[a * kThreads + (threadIdx.x ^ HT)]), s, e);
+            hi[a] = s;
+            float2 &c = lo[a * kThreads + threadIdx.x];
+            c = add2(c, e);
+        }
     }
 
     if (aborted) {
@@ -430,13 +439,11 @@ po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *
 
     pdl_trigger();
 #pragma unroll
-    for (int j = 0; j < TP; ++j) {
-        const long ti = tbase + (long)j * kThreads;
-        if (ti >= nt) continue;
-#pragma unroll
-        for (int a = 0; a < NACC; ++a)
-            part[((long)blockIdx.y * NACC + a) * nt + ti] =
-                (double)hi[j][a] + (double)lo[(a * TP + j) * kThreads + threadIdx.x];
+    for (int a = 0; a < NF; ++a) {
+        const float2 c = lo[a * kThreads + threadIdx.x];
+        double *row = part + ((long)blockIdx.y * NACC + half * NF + a) * nt;
+        if (ti[0] < nt) row[ti[0]] = (double)hi[a].x + (double)c.x;
+        if (ti[1] < nt) row[ti[1]] = (double)hi[a].y + (double)c.y;
     }
 }
 
@@ -603,7 +610,7 @@ __global__ void __launch_bounds__(256) po_fp32_probe_kernel(int iters, float see
 template <int KIND, int T, bool HAS_M>
 static void *pk_ptr()
 {
-    return reinterpret_cast<void *>(&po_pk_kernel<KIND, T, HAS_M, pk_tpt(KIND)>);
+    return reinterpret_cast<void *>(&po_pk_kernel<KIND, T, HAS_M>);
 }
 
 void *pk_kernel(int kind, int t_sign, bool has_m)

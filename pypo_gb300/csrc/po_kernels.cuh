@@ -30,13 +30,18 @@ constexpr int kKindScalar = 2;  // scalar Green's function
 constexpr int kThreads = PO_THREADS;   // threads per CTA
 constexpr int kTile = PO_TILE;         // sources per shared-memory stage
 constexpr int kMinBlocks = PO_MINB;    // resident CTAs per SM asked of ptxas
-#ifndef PO_MINB_M
-// The near-field forward with magnetic currents: 5 CTAs/SM hold it at 90
-// registers (feed -> dish JM forward 0.673 -> 0.624 ms); asking the M = 0
-// kernel for 5 as well slows dish_eh's forward (68.4 -> 70.1 ms).
-#define PO_MINB_M 5
-#endif
-constexpr int kMinBlocksM = PO_MINB_M;
+// The near-field and scalar forward: resident CTAs per SM asked of ptxas and
+// records per iteration. Near field, M = 0, dish to focal plane 251,001 x
+// 90,601, ms: 66.98 at 4 CTAs and 3 records (1 record 67.51, 2 67.43, 4 67.30;
+// 3 CTAs 67.4-68.2, 5 CTAs 67.1-68.0, 6 68.9). With M, 40,602 x 10,100: 2.039
+// at 5 and 4 (1 record 2.084, 3 2.056; 4 CTAs 2.047-2.089). Scalar, same size:
+// 0.443 with 4 records (1 0.478, 2 0.452, 3 0.441; 10,403 x 14,399 0.173,
+// 0.199, 0.177, 0.177).
+__host__ __device__ constexpr int pk_min_blocks(int kind, bool has_m)
+{
+    return kind == kKindScalar ? 1 : (has_m ? 5 : 4);
+}
+__host__ __device__ constexpr int pk_unroll(int kind, bool has_m) { return kind == kKindNF && !has_m ? 3 : 4; }
 #ifndef PO_STAGES
 #define PO_STAGES 3
 #endif
@@ -44,24 +49,15 @@ constexpr int kStages = PO_STAGES;     // TMA pipeline depth
 constexpr int kRec = 6;         // float4 per packed source record (96 B)
 constexpr int kRecScalar = 2;   // float4 per packed scalar record (32 B)
 constexpr int kAcc = 12;        // accumulators per target (E, H re/im x y z)
-constexpr int kRec2 = 11;       // float4 per pair-packed record (two sources), near and far field
-constexpr int kRec2Scalar = 4;  // float4 per pair-packed scalar record
 constexpr int kBoxF = 8;        // floats per source-tile box (lit-tile proof)
 #ifndef PO_MUFU_SINCOS
 #define PO_MUFU_SINCOS 1         // 0: the polynomial sin/cos (accuracy comparisons)
 #endif
-// Targets per thread of the pair-packed kernel (near field, scalar): one; a
-// second costs the near field 0.9 % (162 registers). The far-field kernel
-// (po_farfield.cu) takes two directions per thread.
-__host__ __device__ constexpr int pk_tpt(int) { return 1; }
 constexpr uint32_t kWaitLimit = 1u << 24;   // bounded mbarrier polls
 
 // Adjoint kernels: one source (or target) per thread; 12 current
 // accumulators + 1 displacement accumulator.
 constexpr int kThreadsA = PO_THREADS_A;
-#ifndef PO_UNROLL_F
-#define PO_UNROLL_F 1            // pair records per iteration of the forward pair loop
-#endif
 #ifndef PO_UNROLL_A
 #define PO_UNROLL_A 1            // target pairs per iteration of the adjoint pair loop
 #endif
@@ -92,7 +88,6 @@ constexpr int kFFDirs = 64;   // directions per stage of the far-field adjoint
 // iteration at 5 CTAs/SM: 105.1 ms on 1,002,001 x 160,801 (one record 112.3;
 // at 4 CTAs/SM 109.7 with one, 111.7 with two, 109.4 with four).
 constexpr int kMinBlocksFF0 = 5, kUnrollFF0 = 2;
-constexpr int kUnrollF = PO_UNROLL_F;
 constexpr int kUnrollA = PO_UNROLL_A;   // target pairs per iteration of the adjoint pair loop
 constexpr int kAccAdj = 13;   // the pair formulas' accumulators: 12 of the currents, 1 of the displacement
 // Of those, the ones that a call's kernels keep, as rows of the partials: the
@@ -203,11 +198,20 @@ void *ff_key_kernel();
 void *ff_pack_kernel(bool has_m);
 void *ff_kernel(int t_sign, bool has_m);
 
-// Pair-packed main kernel: stages plus the compensation words.
-inline int pk_smem_bytes(int kind)
+// Source tiles of the near-field and scalar forward (layout in po_kernels.cu):
+// float4 ahead of the records, per record, and of a tile of n sources.
+__host__ __device__ constexpr int pk_head(int kind, bool has_m) { return kind != kKindScalar && !has_m ? kBoxF / 4 : 0; }
+__host__ __device__ constexpr int pk_rec4(int kind, bool has_m) { return kind == kKindScalar ? 2 : (has_m ? 5 : 4); }
+__host__ __device__ constexpr int pk_tile4(int kind, bool has_m, int n)
 {
-    const bool sc = kind == kKindScalar;
-    return kStages * (kTile / 2) * (sc ? kRec2Scalar : kRec2) * 16 + (sc ? 2 : kAcc) * pk_tpt(kind) * kThreads * 4;
+    return pk_head(kind, has_m) + n * pk_rec4(kind, has_m) + (kind != kKindScalar && has_m ? (n + 3) / 4 : 0);
+}
+
+// Stages, the halves' exchange and the compensation words.
+inline int pk_smem_bytes(int kind, bool has_m)
+{
+    const int na = kind == kKindScalar ? 1 : kAcc / 2;
+    return kStages * pk_tile4(kind, has_m, kTile) * 16 + 2 * na * kThreads * 8;
 }
 
 void *pk_kernel(int kind, int t_sign, bool has_m);

@@ -155,14 +155,11 @@ __device__ __forceinline__ void pack_target(long i, long nt, const double *tgt7,
     out[2 * i + 1] = make_float4(l[1], l[2], 0.f, 0.f);
 }
 
-// Blocks 0 .. tiles-1: one tile of kTile sources each, as pair-packed records
-// (layouts in po_kernels.cu; SCALAR: kRec2Scalar float4 per pair, else kRec2),
-// assembled in shared memory and written out in coalesced float4. An odd
-// source count pads the last pair with a copy of the last source carrying
-// zero currents. Near field, M = 0 (near field, M = 0) the tile's box for the
-// lit-tile proof goes into the unused slot 21 of its first four pair
-// records: lowest normal xyz, highest normal xyz, largest n.s, largest |s|_1
-// (s = hi + lo, turns); the padding source changes nothing there.
+// Blocks 0 .. tiles-1: one tile of kTile sources each (layout in
+// po_kernels.cu), assembled in shared memory and written out in coalesced
+// float4. Near field, M = 0: the tile's box for the lit-tile proof goes ahead
+// of the records: lowest normal xyz, highest normal xyz, largest n.s, largest
+// |s|_1 (s = hi + lo, turns).
 // The remaining blocks: kTile targets each. far: no source tiles here (the
 // far field packs them in curve order), and the targets are directions.
 template <bool SCALAR, bool HAS_M>
@@ -171,8 +168,9 @@ po_pack_kernel(long ns, const double *__restrict__ src7, const double *__restric
                const Frame *__restrict__ frp, double fac_re, double fac_im, long tiles,
                float4 *__restrict__ src, long nt, const double *__restrict__ tgt7, int far, float4 *__restrict__ tgt)
 {
-    constexpr int R4 = SCALAR ? kRec2Scalar : kRec2;
-    __shared__ __align__(16) float4 buf[kTile / 2 * R4];
+    constexpr int KIND = SCALAR ? kKindScalar : kKindNF;
+    constexpr int HEAD = pk_head(KIND, HAS_M), R4 = pk_rec4(KIND, HAS_M), T4 = pk_tile4(KIND, HAS_M, kTile);
+    __shared__ __align__(16) float4 buf[T4];
     __shared__ float wbox[kTile / 32][kBoxF];
     pdl_wait();
     const Frame fr = *frp;
@@ -183,41 +181,42 @@ po_pack_kernel(long ns, const double *__restrict__ src7, const double *__restric
         return;
     }
     const long first = (long)blockIdx.x * kTile, i = first + threadIdx.x;
-    const int np = (int)(min((long)kTile, ns - first) + 1) / 2;   // pairs of this tile
-    float v[2 * R4];
-    if ((int)threadIdx.x < 2 * np) {
-        const long k = i < ns ? i : ns - 1;
-        for (int c = 0; c < 3; ++c) split_hi_lo((src7[c * ns + k] - fr.o[c]) * fr.kappa, fr, v[c], v[3 + c]);
-        const double w = i < ns ? trap_weight(k, gmode, ncx, ncy) * src7[6 * ns + k] : 0.0;
+    const int n = (int)min((long)kTile, ns - first);   // sources of this tile
+    const bool real = (int)threadIdx.x < n;
+    float v[4 * R4 + 1];
+    if (real) {
+        for (int c = 0; c < 3; ++c) split_hi_lo((src7[c * ns + i] - fr.o[c]) * fr.kappa, fr, v[c], v[3 + c]);
+        const double w = trap_weight(i, gmode, ncx, ncy) * src7[6 * ns + i];
         const double fr_ = fac_re * w, fi_ = fac_im * w;
         if (SCALAR) {
-            const double re = cur[k], im = cur[ns + k];
+            const double re = cur[i], im = cur[ns + i];
             v[6] = (float)(fr_ * re - fi_ * im);
             v[7] = (float)(fr_ * im + fi_ * re);
         } else {
-            for (int c = 0; c < 3; ++c) v[6 + c] = (float)src7[(3 + c) * ns + k];
+            for (int c = 0; c < 3; ++c) v[6 + c] = (float)src7[(3 + c) * ns + i];
 #pragma unroll
-            for (int q = 0; q < 6; ++q) {
-                if (!HAS_M && q >= 3) {   // the M = 0 kernels do not read M'
-                    v[9 + 2 * q] = v[10 + 2 * q] = 0.f;
-                    continue;
-                }
+            for (int q = 0; q < (HAS_M ? 6 : 3); ++q) {
                 const int grp = q / 3, ax = q % 3;
-                const double re = cur[(grp * 6 + ax) * ns + k];
-                const double im = cur[(grp * 6 + 3 + ax) * ns + k];
+                const double re = cur[(grp * 6 + ax) * ns + i];
+                const double im = cur[(grp * 6 + 3 + ax) * ns + i];
                 v[9 + 2 * q] = (float)(fr_ * re - fi_ * im);
                 v[10 + 2 * q] = (float)(fr_ * im + fi_ * re);
             }
-            v[2 * R4 - 1] = 0.f;
+            if (!HAS_M) v[15] = 0.f;
         }
-        float *o = reinterpret_cast<float *>(buf) + (threadIdx.x >> 1) * (R4 * 4) + (threadIdx.x & 1);
+        // even sources first, then the odd ones
+        const int pos = (threadIdx.x >> 1) + (threadIdx.x & 1) * ((n + 1) / 2);
 #pragma unroll
-        for (int q = 0; q < 2 * R4; ++q) o[2 * q] = v[q];
+        for (int q = 0; q < R4; ++q)
+            buf[HEAD + pos * R4 + q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        if (!SCALAR && HAS_M) reinterpret_cast<float *>(buf + n * R4)[pos] = v[4 * R4];
     }
-    if (!SCALAR && !HAS_M) {
+    if (!SCALAR && HAS_M && (int)threadIdx.x >= n && (int)threadIdx.x < (n + 3) / 4 * 4)
+        reinterpret_cast<float *>(buf + n * R4)[threadIdx.x] = 0.f;
+    if (HEAD > 0) {
         float x[kBoxF] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F,
                           -CUDART_INF_F, 0.0f};
-        if ((int)threadIdx.x < 2 * np) {
+        if (real) {
             float s[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
@@ -242,12 +241,12 @@ po_pack_kernel(long ns, const double *__restrict__ src7, const double *__restric
             const int q = threadIdx.x;
             float r = wbox[0][q];
             for (int w = 1; w < kTile / 32; ++w) r = q < 3 ? fminf(r, wbox[w][q]) : fmaxf(r, wbox[w][q]);
-            if (q / 2 < np) reinterpret_cast<float *>(buf)[(q / 2) * (R4 * 4) + 42 + (q & 1)] = r;
+            reinterpret_cast<float *>(buf)[q] = r;
         }
     }
     __syncthreads();
-    float4 *dst = src + (size_t)blockIdx.x * (kTile / 2) * R4;
-    for (int q = threadIdx.x; q < np * R4; q += kTile) dst[q] = buf[q];
+    float4 *dst = src + (size_t)blockIdx.x * T4;
+    for (int q = threadIdx.x; q < pk_tile4(KIND, HAS_M, n); q += kTile) dst[q] = buf[q];
     pdl_trigger();
 }
 
