@@ -7,7 +7,7 @@
 // point, written straight into the 7-row device layout the propagation entry
 // points take (x, y, z, nx, ny, nz, area; index i*ncy + j). The optional
 // surface error (:852-866) keeps the reference's random sequence, drawn on
-// the device (po_mt_normals_kernel): mt19937 seeded with rms_seed and a fresh
+// the device (normal_deviates_dev): mt19937 seeded with rms_seed and a fresh
 // normal distribution per point (src/include/Random.h:112-116), applied along
 // the normals by a second kernel.
 //
@@ -16,6 +16,8 @@
 // the device at every grid point.
 #include <cuda_runtime.h>
 
+#include <algorithm>
+#include <cmath>
 #include <cstdint>
 #include <string>
 
@@ -220,15 +222,19 @@ int generate_grid_dev(const reflparams &r, double *out7, bool transform, bool sp
 // Marsaglia's polar method, x, y = 2U - 1 until 0 < r2 = x^2 + y^2 <= 1, then
 // y sqrt(-2 ln r2 / r2) stdev, the other deviate of the pair dropped. So each
 // attempt takes four outputs, and a block of 624 outputs is exactly 156
-// attempts. One CTA: per block, the twist in three phases (each phase reads
-// only words that are old or already final), the tempering (thread t holds
-// output t), the 156 attempts in parallel, and a warp-ballot scan that
-// places the accepted deviates in order.
+// attempts, of which pi / 4 are accepted.
+//
+// Only the twist is a serial chain: one CTA writes the generator's words, then
+// all SMs count the accepted attempts and write their deviates in order. (One
+// CTA for all of it waited 13 us per block, most of it for the FP64 logarithm,
+// division and root: 2,070 deviates 174 us, now 22; 200,000 21.1 ms, now 0.39.)
 
 namespace {
 
 constexpr int kMtN = 624;
-constexpr int kMtThreads = 640;
+constexpr int kMtThreads = 256;          // the twist's CTA: 227 threads work
+constexpr long kMtRound = 4096;          // blocks of words kept at a time (10 MB)
+constexpr int kMtAttempts = 256;         // attempts per CTA
 
 __device__ __forceinline__ uint32_t mt_twist(uint32_t cur, uint32_t next, uint32_t tap)
 {
@@ -242,93 +248,144 @@ __device__ __forceinline__ double mt_canonical(uint32_t w0, uint32_t w1)
     return u < 1.0 ? u : 1.0 - 0x1p-53;
 }
 
+__device__ __forceinline__ uint32_t mt_temper(uint32_t w)
+{
+    w ^= w >> 11;
+    w ^= (w << 7) & 0x9d2c5680u;
+    w ^= (w << 15) & 0xefc60000u;
+    return w ^ (w >> 18);
+}
+
+// Attempt a of the round: accepted or not; y and r2 of the polar method.
+__device__ __forceinline__ bool mt_attempt(const uint4 *words, long a, long n, double &y, double &r2)
+{
+    if (a >= n) return false;
+    const uint4 w = words[a];
+    const double x = __dsub_rn(__dmul_rn(2.0, mt_canonical(mt_temper(w.x), mt_temper(w.y))), 1.0);
+    y = __dsub_rn(__dmul_rn(2.0, mt_canonical(mt_temper(w.z), mt_temper(w.w))), 1.0);
+    r2 = __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
+    return r2 <= 1.0 && r2 != 0.0;
+}
+
 }  // namespace
 
+// nblk blocks of the generator's words, before tempering; state: the words of
+// the last block, where a later round goes on (first: from the seed). Word i
+// of a block needs the old words i and i + 1 and the word 227 before it (the
+// old word i + 397 where there is none), so thread t has t, t + 227 and t + 454
+// in one go, and two buffers need one barrier a block.
 __global__ void __launch_bounds__(kMtThreads)
-po_mt_normals_kernel(unsigned seed, long n, double stdev, double *__restrict__ out, int *__restrict__ err)
+po_mt_words_kernel(unsigned seed, int first, long nblk, uint32_t *__restrict__ state, uint32_t *__restrict__ words)
 {
-    __shared__ uint32_t mt[kMtN];
-    __shared__ int warp_ok[kMtThreads / 32];
-    __shared__ int warp_off[kMtThreads / 32];
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    if (t == 0) {
+    __shared__ uint32_t mt[2][kMtN];
+    const int t = threadIdx.x;
+    if (!first) {
+        for (int i = t; i < kMtN; i += kMtThreads) mt[0][i] = state[i];
+    } else if (t == 0) {
         uint32_t v = seed;
-        mt[0] = v;
+        mt[0][0] = v;
         for (int i = 1; i < kMtN; ++i) {
             v = 1812433253u * (v ^ (v >> 30)) + (uint32_t)i;
-            mt[i] = v;
+            mt[0][i] = v;
         }
     }
     __syncthreads();
-    long count = 0;   // block-uniform
-    // 156 attempts a block accept about 122.5 deviates on average: the bound
-    // is never reached in practice, and ends the loop if it were
-    const long max_blocks = n / 100 + 64;
-    for (long b = 0; b < max_blocks && count < n; ++b) {
-        uint32_t v = 0;
-        if (t < 227) v = mt_twist(mt[t], mt[t + 1], mt[t + 397]);
-        __syncthreads();
-        if (t < 227) mt[t] = v;
-        __syncthreads();
-        if (t >= 227 && t < 454) v = mt_twist(mt[t], mt[t + 1], mt[t - 227]);
-        __syncthreads();
-        if (t >= 227 && t < 454) mt[t] = v;
-        __syncthreads();
-        if (t >= 454 && t < 623) v = mt_twist(mt[t], mt[t + 1], mt[t - 227]);
-        else if (t == 623) v = mt_twist(mt[623], mt[0], mt[396]);
-        __syncthreads();
-        if (t >= 454 && t < kMtN) mt[t] = v;
-        __syncthreads();
-        uint32_t w = 0;
-        if (t < kMtN) {
-            w = mt[t];
-            w ^= w >> 11;
-            w ^= (w << 7) & 0x9d2c5680u;
-            w ^= (w << 15) & 0xefc60000u;
-            w ^= w >> 18;
-        }
-        // attempt a = t / 4 takes the outputs of threads 4a .. 4a + 3 (one warp)
-        const int base = lane & ~3;
-        const uint32_t w0 = __shfl_sync(0xffffffffu, w, base), w1 = __shfl_sync(0xffffffffu, w, base + 1);
-        const uint32_t w2 = __shfl_sync(0xffffffffu, w, base + 2), w3 = __shfl_sync(0xffffffffu, w, base + 3);
-        bool ok = false;
-        double val = 0.0;
-        if ((t & 3) == 0 && t < kMtN) {
-            const double x = __dsub_rn(__dmul_rn(2.0, mt_canonical(w0, w1)), 1.0);
-            const double y = __dsub_rn(__dmul_rn(2.0, mt_canonical(w2, w3)), 1.0);
-            const double r2 = __dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y));
-            ok = r2 <= 1.0 && r2 != 0.0;
-            if (ok) val = __dmul_rn(__dmul_rn(y, __dsqrt_rn(__ddiv_rn(__dmul_rn(-2.0, log(r2)), r2))), stdev);
-        }
-        const unsigned ball = __ballot_sync(0xffffffffu, ok);
-        if (lane == 0) warp_ok[warp] = __popc(ball);
-        __syncthreads();
-        if (t == 0) {
-            int o = 0;
-            for (int q = 0; q < kMtThreads / 32; ++q) {
-                warp_off[q] = o;
-                o += warp_ok[q];
+    for (long b = 0; b < nblk; ++b) {
+        const uint32_t *cur = mt[b & 1];
+        uint32_t *nxt = mt[1 - (b & 1)], *out = words + b * kMtN;
+        if (t < 227) {
+            const uint32_t v0 = mt_twist(cur[t], cur[t + 1], cur[t + 397]);
+            const uint32_t v1 = mt_twist(cur[t + 227], cur[t + 228], v0);
+            nxt[t] = v0;
+            nxt[t + 227] = v1;
+            out[t] = v0;
+            out[t + 227] = v1;
+            if (t < 170) {
+                // the last word's successor is the new word 0
+                const uint32_t next = t < 169 ? cur[t + 455] : mt_twist(cur[0], cur[1], cur[397]);
+                const uint32_t v2 = mt_twist(cur[t + 454], next, v1);
+                nxt[t + 454] = v2;
+                out[t + 454] = v2;
             }
         }
         __syncthreads();
-        if (ok) {
-            const long at = count + warp_off[warp] + __popc(ball & ((1u << lane) - 1u));
-            if (at < n) out[at] = val;
-        }
-        count += warp_off[kMtThreads / 32 - 1] + warp_ok[kMtThreads / 32 - 1];
-        __syncthreads();
     }
-    if (t == 0 && count < n) atomicExch(err, kErrRngBound);
+    for (int i = t; i < kMtN; i += kMtThreads) state[i] = mt[nblk & 1][i];
+}
+
+// Accepted attempts of each CTA's kMtAttempts.
+__global__ void __launch_bounds__(kMtAttempts)
+po_mt_count_kernel(const uint4 *__restrict__ words, long na, int *__restrict__ count)
+{
+    double y, r2;
+    const int c = __syncthreads_count(mt_attempt(words, (long)blockIdx.x * kMtAttempts + threadIdx.x, na, y, r2));
+    if (threadIdx.x == 0) count[blockIdx.x] = c;
+}
+
+// The accepted attempts' deviates, in order, from where the rounds before
+// ended (base[0]; the last CTA leaves the new end in base[1] and, at the last
+// round, reports deviates that are missing).
+__global__ void __launch_bounds__(kMtAttempts)
+po_mt_emit_kernel(const uint4 *__restrict__ words, long na, const int *__restrict__ count, long long *__restrict__ base,
+                  int last, long n, double stdev, double *__restrict__ out, int *__restrict__ err)
+{
+    __shared__ unsigned long long before;
+    __shared__ int warp_ok[kMtAttempts / 32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    double y, r2;
+    const bool ok = mt_attempt(words, (long)blockIdx.x * kMtAttempts + t, na, y, r2);
+    const unsigned ball = __ballot_sync(0xffffffffu, ok);
+    if (t == 0) before = (unsigned long long)base[0];
+    if (lane == 0) warp_ok[warp] = __popc(ball);
+    __syncthreads();
+    unsigned long long mine = 0;
+    for (int c = t; c < (int)blockIdx.x; c += kMtAttempts) mine += (unsigned)count[c];
+    if (mine) atomicAdd(&before, mine);
+    __syncthreads();
+    long at = (long)before + __popc(ball & ((1u << lane) - 1u));
+    for (int w = 0; w < warp; ++w) at += warp_ok[w];
+    if (ok && at < n) out[at] = __dmul_rn(__dmul_rn(y, __dsqrt_rn(__ddiv_rn(__dmul_rn(-2.0, log(r2)), r2))), stdev);
+    if (blockIdx.x == gridDim.x - 1 && t == kMtAttempts - 1) {
+        const long end = at + ok;
+        base[1] = end;
+        if (last && end < n) atomicExch(err, kErrRngBound);
+    }
 }
 
 int normal_deviates_dev(unsigned seed, long n, double stdev, double *out, int *err, cudaStream_t s)
 {
     if (n <= 0) return 0;
-    po_mt_normals_kernel<<<1, kMtThreads, 0, s>>>(seed, n, stdev, out, err);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(2, std::string("normal deviates: ") + cudaGetErrorString(e));
-    note_launches(1);
-    return 0;
+    // attempts for n deviates at pi / 4 a piece, with 12 standard deviations to
+    // spare: the bound is never met in practice
+    const double need = n / 0.78539816339744831;
+    const long blocks = (long)((need + 12.0 * sqrt(0.27 * need) + 200.0) / (kMtN / 4)) + 1;
+    const long most = std::min(blocks, kMtRound), na = most * (kMtN / 4);
+    uint32_t *words = nullptr, *state = nullptr;
+    int *count = nullptr;
+    long long *base = nullptr;
+    const long ctas = (na + kMtAttempts - 1) / kMtAttempts, rounds = (blocks + kMtRound - 1) / kMtRound;
+    int rc = 0;
+    if (!(rc = scratch_alloc(reinterpret_cast<void **>(&words), sizeof(uint32_t) * kMtN * (most + 1) +
+                             sizeof(long long) * (rounds + 1) + sizeof(int) * ctas, s))) {
+        // words first (16-byte aligned), then the state, the bases, the counts
+        state = words + kMtN * most;
+        base = reinterpret_cast<long long *>(state + kMtN);
+        count = reinterpret_cast<int *>(base + rounds + 1);
+        cudaError_t e = cudaMemsetAsync(base, 0, sizeof(long long), s);
+        for (long r = 0; r < rounds && e == cudaSuccess; ++r) {
+            const long nb = std::min(kMtRound, blocks - r * kMtRound), a = nb * (kMtN / 4);
+            const unsigned grid = (unsigned)((a + kMtAttempts - 1) / kMtAttempts);
+            const uint4 *w4 = reinterpret_cast<const uint4 *>(words);
+            po_mt_words_kernel<<<1, kMtThreads, 0, s>>>(seed, r == 0, nb, state, words);
+            po_mt_count_kernel<<<grid, kMtAttempts, 0, s>>>(w4, a, count);
+            po_mt_emit_kernel<<<grid, kMtAttempts, 0, s>>>(w4, a, count, base + r, r == rounds - 1, n, stdev, out, err);
+            e = cudaGetLastError();
+            if (e == cudaSuccess) note_launches(3);
+        }
+        if (e != cudaSuccess) rc = fail(2, std::string("normal deviates: ") + cudaGetErrorString(e));
+    }
+    scratch_free(words, s);
+    return rc;
 }
 
 // ------------------------------------------------- correlated surface error
