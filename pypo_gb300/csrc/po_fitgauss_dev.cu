@@ -34,13 +34,15 @@
 //
 // A fit is a chain of a few hundred such launches, each waited for, so a
 // launch's round trip is what counts. The last block writes the sums straight
-// into a page-locked block of the host and then a sequence number, for which
-// the host watches: an empty kernel's round trip is 7.6 us that way, 12.6 with
-// a copy and a stream synchronise (14.5 into pageable memory). The region's
+// into page-locked words of the host, each with the launch's sequence number in
+// its upper half, for which the host watches: an empty kernel's round trip is
+// 7.6 us with the number behind a fence, 12.6 with
+// a copy and a stream synchronise (14.5 into pageable memory); numbers in the
+// words themselves need no fence, 1.3 us less a step. The region's
 // points are spread over the SMs, one warp per 32 points and Gaussian: with
 // 256 consecutive points to a block a region of 1500 sat on six SMs and their
 // FP64 pipes (2 a clock). Measured, a 201 x 201 beam's figures (two fits, LIN):
-// 13.3 -> 5.3 ms, 15 us a simplex step.
+// 13.3 -> 4.7 ms, 13 us a simplex step.
 //
 // Kept from the reference on purpose, with their effects:
 //   * the window's corners are read as x[min(cols), i0], x[max(cols), i0],
@@ -61,6 +63,7 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -108,29 +111,24 @@ __device__ __forceinline__ double gauss_at(const Gauss &g, int scale, double x, 
     return scale == kScaleDb ? __dmul_rn(20.0, log10(e)) : e;
 }
 
-// Where a kernel's results go on the host: `data` in page-locked memory, then
-// `seq` into *flag once they are there. flag null: nowhere (the host copies
-// the device words).
+// Where a kernel's results go on the host: page-locked words, two per result,
+// each half of its bits below the launch's sequence number. A 64-bit store
+// arrives whole, so the host has a result when both its words carry the number,
+// and no fence orders one store behind another. data null: nowhere (the host
+// copies the device words).
 struct Mail {
-    double *data;
-    unsigned *flag;
+    unsigned long long *data;
     unsigned seq;
 };
 
-// The calling thread's v as word q, for the threads that have one, then the
-// sequence number. Called by every thread of one block.
-__device__ void post(const Mail &mail, bool mine, int q, double v)
+// v as result q.
+__device__ __forceinline__ void post(const Mail &mail, int q, double v)
 {
-    if (!mail.flag) return;
-    if (mine) {
-        mail.data[q] = v;
-        __threadfence_system();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence_system();
-        *reinterpret_cast<volatile unsigned *>(mail.flag) = mail.seq;
-    }
+    if (!mail.data) return;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(v), tag = (unsigned long long)mail.seq << 32;
+    volatile unsigned long long *o = mail.data + 2 * q;
+    o[0] = tag | (b & 0xffffffffull);
+    o[1] = tag | (b >> 32);
 }
 
 // The nrow rows of nq partials (stride words apart) added in row order, word
@@ -174,9 +172,11 @@ __device__ void finish_sums(const double (&s)[NS], double *part, double *res, un
     if (!last) return;
     __threadfence();
     const double v = add_rows(part, gridDim.x, NS, NS, sh[0]);
-    if (threadIdx.x < NS) res[threadIdx.x] = v;
+    if (threadIdx.x < NS) {
+        post(mail, threadIdx.x, v);
+        res[threadIdx.x] = v;
+    }
     if (threadIdx.x == 0) *count = 0u;
-    post(mail, threadIdx.x < NS, threadIdx.x, v);
 }
 
 // (value, index) maximum, first index on ties, NaN above every number (as
@@ -243,9 +243,11 @@ __device__ void finish_argmax(double v, long i, double sum, double *part, double
         ss[0] = t;
     }
     const double r = threadIdx.x == 0 ? sv[0] : (threadIdx.x == 1 ? (double)si[0] : ss[0]);
-    if (threadIdx.x < 3) res[threadIdx.x] = r;
+    if (threadIdx.x < 3) {
+        post(mail, threadIdx.x, r);
+        res[threadIdx.x] = r;
+    }
     if (threadIdx.x == 0) *count = 0u;
-    post(mail, threadIdx.x < 3, threadIdx.x, r);
 }
 
 // |E_c| into a; res[0] = max |E_c| (NaN if any is NaN).
@@ -274,10 +276,7 @@ fg_pattern_kernel(long n, const double *__restrict__ a, const double *__restrict
                   double *__restrict__ fit, double *part, double *res, unsigned *count, Mail mail)
 {
     const double m = *amax;
-    if (mail.flag && blockIdx.x == 0 && threadIdx.x == 0) {
-        mail.data[3] = m;
-        __threadfence_system();
-    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) post(mail, 3, m);
     double best = -CUDART_INF;
     long bi = n;
     double s = 0.0;
@@ -433,19 +432,24 @@ fg_compact_kernel(long n, const unsigned char *__restrict__ sel, const int *__re
 }
 
 // Overlap sums of up to kBatch Gaussians over the m compacted points: (sum f
-// Psi, sum Psi^2, sum f^2) per Gaussian. A unit is 32 consecutive points (and
-// those kUnits units further on); block u takes unit u, its warp k Gaussian k,
-// so that a region of a few thousand points spreads over the SMs. The block
+// Psi, sum Psi^2) per Gaussian and, with `ff` (a minimisation's first launch),
+// sum f^2 behind them. A unit is 32 consecutive points (and
+// those kUnits units further on); block u takes unit u, its warp k Gaussian k
+// (the next warp f^2),
+// so that a region of a few thousand points spreads over the SMs. A warp's two
+// sums share the additions of its tree, one in each half of the lanes. The block
 // that finishes last adds the units in order, by eights and then the eights,
 // so that each Gaussian's sums follow one order whatever the grid and
-// whatever else is in the batch.
+// whatever else is in the batch. What counts is the number of dependent FP64
+// operations: f^2 summed for every Gaussian, and three trees a warp, took 4 %
+// longer (301 x 301 beam: 6 %).
 constexpr int kBatch = 8;
 constexpr int kUnits = 152 * 8;
 static_assert(kBatch == kFgThreads / 32, "one warp per Gaussian");
 
 struct GaussBatch {
     Gauss g[kBatch];
-    int k;
+    int k, ff;
 };
 
 __global__ void __launch_bounds__(kFgThreads)
@@ -453,26 +457,31 @@ fg_overlap_kernel(long m, const double *__restrict__ cx, const double *__restric
                   const double *__restrict__ cf, int scale, GaussBatch b, double *part, double *res,
                   unsigned *done, Mail mail)
 {
-    constexpr int NQ = 3 * kBatch;
+    constexpr int NQ = 2 * kBatch + 1;
     __shared__ double eights[kUnits / 8][NQ];
     __shared__ bool last;
-    const int nq = 3 * b.k, lane = threadIdx.x & 31, k = threadIdx.x >> 5;
-    if (k < b.k) {
-        const Gauss g = b.g[k];
-        double s[3] = {0.0, 0.0, 0.0};
-        for (long i = (long)blockIdx.x * 32 + lane; i < m; i += 32L * kUnits) {
-            const double f = cf[i];
-            const double p = gauss_at(g, scale, cx[i], cy[i]);
-            s[0] += __dmul_rn(f, p);
-            s[1] += __dmul_rn(p, p);
-            s[2] += __dmul_rn(f, f);
+    const int nq = 2 * b.k + b.ff, lane = threadIdx.x & 31, k = threadIdx.x >> 5;
+    if (k < b.k + b.ff) {
+        double s0 = 0.0, s1 = 0.0;
+        if (k < b.k) {
+            const Gauss g = b.g[k];
+            for (long i = (long)blockIdx.x * 32 + lane; i < m; i += 32L * kUnits) {
+                const double f = cf[i];
+                const double p = gauss_at(g, scale, cx[i], cy[i]);
+                s0 += __dmul_rn(f, p);
+                s1 += __dmul_rn(p, p);
+            }
+        } else {
+            for (long i = (long)blockIdx.x * 32 + lane; i < m; i += 32L * kUnits) s0 += __dmul_rn(cf[i], cf[i]);
         }
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-            for (int o = 16; o > 0; o >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], o);
-            if (lane == 0) part[(long)blockIdx.x * NQ + 3 * k + q] = s[q];
+        // lane l < 16: s0 of lanes l and l + 16; lane 16 + l: s1 of the same two
+        double v = lane < 16 ? s0 : s1;
+        v += __shfl_xor_sync(0xffffffffu, lane < 16 ? s1 : s0, 16);
+        for (int o = 8; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+        if (lane == 0 || (lane == 16 && k < b.k)) {
+            part[(long)blockIdx.x * NQ + 2 * k + (lane >> 4)] = v;
+            __threadfence();
         }
-        if (lane == 0) __threadfence();
     }
     __syncthreads();
     if (threadIdx.x == 0) last = atomicAdd(done, 1u) == gridDim.x - 1;
@@ -488,13 +497,13 @@ fg_overlap_kernel(long m, const double *__restrict__ cx, const double *__restric
         eights[e][q] = v;
     }
     __syncthreads();
-    double v = 0.0;
     if ((int)threadIdx.x < nq) {
+        double v = 0.0;
         for (int e = 0; e < n8; ++e) v += eights[e][threadIdx.x];
+        post(mail, threadIdx.x, v);
         res[threadIdx.x] = v;
     }
     if (threadIdx.x == 0) *done = 0u;
-    post(mail, (int)threadIdx.x < nq, threadIdx.x, v);
 }
 
 __global__ void fg_generate_kernel(long n, const double *__restrict__ g7, Gauss g, int scale, double *__restrict__ out)
@@ -515,8 +524,8 @@ bool np_index(long r, long dim, long &out)
 // at a time, kept for later ones (at most kMailKeep of them, one per fit that
 // ran at the same time).
 struct MailBox {
-    double data[3 * kBatch];
-    unsigned flag;
+    unsigned long long data[2 * (2 * kBatch + 1)];
+    unsigned seq;   // of the last launch that posted here (host only)
 };
 constexpr size_t kMailKeep = 16;
 std::mutex g_mail_mu;
@@ -537,7 +546,7 @@ MailBox *mailbox_borrow()
         (void)cudaGetLastError();
         return nullptr;   // the fit copies its results instead
     }
-    static_cast<MailBox *>(p)->flag = 0u;
+    *static_cast<MailBox *>(p) = MailBox{};
     return static_cast<MailBox *>(p);
 }
 
@@ -569,7 +578,6 @@ public:
     Fit(int ncx, int ncy, const double *g7, cudaStream_t s)
         : ncx_(ncx), ncy_(ncy), n_((long)ncx * ncy), g7_(g7), s_(s), box_(mailbox_borrow())
     {
-        if (box_) seq_ = box_->flag;
     }
     ~Fit()
     {
@@ -584,7 +592,7 @@ public:
     {
         const size_t nd = (size_t)n_ * sizeof(double);
         const size_t parts = sizeof(double) * kFgBlocks * kFgMaxSums;
-        const size_t bytes = 5 * (nd + 256) + parts + sizeof(double) * (kUnits + 1) * 3 * kBatch + 8 * 256 +
+        const size_t bytes = 5 * (nd + 256) + parts + sizeof(double) * (kUnits + 1) * (2 * kBatch + 1) + 8 * 256 +
                              sizeof(int) * kFgBlocks + 2 * ((size_t)n_ + 256) + (size_t)ncx_ + ncy_ + 256;
         if (int rc = po::scratch_alloc(reinterpret_cast<void **>(&sc_.base), bytes, s_)) return rc;
         char *p = static_cast<char *>(sc_.base);
@@ -602,8 +610,8 @@ public:
         sc_.cy = reinterpret_cast<double *>(take(nd));
         sc_.cf = reinterpret_cast<double *>(take(nd));
         sc_.bcount = reinterpret_cast<int *>(take(sizeof(int) * kFgBlocks));
-        sc_.opart = reinterpret_cast<double *>(take(sizeof(double) * kUnits * 3 * kBatch));
-        sc_.ores = reinterpret_cast<double *>(take(sizeof(double) * 3 * kBatch));
+        sc_.opart = reinterpret_cast<double *>(take(sizeof(double) * kUnits * (2 * kBatch + 1)));
+        sc_.ores = reinterpret_cast<double *>(take(sizeof(double) * (2 * kBatch + 1)));
         sc_.sel = reinterpret_cast<unsigned char *>(take((size_t)n_));
         sc_.lines = reinterpret_cast<unsigned char *>(take((size_t)ncx_ + ncy_));
         const cudaError_t e = cudaMemsetAsync(sc_.count, 0, sizeof(unsigned), s_);
@@ -616,7 +624,7 @@ public:
     {
         if (!box_) return Mail{};
         waiting_ = true;
-        return Mail{box_->data, &box_->flag, ++seq_};
+        return Mail{box_->data, ++box_->seq};
     }
 
     // Launch status, then the first k result words (posted, or res on the device) on the host.
@@ -626,15 +634,14 @@ public:
         if (e == cudaSuccess && box_) {
             // every so often the stream itself is asked, so that an error ends the wait
             for (unsigned spin = 1;; ++spin) {
-                if (__atomic_load_n(&box_->flag, __ATOMIC_ACQUIRE) == seq_) break;
+                if (arrived(h, k)) break;
                 if (spin % 65536u) continue;
                 e = cudaStreamQuery(s_);
                 if (e == cudaErrorNotReady) continue;
-                if (e == cudaSuccess && __atomic_load_n(&box_->flag, __ATOMIC_ACQUIRE) == seq_) break;
+                if (e == cudaSuccess && arrived(h, k)) break;
                 return fail(2, std::string(what) + ": " + (e == cudaSuccess ? "no result" : cudaGetErrorString(e)));
             }
             waiting_ = false;
-            for (int q = 0; q < k; ++q) h[q] = box_->data[q];
             return 0;
         }
         if (e == cudaSuccess) e = cudaMemcpyAsync(h, res, sizeof(double) * k, cudaMemcpyDeviceToHost, s_);
@@ -705,6 +712,7 @@ public:
         nm_init(st, 6, p0, 1e-4, 1e-4, 0, 0);
         double pts[kBatch][6], val[kBatch];
         int npts = 0;
+        f2_ = -1.0;
         while (nm_next(st)) {
             int hit = -1;
             for (int q = 0; q < npts && hit < 0; ++q) {
@@ -748,20 +756,23 @@ public:
         return k;
     }
 
-    // GaussAbs (FitGauss.py:165-195) of each point, one launch.
+    // GaussAbs (FitGauss.py:165-195) of each point, one launch; the first of a
+    // minimisation (at most kBatch - 1 points) sums the region's f^2 as well.
     int values(int scale, const double (*pts)[6], int k, double *val)
     {
         GaussBatch b{};
         b.k = k;
+        b.ff = f2_ < 0.0 ? 1 : 0;
         for (int q = 0; q < k; ++q) b.g[q] = gauss_of(pts[q]);
         const unsigned nblk = (unsigned)std::min<long>(kUnits, std::max(1L, (m_ + 31) / 32));
         fg_overlap_kernel<<<nblk, kFgThreads, 0, s_>>>(m_, sc_.cx, sc_.cy, sc_.cf, scale, b, sc_.opart, sc_.ores,
                                                         sc_.count, mail());
         note_launches(1);
-        double h[3 * kBatch];
-        if (int rc = read(h, 3 * k, sc_.ores, "overlap sums")) return rc;
+        double h[2 * kBatch + 1];
+        if (int rc = read(h, 2 * k + b.ff, sc_.ores, "overlap sums")) return rc;
+        if (b.ff) f2_ = h[2 * k];
         for (int q = 0; q < k; ++q) {
-            const double c00 = h[3 * q] * h[3 * q] / h[3 * q + 2] / h[3 * q + 1];
+            const double c00 = h[2 * q] * h[2 * q] / f2_ / h[2 * q + 1];
             val[q] = std::fabs(1 - std::fabs(c00));
         }
         return 0;
@@ -776,14 +787,27 @@ public:
     }
 
 private:
+    // Whether the last launch's k results are in the box; then h has them.
+    bool arrived(double *h, int k) const
+    {
+        for (int q = 0; q < k; ++q) {
+            const unsigned long long w0 = __atomic_load_n(&box_->data[2 * q], __ATOMIC_RELAXED);
+            const unsigned long long w1 = __atomic_load_n(&box_->data[2 * q + 1], __ATOMIC_RELAXED);
+            if ((unsigned)(w0 >> 32) != box_->seq || (unsigned)(w1 >> 32) != box_->seq) return false;
+            const unsigned long long b = (w1 << 32) | (w0 & 0xffffffffull);
+            std::memcpy(&h[q], &b, sizeof b);
+        }
+        return true;
+    }
+
     int ncx_, ncy_;
     long n_;
     const double *g7_;
     cudaStream_t s_;
     MailBox *box_;
-    unsigned seq_ = 0;
     bool waiting_ = false;
     long m_ = 0;   // points of the current selection
+    double f2_ = -1.0;   // their sum f^2, once a minimisation has it
     FitScratch sc_;
 };
 
