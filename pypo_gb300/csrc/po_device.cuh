@@ -214,6 +214,12 @@ __device__ __forceinline__ double trap_weight(long i, int gmode, int ncx, int nc
     return w;
 }
 
+// Doubles as integers of the same order, and back (its own inverse): the
+// comparisons of a box run on the integer pipe, the FP64 pipe being 32 times
+// slower (161,227 points on 8 SMs: about 30 us of FP64 comparisons).
+__device__ __forceinline__ long long order_key(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffll); }
+constexpr long long kKeyInf = 0x7ff0000000000000ll;   // order_key of +infinity; of -infinity: ~kKeyInf
+
 // A coordinate x (turns, relative to the frame origin) as hi + lo: hi on the
 // frame's quantum q (at most 11 significant bits), lo the small rest.
 __device__ __forceinline__ void split_hi_lo(double x, const Frame &fr, float &h, float &l)

@@ -577,7 +577,7 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
         }
         const int *ord = i_out;
         void *pargs[] = {&ns, &ord, &src7, &cur, &gmode, &ncx, &ncy, &p.frame, &p.fac_re, &p.fac_im, &p.srcpk};
-        if (!rc) rc = launch(ff_pack_kernel(p.has_m), dim3((unsigned)p.tiles), dim3(32), pargs, 0, s);
+        if (!rc) rc = launch(ff_pack_kernel(p.has_m), dim3((unsigned)p.tiles), dim3(kTile), pargs, 0, s);
     }
     const float4 *srcc = p.srcpk, *tgtc = p.tgtpk;
     long ntiles = ns > 0 ? p.tiles : 0;
@@ -791,7 +791,7 @@ int run_adjoint(const AdjArgs &a)
             }
             ff_order = i_out;
             void *fpargs[] = {&ns, &ff_order, &src7, &cur, &gmode, &ncx, &ncy, &frame, &fac_re, &fac_im, &srcpk};
-            if (!rc) rc = launch(ff_pack_kernel(has_m), dim3((unsigned)ntile_s), dim3(32), fpargs, 0, s);
+            if (!rc) rc = launch(ff_pack_kernel(has_m), dim3((unsigned)ntile_s), dim3(kTile), fpargs, 0, s);
         } else {
             long sblk = (ns + 127) / 128;
             double *gam_out = a.mode == kEHP ? nullptr : gam;   // EHP: the cotangents are gam already

@@ -100,106 +100,122 @@ constexpr int kFFKeyBits = 42;
 
 // ------------------------------------------------------------------ packing
 
-// One warp per tile of kTile sources in curve order: the tile's box gives its
-// centre c (FP64, turns) and its box of normals; every source's record holds
-// its offset s - c (FP32) and its currents times the trapezoid weight, the
-// area and the complex prefactor. The tile is assembled in shared memory and
-// written out in coalesced float4. The last tile is padded with copies of the
-// last source carrying zero currents.
+// One CTA per tile of kTile sources in curve order, a thread a source: the
+// tile's box gives its centre c (FP64, turns) and its box of normals; every
+// source's record holds its offset s - c (FP32) and its currents times the
+// trapezoid weight, the area and the complex prefactor. The tile is assembled
+// in shared memory and written out in coalesced float4. The last tile is padded
+// with copies of the last source carrying zero currents. Bound by the latency of
+// the gathered loads and the FP64 chain behind them, so one thread has one
+// source, the box's comparisons are integer ones and one thread does what the
+// tile needs once (318 tiles: 23 -> 18 us against one warp a tile; a far field
+// of 2,652 sources x 1,640 directions 142 -> 129 us).
 template <bool HAS_M>
-__global__ void __launch_bounds__(32)
+__global__ void __launch_bounds__(kTile)
 po_ff_pack_kernel(long ns, const int *__restrict__ order, const double *__restrict__ src7,
                   const double *__restrict__ cur, int gmode, int ncx, int ncy, const Frame *__restrict__ frp,
                   double fac_re, double fac_im, float4 *__restrict__ out)
 {
-    constexpr int R4 = ff_rec4(HAS_M), T4 = ff_tile4(HAS_M);
-    constexpr int PER = kTile / 32;   // sources per lane
+    constexpr int R4 = ff_rec4(HAS_M), T4 = ff_tile4(HAS_M), W = kTile / 32;
     __shared__ __align__(16) float4 buf[T4];
+    __shared__ long long wb[W][6];
+    __shared__ float wn[W][6];
+    __shared__ double tile_c[3], tile_q;   // centre; the wide tile's quantum, or 0
     float *bf = reinterpret_cast<float *>(buf);
     const Frame fr = *frp;
-    const long first = (long)blockIdx.x * kTile;
-    const int lane = threadIdx.x;
+    const long j = (long)blockIdx.x * kTile + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-    double p[PER][3];
-    long src[PER];
-    bool real[PER];
-    double lo[3] = {CUDART_INF, CUDART_INF, CUDART_INF}, hi[3] = {-CUDART_INF, -CUDART_INF, -CUDART_INF};
-    float nlo[3] = {CUDART_INF_F, CUDART_INF_F, CUDART_INF_F}, nhi[3] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
+    const bool real = j < ns;
+    const long k = order[real ? j : ns - 1];
+    double p[3];
+    long long lo[3], hi[3];   // order keys (NaN left out)
+    float nv[3], nlo[3], nhi[3];
 #pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const long j = first + lane + 32 * q;
-        real[q] = j < ns;
-        const long k = order[real[q] ? j : ns - 1];
-        src[q] = k;
+    for (int c = 0; c < 3; ++c) {
+        p[c] = (src7[c * ns + k] - fr.o[c]) * fr.kappa;
+        const long long x = __double_as_longlong(p[c]), y = order_key(x);
+        const bool nan = (x & 0x7fffffffffffffffll) > kKeyInf;
+        lo[c] = nan ? kKeyInf : y;
+        hi[c] = nan ? ~kKeyInf : y;
+        nv[c] = nlo[c] = nhi[c] = (float)src7[(3 + c) * ns + k];
+    }
+    const double w = real ? trap_weight(k, gmode, ncx, ncy) * src7[6 * ns + k] : 0.0;
+    const double fr_ = fac_re * w, fi_ = fac_im * w;
+    float *rec = bf + (kFFHead + (threadIdx.x >> 1) * R4) * 4 + (threadIdx.x & 1);
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            p[q][c] = (src7[c * ns + k] - fr.o[c]) * fr.kappa;
-            lo[c] = fmin(lo[c], p[q][c]);
-            hi[c] = fmax(hi[c], p[q][c]);
-            const float nv = (float)src7[(3 + c) * ns + k];
-            nlo[c] = fminf(nlo[c], nv);
-            nhi[c] = fmaxf(nhi[c], nv);
+    for (int c = 0; c < 3; ++c) {
+        const double jr = cur[c * ns + k], ji = cur[(3 + c) * ns + k];
+        rec[2 * (3 + c)] = (float)(fr_ * jr - fi_ * ji);
+        rec[2 * (6 + c)] = (float)(fr_ * ji + fi_ * jr);
+        rec[2 * (9 + c)] = nv[c];
+        if (HAS_M) {
+            const double mr = cur[(6 + c) * ns + k], mi = cur[(9 + c) * ns + k];
+            rec[2 * (16 + c)] = (float)(fr_ * mr - fi_ * mi);
+            rec[2 * (19 + c)] = (float)(fr_ * mi + fi_ * mr);
         }
     }
+    rec[2 * 15] = 0.0f;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            lo[c] = fmin(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
-            hi[c] = fmax(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
+            lo[c] = min(lo[c], __shfl_xor_sync(0xffffffffu, lo[c], o));
+            hi[c] = max(hi[c], __shfl_xor_sync(0xffffffffu, hi[c], o));
             nlo[c] = fminf(nlo[c], __shfl_xor_sync(0xffffffffu, nlo[c], o));
             nhi[c] = fmaxf(nhi[c], __shfl_xor_sync(0xffffffffu, nhi[c], o));
         }
-    double cen[3], half[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-        cen[c] = 0.5 * (lo[c] + hi[c]);
-        half[c] = 0.5 * (hi[c] - lo[c]);
-    }
-    // narrow: the box's half-diagonal within kFFNarrow turns; a wide tile's
-    // offsets split on the smallest power of two q with max |offset| <= 1024 q
-    const bool wide = !(sqrt(half[0] * half[0] + half[1] * half[1] + half[2] * half[2]) <= (double)kFFNarrow);
-    const double hmax = fmax(half[0], fmax(half[1], half[2]));
-    double qt = 0x1p-40;
-    for (int g = 0; g < 1100 && wide && qt * 1024.0 < hmax; ++g) qt *= 2.0;
-    if (lane < 3) {
-        float h, l;
-        split_hi_lo(cen[lane], fr, h, l);
-        bf[lane] = h;
-        bf[3 + lane] = l;
-        bf[6 + lane] = nlo[lane];
-        bf[9 + lane] = nhi[lane];
-    } else if (lane < 7) {
-        bf[9 + lane] = lane == 3 && wide ? 1.0f : 0.0f;   // float 12: the wide-tile flag; 13-15 spare
-    }
-#pragma unroll
-    for (int q = 0; q < PER; ++q) {
-        const int jt = lane + 32 * q;
-        float *rec = bf + (kFFHead + (jt >> 1) * R4) * 4 + (jt & 1);
-        const long k = src[q];
-        const double w = real[q] ? trap_weight(k, gmode, ncx, ncy) * src7[6 * ns + k] : 0.0;
-        const double fr_ = fac_re * w, fi_ = fac_im * w;
+    if (lane == 0)
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-            const double off = p[q][c] - cen[c];
-            const double oh = wide ? rint(off / qt) * qt : off;
-            rec[2 * c] = (float)oh;
-            rec[2 * (12 + c)] = (float)(off - oh);   // 0 in a narrow tile
-            const double jr = cur[c * ns + k], ji = cur[(3 + c) * ns + k];
-            rec[2 * (3 + c)] = (float)(fr_ * jr - fi_ * ji);
-            rec[2 * (6 + c)] = (float)(fr_ * ji + fi_ * jr);
-            rec[2 * (9 + c)] = (float)src7[(3 + c) * ns + k];
-            if (HAS_M) {
-                const double mr = cur[(6 + c) * ns + k], mi = cur[(9 + c) * ns + k];
-                rec[2 * (16 + c)] = (float)(fr_ * mr - fi_ * mi);
-                rec[2 * (19 + c)] = (float)(fr_ * mi + fi_ * mr);
-            }
+            wb[warp][c] = lo[c];
+            wb[warp][3 + c] = hi[c];
+            wn[warp][c] = nlo[c];
+            wn[warp][3 + c] = nhi[c];
         }
-        rec[2 * 15] = 0.0f;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double half[3];
+        for (int c = 0; c < 3; ++c) {
+            for (int v = 1; v < W; ++v) {
+                lo[c] = min(lo[c], wb[v][c]);
+                hi[c] = max(hi[c], wb[v][3 + c]);
+                nlo[c] = fminf(nlo[c], wn[v][c]);
+                nhi[c] = fmaxf(nhi[c], wn[v][3 + c]);
+            }
+            const double a = __longlong_as_double(order_key(lo[c])), b = __longlong_as_double(order_key(hi[c]));
+            const double cen = 0.5 * (a + b);
+            half[c] = 0.5 * (b - a);
+            float h, l;
+            split_hi_lo(cen, fr, h, l);
+            bf[c] = h;
+            bf[3 + c] = l;
+            bf[6 + c] = nlo[c];
+            bf[9 + c] = nhi[c];
+            tile_c[c] = cen;
+        }
+        // narrow: the box's half-diagonal within kFFNarrow turns; a wide tile's
+        // offsets split on the smallest power of two q with max |offset| <= 1024 q
+        const bool wide = !(sqrt(half[0] * half[0] + half[1] * half[1] + half[2] * half[2]) <= (double)kFFNarrow);
+        const double hmax = fmax(half[0], fmax(half[1], half[2]));
+        double qt = 0x1p-40;
+        for (int g = 0; g < 1100 && wide && qt * 1024.0 < hmax; ++g) qt *= 2.0;
+        tile_q = wide ? qt : 0.0;
+        bf[12] = wide ? 1.0f : 0.0f;   // the wide-tile flag; 13-15 spare
+        bf[13] = bf[14] = bf[15] = 0.0f;
     }
-    __syncwarp();
+    __syncthreads();
+    const double qt = tile_q;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        const double off = p[c] - tile_c[c];
+        const double oh = qt > 0.0 ? rint(off / qt) * qt : off;
+        rec[2 * c] = (float)oh;
+        rec[2 * (12 + c)] = (float)(off - oh);   // 0 in a narrow tile
+    }
+    __syncthreads();
     float4 *dst = out + (size_t)blockIdx.x * T4;
-    for (int q = lane; q < T4; q += 32) dst[q] = buf[q];
+    for (int q = threadIdx.x; q < T4; q += kTile) dst[q] = buf[q];
 }
 
 // ---------------------------------------------------------------- main kernel

@@ -37,12 +37,6 @@ __device__ __forceinline__ void st_cluster(long long *p, uint32_t rank, long lon
     asm volatile("st.shared::cluster.s64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
 }
 
-// Doubles as integers of the same order, and back (its own inverse): the
-// comparisons of a box run on the integer pipe, the FP64 pipe being 32 times
-// slower (161,227 points on 8 SMs: about 30 us of FP64 comparisons).
-__device__ __forceinline__ long long order_key(long long b) { return b ^ ((b >> 63) & 0x7fffffffffffffffll); }
-constexpr long long kKeyInf = 0x7ff0000000000000ll;   // order_key of +infinity; of -infinity: ~kKeyInf
-
 // Smallest power of two q >= need, at least 2^-40 (need NaN: 2^-40; need
 // infinite or past the largest power of two: infinity).
 __device__ __forceinline__ double quantum(double need)
