@@ -130,13 +130,14 @@ static int device_info(DeviceInfo *&out)
     return 0;
 }
 
-// Share of a chunk that the last wave is expected to idle (choose_split). Near
-// field and scalar: 0.3 (scalar 10,403 -> 14,399 0.197 -> 0.185 ms, feed ->
-// dish step 2.00 -> 1.97 against 0). The far-field forward's tiles differ
-// more in cost (narrow, wide, lit): 0.5 (122,500 -> 22,650 2.74 -> 2.58 ms).
-// Its adjoint, whose stages are alike, is best left at 0 (17.59 against 17.78
-// ms on 251,001 x 40,803 with 0.3).
-constexpr double kTailNF = 0.3, kTailFF = 0.5;
+// Share of a chunk that the last wave is expected to idle (choose_split): the
+// near field's adjoint. The far field's, whose stages are alike, is best left
+// at 0 (17.59 against 17.78 ms on 251,001 x 40,803 with 0.3).
+constexpr double kTailAdj = 0.3;
+
+// Chunks that an SM's last CTAs cost (load_split). The far field's tiles differ
+// more in cost (narrow, wide, lit).
+constexpr double kTailNF = 1.0, kTailFF = 3.0;
 
 // Resident CTAs per SM of a kernel (and its shared-memory attribute), looked
 // up once per device and kernel.
@@ -173,6 +174,36 @@ long choose_split(long nb, long ns, long slots, long max_chunks, long tile, doub
         if (real != s) continue;
         const long waves = (nb * real + slots - 1) / slots;
         const double cost = (double)waves * (chunk + start) + tail * chunk + per_chunk * real;
+        if (cost < best_cost - 1e-9) {
+            best_cost = cost;
+            best = real;
+        }
+    }
+    return best;
+}
+
+// The same for the forwards and the scalar adjoint, by the load of the fullest
+// SM: with about 8 CTAs or more to hide latencies an SM works at one rate
+// whatever their number, so the cost is its CTAs times their tiles; where they
+// are not all resident at once (occ) the last ones run with fewer beside them,
+// which costs about `tail` chunks; a CTA's start and partials cost 0.2 of a
+// tile. Fitted to every split of 92 sizes (40^2 to 301^2 points a side; near
+// field with and without M, scalar, far field): on average 0.2 to 0.9 % slower
+// than the best split and 3 % at most, where counting waves of resident CTAs
+// was 1 to 3 % and 14 % (4,422 x 4,356 with M 146.8 us, best 128.4). The
+// near field's adjoint, with 2 or 3 CTAs an SM, keeps the waves (1.3 % against 2 %).
+long load_split(long nb, long ns, long sms, long occ, long max_chunks, long tile, double tail)
+{
+    const long tiles = std::max(1L, (ns + tile - 1) / tile);
+    long best = 1;
+    double best_cost = 1e300;
+    for (long s = 1; s <= std::min(tiles, std::min(std::max(1L, max_chunks), 1024L)); ++s) {
+        const long chunk = (tiles + s - 1) / s;
+        const long real = (tiles + chunk - 1) / chunk;
+        if (real != s) continue;
+        const long ctas = nb * real;
+        const double load = (double)std::max((ctas + sms - 1) / sms, 8L) + (ctas > sms * occ ? tail : 0.0);
+        const double cost = chunk * load + 0.2 * ctas / sms;
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = real;
@@ -533,7 +564,7 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
     const int occ = p.far ? di->occ_ff[p.ts > 0][p.has_m ? 1 : 0] : di->occ2[p.kind][p.ts > 0][p.has_m ? 1 : 0];
     const size_t room = std::min(sc.room(), (size_t)1 << 30);
     const long max_chunks = std::max(1L, (long)(room / ((size_t)p.nacc * nt * sizeof(double))));
-    p.nsplit = choose_split(p.ntb, ns, (long)di->sms * occ, max_chunks, kTile, p.far ? kTailFF : kTailNF);
+    p.nsplit = load_split(p.ntb, ns, di->sms, occ, max_chunks, kTile, p.far ? kTailFF : kTailNF);
     const long chunk_tiles = (p.tiles + p.nsplit - 1) / p.nsplit;
     p.chunk = chunk_tiles * (p.far ? 1 : kTile);   // tiles (far field) or sources per chunk
     if ((rc = sc.get(&p.part, (size_t)p.nsplit * p.nacc * nt))) return rc;
@@ -682,8 +713,10 @@ int run_adjoint(const AdjArgs &a)
     int occ = 1, rc = 0;
     if ((rc = kernel_occupancy(di, fk, threads, smem, occ))) return rc;
     const long nsb = (ns + per_block - 1) / per_block;
-    const long split = choose_split(nsb, nt, (long)di->sms * occ, partial_cap(ns, std::max(rows, 1)), tile_t,
-                                    far ? 0.0 : kTailNF);
+    const long cap = partial_cap(ns, std::max(rows, 1));
+    const long split = kind == kKindScalar && !fp64
+                           ? load_split(nsb, nt, di->sms, occ, cap, tile_t, kTailNF)
+                           : choose_split(nsb, nt, (long)di->sms * occ, cap, tile_t, far ? 0.0 : kTailAdj);
     const long tiles_t = std::max(1L, (nt + tile_t - 1) / tile_t);
     const long per_chunk = (tiles_t + split - 1) / split;
     long chunk = !fp64 && far ? per_chunk : per_chunk * tile_t;   // stages (mixed far field) or targets

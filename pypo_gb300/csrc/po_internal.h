@@ -130,6 +130,9 @@ cudaError_t ff_sort(void *temp, size_t *temp_bytes, const unsigned long long *ke
 // chunk length, with a cost per CTA and per extra chunk, and `tail` of a chunk
 // for the last wave; at most max_chunks.
 long choose_split(long nb, long ns, long slots, long max_chunks, long tile, double tail);
+// The same by the load of the fullest SM, for kernels with several CTAs an SM
+// (occ resident at most).
+long load_split(long nb, long ns, long sms, long occ, long max_chunks, long tile, double tail);
 
 // FP64 grid generation on the device into a 7-row layout (po_grid_dev.cu).
 int generate_grid_dev(const reflparams &r, double *out7, bool transform, bool spheric, cudaStream_t s);
