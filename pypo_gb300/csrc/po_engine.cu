@@ -130,14 +130,10 @@ static int device_info(DeviceInfo *&out)
     return 0;
 }
 
-// Share of a chunk that the last wave is expected to idle (choose_split): the
-// near field's adjoint. The far field's, whose stages are alike, is best left
-// at 0 (17.59 against 17.78 ms on 251,001 x 40,803 with 0.3).
-constexpr double kTailAdj = 0.3;
-
-// Chunks that an SM's last CTAs cost (load_split). The far field's tiles differ
-// more in cost (narrow, wide, lit).
-constexpr double kTailNF = 1.0, kTailFF = 3.0;
+// load_split's costs: near-field and scalar forward, scalar adjoint; far-field
+// forward (its tiles differ more in cost: narrow, wide, lit); near-field
+// adjoint, at 2 to 4 CTAs an SM; the FP64 kernels, whose pipe two CTAs fill.
+constexpr LoadCost kLoadNF = {8, 1.0, 0.2}, kLoadFF = {8, 3.0, 0.2}, kLoadAdj = {4, 0.2, 0.15}, kLoad64 = {2, 0.0, 0.03};
 
 // Resident CTAs per SM of a kernel (and its shared-memory attribute), looked
 // up once per device and kernel.
@@ -156,16 +152,14 @@ static int kernel_occupancy(DeviceInfo *di, void *fk, int threads, int smem, int
     return 0;
 }
 
-long choose_split(long nb, long ns, long slots, long max_chunks, long tile, double tail)
+// The far field's adjoint: waves of resident CTAs, with 0.3 of a stage for a
+// CTA's start, 0.3 of a chunk for the last wave's idle share and 0.1 of a stage
+// for a chunk's partials. Fitted to every split of 14 sizes (45^2 to 169^2
+// points a side): 1.8 % slower than the best on average and 6 % at most (3 %
+// and 11 % with 0.002 to 0.05 for the partials and no idle share).
+long choose_split(long nb, long ns, long slots, long max_chunks, long tile)
 {
     const long tiles = std::max(1L, (ns + tile - 1) / tile);
-    // a chunk's partials cost the epilogue about 0.05 of a full wave's tile,
-    // less where the owning blocks fill only part of a wave
-    const double per_chunk = 0.002 + 0.048 * std::min(1.0, (double)nb / (double)slots);
-    // a CTA's start (barriers, its first copies) costs about 0.3 of a tile:
-    // without it, 10,201 sources -> 40,401 targets went to 40 chunks of 2 tiles
-    // (2.10 ms; 2.06 with 12 of 7)
-    const double start = 0.3;
     long best = 1;
     double best_cost = 1e300;
     for (long s = 1; s <= std::min(tiles, std::min(std::max(1L, max_chunks), 1024L)); ++s) {
@@ -173,7 +167,7 @@ long choose_split(long nb, long ns, long slots, long max_chunks, long tile, doub
         const long real = (tiles + chunk - 1) / chunk;
         if (real != s) continue;
         const long waves = (nb * real + slots - 1) / slots;
-        const double cost = (double)waves * (chunk + start) + tail * chunk + per_chunk * real;
+        const double cost = waves * (chunk + 0.3) + 0.3 * chunk + 0.1 * real;
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = real;
@@ -182,17 +176,17 @@ long choose_split(long nb, long ns, long slots, long max_chunks, long tile, doub
     return best;
 }
 
-// The same for the forwards and the scalar adjoint, by the load of the fullest
-// SM: with about 8 CTAs or more to hide latencies an SM works at one rate
-// whatever their number, so the cost is its CTAs times their tiles; where they
-// are not all resident at once (occ) the last ones run with fewer beside them,
-// which costs about `tail` chunks; a CTA's start and partials cost 0.2 of a
-// tile. Fitted to every split of 92 sizes (40^2 to 301^2 points a side; near
-// field with and without M, scalar, far field): on average 0.2 to 0.9 % slower
-// than the best split and 3 % at most, where counting waves of resident CTAs
-// was 1 to 3 % and 14 % (4,422 x 4,356 with M 146.8 us, best 128.4). The
-// near field's adjoint, with 2 or 3 CTAs an SM, keeps the waves (1.3 % against 2 %).
-long load_split(long nb, long ns, long sms, long occ, long max_chunks, long tile, double tail)
+// The other kernels: the load of the fullest SM. With `busy` CTAs or more to
+// hide latencies an SM works at one rate whatever their number, so the cost is
+// its CTAs times their tiles; where they are not all resident at once (occ) the
+// last ones run with fewer beside them, which costs about `tail` chunks; a
+// CTA's start and partials cost `start` tiles. Fitted to every split of 134
+// sizes (40^2 to 301^2 points a side): the forwards and the scalar adjoint are
+// 0.2 to 0.9 % slower than the best split on average and 3 % at most, where
+// counting waves of resident CTAs was 1 to 3 % and 14 % (4,422 x 4,356 with M
+// 146.8 us, best 128.4); the near field's adjoint 1.1 % and 5 % (2.3 % and
+// 18 %). FP64, 9,999 sources -> 1,763 targets, forward and adjoint 13.45 -> 12.79 ms.
+long load_split(long nb, long ns, long sms, long occ, long max_chunks, long tile, LoadCost k)
 {
     const long tiles = std::max(1L, (ns + tile - 1) / tile);
     long best = 1;
@@ -202,8 +196,8 @@ long load_split(long nb, long ns, long sms, long occ, long max_chunks, long tile
         const long real = (tiles + chunk - 1) / chunk;
         if (real != s) continue;
         const long ctas = nb * real;
-        const double load = (double)std::max((ctas + sms - 1) / sms, 8L) + (ctas > sms * occ ? tail : 0.0);
-        const double cost = chunk * load + 0.2 * ctas / sms;
+        const double load = (double)std::max((ctas + sms - 1) / sms, k.busy) + (ctas > sms * occ ? k.tail : 0.0);
+        const double cost = chunk * load + k.start * ctas / sms;
         if (cost < best_cost - 1e-9) {
             best_cost = cost;
             best = real;
@@ -495,7 +489,7 @@ int run_device(const RunArgs &a)
     int occ = 1;
     if ((rc = device_info(di)) || (rc = kernel_occupancy(di, fk, kThreadsD, 0, occ))) return rc;
     const long ntb = (nt + kThreadsD - 1) / kThreadsD;
-    const long nsplit = choose_split(ntb, ns, (long)di->sms * occ, partial_cap(nt, nacc), kChunkD, 0.0);
+    const long nsplit = load_split(ntb, ns, di->sms, occ, partial_cap(nt, nacc), kChunkD, kLoad64);
     const long tiles = std::max(1L, (ns + kChunkD - 1) / kChunkD);
     long chunk = (tiles + nsplit - 1) / nsplit * kChunkD;
     double *srcd = nullptr, *part = nullptr;
@@ -564,7 +558,7 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
     const int occ = p.far ? di->occ_ff[p.ts > 0][p.has_m ? 1 : 0] : di->occ2[p.kind][p.ts > 0][p.has_m ? 1 : 0];
     const size_t room = std::min(sc.room(), (size_t)1 << 30);
     const long max_chunks = std::max(1L, (long)(room / ((size_t)p.nacc * nt * sizeof(double))));
-    p.nsplit = load_split(p.ntb, ns, di->sms, occ, max_chunks, kTile, p.far ? kTailFF : kTailNF);
+    p.nsplit = load_split(p.ntb, ns, di->sms, occ, max_chunks, kTile, p.far ? kLoadFF : kLoadNF);
     const long chunk_tiles = (p.tiles + p.nsplit - 1) / p.nsplit;
     p.chunk = chunk_tiles * (p.far ? 1 : kTile);   // tiles (far field) or sources per chunk
     if ((rc = sc.get(&p.part, (size_t)p.nsplit * p.nacc * nt))) return rc;
@@ -714,9 +708,10 @@ int run_adjoint(const AdjArgs &a)
     if ((rc = kernel_occupancy(di, fk, threads, smem, occ))) return rc;
     const long nsb = (ns + per_block - 1) / per_block;
     const long cap = partial_cap(ns, std::max(rows, 1));
-    const long split = kind == kKindScalar && !fp64
-                           ? load_split(nsb, nt, di->sms, occ, cap, tile_t, kTailNF)
-                           : choose_split(nsb, nt, (long)di->sms * occ, cap, tile_t, far ? 0.0 : kTailAdj);
+    const LoadCost load = fp64 ? kLoad64 : (kind == kKindScalar ? kLoadNF : kLoadAdj);
+    const long split = !far || fp64
+                           ? load_split(nsb, nt, di->sms, occ, cap, tile_t, load)
+                           : choose_split(nsb, nt, (long)di->sms * occ, cap, tile_t);
     const long tiles_t = std::max(1L, (nt + tile_t - 1) / tile_t);
     const long per_chunk = (tiles_t + split - 1) / split;
     long chunk = !fp64 && far ? per_chunk : per_chunk * tile_t;   // stages (mixed far field) or targets

@@ -126,13 +126,16 @@ cudaError_t ff_sort(void *temp, size_t *temp_bytes, const unsigned long long *ke
                     const int *idx_in, int *idx_out, long n, cudaStream_t s);
 
 // Number of chunks of a streamed axis (ns items in tiles of `tile`) for a
-// grid of `nb` owning blocks on `slots` resident CTAs: minimises waves times
-// chunk length, with a cost per CTA and per extra chunk, and `tail` of a chunk
-// for the last wave; at most max_chunks.
-long choose_split(long nb, long ns, long slots, long max_chunks, long tile, double tail);
-// The same by the load of the fullest SM, for kernels with several CTAs an SM
-// (occ resident at most).
-long load_split(long nb, long ns, long sms, long occ, long max_chunks, long tile, double tail);
+// grid of `nb` owning blocks, at most max_chunks: by waves of `slots` resident
+// CTAs.
+long choose_split(long nb, long ns, long slots, long max_chunks, long tile);
+// The same by the load of the fullest SM (occ CTAs of it resident at most).
+struct LoadCost {
+    long busy;     // CTAs that keep an SM busy
+    double tail;   // chunks that the last CTAs cost where not all are resident
+    double start;  // tiles that a CTA's start and partials cost
+};
+long load_split(long nb, long ns, long sms, long occ, long max_chunks, long tile, LoadCost k);
 
 // FP64 grid generation on the device into a 7-row layout (po_grid_dev.cu).
 int generate_grid_dev(const reflparams &r, double *out7, bool transform, bool spheric, cudaStream_t s);
