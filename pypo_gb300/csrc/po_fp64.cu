@@ -105,8 +105,13 @@ __device__ __forceinline__ Geo64 geo64(const double *t, const double *s)
 
 // The reference's illumination decision (lit_fp64) of a pair with n . d = nd:
 // clear of zero by far more than any rounding, or decided with its rounding.
+// Almost every pair is clear by its exponents alone (|nd| >= 2^(en - 1023) and
+// R < 2^(er - 1022), so en >= er - 38 gives |nd| > 1e-12 R), which takes no FP64
+// operation where the comparisons take three.
 __device__ __forceinline__ bool lit64(const double *n, const Geo64 &g, double nd)
 {
+    const int h = __double2hiint(nd), en = (h >> 20) & 0x7ff, er = (__double2hiint(g.R) >> 20) & 0x7ff;
+    if (en > 0 && en < 0x7ff && er < 0x7ff && en + 38 >= er) return h >= 0;
     const double thr = 1e-12 * g.R;
     if (nd > thr) return true;
     if (nd < -thr) return false;
@@ -119,6 +124,9 @@ __device__ __forceinline__ bool lit64(const double *n, const Geo64 &g, double nd
 // products summed left to right, no FMA).
 __device__ __forceinline__ bool lit64_ff(const double *n, const double *r, double nd)
 {
+    // 2^-39 > 1e-12; not NaN or infinite
+    const int h = __double2hiint(nd), en = (h >> 20) & 0x7ff;
+    if (en >= 1023 - 39 && en < 0x7ff) return h >= 0;
     if (nd > 1e-12) return true;
     if (nd < -1e-12) return false;
     return !(__dadd_rn(__dadd_rn(__dmul_rn(n[0], r[0]), __dmul_rn(n[1], r[1])), __dmul_rn(n[2], r[2])) < 0.0);
