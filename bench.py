@@ -571,8 +571,9 @@ def run_ours(args):
         torch.cuda.synchronize()
         peak = max(peak, blocks * 256 * iters * 16 / (p0.elapsed_time(p1) * 1e-3) / 1e12)
     mk = ("EH" if not far else "FF", not m_zero)
-    # pair-packed forward and adjoint (near field: the fused adjoint)
-    names = ["forward " + ("po_ff_kernel" if far else "po_pk_kernel"), "adjoint po_adj_pk_kernel"]
+    # forward and adjoint main kernels (near field: the fused adjoint)
+    names = ["forward " + (("po_ff0_kernel" if m_zero else "po_ff_kernel") if far else "po_pk_kernel"),
+             "adjoint " + ("po_ff_adj_kernel" if far else "po_adj_pk_kernel")]
     flops = [FWD_FLOPS[mk], ADJ_FLOPS[mk]]
     kernels = []
     for j in range(kernels_per_step):

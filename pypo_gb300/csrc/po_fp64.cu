@@ -20,7 +20,7 @@
 //   * a grid over (owning blocks, streamed chunks), so that a few thousand
 //     points still fill the GPU; the epilogues add the chunks in order.
 // Measured (one GB300): 101 x 99 sources -> 41 x 43 targets, EH, M = 0 (1.76e7
-// pairs), forward and every gradient 13.5 ms (229 ms with one block per 128
+// pairs), forward and every gradient 12.6 ms (229 ms with one block per 128
 // points, magnetic terms always and separate adjoint sides); 201 x 201 ->
 // 101 x 101, JMEH with M (4.1e8 pairs), forward 115 ms (295 ms), about 165
 // FP64 instructions a pair at 93 % of 2 per clock and SM.

@@ -25,7 +25,7 @@
 //     (tile_lit; the boxes travel ahead of the tile's records);
 //   * the per-pair test counts a pair lit when n . d >= 1e-6 R and unlit
 //     below -1e-6 R; a pair in between is left out, its tile flagged, and the
-//     rare path after the tile's fold lists it (nf_band_scan) for
+//     rare path after the tile's loop lists it (nf_band_scan) for
 //     po_band_fixup_kernel, which decides it with the reference's FP64
 //     rounding and adds its FP64 term;
 //   * a source chunk (blockIdx.y) writes its totals as doubles; the epilogue

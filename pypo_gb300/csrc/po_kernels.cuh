@@ -109,9 +109,8 @@ __host__ __device__ constexpr int adj_row(int kind, bool c, bool d, int a)
 constexpr int kThreadsD = 128;
 constexpr int kTileD = 64;
 // Granularity of a chunk of the streamed axis: 16 lets a few hundred points
-// fill the GPU and evens the last wave (101 x 99 -> 41 x 43 forward and
-// adjoint: 13.3 ms; 14.9 with 64, 12.8 with 32, but 13 x 13 -> 5 x 5: 0.45,
-// 0.78 and 0.61 ms).
+// fill the GPU (13 x 13 -> 5 x 5 forward and adjoint 0.45 ms; 0.61 with 32,
+// 0.78 with 64) and even the SMs' loads (101 x 99 -> 41 x 43: 12.6 ms).
 constexpr int kChunkD = 16;
 constexpr int kRecD = 18;       // x y z nx ny nz, J' 6, M' 6 (doubles)
 // Doubles per source record (scalar: point, normal, S'; M = 0: no M') and
