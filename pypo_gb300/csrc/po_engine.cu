@@ -565,6 +565,22 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
     return sc.commit();
 }
 
+// Indices of the sources in the order of their keys, into i_out (k_in, i_in:
+// ff_key_kernel's).
+static int ff_order(long ns, unsigned long long *k_in, unsigned long long *k_out, int *i_in, int *i_out, void *tmp,
+                    size_t tmp_bytes, cudaStream_t s)
+{
+    if (ns <= kFFRankMax) {
+        int n = (int)ns;
+        void *args[] = {&n, &k_in, &i_out};
+        return launch_pdl(ff_rank_kernel(), dim3((unsigned)((n + 31) / 32)), dim3(256), args, 0, s);
+    }
+    const cudaError_t e = ff_sort(tmp, &tmp_bytes, k_in, k_out, i_in, i_out, ns, s);
+    if (e != cudaSuccess) return fail(2, std::string("source sort: ") + err_str(e));
+    note_launches(1);
+    return 0;
+}
+
 int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
 {
     cudaStream_t s = a.stream;
@@ -595,14 +611,10 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
         int *i_in = p.order, *i_out = p.order + ns;
         void *kargs[] = {&ns, &src7, &p.frame, &k_in, &i_in};
         if (!rc) rc = launch_pdl(ff_key_kernel(), dim3(nblk_s), dim3(256), kargs, 0, s);
-        if (!rc) {
-            cudaError_t e = ff_sort(p.sort_tmp, &p.sort_bytes, k_in, k_out, i_in, i_out, ns, s);
-            if (e != cudaSuccess) rc = fail(2, std::string("source sort: ") + err_str(e));
-            else note_launches(1);
-        }
+        if (!rc) rc = ff_order(ns, k_in, k_out, i_in, i_out, p.sort_tmp, p.sort_bytes, s);
         const int *ord = i_out;
         void *pargs[] = {&ns, &ord, &src7, &cur, &gmode, &ncx, &ncy, &p.frame, &p.fac_re, &p.fac_im, &p.srcpk};
-        if (!rc) rc = launch(ff_pack_kernel(p.has_m), dim3((unsigned)p.tiles), dim3(kTile), pargs, 0, s);
+        if (!rc) rc = launch_pdl(ff_pack_kernel(p.has_m), dim3((unsigned)p.tiles), dim3(kTile), pargs, 0, s);
     }
     const float4 *srcc = p.srcpk, *tgtc = p.tgtpk;
     long ntiles = ns > 0 ? p.tiles : 0;
@@ -777,7 +789,7 @@ int run_adjoint(const AdjArgs &a)
     }
     int nspl = (int)split;
     double dsc = 1.0, tsc = 1.0;   // gradient per mm from the kernels' units
-    const int *ff_order = nullptr;   // far field: curve position -> source
+    const int *curve = nullptr;   // far field: curve position -> source
 
     if (fp64) {
         dsc = far ? 1.0 : -1.0;
@@ -812,14 +824,10 @@ int run_adjoint(const AdjArgs &a)
             int *i_in = ord, *i_out = ord + ns;
             void *kargs[] = {&ns, &src7, &frame, &k_in, &i_in};
             if (!rc) rc = launch_pdl(ff_key_kernel(), dim3(nblk_s), dim3(256), kargs, 0, s);
-            if (!rc) {
-                cudaError_t e = ff_sort(sort_tmp, &sort_bytes, k_in, k_out, i_in, i_out, ns, s);
-                if (e != cudaSuccess) rc = fail(2, std::string("source sort: ") + err_str(e));
-                else note_launches(1);
-            }
-            ff_order = i_out;
-            void *fpargs[] = {&ns, &ff_order, &src7, &cur, &gmode, &ncx, &ncy, &frame, &fac_re, &fac_im, &srcpk};
-            if (!rc) rc = launch(ff_pack_kernel(has_m), dim3((unsigned)ntile_s), dim3(kTile), fpargs, 0, s);
+            if (!rc) rc = ff_order(ns, k_in, k_out, i_in, i_out, sort_tmp, sort_bytes, s);
+            curve = i_out;
+            void *fpargs[] = {&ns, &curve, &src7, &cur, &gmode, &ncx, &ncy, &frame, &fac_re, &fac_im, &srcpk};
+            if (!rc) rc = launch_pdl(ff_pack_kernel(has_m), dim3((unsigned)ntile_s), dim3(kTile), fpargs, 0, s);
         } else {
             long sblk = (ns + 127) / 128;
             double *gam_out = a.mode == kEHP ? nullptr : gam;   // EHP: the cotangents are gam already
@@ -830,7 +838,7 @@ int run_adjoint(const AdjArgs &a)
         }
         const float4 *srcc = srcpk, *trc = reinterpret_cast<const float4 *>(trec);
         void *nfargs[] = {&srcc, &ns, &trc, &nt, &chunk, &part, &gt, &err, &band};
-        void *ffargs[] = {&srcc, &ns, &trc, &nstage, &chunk, &nt, &part, &err, &band, &ff_order};
+        void *ffargs[] = {&srcc, &ns, &trc, &nstage, &chunk, &nt, &part, &err, &band, &curve};
         timing_mark(s, true);
         if (!rc) rc = launch_pdl(fk, dim3((unsigned)nsb, (unsigned)split), dim3((unsigned)threads),
                                  far ? ffargs : nfargs, smem, s);

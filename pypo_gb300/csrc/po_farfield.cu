@@ -97,6 +97,48 @@ __global__ void po_ff_key_kernel(long ns, const double *__restrict__ src7, const
 
 // Bits of the sort key.
 constexpr int kFFKeyBits = 42;
+constexpr int kFFRankBits = 64 - kFFKeyBits;
+static_assert(kFFRankMax <= 1 << kFFRankBits, "a source's index fits behind its key");
+
+// The same order for few sources (kFFRankMax), as a stable sort of the keys
+// gives it: a source's place is the number of sources ahead of it, by (key,
+// index). A radix sort is eight dependent launches of 2 to 9 us however short
+// its input (58 us together); n^2 comparisons on all SMs are one launch of a
+// few us at some thousand sources. A CTA has 32 sources, one per lane; its warps
+// share the others, which pass through shared memory and are read by all lanes
+// at once.
+constexpr int kRankThreads = 256, kRankTile = 2048;
+
+__global__ void __launch_bounds__(kRankThreads)
+po_ff_rank_kernel(int n, const unsigned long long *__restrict__ key, int *__restrict__ order)
+{
+    constexpr int W = kRankThreads / 32;
+    __shared__ __align__(16) unsigned long long tile[kRankTile];
+    __shared__ int count[32];
+    pdl_wait();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+    // (key, index) in one word; the padding is behind every source
+    auto word = [&](int j) { return j < n ? key[j] << kFFRankBits | (unsigned long long)j : ~0ull; };
+    const unsigned long long own = word(i);
+    if (warp == 0) count[lane] = 0;
+    int c = 0;
+    for (int b = 0; b < n; b += kRankTile) {
+        const int pairs = (min(kRankTile, n - b) + 2 * W - 1) / (2 * W);   // a warp's share, in pairs
+        __syncthreads();
+        for (int q = threadIdx.x; q < 2 * W * pairs; q += kRankThreads) tile[q] = word(b + q);
+        __syncthreads();
+        const ulonglong2 *t = reinterpret_cast<const ulonglong2 *>(tile) + warp * pairs;
+#pragma unroll 8
+        for (int q = 0; q < pairs; ++q) {
+            const ulonglong2 v = t[q];
+            c += (v.x < own) + (v.y < own);
+        }
+    }
+    atomicAdd(&count[lane], c);
+    __syncthreads();
+    if (warp == 0 && i < n) order[count[lane]] = i;
+    pdl_trigger();
+}
 
 // ------------------------------------------------------------------ packing
 
@@ -122,6 +164,7 @@ po_ff_pack_kernel(long ns, const int *__restrict__ order, const double *__restri
     __shared__ float wn[W][6];
     __shared__ double tile_c[3], tile_q;   // centre; the wide tile's quantum, or 0
     float *bf = reinterpret_cast<float *>(buf);
+    pdl_wait();
     const Frame fr = *frp;
     const long j = (long)blockIdx.x * kTile + threadIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -734,6 +777,8 @@ po_ff0_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const flo
 int ff_smem_bytes(bool has_m) { return kStages * ff_tile4(has_m) * 16 + (has_m ? 12 : 6) * 2 * kThreads * 4; }
 
 void *ff_key_kernel() { return reinterpret_cast<void *>(&po_ff_key_kernel); }
+
+void *ff_rank_kernel() { return reinterpret_cast<void *>(&po_ff_rank_kernel); }
 
 void *ff_pack_kernel(bool has_m)
 {
