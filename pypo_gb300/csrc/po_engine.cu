@@ -107,9 +107,11 @@ static int device_info(DeviceInfo *&out)
             for (int ts = 0; ts < 2; ++ts)
                 for (int hm = 0; hm < 2; ++hm) {
                     if (kind == kKindFF || (kind == kKindScalar && hm)) continue;   // FF: occ_ff below
-                    void *fn = pk_kernel(kind, ts ? 1 : -1, hm != 0);
+                    void *fn = pk_kernel(kind, ts ? 1 : -1, hm != 0, false);
                     const int smem = pk_smem_bytes(kind, hm != 0);
                     PO_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+                    PO_CK(cudaFuncSetAttribute(pk_kernel(kind, ts ? 1 : -1, hm != 0, true),
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
                     int nb = 0;
                     PO_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kThreads, smem));
                     di.occ2[kind][ts][hm] = std::max(nb, 1);
@@ -559,6 +561,7 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
     const size_t room = std::min(sc.room(), (size_t)1 << 30);
     const long max_chunks = std::max(1L, (long)(room / ((size_t)p.nacc * nt * sizeof(double))));
     p.nsplit = load_split(p.ntb, ns, di->sms, occ, max_chunks, kTile, p.far ? kLoadFF : kLoadNF);
+    p.few = p.ntb * p.nsplit <= 2L * di->sms;
     const long chunk_tiles = (p.tiles + p.nsplit - 1) / p.nsplit;
     p.chunk = chunk_tiles * (p.far ? 1 : kTile);   // tiles (far field) or sources per chunk
     if ((rc = sc.get(&p.part, (size_t)p.nsplit * p.nacc * nt))) return rc;
@@ -627,8 +630,8 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
             rc = launch_pdl(ff_kernel(p.ts, p.has_m), dim3((unsigned)p.ntb, (unsigned)p.nsplit), dim3(kThreads), margs,
                         ff_smem_bytes(p.has_m), s);
         else
-            rc = launch_pdl(pk_kernel(p.kind, p.ts, p.has_m), dim3((unsigned)p.ntb, (unsigned)p.nsplit), dim3(kThreads),
-                        margs, pk_smem_bytes(p.kind, p.has_m), s);
+            rc = launch_pdl(pk_kernel(p.kind, p.ts, p.has_m, p.few), dim3((unsigned)p.ntb, (unsigned)p.nsplit),
+                        dim3(kThreads), margs, pk_smem_bytes(p.kind, p.has_m), s);
     }
     timing_mark(s, false);
     if (!rc && p.band.count && ns > 0) {

@@ -104,6 +104,7 @@ public:
 struct MixedPlan {
     int kind = 0, nacc = 0, ts = -1;
     bool far = false, has_m = false;
+    bool few = false;   // main kernel: at most two CTAs an SM
     double kappa = 0, fac_re = 0, fac_im = 0, zeta_inv = 0;
     long tiles = 0, ntb = 0, nsplit = 1, chunk = 0;
     double *part = nullptr;

@@ -260,8 +260,8 @@ __device__ __forceinline__ bool tile_lit(const float4 *tile, const float *tb)
 // and fold the sums into their float-float totals. With `boxes`, a near-field
 // tile proven lit for the CTA skips the per-pair illumination test (M = 0
 // kernels). The far field has its own kernel (po_farfield.cu).
-template <int KIND, int T, bool HAS_M>
-__global__ void __launch_bounds__(kThreads, pk_min_blocks(KIND, HAS_M))
+template <int KIND, int T, bool HAS_M, bool FEW>
+__global__ void __launch_bounds__(kThreads, pk_min_blocks(KIND, HAS_M, FEW))
 po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *__restrict__ tgt, long nt,
              double *__restrict__ part, int *__restrict__ err, int boxes, BandList bl)
 {
@@ -270,7 +270,7 @@ po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *
     constexpr int NF = NACC / 2;          // accumulators that a thread folds
     constexpr int HT = kThreads / 2;      // threads of a half
     constexpr int NR = 4 * R4 + (HAS_M ? 1 : 0);
-    constexpr int UNROLL = pk_unroll(KIND, HAS_M);
+    constexpr int UNROLL = pk_unroll(KIND, HAS_M, FEW);
     extern __shared__ __align__(128) float4 stage[];   // kStages tiles, the exchange, the compensation words
     __shared__ __align__(8) uint64_t full[kStages];
     pdl_wait();
@@ -607,19 +607,21 @@ __global__ void __launch_bounds__(256) po_fp32_probe_kernel(int iters, float see
 
 // ----------------------------------------------------------- instantiations
 
-template <int KIND, int T, bool HAS_M>
-static void *pk_ptr()
+template <int T, bool HAS_M>
+static void *pk_nf(bool few)
 {
-    return reinterpret_cast<void *>(&po_pk_kernel<KIND, T, HAS_M>);
+    return few ? reinterpret_cast<void *>(&po_pk_kernel<kKindNF, T, HAS_M, true>)
+               : reinterpret_cast<void *>(&po_pk_kernel<kKindNF, T, HAS_M, false>);
 }
 
-void *pk_kernel(int kind, int t_sign, bool has_m)
+void *pk_kernel(int kind, int t_sign, bool has_m, bool few)
 {
     if (kind == kKindNF) {
-        if (t_sign < 0) return has_m ? pk_ptr<kKindNF, -1, true>() : pk_ptr<kKindNF, -1, false>();
-        return has_m ? pk_ptr<kKindNF, 1, true>() : pk_ptr<kKindNF, 1, false>();
+        if (t_sign < 0) return has_m ? pk_nf<-1, true>(few) : pk_nf<-1, false>(few);
+        return has_m ? pk_nf<1, true>(few) : pk_nf<1, false>(few);
     }
-    return t_sign < 0 ? pk_ptr<kKindScalar, -1, false>() : pk_ptr<kKindScalar, 1, false>();
+    return t_sign < 0 ? reinterpret_cast<void *>(&po_pk_kernel<kKindScalar, -1, false, false>)
+                      : reinterpret_cast<void *>(&po_pk_kernel<kKindScalar, 1, false, false>);
 }
 
 // Precision conversions of the float drop-in ABI's buffers (n elements).

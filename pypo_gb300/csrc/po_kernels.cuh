@@ -37,11 +37,18 @@ constexpr int kMinBlocks = PO_MINB;    // resident CTAs per SM asked of ptxas
 // at 5 and 4 (1 record 2.084, 3 2.056; 4 CTAs 2.047-2.089). Scalar, same size:
 // 0.443 with 4 records (1 0.478, 2 0.452, 3 0.441; 10,403 x 14,399 0.173,
 // 0.199, 0.177, 0.177).
-__host__ __device__ constexpr int pk_min_blocks(int kind, bool has_m)
+// FEW: a grid that leaves an SM two CTAs or fewer has nothing to hide a warp's
+// latencies but its own instructions, so the near field then takes eight
+// records at a time and the registers that this needs (156): 1,023 x 899 with M
+// 35.8 -> 34.0 us, M = 0 1 to 4 % (at four CTAs an SM up to 30 % slower).
+__host__ __device__ constexpr int pk_min_blocks(int kind, bool has_m, bool few)
 {
-    return kind == kKindScalar ? 1 : (has_m ? 5 : 4);
+    return kind == kKindScalar || few ? 1 : (has_m ? 5 : 4);
 }
-__host__ __device__ constexpr int pk_unroll(int kind, bool has_m) { return kind == kKindNF && !has_m ? 3 : 4; }
+__host__ __device__ constexpr int pk_unroll(int kind, bool has_m, bool few)
+{
+    return few ? 8 : (kind == kKindNF && !has_m ? 3 : 4);
+}
 #ifndef PO_STAGES
 #define PO_STAGES 3
 #endif
@@ -219,7 +226,7 @@ inline int pk_smem_bytes(int kind, bool has_m)
     return kStages * pk_tile4(kind, has_m, kTile) * 16 + 2 * na * kThreads * 8;
 }
 
-void *pk_kernel(int kind, int t_sign, bool has_m);
+void *pk_kernel(int kind, int t_sign, bool has_m, bool few);
 void *pack_kernel(bool scalar, bool has_m);   // source tiles (near field, scalar) and targets
 void *fp64_kernel(int kind, bool has_m);
 void *frame_kernel();
