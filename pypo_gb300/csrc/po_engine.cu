@@ -118,9 +118,11 @@ static int device_info(DeviceInfo *&out)
                 }
         for (int ts = 0; ts < 2; ++ts)
             for (int hm = 0; hm < 2; ++hm) {
-                void *fn = ff_kernel(ts ? 1 : -1, hm != 0);
+                void *fn = ff_kernel(ts ? 1 : -1, hm != 0, false);
                 const int smem = ff_smem_bytes(hm != 0);
                 PO_CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+                PO_CK(cudaFuncSetAttribute(ff_kernel(ts ? 1 : -1, hm != 0, true),
+                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
                 int nb = 0;
                 PO_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kThreads, smem));
                 di.occ_ff[ts][hm] = std::max(nb, 1);
@@ -627,8 +629,8 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
     timing_mark(s, true);
     if (!rc) {
         if (p.far)
-            rc = launch_pdl(ff_kernel(p.ts, p.has_m), dim3((unsigned)p.ntb, (unsigned)p.nsplit), dim3(kThreads), margs,
-                        ff_smem_bytes(p.has_m), s);
+            rc = launch_pdl(ff_kernel(p.ts, p.has_m, p.few), dim3((unsigned)p.ntb, (unsigned)p.nsplit),
+                        dim3(kThreads), margs, ff_smem_bytes(p.has_m), s);
         else
             rc = launch_pdl(pk_kernel(p.kind, p.ts, p.has_m, p.few), dim3((unsigned)p.ntb, (unsigned)p.nsplit),
                         dim3(kThreads), margs, pk_smem_bytes(p.kind, p.has_m), s);

@@ -517,14 +517,15 @@ po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const floa
 // ms on 249,999 x 40,803), so po_ff_kernel stays for those.
 // `boxes`: the tiles' normal boxes may prove a tile lit for the CTA's
 // directions, which skips the per-pair illumination test.
-template <int T>
-__global__ void __launch_bounds__(kThreads, kMinBlocksFF0)
+template <int T, bool FEW>
+__global__ void __launch_bounds__(kThreads, ff0_min_blocks(FEW))
 po_ff0_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const float4 *__restrict__ tgt, long nt,
              double *__restrict__ part, int *__restrict__ err, int boxes, BandList bl, long ns,
              const int *__restrict__ order)
 {
     constexpr int R4 = ff_rec4(false), T4 = ff_tile4(false), TP = 2;
     constexpr int NA = 6;   // S_J (re xyz, im xyz)
+    constexpr int UNROLL = ff0_unroll(FEW);
     extern __shared__ __align__(128) float4 stage[];   // kStages tiles, then the compensation words
     __shared__ __align__(8) uint64_t full[kStages];
     __shared__ float tbox_w[kThreads / 32][6];
@@ -640,7 +641,7 @@ po_ff0_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const flo
             // unless the tile is proven lit; the lo offsets in a wide tile)
             constexpr int NLD = VAR == 0 ? 5 : (VAR == 1 ? 6 : 8);
             const float4 *recs = tile + kFFHead;
-#pragma unroll kUnrollFF0
+#pragma unroll UNROLL
             for (int s = 0; s < kTile / 2; ++s) {
                 float rec[2][2 * NLD];
 #pragma unroll
@@ -786,11 +787,16 @@ void *ff_pack_kernel(bool has_m)
                  : reinterpret_cast<void *>(&po_ff_pack_kernel<false>);
 }
 
-void *ff_kernel(int t_sign, bool has_m)
+template <int T>
+static void *ff0_sel(bool few)
 {
-    if (t_sign < 0)
-        return has_m ? reinterpret_cast<void *>(&po_ff_kernel<-1>) : reinterpret_cast<void *>(&po_ff0_kernel<-1>);
-    return has_m ? reinterpret_cast<void *>(&po_ff_kernel<1>) : reinterpret_cast<void *>(&po_ff0_kernel<1>);
+    return few ? reinterpret_cast<void *>(&po_ff0_kernel<T, true>) : reinterpret_cast<void *>(&po_ff0_kernel<T, false>);
+}
+
+void *ff_kernel(int t_sign, bool has_m, bool few)
+{
+    if (t_sign < 0) return has_m ? reinterpret_cast<void *>(&po_ff_kernel<-1>) : ff0_sel<-1>(few);
+    return has_m ? reinterpret_cast<void *>(&po_ff_kernel<1>) : ff0_sel<1>(few);
 }
 
 // Radix sort of (key, index) pairs on `s`; with temp == nullptr only sets

@@ -94,7 +94,10 @@ constexpr int kFFDirs = 64;   // directions per stage of the far-field adjoint
 // The far-field forward without magnetic currents, two pair records an
 // iteration at 5 CTAs/SM: 105.1 ms on 1,002,001 x 160,801 (one record 112.3;
 // at 4 CTAs/SM 109.7 with one, 111.7 with two, 109.4 with four).
-constexpr int kMinBlocksFF0 = 5, kUnrollFF0 = 2;
+// FEW (at most two CTAs an SM), as in the near field: eight pair records an
+// iteration, 2,652 x 1,722 61.2 -> 58.9 us.
+__host__ __device__ constexpr int ff0_min_blocks(bool few) { return few ? 1 : 5; }
+__host__ __device__ constexpr int ff0_unroll(bool few) { return few ? 8 : 2; }
 constexpr int kUnrollA = PO_UNROLL_A;   // target pairs per iteration of the adjoint pair loop
 constexpr int kAccAdj = 13;   // the pair formulas' accumulators: 12 of the currents, 1 of the displacement
 // Of those, the ones that a call's kernels keep, as rows of the partials: the
@@ -208,7 +211,7 @@ constexpr long kFFRankMax = 20000;
 void *ff_key_kernel();
 void *ff_rank_kernel();
 void *ff_pack_kernel(bool has_m);
-void *ff_kernel(int t_sign, bool has_m);
+void *ff_kernel(int t_sign, bool has_m, bool few);
 
 // Source tiles of the near-field and scalar forward (layout in po_kernels.cu):
 // float4 ahead of the records, per record, and of a tile of n sources.
