@@ -87,10 +87,10 @@ __global__ void po_adj_ehp_cot_kernel(long nt, const double *__restrict__ cot, c
 // is 0 (of the N = 1 instance).
 template <int G, int N>
 __global__ void __launch_bounds__(kEpiThreads)
-po_adj_epilogue_kernel(int kind, int nsplit, long ns, const double *__restrict__ part,
+po_adj_epilogue_kernel(int kind, int nsplit, long ns, const double *part,
                        const double *__restrict__ src7, int gmode, int ncx, int ncy, double fac_re, double fac_im,
                        double dscale, double *__restrict__ grad_cur, double *__restrict__ grad_ds, long nblk_s, long nt,
-                       const double *__restrict__ gt, double tscale, double *__restrict__ grad_dt)
+                       const double *gt, double tscale, double *__restrict__ grad_dt)
 {
     constexpr int SB = kEpiThreads / G;   // sources per block
     __shared__ double sh[G > 1 ? G / 2 : 1][G > 1 ? N : 1][G > 1 ? SB : 1];
@@ -161,7 +161,7 @@ po_adj_epilogue_kernel(int kind, int nsplit, long ns, const double *__restrict__
 // po_adjoint_pk.cu, rec4 float4 per pair); its sum gt cleared.
 __global__ void __launch_bounds__(128)
 po_adj_pack_kernel(long ns, const double *__restrict__ src7, const double *__restrict__ cur, int gmode, int ncx,
-                   int ncy, const Frame *__restrict__ frp, double fac_re, double fac_im, int scalar, long sblk,
+                   int ncy, const Frame *frp, double fac_re, double fac_im, int scalar, long sblk,
                    float4 *__restrict__ src, int mode, long nt, const double *__restrict__ tgt7,
                    const double *__restrict__ cot, double t, double *__restrict__ gam, int rec4,
                    float *__restrict__ tgt, double *__restrict__ gt)

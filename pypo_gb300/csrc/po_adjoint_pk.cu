@@ -321,7 +321,7 @@ __device__ __forceinline__ void adj_band_scan(const float4 *tile, int cnt, long 
 template <int KIND, int T, bool HAS_M, bool WANT_C, bool WANT_D, bool WANT_T>
 __global__ void __launch_bounds__(kThreadsA, WANT_C ? (HAS_M ? kMinBlocksA2M : kMinBlocksA2)
                                                     : (HAS_M ? kMinBlocksA2MN : kMinBlocksA2N))
-po_adj_pk_kernel(const float4 *__restrict__ srcpk, long ns, const float4 *__restrict__ trec, long nt, long chunk,
+po_adj_pk_kernel(const float4 *srcpk, long ns, const float4 *trec, long nt, long chunk,
                  double *__restrict__ part, double *__restrict__ gt, int *__restrict__ err, BandList bl)
 {
     constexpr int RT = adj2_rec(HAS_M, WANT_T);

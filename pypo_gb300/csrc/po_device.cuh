@@ -59,7 +59,10 @@ __device__ __forceinline__ void fence_proxy_async()
 // Programmatic dependent launch. A kernel launched after another one with
 // programmatic stream serialisation may start while that one runs: it begins
 // with pdl_wait(), which returns when every earlier kernel's writes are
-// visible. pdl_trigger() lets the next kernel's blocks be scheduled once every
+// visible. What those write is therefore not constant for its lifetime, and
+// only the caller's inputs may be `const T *__restrict__` parameters of it (a
+// promise that lets the compiler read early or through the non-coherent path).
+// pdl_trigger() lets the next kernel's blocks be scheduled once every
 // block of this one has called it or ended; without a dependent both do
 // nothing. It stands at a kernel's end: called at the start of a kernel of
 // many blocks, it has the next kernel's few blocks placed on whichever SMs

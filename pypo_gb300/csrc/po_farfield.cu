@@ -71,7 +71,7 @@ __device__ __forceinline__ unsigned long long hilbert_index(uint32_t x, uint32_t
 
 // Sort keys of the sources: the Hilbert index of their projection onto the
 // two axes along which their box is widest, on one common scale.
-__global__ void po_ff_key_kernel(long ns, const double *__restrict__ src7, const Frame *__restrict__ frp,
+__global__ void po_ff_key_kernel(long ns, const double *__restrict__ src7, const Frame *frp,
                                  unsigned long long *__restrict__ key, int *__restrict__ idx)
 {
     pdl_wait();
@@ -110,7 +110,7 @@ static_assert(kFFRankMax <= 1 << kFFRankBits, "a source's index fits behind its 
 constexpr int kRankThreads = 256, kRankTile = 2048;
 
 __global__ void __launch_bounds__(kRankThreads)
-po_ff_rank_kernel(int n, const unsigned long long *__restrict__ key, int *__restrict__ order)
+po_ff_rank_kernel(int n, const unsigned long long *key, int *__restrict__ order)
 {
     constexpr int W = kRankThreads / 32;
     __shared__ __align__(16) unsigned long long tile[kRankTile];
@@ -154,8 +154,8 @@ po_ff_rank_kernel(int n, const unsigned long long *__restrict__ key, int *__rest
 // of 2,652 sources x 1,640 directions 142 -> 129 us).
 template <bool HAS_M>
 __global__ void __launch_bounds__(kTile)
-po_ff_pack_kernel(long ns, const int *__restrict__ order, const double *__restrict__ src7,
-                  const double *__restrict__ cur, int gmode, int ncx, int ncy, const Frame *__restrict__ frp,
+po_ff_pack_kernel(long ns, const int *order, const double *__restrict__ src7,
+                  const double *__restrict__ cur, int gmode, int ncx, int ncy, const Frame *frp,
                   double fac_re, double fac_im, float4 *__restrict__ out)
 {
     constexpr int R4 = ff_rec4(HAS_M), T4 = ff_tile4(HAS_M), W = kTile / 32;
@@ -279,7 +279,7 @@ __device__ __forceinline__ float2 ff_ndr2(const float2 *r, const float2 *rf)
 // curve position of its first source.
 template <int TP, int R4>
 __device__ __forceinline__ void ff_band_scan(const float4 *recs, long pos0, const float2 (*rf)[3], long tbase, long ns,
-                                             long nt, const int *__restrict__ order, BandList bl)
+                                             long nt, const int *order, BandList bl)
 {
 #pragma unroll 1
     for (int s = 0; s < kTile / 2; ++s) {
@@ -307,9 +307,9 @@ __device__ __forceinline__ void ff_band_scan(const float4 *recs, long pos0, cons
 // operation of the pair loop.
 template <int T>
 __global__ void __launch_bounds__(kThreads, kMinBlocks)
-po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const float4 *__restrict__ tgt, long nt,
+po_ff_kernel(const float4 *src, long ntiles, long chunk, const float4 *tgt, long nt,
              double *__restrict__ part, int *__restrict__ err, int, BandList bl, long ns,
-             const int *__restrict__ order)
+             const int *order)
 {
     constexpr int R4 = ff_rec4(true), T4 = ff_tile4(true), TP = 2;
     constexpr int NA = 12;   // S_J (re xyz, im xyz), then S_M
@@ -519,9 +519,9 @@ po_ff_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const floa
 // directions, which skips the per-pair illumination test.
 template <int T, bool FEW>
 __global__ void __launch_bounds__(kThreads, ff0_min_blocks(FEW))
-po_ff0_kernel(const float4 *__restrict__ src, long ntiles, long chunk, const float4 *__restrict__ tgt, long nt,
+po_ff0_kernel(const float4 *src, long ntiles, long chunk, const float4 *tgt, long nt,
              double *__restrict__ part, int *__restrict__ err, int boxes, BandList bl, long ns,
-             const int *__restrict__ order)
+             const int *order)
 {
     constexpr int R4 = ff_rec4(false), T4 = ff_tile4(false), TP = 2;
     constexpr int NA = 6;   // S_J (re xyz, im xyz)

@@ -218,9 +218,9 @@ __device__ __forceinline__ void ff_rotate_cot(float *r, const float *c)
 // both 1.61, the currents' alone 1.09, the displacement's alone 0.88).
 template <int T, bool HAS_M, bool WANT_C, bool WANT_D>
 __global__ void __launch_bounds__(kThreadsFA, HAS_M ? kMinBlocksFAM : kMinBlocksFA)
-po_ff_adj_kernel(const float4 *__restrict__ tiles, long ns, const float4 *__restrict__ dirs, long nstage, long chunk,
+po_ff_adj_kernel(const float4 *tiles, long ns, const float4 *dirs, long nstage, long chunk,
                  long nt, double *__restrict__ part, int *__restrict__ err, BandList bl,
-                 const int *__restrict__ order)
+                 const int *order)
 {
     constexpr int R4 = ff_rec4(HAS_M), T4 = ff_tile4(HAS_M);
     constexpr int NA = adj_rows(kKindFF, WANT_C, WANT_D);

@@ -617,7 +617,7 @@ template <int KIND, bool WANT_T>
 __global__ void __launch_bounds__(256)
 po_adj_band_fixup_kernel(BandList bl, long ns, const double *__restrict__ src7, const double *__restrict__ cur,
                          int gmode, int ncx, int ncy, double fac_re, double fac_im, long nt,
-                         const double *__restrict__ tgt7, const double *__restrict__ gam, Wave64 w,
+                         const double *__restrict__ tgt7, const double *gam, Wave64 w,
                          double inv_kappa, int want_c, int want_d, double *__restrict__ part,
                          double *__restrict__ gt, int *__restrict__ err)
 {

@@ -262,7 +262,7 @@ __device__ __forceinline__ bool tile_lit(const float4 *tile, const float *tb)
 // kernels). The far field has its own kernel (po_farfield.cu).
 template <int KIND, int T, bool HAS_M, bool FEW>
 __global__ void __launch_bounds__(kThreads, pk_min_blocks(KIND, HAS_M, FEW))
-po_pk_kernel(const float4 *__restrict__ src, long ns, long chunk, const float4 *__restrict__ tgt, long nt,
+po_pk_kernel(const float4 *src, long ns, long chunk, const float4 *tgt, long nt,
              double *__restrict__ part, int *__restrict__ err, int boxes, BandList bl)
 {
     constexpr int HEAD = pk_head(KIND, HAS_M), R4 = pk_rec4(KIND, HAS_M), T4 = pk_tile4(KIND, HAS_M, kTile);
@@ -482,7 +482,7 @@ __device__ __forceinline__ void cross_d(const double a[3], const double b[3], do
 // loads and one SM's FP64 additions.
 template <int G>
 __global__ void __launch_bounds__(kEpiThreads)
-po_epilogue_kernel(int mode, int nacc, int nsplit, long nt, const double *__restrict__ part,
+po_epilogue_kernel(int mode, int nacc, int nsplit, long nt, const double *part,
                    const double *__restrict__ tgt7, double t, double zeta_inv, double *__restrict__ out)
 {
     constexpr int TB = kEpiThreads / G;   // targets per block

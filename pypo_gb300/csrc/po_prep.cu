@@ -159,7 +159,7 @@ __device__ __forceinline__ void pack_target(long i, long nt, const double *tgt7,
 template <bool SCALAR, bool HAS_M>
 __global__ void __launch_bounds__(kTile)
 po_pack_kernel(long ns, const double *__restrict__ src7, const double *__restrict__ cur, int gmode, int ncx, int ncy,
-               const Frame *__restrict__ frp, double fac_re, double fac_im, long tiles,
+               const Frame *frp, double fac_re, double fac_im, long tiles,
                float4 *__restrict__ src, long nt, const double *__restrict__ tgt7, int far, float4 *__restrict__ tgt)
 {
     constexpr int KIND = SCALAR ? kKindScalar : kKindNF;
