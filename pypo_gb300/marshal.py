@@ -56,12 +56,13 @@ def fill_reflparams(refl, ctype=ctypes.c_double):
     return st, keep
 
 
-def _point_rows(st, first, block):
-    """Point the struct's consecutive pointer members, from the one named
-    `first` on, at the rows of `block` (one write of all the addresses: a
-    ctypes pointer object per member takes 4 us each)."""
+def _point_rows(st, first, n, block):
+    """Point the struct's n consecutive pointer members, from the one named
+    `first` on, at the first n rows of `block` (one write of all the addresses:
+    a ctypes pointer object per member takes 4 us each)."""
+    if block.shape[0] < n:
+        raise IndexError(f"a block of {n} rows is needed, this one has {block.shape[0]}")
     at = getattr(type(st), first).offset
-    n = block.shape[0]
     np.ndarray((n,), np.uintp, buffer=st, offset=at)[:] = block.ctypes.data + block.strides[0] * np.arange(n)
 
 
@@ -70,7 +71,7 @@ def alloc_container(n, ctype=ctypes.c_double):
     st = S.reflcontainer() if ctype is ctypes.c_double else S.reflcontainerf()
     block = np.zeros((7, n), dtype=_NP[ctype])
     st.size = n
-    _point_rows(st, "x", block)
+    _point_rows(st, "x", 7, block)
     st._block = block
     return st, block
 
@@ -80,7 +81,7 @@ def fill_container(block, ctype=ctypes.c_double):
     block = np.ascontiguousarray(block, dtype=_NP[ctype])
     st = S.reflcontainer() if ctype is ctypes.c_double else S.reflcontainerf()
     st.size = block.shape[1]
-    _point_rows(st, "x", block)
+    _point_rows(st, "x", 7, block)
     st._block = block
     return st, block
 
@@ -91,7 +92,7 @@ def bundle(cls, block, ctype):
     alive as long as the struct does."""
     st = cls()
     assert block.shape[0] == len(cls._fields_)
-    _point_rows(st, cls._fields_[0][0], block)
+    _point_rows(st, cls._fields_[0][0], len(cls._fields_), block)
     st._block = block
     return st
 
