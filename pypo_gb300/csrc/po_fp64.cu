@@ -56,12 +56,28 @@ __device__ __forceinline__ void rsqrt64(double x, double &rinv, double &root)
     root = fma(fma(-h, h, x), 0.5 * rinv, h);
 }
 
-// cos and sin of the angle x. X = x 2/pi quarter turns, n = rint(X) from one
+// cos and sin past sincos64's range: the general reduction.
+__device__ __noinline__ double2 sincos64_far(double x)
+{
+    double s, c;
+    sincos(x, &s, &c);
+    return make_double2(c, s);
+}
+
+// cos and sin of the angle x. Past 2^51, infinite or NaN: the call above (one
+// integer comparison a pair, 0.1 % on average over 39 sizes and 0.8 % at most,
+// the near field's adjoint). Up to there: X = x 2/pi quarter turns, n = rint(X) from one
 // fma against 1.5 2^52, y = X - n exact but for 2/pi's 2^-106; sin and cos of
 // y pi/2, |y| <= 1/2, by polynomials in y^2 (minimax fits by Remez exchange,
 // errors 4e-18 and 4e-20 before rounding), placed by n mod 4.
 __device__ __forceinline__ void sincos64(double x, double &cs, double &sn)
 {
+    if ((__double2hiint(x) & 0x7fffffff) >= 0x43200000) {
+        const double2 f = sincos64_far(x);
+        cs = f.x;
+        sn = f.y;
+        return;
+    }
     const double magic = 6755399441055744.0;
     const double h = 0.6366197723675814, l = -3.935735335036497e-17;   // 2/pi
     const double t = fma(x, h, magic);
