@@ -154,7 +154,10 @@ po_adj_epilogue_kernel(int kind, int nsplit, long ns, const double *part,
 //   r4 = (My.re, My.im, Mz.re, Mz.im)
 //   r5 = (n.z, 0, 0, 0)
 // (scalar: S' in the J.x slot, the rest zero); fac: complex factor folded into
-// the currents (times weight * area). The remaining blocks: a target each
+// the currents (times weight * area). The last block's threads past the sources
+// pack a record without normal and currents at 4096 quanta, where no target is
+// (they reach to 1025), so that the pair kernel's thread for it adds zeros, not
+// 0 / 0, to the target sums. The remaining blocks: a target each
 // thread (an odd count's last pair padded with the last target carrying no
 // cotangent): its cotangents mapped onto E and H, written to gam (unless null)
 // for the near-tangent pairs and into the pair-packed records (layout in
@@ -170,7 +173,14 @@ po_adj_pack_kernel(long ns, const double *__restrict__ src7, const double *__res
     const Frame fr = *frp;
     if ((long)blockIdx.x < sblk) {
         const long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-        if (i >= ns) return;
+        if (i >= ns) {
+            float4 *o = src + (size_t)kRec * i;
+            o[0] = make_float4(0.f, 0.f, (float)(4096.0 * fr.q), 0.f);
+#pragma unroll
+            for (int q = 1; q < kRec; ++q) o[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+            pdl_trigger();
+            return;
+        }
         float h[3], l[3];
         for (int c = 0; c < 3; ++c) split_hi_lo((src7[c * ns + i] - fr.o[c]) * fr.kappa, fr, h[c], l[c]);
         const double w = trap_weight(i, gmode, ncx, ncy) * src7[6 * ns + i];

@@ -338,8 +338,7 @@ po_adj_pk_kernel(const float4 *srcpk, long ns, const float4 *trec, long nt, long
     {
         float4 q[kRec];
 #pragma unroll
-        for (int c = 0; c < kRec; ++c) q[c] = si < ns ? srcpk[(size_t)kRec * si + c] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if (si >= ns) q[0].z = 1e3f;   // idle lanes: keep R > 0 (zero currents)
+        for (int c = 0; c < kRec; ++c) q[c] = srcpk[(size_t)kRec * si + c];   // a record for each thread
         s.sh[0] = q[0].x; s.sh[1] = q[0].y; s.sh[2] = q[0].z;
         s.sl[0] = q[1].x; s.sl[1] = q[1].y; s.sl[2] = q[1].z;
         s.n[0] = q[0].w; s.n[1] = q[1].w; s.n[2] = q[5].x;

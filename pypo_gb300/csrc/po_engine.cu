@@ -769,7 +769,7 @@ int run_adjoint(const AdjArgs &a)
             sc.get(&srcpk, (size_t)ntile_s * ff_tile4(has_m));
             sc.get(&trec, (size_t)nstage * ff_adj_stage4() * 4);
         } else {
-            sc.get(&srcpk, (size_t)ns * kRec);
+            sc.get(&srcpk, (size_t)nsb * threads * kRec);
             sc.get(&trec, (size_t)npair * rec4 * 4);
         }
     }
@@ -834,7 +834,7 @@ int run_adjoint(const AdjArgs &a)
             void *fpargs[] = {&ns, &curve, &src7, &cur, &gmode, &ncx, &ncy, &frame, &fac_re, &fac_im, &srcpk};
             if (!rc) rc = launch_pdl(ff_pack_kernel(has_m), dim3((unsigned)ntile_s), dim3(kTile), fpargs, 0, s);
         } else {
-            long sblk = (ns + 127) / 128;
+            long sblk = nsb;
             double *gam_out = a.mode == kEHP ? nullptr : gam;   // EHP: the cotangents are gam already
             void *pargs[] = {&ns, &src7, &cur, &gmode, &ncx, &ncy, &frame, &fac_re, &fac_im, (void *)&scalar, &sblk,
                              &srcpk, &mode, &nt, &tgt7, &cot, &t, &gam_out, &rec4, &trec, &gt};
