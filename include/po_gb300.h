@@ -340,8 +340,9 @@ int po_run_dev_static(int mode, long ns, const double *src7, int gmode, int ncx,
  * EH forward again and maps the cotangents through the EHP reflection's
  * Jacobian there (forward-mode dual numbers) before the EH adjoint. The
  * Green's function is recomputed, nothing of size ns*nt is stored.
- * precision 0 mixed, 1 plain FP64. flags bit 0: M == 0 on the source.
- * po_adjoint_dev queues on `stream` (device pointers); po_adjoint_d takes host
+ * precision 0 mixed, 1 plain FP64 (the same bits each time; mixed sums grad_dt
+ * with atomics, its last bits vary between runs). flags bit 0: M == 0 on the
+ * source. po_adjoint_dev queues on `stream` (device pointers); po_adjoint_d takes host
  * buffers and synchronises. */
 int po_adjoint_dev(int mode, long ns, const double *src7, int gmode, int ncx, int ncy,
                    const double *cur, long nt, const double *tgt7,

@@ -724,10 +724,13 @@ int run_adjoint(const AdjArgs &a)
     int occ = 1, rc = 0;
     if ((rc = kernel_occupancy(di, fk, threads, smem, occ))) return rc;
     const long nsb = (ns + per_block - 1) / per_block;
+    // FP64 target sums, a row of nt a source block: as many blocks a launch as
+    // partial_cap has rows for (all of them but for the largest calls)
+    const long nsb_l = fp64 && want_t ? std::min(nsb, partial_cap(nt, 1)) : nsb;
     const long cap = partial_cap(ns, std::max(rows, 1));
     const LoadCost load = fp64 ? kLoad64 : (kind == kKindScalar ? kLoadNF : kLoadAdj);
     const long split = !far || fp64
-                           ? load_split(nsb, nt, di->sms, occ, cap, tile_t, load)
+                           ? load_split(nsb_l, nt, di->sms, occ, cap, tile_t, load)
                            : choose_split(nsb, nt, (long)di->sms * occ, cap, tile_t);
     const long tiles_t = std::max(1L, (nt + tile_t - 1) / tile_t);
     const long per_chunk = (tiles_t + split - 1) / split;
@@ -735,6 +738,7 @@ int run_adjoint(const AdjArgs &a)
 
     PoolScratch sc(s);
     double *gam = nullptr, *eh = nullptr, *part = nullptr, *gt = nullptr, *srcd = nullptr, *trecd = nullptr;
+    double *tsum = nullptr;
     Frame *frame = nullptr;
     float4 *srcpk = nullptr;
     float *trec = nullptr;
@@ -753,6 +757,7 @@ int run_adjoint(const AdjArgs &a)
     if (fp64) {
         sc.get(&srcd, (size_t)ns * rec);
         sc.get(&trecd, (size_t)nt * adj64_rec(kind));
+        if (want_t) sc.get(&tsum, (size_t)nsb_l * nt);
     } else {
         sc.get(&frame, 1);
         if (kind != kKindScalar) {
@@ -807,11 +812,17 @@ int run_adjoint(const AdjArgs &a)
         if (!rc) rc = launch(pack_src_d_kernel(), dim3(nblk_s), dim3(256), pargs, 0, s);
         void *tpargs[] = {&nt, &tgt7, &gam, &trecd};
         if (!rc) rc = launch(adj_pack_tgt_d_kernel(kind), dim3(nblk_t), dim3(256), tpargs, 0, s);
-        if (want_t) PO_CK_RC(cudaMemsetAsync(gt, 0, sizeof(double) * nt, s));
-        void *sargs[] = {&srcd, &ns, &trecd, &nt, &chunk, &w, &part, &gt};
-        timing_mark(s, true);
-        if (!rc) rc = launch(fk, dim3((unsigned)nsb, (unsigned)split), dim3((unsigned)threads), sargs, 0, s);
-        timing_mark(s, false);
+        for (long first = 0; first < nsb && !rc; first += nsb_l) {
+            long blocks = std::min(nsb_l, nsb - first);
+            void *sargs[] = {&srcd, &ns, &first, &trecd, &nt, &chunk, &w, &part, &tsum};
+            timing_mark(s, true);
+            rc = launch(fk, dim3((unsigned)blocks, (unsigned)split), dim3((unsigned)threads), sargs, 0, s);
+            timing_mark(s, false);
+            int add = first > 0;
+            void *gargs[] = {&blocks, &nt, &tsum, &add, &gt};
+            if (!rc && want_t)
+                rc = launch_pdl(adj_tsum_kernel(), dim3((unsigned)((nt + 31) / 32)), dim3(256), gargs, 0, s);
+        }
     } else {
         dsc = far ? kappa : -kappa;
         tsc = kappa;

@@ -65,11 +65,11 @@ __device__ __noinline__ double2 sincos64_far(double x)
 }
 
 // cos and sin of the angle x. Past 2^51, infinite or NaN: the call above (one
-// integer comparison a pair, 0.1 % on average over 39 sizes and 0.8 % at most,
-// the near field's adjoint). Up to there: X = x 2/pi quarter turns, n = rint(X) from one
-// fma against 1.5 2^52, y = X - n exact but for 2/pi's 2^-106; sin and cos of
-// y pi/2, |y| <= 1/2, by polynomials in y^2 (minimax fits by Remez exchange,
-// errors 4e-18 and 4e-20 before rounding), placed by n mod 4.
+// integer comparison a pair, whose cost does not show). Up to there: X = x 2/pi
+// quarter turns, n = rint(X) from one fma against 1.5 2^52, y = X - n exact but
+// for 2/pi's 2^-106; sin and cos of y pi/2, |y| <= 1/2, by polynomials in y^2
+// (minimax fits by Remez exchange, errors 4e-18 and 4e-20 before rounding),
+// placed by n mod 4.
 __device__ __forceinline__ void sincos64(double x, double &cs, double &sn)
 {
     if ((__double2hiint(x) & 0x7fffffff) >= 0x43200000) {
@@ -562,24 +562,25 @@ __global__ void po_adj_pack_tgt_d_kernel(long nt, const double *__restrict__ tgt
     if (i < nt) adj_record64<KIND>(i, nt, tgt7, gam, out + (size_t)adj64_rec(KIND) * i);
 }
 
-// Grid = (source blocks, target chunks of `chunk` targets). One source per
-// thread, its record in registers; the chunk's target records pass through
-// shared memory kFlushD at a time. WANT_T: each target's
-// values are summed over the CTA's sources through shared memory and added
-// to gt with one atomicAdd (the order of those varies between runs: gt is
-// reproducible to ~1e-16, not bitwise). Only the accumulators of the
+// Grid = (source blocks from `first` on, target chunks of `chunk` targets). One
+// source per thread, its record in registers; the chunk's target records pass
+// through shared memory kFlushD at a time. WANT_T: each target's values are
+// summed over the CTA's sources through shared memory into the block's row of
+// tsum, and po_adj_tsum_kernel adds the rows in order, so that grad_dt is the
+// same bits each time, as the FP64 path is for comparisons (an atomicAdd a CTA
+// and target, whose order varies: the same time). Only the accumulators of the
 // gradients asked for are kept (8,000 sources x 8,000 targets, near field, ms:
 // all three 33.0, the two displacements 22.2, the currents and grad_dt 29.7,
 // grad_dt alone 19.4).
 template <int KIND, bool HAS_M, bool WANT_C, bool WANT_D, bool WANT_T>
 __global__ void __launch_bounds__(kThreadsD)
-po_adj_fp64_kernel(const double *__restrict__ src, long ns, const double *__restrict__ trec, long nt, long chunk,
-                   Wave64 w, double *__restrict__ part, double *__restrict__ gt)
+po_adj_fp64_kernel(const double *__restrict__ src, long ns, long first, const double *__restrict__ trec, long nt,
+                   long chunk, Wave64 w, double *__restrict__ part, double *__restrict__ tsum)
 {
     constexpr int SR = fp64_rec(KIND, HAS_M), TR = adj64_rec(KIND);
     __shared__ double tile[kFlushD * TR];
     __shared__ double vbuf[WANT_T ? kFlushD * (kThreadsD + 1) : 1];
-    const long si = (long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long si = (first + blockIdx.x) * blockDim.x + threadIdx.x;
     double s[SR];
 #pragma unroll
     for (int q = 0; q < SR; ++q) s[q] = si < ns ? src[(size_t)SR * si + q] : 0.0;
@@ -612,7 +613,7 @@ po_adj_fp64_kernel(const double *__restrict__ src, long ns, const double *__rest
                 for (int j = 0; j < kFlushD; ++j) sum += vbuf[q * (kThreadsD + 1) + j * SEG + g];
 #pragma unroll
             for (int m = 1; m < SEG; m <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
-            if (g == 0 && q < cnt) atomicAdd(&gt[base + q], sum);
+            if (g == 0 && q < cnt) tsum[blockIdx.x * nt + base + q] = sum;
         }
     }
     if (si >= ns) return;
@@ -621,6 +622,26 @@ po_adj_fp64_kernel(const double *__restrict__ src, long ns, const double *__rest
         const int r = adj_row(KIND, WANT_C, WANT_D, a);
         if (r >= 0) part[((long)blockIdx.y * adj_rows(KIND, WANT_C, WANT_D) + r) * ns + si] = acc[a];
     }
+}
+
+// gt (with `add`, added to) = the sum of tsum's rows, in their order by eighths
+// (row r in eighth r mod 8), then the eighths. A block has 32 targets.
+__global__ void __launch_bounds__(256)
+po_adj_tsum_kernel(long rows, long nt, const double *tsum, int add, double *__restrict__ gt)
+{
+    __shared__ double sh[8][32];
+    pdl_wait();
+    const int l = threadIdx.x & 31, g = threadIdx.x >> 5;
+    const long j = (long)blockIdx.x * 32 + l;
+    double v = 0.0;
+    if (j < nt)
+#pragma unroll 4
+        for (long r = g; r < rows; r += 8) v += tsum[r * nt + j];
+    sh[g][l] = v;
+    __syncthreads();
+    if (g > 0 || j >= nt) return;
+    for (int q = 1; q < 8; ++q) v += sh[q][l];
+    gt[j] = add ? gt[j] + v : v;
 }
 
 // The pairs the mixed adjoint left out as inside the tangent band: each is
@@ -709,6 +730,8 @@ void *adj_fp64_kernel(int kind, bool has_m, bool want_c, bool want_d, bool want_
     return has_m ? adj_fp64_c<kKindFF, true>(want_c, want_d, want_t)
                  : adj_fp64_c<kKindFF, false>(want_c, want_d, want_t);
 }
+
+void *adj_tsum_kernel() { return reinterpret_cast<void *>(&po_adj_tsum_kernel); }
 
 void *adj_pack_tgt_d_kernel(int kind)
 {

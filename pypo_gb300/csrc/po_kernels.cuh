@@ -243,6 +243,7 @@ void *band_fixup_kernel(int kind, bool has_m);
 void *adj_band_fixup_kernel(int kind, bool want_t);
 void *wait_selftest_kernel();
 void *adj_fp64_kernel(int kind, bool has_m, bool want_c, bool want_d, bool want_t);
+void *adj_tsum_kernel();
 void *adj_pack_tgt_d_kernel(int kind);
 void *adj_cot_kernel();
 void *adj_pack_kernel();                 // near field, scalar: sources, targets and cotangents
