@@ -111,15 +111,16 @@ int m_is_zero(const double *h_cur, const double *d_cur, long ns, cudaStream_t s,
         if ((rc = po::scratch_alloc(reinterpret_cast<void **>(&ptr), (bytes), s))) goto done; \
     } while (0)
 
-// Host slots read back by a host-buffer call: the frame's half-extent and
-// the number of near-tangent pairs. They are page-locked so that the copies
-// stay asynchronous: a device-to-host copy into pageable memory makes the
-// host wait for all of the call's kernels before it can queue the output
-// copies. Pageable (the caller's slots) if pinning fails. One small
-// page-locked block per calling thread, kept.
+// Host slots read back by a host-buffer call: the frame's half-extent, the
+// number of near-tangent pairs and the device error words. They are
+// page-locked so that the copies stay asynchronous: a device-to-host copy into
+// pageable memory makes the host wait for all of the call's kernels before it
+// can queue the output copies. Pageable (the caller's slots) if pinning fails.
+// One small page-locked block per calling thread, kept.
 struct HostSlots {
     double extent;
     unsigned band;
+    int words[2];
 };
 
 HostSlots *host_slots(HostSlots *pageable)
@@ -209,7 +210,7 @@ int run_host(int mode, long ns, const double *src7, int gmode, int ncx, int ncy,
     rc = po::run_device(a);
     if (rc) goto done;
     CK(cudaMemcpyAsync(out, d_out, sizeof(double) * nout * nt, cudaMemcpyDeviceToHost, s));
-    rc = po::read_device_error(s, &code);   // the call's one synchronisation
+    rc = po::read_device_error(s, &code, hs->words);   // the call's one synchronisation
     if (!rc && precision == 0) {
         t_extent = hs->extent;
         t_band = hs->band;
@@ -417,7 +418,7 @@ int drop_in(int mode, float *const *res, reflparamsf source, reflparamsf target,
     else
         for (int r = 0; r < nout; ++r)
             CK(cudaMemcpyAsync(res[r], d_f + (size_t)r * nt, sizeof(float) * nt, cudaMemcpyDeviceToHost, s));
-    rc = po::read_device_error(s, &code);   // the kernels' one synchronisation
+    rc = po::read_device_error(s, &code, hs->words);   // the kernels' one synchronisation
     if (!rc && code) rc = fail(4, device_error_text(code));
     if (rc) goto done;
     t_extent = hs->extent;
@@ -657,7 +658,7 @@ int po_adjoint_d(int mode, long ns, const double *src7, int gmode, int ncx, int 
         CK(cudaMemcpyAsync(grad_cur, d_gc, sizeof(double) * ncur * ns, cudaMemcpyDeviceToHost, s));
     if (grad_ds && ns > 0) CK(cudaMemcpyAsync(grad_ds, d_gs, sizeof(double) * ns, cudaMemcpyDeviceToHost, s));
     if (grad_dt && nt > 0) CK(cudaMemcpyAsync(grad_dt, d_gt, sizeof(double) * nt, cudaMemcpyDeviceToHost, s));
-    rc = po::read_device_error(s, &code);   // the call's one synchronisation
+    rc = po::read_device_error(s, &code, hs->words);   // the call's one synchronisation
     if (!rc && precision == 0) {
         t_extent = hs->extent;
         t_band = hs->band;

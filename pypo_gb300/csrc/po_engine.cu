@@ -387,26 +387,16 @@ static int *error_word_impl(bool create)
 
 int *error_word() { return error_word_impl(true); }
 
-int read_device_error(cudaStream_t s, int *code)
+int read_device_error(cudaStream_t s, int *code, int *words)
 {
     // Both words: the allocating paths' (if it exists yet) and the
     // allocation-free entry's (if it has set up on this device). Nothing is
-    // allocated on the device here, so callers of the allocation-free entry
-    // can use it. The words are read into page-locked memory (one small block
-    // per calling thread, kept; the stack where that fails: a copy into
-    // pageable memory waits for the stream and costs 10 us more), and cleared
-    // only where one is set.
-    thread_local int *pinned = nullptr;
-    thread_local bool tried = false;
-    if (!tried) {
-        tried = true;
-        if (cudaMallocHost(&pinned, 2 * sizeof(int)) != cudaSuccess) {
-            pinned = nullptr;
-            (void)cudaGetLastError();
-        }
-    }
+    // allocated here, on the device or page-locked, so callers of the
+    // allocation-free entry can use it. They are read into the caller's
+    // page-locked `words` (a copy into pageable memory waits for the stream and
+    // costs 10 us more) or the stack, and cleared only where one is set.
     int local[2];
-    int *got = pinned ? pinned : local;
+    int *got = words ? words : local;
     int *w[2] = {error_word_impl(false), static_status_word()};
     got[0] = got[1] = 0;
     for (int i = 0; i < 2; ++i)

@@ -59,8 +59,9 @@ int timing_collect(float *ms, int max);
 
 // Synchronises `s`, returns and clears the device error words (wait
 // timeouts): the allocating paths' word and, once the allocation-free entry
-// has set up on this device, its static status word. Allocates nothing.
-int read_device_error(cudaStream_t s, int *code);
+// has set up on this device, its static status word. Allocates nothing; words:
+// two page-locked ints of the caller to read them into, or null.
+int read_device_error(cudaStream_t s, int *code, int *words = nullptr);
 // The allocating paths' error word of the current device (allocated once).
 int *error_word();
 // The allocation-free entry's status word on the current device, or null
