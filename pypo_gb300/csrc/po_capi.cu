@@ -226,40 +226,38 @@ done:
 }
 
 // Page-locked staging of the drop-in calls: blocks of kStageBytes, borrowed by
-// one call at a time and kept for later ones (at most kStageKeep).
+// one call at a time and kept until the process exits, kStageMost of them. A
+// call that finds them all taken copies its rows directly: making and freeing
+// a block per call would cost more, and freeing one waits for the device.
 constexpr size_t kStageBytes = size_t(8) << 20;
-constexpr size_t kStageKeep = 4;
+constexpr int kStageMost = 4;
 std::mutex g_stage_mu;
-std::vector<void *> g_stage_free;
+void *g_stage_free[kStageMost];   // not borrowed
+int g_stage_nfree = 0, g_stage_made = 0;
 
 class Staging {
 public:
     ~Staging()
     {
         if (!p_) return;
-        {
-            std::lock_guard<std::mutex> lk(g_stage_mu);
-            if (g_stage_free.size() < kStageKeep) {
-                g_stage_free.push_back(p_);
-                return;
-            }
-        }
-        cudaFreeHost(p_);
+        std::lock_guard<std::mutex> lk(g_stage_mu);
+        g_stage_free[g_stage_nfree++] = p_;
     }
-    // A block for `bytes`, or null (too many, or no page-locked memory).
+    // A block for `bytes`, or null (too many, all taken, or no page-locked memory).
     float *borrow(size_t bytes)
     {
         if (bytes > kStageBytes) return nullptr;
         {
             std::lock_guard<std::mutex> lk(g_stage_mu);
-            if (!g_stage_free.empty()) {
-                p_ = g_stage_free.back();
-                g_stage_free.pop_back();
-            }
+            if (g_stage_nfree > 0) p_ = g_stage_free[--g_stage_nfree];
+            else if (g_stage_made == kStageMost) return nullptr;
+            else ++g_stage_made;
         }
         if (!p_ && cudaHostAlloc(&p_, kStageBytes, cudaHostAllocPortable) != cudaSuccess) {
             p_ = nullptr;
             (void)cudaGetLastError();
+            std::lock_guard<std::mutex> lk(g_stage_mu);
+            --g_stage_made;
         }
         return static_cast<float *>(p_);
     }
@@ -320,7 +318,8 @@ void widen(const reflparamsf &f, Widened &w)
 // rows and containers cs / ct, as the reference leaves them. Up to
 // kStageBytes the caller's rows go through page-locked staging, one copy each
 // way and one synchronisation (31 x 33 -> 31 x 31: 38 copies of pageable rows
-// took 0.4 of the call's 0.64 ms); larger calls copy row by row.
+// took 0.4 of the call's 0.64 ms); larger calls, and those that find no staging
+// block, copy row by row.
 int drop_in(int mode, float *const *res, reflparamsf source, reflparamsf target, reflcontainerf *cs,
             reflcontainerf *ct, float *const *inp, float k, float epsilon, float t)
 {
