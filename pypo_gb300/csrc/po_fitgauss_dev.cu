@@ -521,29 +521,31 @@ bool np_index(long r, long dim, long &out)
 }
 
 // A page-locked block that the kernels post results into: borrowed by one fit
-// at a time, kept for later ones (at most kMailKeep of them, one per fit that
-// ran at the same time).
+// at a time and kept until the process exits, kMailMost of them. A fit that
+// finds them all taken copies its results: freeing page-locked memory waits for
+// the device.
 struct MailBox {
     unsigned long long data[2 * (2 * kBatch + 1)];
     unsigned seq;   // of the last launch that posted here (host only)
 };
-constexpr size_t kMailKeep = 16;
+constexpr int kMailMost = 16;
 std::mutex g_mail_mu;
-std::vector<MailBox *> g_mail_free;
+MailBox *g_mail_free[kMailMost];   // not borrowed
+int g_mail_nfree = 0, g_mail_made = 0;
 
 MailBox *mailbox_borrow()
 {
     {
         std::lock_guard<std::mutex> lk(g_mail_mu);
-        if (!g_mail_free.empty()) {
-            MailBox *m = g_mail_free.back();
-            g_mail_free.pop_back();
-            return m;
-        }
+        if (g_mail_nfree > 0) return g_mail_free[--g_mail_nfree];
+        if (g_mail_made == kMailMost) return nullptr;
+        ++g_mail_made;
     }
     void *p = nullptr;
     if (cudaHostAlloc(&p, sizeof(MailBox), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
         (void)cudaGetLastError();
+        std::lock_guard<std::mutex> lk(g_mail_mu);
+        --g_mail_made;
         return nullptr;   // the fit copies its results instead
     }
     *static_cast<MailBox *>(p) = MailBox{};
@@ -553,14 +555,8 @@ MailBox *mailbox_borrow()
 void mailbox_return(MailBox *m)
 {
     if (!m) return;
-    {
-        std::lock_guard<std::mutex> lk(g_mail_mu);
-        if (g_mail_free.size() < kMailKeep) {
-            g_mail_free.push_back(m);
-            return;
-        }
-    }
-    cudaFreeHost(m);
+    std::lock_guard<std::mutex> lk(g_mail_mu);
+    g_mail_free[g_mail_nfree++] = m;
 }
 
 // Scratch of one fit, one allocation.
