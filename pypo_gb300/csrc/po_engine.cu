@@ -34,6 +34,7 @@ thread_local int t_launches = 0;
 struct DeviceInfo {
     bool ready = false;
     int sms = 0;
+    bool cluster = false;           // the device can hold the frame's cluster
     cudaMemPool_t pool = nullptr;   // the library's own scratch pool
     int occ2[3][2][2] = {};  // near-field and scalar kernels, [kind][t>0][has_m]
     int occ_ff[2][2] = {};   // far-field tile kernels, [t>0][has_m]
@@ -94,6 +95,26 @@ int n_out(int mode)
         if (e_ != cudaSuccess) return fail(2, std::string(#expr) + ": " + err_str(e_));     \
     } while (0)
 
+// Whether the frame's cluster can run on the current device or the share of it
+// that this context has (a cluster's CTAs need their SMs in one GPC).
+static bool frame_cluster_fits()
+{
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(kFrameCtas);
+    c.blockDim = dim3(kFrameThreads);
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kFrameCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    c.attrs = at;
+    c.numAttrs = 1;
+    int n = 0;
+    const bool ok = cudaFuncSetAttribute(frame_kernel(), cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                    cudaOccupancyMaxActiveClusters(&n, frame_kernel(), &c) == cudaSuccess && n > 0;
+    if (!ok) (void)cudaGetLastError();
+    return ok;
+}
+
 static int device_info(DeviceInfo *&out)
 {
     int dev = 0;
@@ -127,7 +148,7 @@ static int device_info(DeviceInfo *&out)
                 PO_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, kThreads, smem));
                 di.occ_ff[ts][hm] = std::max(nb, 1);
             }
-        PO_CK(cudaFuncSetAttribute(frame_kernel(), cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        di.cluster = frame_cluster_fits();
         di.ready = true;
     }
     out = &di;
@@ -503,6 +524,28 @@ int run_device(const RunArgs &a)
     return rc;
 }
 
+// CTAs of the box kernel for n points, or 0 where the frame comes from its cluster.
+static int box_ctas(const DeviceInfo *di, long n)
+{
+    if (di->cluster && n <= kFrameClusterMax) return 0;
+    return (int)std::max(1L, std::min((long)di->sms, (n + kFrameThreads - 1) / kFrameThreads));
+}
+
+// The frame of the sources' and nb targets' box (po_prep.cu), `zero` cleared.
+// boxes: 48 bytes for each of the nbox CTAs, free until the frame is written.
+static int launch_frame(const double *src7, long ns, const double *tgt7, long nb, double kappa, int centred, Frame *frame,
+                        unsigned *zero, int nbox, long long *boxes, cudaStream_t s)
+{
+    if (nbox == 0) {
+        void *args[] = {&src7, &ns, &tgt7, &nb, &kappa, &centred, &frame, &zero};
+        return launch(frame_kernel(), dim3(kFrameCtas), dim3(kFrameThreads), args, 0, s);
+    }
+    void *bargs[] = {&src7, &ns, &tgt7, &nb, &boxes};
+    if (int rc = launch(box_kernel(), dim3((unsigned)nbox), dim3(kFrameThreads), bargs, 0, s)) return rc;
+    void *fargs[] = {&boxes, &nbox, &kappa, &centred, &frame, &zero};
+    return launch_pdl(box_frame_kernel(), dim3(1), dim3(192), fargs, 0, s);
+}
+
 int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
 {
     DeviceInfo *di = nullptr;
@@ -556,8 +599,11 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
     p.few = p.ntb * p.nsplit <= 2L * di->sms;
     const long chunk_tiles = (p.tiles + p.nsplit - 1) / p.nsplit;
     p.chunk = chunk_tiles * (p.far ? 1 : kTile);   // tiles (far field) or sources per chunk
-    if ((rc = sc.get(&p.part, (size_t)p.nsplit * p.nacc * nt))) return rc;
-    return sc.commit();
+    if ((rc = sc.get(&p.part, (size_t)p.nsplit * p.nacc * nt)) || (rc = sc.commit())) return rc;
+    // the boxes where the pack kernel writes the more numerous points' records (16 bytes a point and more)
+    p.nbox = box_ctas(di, p.far ? ns : ns + nt);
+    p.boxes = reinterpret_cast<long long *>(p.far || ns >= nt ? p.srcpk : p.tgtpk);
+    return 0;
 }
 
 // Indices of the sources in the order of their keys, into i_out (k_in, i_in:
@@ -591,8 +637,7 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
     // field; the far field keeps the coordinate origin (its phase reference)
     long nb = p.far ? 0 : nt;
     int centred = p.far ? 0 : 1, farflag = p.far ? 1 : 0;
-    void *frargs[] = {&src7, &ns, &tgt7, &nb, &p.kappa, &centred, &p.frame, &p.band.count};
-    rc = launch(frame_kernel(), dim3(kFrameCtas), dim3(kFrameThreads), frargs, 0, s);
+    rc = launch_frame(src7, ns, tgt7, nb, p.kappa, centred, p.frame, p.band.count, p.nbox, p.boxes, s);
     int boxes = !scalar && !p.has_m && ns > 0;   // the lit-tile proof serves the M = 0 kernels
     // ---- sources (near field, scalar) and targets
     long stiles = p.far || ns == 0 ? 0 : p.tiles;
@@ -817,10 +862,9 @@ int run_adjoint(const AdjArgs &a)
         dsc = far ? kappa : -kappa;
         tsc = kappa;
         long nb = far ? 0 : nt;
-        double kap = kappa;
-        int centred = far ? 0 : 1;
-        void *frargs[] = {&src7, &ns, &tgt7, &nb, &kap, &centred, &frame, &band.count};
-        if (!rc) rc = launch(frame_kernel(), dim3(kFrameCtas), dim3(kFrameThreads), frargs, 0, s);
+        // the boxes where the pack kernels write the more numerous points' records
+        long long *boxes = reinterpret_cast<long long *>(far || ns >= nt ? (void *)srcpk : (void *)trec);
+        if (!rc) rc = launch_frame(src7, ns, tgt7, nb, kappa, far ? 0 : 1, frame, band.count, box_ctas(di, ns + nb), boxes, s);
         if (far) {
             // sources in Hilbert order, in the forward's tile records: one adjoint
             // CTA per tile, whose centre's phase goes into the cotangents

@@ -135,9 +135,14 @@ struct Wave64 {
 Wave64 wave64(double k, double t);
 
 // The frame kernel: one thread-block cluster (16 is the most a cluster may
-// have, past the portable 8).
+// have, past the portable 8). Past kFrameClusterMax points, and where a context's
+// share of the device cannot hold the cluster, the box comes from a CTA an SM and
+// the frame from a second kernel. A call of n sources and 25 targets, cluster /
+// two kernels, in us: 4,000 28.6 / 29.5, 48,000 54.8 / 55.3, 64,000 67.8 / 67.8,
+// 161,202 126.2 / 122.1, 1,002,001 600 / 554.
 constexpr int kFrameThreads = 512;
 constexpr int kFrameCtas = 16;
+constexpr long kFrameClusterMax = 60000;
 
 // Illumination test of the mixed-precision kernels: a pair with
 // n . R_hat >= kTangentBand is lit, one below -kTangentBand is not (the FP32
@@ -233,6 +238,8 @@ void *pk_kernel(int kind, int t_sign, bool has_m, bool few);
 void *pack_kernel(bool scalar, bool has_m);   // source tiles (near field, scalar) and targets
 void *fp64_kernel(int kind, bool has_m);
 void *frame_kernel();
+void *box_kernel();
+void *box_frame_kernel();   // 192 threads
 void *pack_src_d_kernel();
 constexpr int kEpiThreads = 256;
 void *epilogue_kernel(int groups);   // 1, 8, 32 or 64 threads share a target's chunks

@@ -48,29 +48,18 @@ __device__ __forceinline__ double quantum(double need)
     return __longlong_as_double(((bits & 0xfffffffffffffll) ? e + 1 : e) << 52);
 }
 
-}  // namespace
-
-// Box of the points of a (na) and b (nb; rows x, y, z first), and from it the
-// frame: origin, scale and quantum. One cluster of kFrameCtas CTAs: minima and
-// maxima are exact in any order, so the split does not show in the result
-// (NaN coordinates are left out). centred: origin at the box centre (near
-// field, scalar); otherwise origin 0 (far field: the phase reference is the
-// coordinate origin). zero: a word cleared for the call's later kernels (the
-// band list's count), or null.
-__global__ void __launch_bounds__(kFrameThreads) __cluster_dims__(kFrameCtas, 1, 1)
-po_frame_kernel(const double *__restrict__ a, long na, const double *__restrict__ b, long nb, double kappa,
-                int centred, Frame *__restrict__ fr, unsigned *__restrict__ zero)
+// The box of the points of a (na) and b (nb; rows x, y, z first) that the CTAs
+// first, first + step, ... of THREADS threads take, THREADS points at a time: thread
+// q < 6 returns lowest x, y, z, highest x, y, z as order keys (NaN coordinates
+// are left out). wbox: shared.
+template <int THREADS>
+__device__ __forceinline__ long long cta_box(const double *__restrict__ a, long na, const double *__restrict__ b,
+                                             long nb, long first, long step, long long (*wbox)[THREADS / 32])
 {
-    __shared__ long long box[6][kFrameCtas];   // rank 0's copy gathers the cluster's
-    __shared__ long long wbox[6][kFrameThreads / 32];
-    pdl_trigger();
-    cluster_arrive();   // completed below: every CTA has started before one writes into rank 0's memory
-    const uint32_t rank = cluster_rank();
-    if (rank == 0 && threadIdx.x == 0 && zero) *zero = 0u;
     long long v[6] = {kKeyInf, kKeyInf, kKeyInf, ~kKeyInf, ~kKeyInf, ~kKeyInf};
     auto scan = [&](const double *__restrict__ p, long n) {
 #pragma unroll 4
-        for (long i = (long)rank * kFrameThreads + threadIdx.x; i < n; i += (long)kFrameCtas * kFrameThreads)
+        for (long i = first * THREADS + threadIdx.x; i < n; i += step * THREADS)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 const long long x = __double_as_longlong(p[c * n + i]), y = order_key(x);
@@ -91,30 +80,27 @@ po_frame_kernel(const double *__restrict__ a, long na, const double *__restrict_
         if ((threadIdx.x & 31) == 0) wbox[q][threadIdx.x >> 5] = v[q];
     }
     __syncthreads();
-    cluster_wait();
+    long long r = 0;
     if (threadIdx.x < 6) {
         const int q = threadIdx.x;
-        long long r = wbox[q][0];
-        for (int w = 1; w < kFrameThreads / 32; ++w) r = q < 3 ? min(r, wbox[q][w]) : max(r, wbox[q][w]);
-        st_cluster(&box[q][rank], 0, r);
+        r = wbox[q][0];
+        for (int w = 1; w < THREADS / 32; ++w) r = q < 3 ? min(r, wbox[q][w]) : max(r, wbox[q][w]);
     }
-    __syncwarp();
-    cluster_arrive();
-    cluster_wait();
-    if (rank != 0 || threadIdx.x != 0) return;
-    double lo[3], hi[3], m = 0.0;
+    return r;
+}
+
+// The frame of the box k (order keys: lowest x, y, z, highest x, y, z).
+__device__ __forceinline__ void write_frame(const long long *k, double kappa, int centred, Frame *fr)
+{
+    double m = 0.0;
     for (int c = 0; c < 3; ++c) {
-        long long l = box[c][0], h = box[3 + c][0];
-        for (int r = 1; r < kFrameCtas; ++r) {
-            l = min(l, box[c][r]);
-            h = max(h, box[3 + c][r]);
-        }
-        lo[c] = __longlong_as_double(order_key(l));
-        hi[c] = __longlong_as_double(order_key(h));
+        const double lo = __longlong_as_double(order_key(k[c])), hi = __longlong_as_double(order_key(k[3 + c]));
         double o = 0.0;
-        if (centred && lo[c] <= hi[c]) o = 0.5 * (lo[c] + hi[c]);
+        if (centred && lo <= hi) o = 0.5 * (lo + hi);
         fr->o[c] = o;
-        if (lo[c] <= hi[c]) m = fmax(m, fmax(fabs(hi[c] - o), fabs(lo[c] - o)));
+        if (lo <= hi) m = fmax(m, fmax(fabs(hi - o), fabs(lo - o)));
+        fr->lo[c] = lo;
+        fr->hi[c] = hi;
     }
     m *= kappa;
     // 2 m / q <= 2048, so |hi/q| <= 1024.5
@@ -123,10 +109,77 @@ po_frame_kernel(const double *__restrict__ a, long na, const double *__restrict_
     fr->q = q;
     fr->inv_q = 1.0 / q;
     fr->m = m;
-    for (int c = 0; c < 3; ++c) {
-        fr->lo[c] = lo[c];
-        fr->hi[c] = hi[c];
+}
+
+}  // namespace
+
+// Box of the points of a (na) and b (nb; rows x, y, z first), and from it the
+// frame: origin, scale and quantum. One cluster of kFrameCtas CTAs: minima and
+// maxima are exact in any order, so the split does not show in the result.
+// centred: origin at the box centre (near field, scalar); otherwise origin 0
+// (far field: the phase reference is the coordinate origin). zero: a word
+// cleared for the call's later kernels (the band list's count), or null.
+__global__ void __launch_bounds__(kFrameThreads) __cluster_dims__(kFrameCtas, 1, 1)
+po_frame_kernel(const double *__restrict__ a, long na, const double *__restrict__ b, long nb, double kappa,
+                int centred, Frame *__restrict__ fr, unsigned *__restrict__ zero)
+{
+    __shared__ long long box[6][kFrameCtas];   // rank 0's copy gathers the cluster's
+    __shared__ long long wbox[6][kFrameThreads / 32];
+    pdl_trigger();
+    cluster_arrive();   // completed below: every CTA has started before one writes into rank 0's memory
+    const uint32_t rank = cluster_rank();
+    if (rank == 0 && threadIdx.x == 0 && zero) *zero = 0u;
+    const long long r = cta_box<kFrameThreads>(a, na, b, nb, rank, kFrameCtas, wbox);
+    cluster_wait();
+    if (threadIdx.x < 6) st_cluster(&box[threadIdx.x][rank], 0, r);
+    __syncwarp();
+    cluster_arrive();
+    cluster_wait();
+    if (rank != 0 || threadIdx.x != 0) return;
+    long long k[6];
+    for (int q = 0; q < 6; ++q) {
+        k[q] = box[q][0];
+        for (int c = 1; c < kFrameCtas; ++c) k[q] = q < 3 ? min(k[q], box[q][c]) : max(k[q], box[q][c]);
     }
+    write_frame(k, kappa, centred, fr);
+}
+
+// The same in two kernels, for many points and for devices that cannot hold the
+// cluster: the boxes of gridDim.x CTAs, then the frame of their box.
+__global__ void __launch_bounds__(kFrameThreads)
+po_box_kernel(const double *__restrict__ a, long na, const double *__restrict__ b, long nb,
+              long long *__restrict__ boxes)
+{
+    __shared__ long long wbox[6][kFrameThreads / 32];
+    const long long r = cta_box<kFrameThreads>(a, na, b, nb, blockIdx.x, gridDim.x, wbox);
+    if (threadIdx.x < 6) boxes[6L * blockIdx.x + threadIdx.x] = r;
+    pdl_trigger();
+}
+
+__global__ void __launch_bounds__(192)
+po_box_frame_kernel(const long long *boxes, int n, double kappa, int centred, Frame *__restrict__ fr,
+                    unsigned *__restrict__ zero)
+{
+    __shared__ long long k[6];
+    pdl_wait();
+    pdl_trigger();
+    // warp q: word q of the boxes
+    const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    long long v = q < 3 ? kKeyInf : ~kKeyInf;
+    for (int i = lane; i < n; i += 32) {
+        const long long u = boxes[6L * i + q];
+        v = q < 3 ? min(v, u) : max(v, u);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const long long u = __shfl_xor_sync(0xffffffffu, v, o);
+        v = q < 3 ? min(v, u) : max(v, u);
+    }
+    if (lane == 0) k[q] = v;
+    __syncthreads();
+    if (threadIdx.x > 0) return;
+    if (zero) *zero = 0u;
+    write_frame(k, kappa, centred, fr);
 }
 
 // Packed target i. Near field / scalar: hi/lo split position in the frame.
@@ -245,6 +298,8 @@ po_pack_kernel(long ns, const double *__restrict__ src7, const double *__restric
 }
 
 void *frame_kernel() { return reinterpret_cast<void *>(&po_frame_kernel); }
+void *box_kernel() { return reinterpret_cast<void *>(&po_box_kernel); }
+void *box_frame_kernel() { return reinterpret_cast<void *>(&po_box_frame_kernel); }
 
 void *pack_kernel(bool scalar, bool has_m)
 {
