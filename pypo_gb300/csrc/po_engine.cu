@@ -454,12 +454,12 @@ int validate(const RunArgs &a)
 // on, and more where few targets (fewer blocks than SMs, each bound by its
 // SM's FP64 additions) have many chunks: 25 targets, 630 chunks: 30 us with
 // 32 threads, 18 us with 64.
-static int launch_epilogue(int mode, int nacc, int nsplit, long nt, const double *part, const double *tgt7, double t,
-                           double zeta_inv, double *out, cudaStream_t s)
+static int launch_epilogue(long sms, int mode, int nacc, int nsplit, long nt, const double *part, const double *tgt7,
+                           double t, double zeta_inv, double *out, cudaStream_t s)
 {
     int groups = nsplit < 8 ? 1 : 8;
-    if (nsplit >= 32 && nt <= 152L * (kEpiThreads / 32)) groups = 32;
-    if (nsplit >= 64 && nt <= 152L * (kEpiThreads / 64)) groups = 64;
+    if (nsplit >= 32 && nt <= sms * (kEpiThreads / 32)) groups = 32;
+    if (nsplit >= 64 && nt <= sms * (kEpiThreads / 64)) groups = 64;
     const long per = kEpiThreads / groups;
     void *args[] = {&mode, &nacc, &nsplit, &nt, &part, &tgt7, &t, &zeta_inv, &out};
     return launch_pdl(epilogue_kernel(groups), dim3((unsigned)((nt + per - 1) / per)), dim3(kEpiThreads), args, 0, s);
@@ -520,7 +520,7 @@ int run_device(const RunArgs &a)
     if (!rc) rc = launch(fk, dim3((unsigned)ntb, (unsigned)nsplit), dim3(kThreadsD), fargs, 0, s);
     timing_mark(s, false);
     int nspl = (int)nsplit;
-    if (!rc) rc = launch_epilogue(mode, nacc, nspl, nt, part, tgt7, t, zeta_inv, out, s);
+    if (!rc) rc = launch_epilogue(di->sms, mode, nacc, nspl, nt, part, tgt7, t, zeta_inv, out, s);
     return rc;
 }
 
@@ -596,6 +596,7 @@ int mixed_prepare(const RunArgs &a, Scratch &sc, MixedPlan &p)
     const size_t room = std::min(sc.room(), (size_t)1 << 30);
     const long max_chunks = std::max(1L, (long)(room / ((size_t)p.nacc * nt * sizeof(double))));
     p.nsplit = load_split(p.ntb, ns, di->sms, occ, max_chunks, kTile, p.far ? kLoadFF : kLoadNF);
+    p.sms = di->sms;
     p.few = p.ntb * p.nsplit <= 2L * di->sms;
     const long chunk_tiles = (p.tiles + p.nsplit - 1) / p.nsplit;
     p.chunk = chunk_tiles * (p.far ? 1 : kTile);   // tiles (far field) or sources per chunk
@@ -679,7 +680,7 @@ int mixed_launch(const RunArgs &a, MixedPlan &p, int *err)
         rc = launch_pdl(band_fixup_kernel(p.kind, p.has_m), dim3(kFixupBlocks), dim3(256), xargs, 0, s);
     }
     int nspl = (int)p.nsplit;
-    if (!rc) rc = launch_epilogue(mode, p.nacc, nspl, nt, p.part, tgt7, t, p.zeta_inv, out, s);
+    if (!rc) rc = launch_epilogue(p.sms, mode, p.nacc, nspl, nt, p.part, tgt7, t, p.zeta_inv, out, s);
     if (!rc && a.extent_host) PO_CK_RC(cudaMemcpyAsync(a.extent_host, &p.frame->m, sizeof(double),
                                                        cudaMemcpyDeviceToHost, s));
     if (!rc && a.band_host && p.band.count)
@@ -904,7 +905,7 @@ int run_adjoint(const AdjArgs &a)
         }
     }
     long nt_e = want_t ? nt : 0;
-    const int groups = nspl >= 8 && ns <= 152L * kEpiThreads ? 8 : 1;   // fewer blocks than SMs: share the chunks
+    const int groups = nspl >= 8 && ns <= (long)di->sms * kEpiThreads ? 8 : 1;   // fewer blocks than SMs: share the chunks
     const long per = kEpiThreads / groups;
     long nblk_e = rows > 0 ? (ns + per - 1) / per : 0;
     void *eargs[] = {(void *)&kind, &nspl, &ns, &part, &src7, &gmode, &ncx, &ncy, &fac_re, &fac_im, &dsc,

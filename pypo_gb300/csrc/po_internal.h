@@ -110,6 +110,7 @@ struct MixedPlan {
     long tiles = 0, ntb = 0, nsplit = 1, chunk = 0;
     double *part = nullptr;
     Frame *frame = nullptr;
+    int sms = 0;                // of the device
     int nbox = 0;               // CTAs of the box kernel; 0: the frame's cluster
     long long *boxes = nullptr; // their boxes, in memory that the pack kernel fills afterwards
     float4 *srcpk = nullptr, *tgtpk = nullptr;
