@@ -54,7 +54,6 @@ __host__ __device__ constexpr int pk_unroll(int kind, bool has_m, bool few)
 #endif
 constexpr int kStages = PO_STAGES;     // TMA pipeline depth
 constexpr int kRec = 6;         // float4 per packed source record (96 B)
-constexpr int kRecScalar = 2;   // float4 per packed scalar record (32 B)
 constexpr int kAcc = 12;        // accumulators per target (E, H re/im x y z)
 constexpr int kBoxF = 8;        // floats per source-tile box (lit-tile proof)
 #ifndef PO_MUFU_SINCOS
