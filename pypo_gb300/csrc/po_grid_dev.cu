@@ -9,7 +9,7 @@
 // surface error (:852-866) keeps the reference's random sequence, drawn on
 // the device (normal_deviates_dev): mt19937 seeded with rms_seed and a fresh
 // normal distribution per point (src/include/Random.h:112-116), applied along
-// the normals by a second kernel.
+// the normals where the deviates are formed.
 //
 // The correlated surface error (po_correlated_error_dev) is a spectral
 // synthesis over random modes drawn from the same generator, evaluated on
@@ -152,17 +152,6 @@ __global__ void po_grid_kernel(GridSpec g, double *__restrict__ out)
     out[6 * n + idx] = area;
 }
 
-// Normal-direction surface error: point += s_i * n_i.
-__global__ void po_grid_error_kernel(long n, const double *__restrict__ s, double *__restrict__ out)
-{
-    const long idx = (long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= n) return;
-    const double d = s[idx];
-    out[idx] += d * out[3 * n + idx];
-    out[n + idx] += d * out[4 * n + idx];
-    out[2 * n + idx] += d * out[5 * n + idx];
-}
-
 int generate_grid_dev(const reflparams &r, double *out7, bool transform, bool spheric, cudaStream_t s)
 {
     if (!r.n_cells || r.n_cells[0] < 1 || r.n_cells[1] < 1) return fail(1, "bad n_cells");
@@ -197,19 +186,9 @@ int generate_grid_dev(const reflparams &r, double *out7, bool transform, bool sp
     if (e != cudaSuccess) return fail(2, std::string("grid kernel launch: ") + cudaGetErrorString(e));
     note_launches(1);
     if (r.rms > 0) {
-        double *d = nullptr;
         int *err = error_word();
         if (!err) return fail(2, "could not allocate the device error word");
-        if (int rc = scratch_alloc(reinterpret_cast<void **>(&d), sizeof(double) * n, s)) return rc;
-        int rc = normal_deviates_dev((unsigned)r.rms_seed, n, r.rms, d, err, s);
-        if (!rc) {
-            po_grid_error_kernel<<<nblk, 256, 0, s>>>(n, d, out7);
-            e = cudaGetLastError();
-            if (e == cudaSuccess) note_launches(1);
-            else rc = fail(2, std::string("surface error: ") + cudaGetErrorString(e));
-        }
-        scratch_free(d, s);
-        return rc;
+        return normal_deviates_dev((unsigned)r.rms_seed, n, r.rms, nullptr, out7, err, s);
     }
     return 0;
 }
@@ -235,6 +214,10 @@ constexpr int kMtN = 624;
 constexpr int kMtThreads = 256;          // the twist's CTA: 227 threads work
 constexpr long kMtRound = 4096;          // blocks of words kept at a time (10 MB)
 constexpr int kMtAttempts = 256;         // attempts per CTA
+// CTAs from which a kernel of its own counts the accepted attempts: 121 deviates
+// (2 CTAs) take 5 us less without it, 289 (4 CTAs, whose attempts one CTA would
+// try one after the other) 4 us more.
+constexpr unsigned kMtCountFrom = 3;
 
 __device__ __forceinline__ uint32_t mt_twist(uint32_t cur, uint32_t next, uint32_t tap)
 {
@@ -270,18 +253,21 @@ __device__ __forceinline__ bool mt_attempt(const uint4 *words, long a, long n, d
 }  // namespace
 
 // nblk blocks of the generator's words, before tempering; state: the words of
-// the last block, where a later round goes on (first: from the seed). Word i
+// the last block, where a later round goes on (start: from the seed, and the
+// deviates' count *start is cleared). Word i
 // of a block needs the old words i and i + 1 and the word 227 before it (the
 // old word i + 397 where there is none), so thread t has t, t + 227 and t + 454
 // in one go, and two buffers need one barrier a block.
 __global__ void __launch_bounds__(kMtThreads)
-po_mt_words_kernel(unsigned seed, int first, long nblk, uint32_t *__restrict__ state, uint32_t *__restrict__ words)
+po_mt_words_kernel(unsigned seed, long long *__restrict__ start, long nblk, uint32_t *__restrict__ state,
+                   uint32_t *__restrict__ words)
 {
     __shared__ uint32_t mt[2][kMtN];
     const int t = threadIdx.x;
-    if (!first) {
+    if (!start) {
         for (int i = t; i < kMtN; i += kMtThreads) mt[0][i] = state[i];
     } else if (t == 0) {
+        *start = 0;
         uint32_t v = seed;
         mt[0][0] = v;
         for (int i = 1; i < kMtN; ++i) {
@@ -324,10 +310,13 @@ po_mt_count_kernel(const uint4 *__restrict__ words, long na, int *__restrict__ c
 
 // The accepted attempts' deviates, in order, from where the rounds before
 // ended (base[0]; the last CTA leaves the new end in base[1] and, at the last
-// round, reports deviates that are missing).
+// round, reports deviates that are missing). Without counts (a few CTAs) each
+// CTA counts the attempts before its own itself. Deviate i goes into out[i] or,
+// with g7 (7 rows of n), moves point i along its normal.
 __global__ void __launch_bounds__(kMtAttempts)
 po_mt_emit_kernel(const uint4 *__restrict__ words, long na, const int *__restrict__ count, long long *__restrict__ base,
-                  int last, long n, double stdev, double *__restrict__ out, int *__restrict__ err)
+                  int last, long n, double stdev, double *__restrict__ out, double *__restrict__ g7,
+                  int *__restrict__ err)
 {
     __shared__ unsigned long long before;
     __shared__ int warp_ok[kMtAttempts / 32];
@@ -339,12 +328,24 @@ po_mt_emit_kernel(const uint4 *__restrict__ words, long na, const int *__restric
     if (lane == 0) warp_ok[warp] = __popc(ball);
     __syncthreads();
     unsigned long long mine = 0;
-    for (int c = t; c < (int)blockIdx.x; c += kMtAttempts) mine += (unsigned)count[c];
+    if (count)
+        for (int c = t; c < (int)blockIdx.x; c += kMtAttempts) mine += (unsigned)count[c];
+    else
+        for (int c = 0; c < (int)blockIdx.x; ++c) {
+            double u, v;
+            mine += mt_attempt(words, (long)c * kMtAttempts + t, na, u, v);
+        }
     if (mine) atomicAdd(&before, mine);
     __syncthreads();
     long at = (long)before + __popc(ball & ((1u << lane) - 1u));
     for (int w = 0; w < warp; ++w) at += warp_ok[w];
-    if (ok && at < n) out[at] = __dmul_rn(__dmul_rn(y, __dsqrt_rn(__ddiv_rn(__dmul_rn(-2.0, log(r2)), r2))), stdev);
+    if (ok && at < n) {
+        const double d = __dmul_rn(__dmul_rn(y, __dsqrt_rn(__ddiv_rn(__dmul_rn(-2.0, log(r2)), r2))), stdev);
+        if (g7)
+            for (int c = 0; c < 3; ++c) g7[c * n + at] += d * g7[(3 + c) * n + at];
+        else
+            out[at] = d;
+    }
     if (blockIdx.x == gridDim.x - 1 && t == kMtAttempts - 1) {
         const long end = at + ok;
         base[1] = end;
@@ -352,7 +353,7 @@ po_mt_emit_kernel(const uint4 *__restrict__ words, long na, const int *__restric
     }
 }
 
-int normal_deviates_dev(unsigned seed, long n, double stdev, double *out, int *err, cudaStream_t s)
+int normal_deviates_dev(unsigned seed, long n, double stdev, double *out, double *g7, int *err, cudaStream_t s)
 {
     if (n <= 0) return 0;
     // attempts for n deviates at pi / 4 a piece, with 12 standard deviations to
@@ -371,16 +372,18 @@ int normal_deviates_dev(unsigned seed, long n, double stdev, double *out, int *e
         state = words + kMtN * most;
         base = reinterpret_cast<long long *>(state + kMtN);
         count = reinterpret_cast<int *>(base + rounds + 1);
-        cudaError_t e = cudaMemsetAsync(base, 0, sizeof(long long), s);
+        cudaError_t e = cudaSuccess;
         for (long r = 0; r < rounds && e == cudaSuccess; ++r) {
             const long nb = std::min(kMtRound, blocks - r * kMtRound), a = nb * (kMtN / 4);
             const unsigned grid = (unsigned)((a + kMtAttempts - 1) / kMtAttempts);
             const uint4 *w4 = reinterpret_cast<const uint4 *>(words);
-            po_mt_words_kernel<<<1, kMtThreads, 0, s>>>(seed, r == 0, nb, state, words);
-            po_mt_count_kernel<<<grid, kMtAttempts, 0, s>>>(w4, a, count);
-            po_mt_emit_kernel<<<grid, kMtAttempts, 0, s>>>(w4, a, count, base + r, r == rounds - 1, n, stdev, out, err);
+            const bool counts = grid >= kMtCountFrom;
+            po_mt_words_kernel<<<1, kMtThreads, 0, s>>>(seed, r == 0 ? base : nullptr, nb, state, words);
+            if (counts) po_mt_count_kernel<<<grid, kMtAttempts, 0, s>>>(w4, a, count);
+            po_mt_emit_kernel<<<grid, kMtAttempts, 0, s>>>(w4, a, counts ? count : nullptr, base + r, r == rounds - 1, n, stdev,
+                                                          out, g7, err);
             e = cudaGetLastError();
-            if (e == cudaSuccess) note_launches(3);
+            if (e == cudaSuccess) note_launches(counts ? 3 : 2);
         }
         if (e != cudaSuccess) rc = fail(2, std::string("normal deviates: ") + cudaGetErrorString(e));
     }
@@ -548,7 +551,7 @@ int correlated_error_dev(long n, double *g7, double rms, double corr_len, unsign
         scratch_free(modes, s);
         return rc;
     }
-    rc = normal_deviates_dev(seed, 4L * n_modes, 1.0, g, err, s);
+    rc = normal_deviates_dev(seed, 4L * n_modes, 1.0, g, nullptr, err, s);
     if (!rc) {
         po_modes_kernel<<<(std::max(n_modes, kCosN) + 127) / 128, 128, 0, s>>>(n_modes, g, 1.0 / corr_len, modes, tab);
         po_correlated_kernel<<<(unsigned)((n + kCorrPoints - 1) / kCorrPoints), 256, 0, s>>>(

@@ -145,8 +145,9 @@ long load_split(long nb, long ns, long sms, long occ, long max_chunks, long tile
 // FP64 grid generation on the device into a 7-row layout (po_grid_dev.cu).
 int generate_grid_dev(const reflparams &r, double *out7, bool transform, bool spheric, cudaStream_t s);
 // n normal deviates N(0, stdev) in the reference's sequence (mt19937 seeded
-// with `seed`, a fresh distribution per draw), on the device.
-int normal_deviates_dev(unsigned seed, long n, double stdev, double *out, int *err, cudaStream_t s);
+// with `seed`, a fresh distribution per draw), on the device: into out or, with
+// g7 (7 rows of n points), as displacements of the points along their normals.
+int normal_deviates_dev(unsigned seed, long n, double stdev, double *out, double *g7, int *err, cudaStream_t s);
 // Correlated surface error at the n points of a 7-row device grid (delta
 // and/or the points moved along their normals), and its host twin (po_grid.cpp).
 int correlated_error_dev(long n, double *g7, double rms, double corr_len, unsigned seed, int n_modes, double *delta,
