@@ -64,8 +64,9 @@ __device__ __forceinline__ void fence_proxy_async()
 // promise that lets the compiler read early or through the non-coherent path).
 // pdl_trigger() lets the next kernel's blocks be scheduled once every
 // block of this one has called it or ended; without a dependent both do
-// nothing. It stands at a kernel's end: called at the start of a kernel of
-// many blocks, it has the next kernel's few blocks placed on whichever SMs
+// nothing. It stands at a kernel's end (in the pair kernels ahead of their
+// stores), but for the frame's one cluster or block: called at the start of a
+// kernel of many blocks, it has the next kernel's few blocks placed on whichever SMs
 // are free at that moment instead of one to an SM (161,202 sources -> 25
 // targets: the 158 blocks of the pair kernel took 142 us alone and the call
 // 380 us; an epilogue of 333 blocks that reads 570 MB took 0.25 ms longer).

@@ -2,10 +2,11 @@
 // split representation, and the packed records of sources and targets.
 //
 // A small propagation is bound by its launches (2.1 us each on the device,
-// and as much per stream-ordered allocation), so the set-up is two kernels:
+// and as much per stream-ordered allocation), so its set-up is two kernels:
 // the frame in one thread-block cluster (no partial buffer, no second
 // launch), and one pack kernel for the source records, their tile boxes and
-// the targets. Each later kernel of a call is launched with programmatic
+// the targets. Many points take their box from all SMs, in one kernel more.
+// Each later kernel of a call is launched with programmatic
 // stream serialisation and begins with pdl_wait().
 #include <cuda_runtime.h>
 #include <math_constants.h>
